@@ -152,6 +152,8 @@ struct RecLayout {
 RecLayout rec_layout(const dv_step_params& p);
 // Doubles of the split residual's scratch (per-cell properties + per-face fluxes).
 int64_t split_doubles(const dv_step_params& p);
+// Doubles of the finite-difference Jacobian's scratch (seven variants of the cell properties, faces).
+int64_t jac_scratch_doubles(const dv_step_params& p);
 
 }  // namespace dv
 
@@ -163,6 +165,9 @@ struct dv_model {
     dv::RecLayout rl;
     double* d_rec;                  // internal record scratch (accumulators)
     double* d_split;                // per-cell properties and per-face fluxes of the split residual
+    double* d_jac;                  // scratch of the finite-difference Jacobian
+    cudaEvent_t jac_ev;             // end of the last Jacobian (its scratch is free for another stream)
+    int jac_used;                   // jac_ev has been recorded
     double* d_diag;                 // diagnostics record of the outlet summary (dv_outlet_row)
     double* d_acc;                  // DV_NACC
     int64_t nfev;

@@ -212,55 +212,6 @@ __global__ void __launch_bounds__(256) k_accumulators(dv_step_params p, const do
         for (int q = 0; q < DV_NACC; ++q) acc[q] = a[q];
 }
 
-// All colour perturbations of the forward-difference Jacobian in one launch.
-// blockIdx.y = slot * 7 + col_var: the perturbed column is unknown `col_var` of neighbour `slot`
-// of the row cell.  With a distance-2 colouring every row sees exactly one perturbed column of
-// each colour, so evaluating the row cell with that single column perturbed reproduces the
-// coloured evaluation of core/jacobian.py:78-84 (colour = colour[column]).
-template <class TJ>
-__global__ void __launch_bounds__(128) k_fd_jacobian(dv_step_params p, Aux aux, double t, const double* __restrict__ y,
-                                                     const double* __restrict__ f0, TJ* __restrict__ J) {
-    const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz;
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nc) return;
-    const int slot = blockIdx.y / DV_NB, cv = blockIdx.y % DV_NB;
-    int i, j, k;
-    cell_ijk(p, c, i, j, k);
-    int ni = i, nj = j, nk = k;
-    bool ok = true;
-    switch (slot) {
-        case 0: break;
-        case 1: nk = k - 1; ok = nk >= 0; break;
-        case 2: nk = k + 1; ok = nk < p.Nz; break;
-        case 3: nk = k - 2; ok = nk >= 0; break;
-        case 4: nk = k + 2; ok = nk < p.Nz; break;
-        case 5: ni = i - 1; ok = ni >= 0; break;
-        case 6: ni = i + 1; ok = ni < p.Nr; break;
-        case 7: ok = p.Nth > 1; nj = (j == 0) ? p.Nth - 1 : j - 1; break;
-        default: ok = p.Nth > 1; nj = (j == p.Nth - 1) ? 0 : j + 1; break;
-    }
-    if (cv == DV_NV) ok = ok && p.wall_on && (ni == p.Nr - 1);
-    TJ* Jb = J + ((int64_t)slot * DV_NB * DV_NB + cv) * nc + c;         // row stride DV_NB*nc
-    if (!ok) {
-#pragma unroll
-        for (int rv = 0; rv < DV_NB; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)0.0;
-        return;
-    }
-    const int64_t ncell_n = ((int64_t)ni * p.Nth + nj) * p.Nz + nk;
-    const int64_t col = (cv < DV_NV) ? (int64_t)cv * nc + ncell_n : (int64_t)DV_NV * nc + (int64_t)nj * p.Nz + nk;
-    const double yv = y[col];
-    double h = 1.5e-8 * npmax(fabs(yv), p.typ[cv]);
-    h = (yv + h) - yv;                                   // core/jacobian.py:75-76
-    LoadPert ld{y, col, h};
-    double f[DV_NV], fw = 0.0;
-    const bool outer_wall = (i == p.Nr - 1) && p.wall_on;
-    cell_eval(p, aux, ld, t, i, j, k, f, outer_wall ? &fw : nullptr, (const Rec*)nullptr);
-#pragma unroll
-    for (int rv = 0; rv < DV_NV; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)((f[rv] - f0[rv * nc + c]) / h);
-    Jb[(int64_t)DV_NV * DV_NB * nc] =
-        (TJ)(outer_wall ? (fw - f0[(int64_t)DV_NV * nc + (int64_t)j * p.Nz + k]) / h : 0.0);
-}
-
 // ---------------------------------------------------------------- split residual
 // The residual as three launches with short per-thread chains: per-cell properties and uptake
 // (k_cprops), the flux through every face once (k_faces), per-cell divergence and sources
@@ -399,28 +350,16 @@ __device__ __forceinline__ void cprops_block(const dv_step_params& p, const Spli
 // bit-identical to the one-thread-per-cell evaluation.
 #define CP_WARPS 8
 static_assert(DV_NG == 3 && CP_WARPS == 8, "the warp roles assume three gases");
-template <int MODE>
-__device__ __forceinline__ void cprops_split(const dv_step_params& p, const Split& S, const double* __restrict__ y,
-                                             const double* __restrict__ u, const double* __restrict__ sc,
-                                             const double* __restrict__ scal, int64_t vb) {
+template <class L>
+__device__ __forceinline__ void cprops_split(const dv_step_params& p, const Split& S, const L& ld, int64_t vb) {
     __shared__ double xk[DV_NG][32], xdcw[32], xqw[32], xqd[32], xqwet[32];
     const int64_t nc = S.nc;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t c = vb * 32 + lane;
     const bool in = c < nc;
-    if (MODE == M_MATVEC && scal[0] == 0.0) return;    // zero direction (grid-uniform): k_assemble writes zeros
     Cell s;
-    if (in) {
-        if (MODE == M_MATVEC) {
-            LoadDir ld{y, u, sc, matvec_sig(scal)};
-            load_cell(ld, nc, c, s);
-        } else {
-            LoadPlain ld{y};
-            load_cell(ld, nc, c, s);
-        }
-    } else {
-        s = Cell{};
-    }
+    if (in) load_cell(ld, nc, c, s);
+    else s = Cell{};
     Props o;
     double ycl[DV_NG];
     props_state(p, s, o, ycl);
@@ -496,7 +435,12 @@ __global__ void __launch_bounds__(CP_WARPS * 32) k_cprops(dv_step_params p, Spli
                                                           const double* __restrict__ scal) {
     pdl_wait();                             // (launched programmatically inside the GMRES graph)
     pdl_trigger();
-    cprops_split<MODE>(p, S, y, u, sc, scal, blockIdx.x);
+    if (MODE == M_MATVEC) {
+        if (scal[0] == 0.0) return;         // zero direction (grid-uniform): k_assemble writes zeros
+        cprops_split(p, S, LoadDir{y, u, sc, matvec_sig(scal)}, blockIdx.x);
+    } else {
+        cprops_split(p, S, LoadPlain{y}, blockIdx.x);
+    }
 }
 
 // MUSCL slope of cell kk of a column starting at cell index base (zero next to the ends).
@@ -721,6 +665,260 @@ __global__ void __launch_bounds__(64) k_matvec_coop(dv_step_params p, Aux aux, S
         assemble_at<M_MATVEC, false>(p, aux, S, rec, 0.0, z, u, sc, f0, scal, 0.0, out, dargs, vb * 64 + threadIdx.x);
 }
 
+// ---------------------------------------------------------------- finite-difference Jacobian
+// Forward differences of every column (core/jacobian.py:71-86).  With a distance-2
+// colouring every row sees exactly one perturbed column of each colour, so a row evaluated with that
+// single column perturbed reproduces the coloured evaluation (core/jacobian.py:78-84).  Perturbing one
+// unknown of cell n changes the properties of n alone, and through them at most two of the six faces of
+// a row cell, so nothing else is evaluated again:
+//   k_jac_props  properties and uptake of every cell, unperturbed and with each of its six unknowns
+//                perturbed (seven variants)
+//   k_jac_faces  the flux of every face, unperturbed and for each unknown of each cell it depends on, and
+//                the wall resistance of the outer cells' variants
+//   k_jac_rows   per (row cell, neighbour slot, column): the row's six fluxes, the balances, the
+//                difference quotients
+// Every expression has the operands it has in an evaluation of the whole row (cell_eval), so the entries
+// are the same bits.  One thread evaluating its whole row for each of the 63 (slot, column) pairs took
+// 441 property evaluations and 378 faces a cell against 7 and 51 here: 155 -> 34 us at 8x8x32 and
+// 1270 -> 172 us at 16x16x64 (props 50, faces 63, rows 59; 58 MB of entries, 9 us at the copy bandwidth).
+// (Faces evaluated by the row threads, 99 a cell at one 224-thread block per SM: 56 and 374 us.)  What
+// bounds it: FP64 latency at 2 instructions per cycle (FP64 pipe 15-32 % busy), divisions first.
+constexpr int JAC_VAR = DV_NV + 1;          // unperturbed + the six cell unknowns
+
+// y with one unknown `v` of every cell perturbed by the step of core/jacobian.py:75-76 (v < 0: none)
+static __device__ __forceinline__ double fd_step(const dv_step_params& p, double yv, int v) {
+    const double h = 1.5e-8 * npmax(fabs(yv), p.typ[v]);
+    return (yv + h) - yv;
+}
+struct LoadVar {
+    const dv_step_params& p;
+    const double* y;
+    int64_t nc;
+    int v;
+    __device__ __forceinline__ double operator()(int64_t i) const {
+        const double x = y[i];
+        return (v >= 0 && i >= v * nc && i < (v + 1) * nc) ? x + fd_step(p, x, v) : x;
+    }
+};
+
+// Scratch of the Jacobian: the split residual's layout with seven variants of the cell properties
+// (variant-major); the wall resistances [JAC_VAR][Nth Nz]; the perturbed fluxes: z faces
+// [rel 0..3][var][4][nzf], cell kf - 2 + rel of the column perturbed at face kf, then r and theta faces
+// [side][var][4][..], the face's lower or upper cell perturbed.
+struct JacScratch {
+    Split S;
+    double *rbed, *zp, *rp, *tp;
+};
+constexpr int JAC_ZREL = 4;
+int64_t jac_scratch_doubles(const dv_step_params& p) {
+    const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz, nzf = (int64_t)p.Nr * p.Nth * (p.Nz + 1);
+    const int64_t nrf = (int64_t)(p.Nr - 1) * p.Nth * p.Nz;
+    return split_doubles(p) + (JAC_VAR - 1) * SP_NCELL * nc + JAC_VAR * (int64_t)p.Nth * p.Nz +
+           4 * DV_NV * (JAC_ZREL * nzf + 2 * nrf + 2 * nc);
+}
+static JacScratch jac_scratch_of(const dv_step_params& p, double* base) {
+    const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz;
+    JacScratch j;
+    j.S = split_of(p, base + (JAC_VAR - 1) * SP_NCELL * nc);
+    j.S.cell = base;
+    j.rbed = j.S.tf + 4 * j.S.ntf;
+    j.zp = j.rbed + JAC_VAR * (int64_t)p.Nth * p.Nz;
+    j.rp = j.zp + 4 * DV_NV * JAC_ZREL * j.S.nzf;
+    j.tp = j.rp + 4 * DV_NV * 2 * j.S.nrf;
+    return j;
+}
+static __device__ __forceinline__ Split jac_variant(const Split& S, int var) {
+    Split V = S;
+    V.cell = S.cell + (int64_t)var * SP_NCELL * S.nc;
+    return V;
+}
+
+__global__ void __launch_bounds__(CP_WARPS * 32) k_jac_props(dv_step_params p, Split S, const double* __restrict__ y) {
+    const int var = blockIdx.y;
+    cprops_split(p, jac_variant(S, var), LoadVar{p, y, S.nc, var - 1}, blockIdx.x);
+}
+
+// Flux through the interior z face between cells kL and kL + 1 of a column with cell kp of that column
+// taken from V (the perturbed variant) and all others from S.
+static __device__ __forceinline__ void jac_zface(const dv_step_params& p, const Split& S, const Split& V, int i,
+                                                 int64_t base, int kL, int kp, bool muscl, double N_nom, Flux& F) {
+    const int64_t nc = S.nc;
+    auto at = [&](int row, int kk) { return ((kk == kp) ? V.cell : S.cell)[row * nc + base + kk]; };
+    double s[2][4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {           // the slopes of sp_slope
+        const int kk = kL + e;
+        s[e][0] = s[e][1] = s[e][2] = s[e][3] = 0.0;
+        if (!muscl || kk < 1 || kk > p.Nz - 2) continue;
+#pragma unroll
+        for (int q = 0; q < DV_NG; ++q) {
+            const double x = at(SP_C0 + q, kk);
+            s[e][q] = limited_slope(p.limiter, x - at(SP_C0 + q, kk - 1), at(SP_C0 + q, kk + 1) - x);
+        }
+        const double T = at(SP_T, kk);
+        s[e][3] = limited_slope(p.limiter, T - at(SP_T, kk - 1), at(SP_T, kk + 1) - T);
+    }
+    Cell a, b;
+    Props L, R;
+    sp_get(kL == kp ? V : S, base + kL, a, L);
+    sp_get(kL + 1 == kp ? V : S, base + kL + 1, b, R);
+    double uz;
+    zface(p, i, L, R, a, b, s[0], s[1], muscl, N_nom, F, &uz);
+}
+
+// blockIdx.y: 0..3 z faces with cell kf - 2 + y perturbed; 4, 5 r faces and 6, 7 theta faces with the
+// lower / upper cell perturbed; 8 the unperturbed faces (the index space of faces_at), then (variant,
+// wall node).  y < 8: a block takes 32 faces, its warps the six unknowns, so a block runs one kind of
+// face and its warps share the unperturbed cells through L1.
+constexpr int JF_THREADS = DV_NV * 32;
+__global__ void __launch_bounds__(JF_THREADS, 3) k_jac_faces(dv_step_params p, Aux aux, JacScratch X, double t,
+                                                             int64_t nfaces) {
+    const Split& S = X.S;
+    const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
+    const int64_t nw = (int64_t)Nth * Nz;
+    const int kind = blockIdx.y;
+    if (kind == 8) {
+        int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+        if (g < nfaces) {
+            faces_at<false>(p, aux, S, Rec{}, t, nullptr, nullptr, g);
+            return;
+        }
+        g -= nfaces;
+        if (g >= JAC_VAR * nw) return;
+        const int var = (int)(g / nw);
+        Cell s;
+        Props o;
+        sp_get(jac_variant(S, var), (int64_t)(Nr - 1) * nw + (g - var * nw), s, o);
+        X.rbed[g] = wall_R_bed(p, o);
+        return;
+    }
+    const int v = threadIdx.x >> 5;
+    const int64_t g = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    const Split V = jac_variant(S, v + 1);
+    Flux F;
+    if (kind < JAC_ZREL) {
+        if (g >= S.nzf) return;
+        const int64_t col = g / (Nz + 1);
+        const int kf = (int)(g - col * (Nz + 1)), kp = kf - 2 + kind;
+        if (kp < 0 || kp >= Nz) return;
+        const int i = (int)(col / Nth);
+        if (kf > 0 && kf < Nz) {
+            const bool muscl = (Nz >= 3 && p.limiter != DV_LIM_UPWIND);
+            jac_zface(p, S, V, i, col * Nz, kf - 1, kp, muscl, aux.n_nom[col], F);
+        } else {                            // a column end: depends on its own cell only
+            if (kp != (kf == 0 ? 0 : Nz - 1)) return;
+            Cell s;
+            Props o;
+            sp_get(V, col * Nz + kp, s, o);
+            double F_in[DV_NG], H_in;
+            end_face(p, p.ends[kf == 0 ? 0 : 1], t, i, s, o, aux.feed_flux[col], F_in, H_in, nullptr, 0);
+#pragma unroll
+            for (int q = 0; q < DV_NG; ++q) F.F[q] = (kf == 0) ? F_in[q] : -F_in[q];
+            F.H = (kf == 0) ? H_in : -H_in;
+        }
+        flux_put(X.zp + (int64_t)(kind * DV_NV + v) * 4 * S.nzf, S.nzf, g, F);
+        return;
+    }
+    const bool theta = kind >= 6, upper = kind & 1;
+    if (g >= (theta ? (Nth > 1 ? S.ntf : 0) : (Nr > 1 ? S.nrf : 0))) return;
+    int i, j, k;
+    cell_ijk(p, g, i, j, k);                // the face's lower cell
+    const int jp = (j == Nth - 1) ? 0 : j + 1;
+    const int64_t gb = theta ? ((int64_t)i * Nth + jp) * Nz + k : g + nw;
+    Cell a, b;
+    Props A, B;
+    sp_get(upper ? S : V, g, a, A);
+    sp_get(upper ? V : S, gb, b, B);
+    double u;
+    tface(p, A, B, a, b, theta ? p.arc[i] : p.drc[i], theta ? p.Ath[i] : p.Ar[i], F, &u);
+    const int64_t nf = theta ? S.ntf : S.nrf;
+    flux_put((theta ? X.tp : X.rp) + (int64_t)((upper ? 1 : 0) * DV_NV + v) * 4 * nf, nf, g, F);
+}
+
+// A row difference over the step: rows the column does not reach difference to an exact zero, which is
+// the quotient (h is positive and finite wherever the unknown is), without the division.
+static __device__ __forceinline__ double jac_quot(double d, double h) {
+    return (d == 0.0 && h > 0.0 && h < 1e300) ? d : d / h;
+}
+
+// One warp per column variable cv (0..6) of a tile of 32 row cells, blockIdx.y = neighbour slot: the
+// seven warps read the same unperturbed fluxes and properties (one of them from L2, the others from L1)
+// and each (row, column) plane of J is written coalesced.
+template <class TJ>
+__global__ void __launch_bounds__(DV_NB * 32, 3) k_jac_rows(dv_step_params p, Aux aux, JacScratch X, double t,
+                                                            const double* __restrict__ y,
+                                                            const double* __restrict__ f0, TJ* __restrict__ J) {
+    const Split& S = X.S;
+    const int64_t nc = S.nc;
+    const int cv = threadIdx.x >> 5, slot = blockIdx.y;
+    const int64_t c = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    if (c >= nc) return;
+    int i, j, k;
+    cell_ijk(p, c, i, j, k);
+    const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
+    const int jm = (j == 0) ? Nth - 1 : j - 1;
+    int ni = i, nj = j, nk = k;
+    bool ok = true;
+    switch (slot) {
+        case 0: break;
+        case 1: nk = k - 1; ok = nk >= 0; break;
+        case 2: nk = k + 1; ok = nk < Nz; break;
+        case 3: nk = k - 2; ok = nk >= 0; break;
+        case 4: nk = k + 2; ok = nk < Nz; break;
+        case 5: ni = i - 1; ok = ni >= 0; break;
+        case 6: ni = i + 1; ok = ni < Nr; break;
+        case 7: ok = Nth > 1; nj = jm; break;
+        default: ok = Nth > 1; nj = (j == Nth - 1) ? 0 : j + 1; break;
+    }
+    if (cv == DV_NV) ok = ok && p.wall_on && (ni == Nr - 1);
+    TJ* Jb = J + ((int64_t)slot * DV_NB * DV_NB + cv) * nc + c;         // row stride DV_NB*nc
+    if (!ok) {
+#pragma unroll
+        for (int rv = 0; rv < DV_NB; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)0.0;
+        return;
+    }
+    const int64_t n = ((int64_t)ni * Nth + nj) * Nz + nk;               // the column's cell
+    const int64_t col = (cv < DV_NV) ? (int64_t)cv * nc + n : (int64_t)DV_NV * nc + (int64_t)nj * Nz + nk;
+    const double h = fd_step(p, y[col], cv);
+    const LoadPert ld{y, col, h};
+    const bool own = slot == 0, cellv = cv < DV_NV;      // (a wall column changes no flux and no property)
+    const int var = (own && cellv) ? cv + 1 : 0;         // variant of the row cell's properties
+    const double* cell = S.cell + (int64_t)var * SP_NCELL * nc;
+    Props P0;
+    P0.T = cell[SP_T * nc + c];                          // (all that the balances read with R_bed given)
+    double rate[DV_NA], qstar[DV_NA] = {0.0, 0.0};       // (qstar goes to the records only)
+#pragma unroll
+    for (int q = 0; q < DV_NA; ++q) rate[q] = cell[(SP_RATE0 + q) * nc + c];
+    const int64_t ccol = (int64_t)i * Nth + j;
+    // the row's fluxes: the perturbed ones of the faces the column reaches.  z: the own cell and its z
+    // neighbours reach both faces (k +- 1 through the own slope), the cells two planes away the nearer one
+    auto face = [&](const double* f, const double* fp, bool pert, int which, int64_t nf, int64_t g, Flux& F) {
+        flux_get(pert ? fp + (int64_t)(which * DV_NV + cv) * 4 * nf : f, nf, g, F);
+    };
+    Flux Fzm, Fzp, Frm, Frp, Ftm, Ftp;
+    face(S.zf, X.zp, cellv && (own || (k > 0 && slot <= 3)), nk - k + 2, S.nzf, ccol * (Nz + 1) + k, Fzm);
+    face(S.zf, X.zp, cellv && (own || (k < Nz - 1 && (slot <= 2 || slot == 4))), nk - k + 1, S.nzf,
+         ccol * (Nz + 1) + k + 1, Fzp);
+    if (Nr > 1) {
+        if (i > 0) face(S.rf, X.rp, cellv && (own || slot == 5), own ? 1 : 0, S.nrf, c - (int64_t)Nth * Nz, Frm);
+        if (i < Nr - 1) face(S.rf, X.rp, cellv && (own || slot == 6), own ? 0 : 1, S.nrf, c, Frp);
+    }
+    if (Nth > 1) {
+        face(S.tf, X.tp, cellv && (own || slot == 7), own ? 1 : 0, S.ntf, ((int64_t)i * Nth + jm) * Nz + k, Ftm);
+        face(S.tf, X.tp, cellv && (own || slot == 8), own ? 0 : 1, S.ntf, c, Ftp);
+    }
+    const bool outer_wall = (i == Nr - 1) && p.wall_on;
+    const int64_t nw = (int64_t)Nth * Nz;
+    const double R_bed = (i == Nr - 1) ? X.rbed[var * nw + (int64_t)j * Nz + k] : 0.0;
+    double f[DV_NV], fw = 0.0;
+    cell_tail(p, aux, ld, t, i, j, k, P0, rate, qstar, Fzm, Fzp, Frm, Frp, Ftm, Ftp, f, outer_wall ? &fw : nullptr,
+              (const Rec*)nullptr, &R_bed);
+#pragma unroll
+    for (int rv = 0; rv < DV_NV; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)jac_quot(f[rv] - f0[rv * nc + c], h);
+    Jb[(int64_t)DV_NV * DV_NB * nc] =
+        (TJ)(outer_wall ? jac_quot(fw - f0[(int64_t)DV_NV * nc + (int64_t)j * Nz + k], h) : 0.0);
+}
+
 static Aux aux_of(const dv_model* m) { return Aux{m->aux.feed_flux, m->aux.n_nom, m->aux.cov}; }
 
 static unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -857,22 +1055,38 @@ int matvec_capture(dv_model* m, const double* dargs, const double* z, const doub
     return DV_OK;
 }
 
-static int fdjac_block(const dv_model* m) { return m->tune.fdjac_block == 64 ? 64 : 128; }
-
-int launch_fd_jacobian(dv_model* m, double t, const double* y, const double* f0, double* J, cudaStream_t s) {
-    const int bl = fdjac_block(m);
-    dim3 grid(nblk(m->nc, bl), DV_NSLOT * DV_NB);
-    DV_LAUNCH(dv::K_FDJAC, s, k_fd_jacobian<double><<<grid, bl, 0, s>>>(m->p, aux_of(m), t, y, f0, J));
+template <class TJ>
+static int fd_jacobian(dv_model* m, double t, const double* y, const double* f0, TJ* J, cudaStream_t s) {
+    const dv_step_params& p = m->p;
+    const JacScratch X = jac_scratch_of(p, m->d_jac);
+    const Split& S = X.S;
+    const int64_t ncol = (int64_t)p.Nr * p.Nth, nw = (int64_t)p.Nth * p.Nz;
+    const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol;
+    // the scratch belongs to one Jacobian at a time: a call on another stream waits for the last one
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    DV_CUDA(cudaStreamIsCapturing(s, &cap));
+    const bool order = cap == cudaStreamCaptureStatusNone;
+    if (order && m->jac_used) DV_CUDA(cudaStreamWaitEvent(s, m->jac_ev, 0));
+    DV_LAUNCH(dv::K_FDJAC, s, k_jac_props<<<dim3(nblk(m->nc, 32), JAC_VAR), CP_WARPS * 32, 0, s>>>(p, S, y));
+    // x covers the z faces (the most of the perturbed kinds) and the unperturbed index space
+    const unsigned gx = std::max(nblk(S.nzf, 32), nblk(nfaces + JAC_VAR * nw, JF_THREADS));
+    DV_LAUNCH(dv::K_FDJAC, s, k_jac_faces<<<dim3(gx, 9), JF_THREADS, 0, s>>>(p, aux_of(m), X, t, nfaces));
+    DV_LAUNCH(dv::K_FDJAC, s, k_jac_rows<TJ><<<dim3(nblk(m->nc, 32), DV_NSLOT), DV_NB * 32, 0, s>>>(p, aux_of(m), X, t, y,
+                                                                                                 f0, J));
     DV_CUDA(cudaGetLastError());
+    if (order) {
+        DV_CUDA(cudaEventRecord(m->jac_ev, s));
+        m->jac_used = 1;
+    }
     return DV_OK;
 }
 
+int launch_fd_jacobian(dv_model* m, double t, const double* y, const double* f0, double* J, cudaStream_t s) {
+    return fd_jacobian<double>(m, t, y, f0, J, s);
+}
+
 int launch_fd_jacobian32(dv_model* m, double t, const double* y, const double* f0, float* J, cudaStream_t s) {
-    const int bl = fdjac_block(m);
-    dim3 grid(nblk(m->nc, bl), DV_NSLOT * DV_NB);
-    DV_LAUNCH(dv::K_FDJAC, s, k_fd_jacobian<float><<<grid, bl, 0, s>>>(m->p, aux_of(m), t, y, f0, J));
-    DV_CUDA(cudaGetLastError());
-    return DV_OK;
+    return fd_jacobian<float>(m, t, y, f0, J, s);
 }
 
 // ---------------------------------------------------------------- outlet record

@@ -67,13 +67,16 @@ static __device__ __forceinline__ void slope4(int lim, const Cell& m, const doub
 
 // Divergence of the face fluxes, sorption sinks, wall / jacket / exchanger terms and records of
 // cell (i,j,k) (core/residual.py:298-365): f[0..5]; *fw = dTw/dt of its wall node.  Shared by the
-// thread-per-cell residual and the split residual's assembly, so both add in the same order.
+// thread-per-cell residual, the split residual's assembly and the Jacobian's rows, so all add in the
+// same order.  R_pre: the outer-ring cell's wall resistance where it has been evaluated already (the
+// same expression on the same properties), else null.
 template <class L>
 static __device__ __forceinline__ void cell_tail(const dv_step_params& p, const Aux& aux, const L& ld, double t, int i,
                                                  int j, int k, const Props& P0, const double rate[DV_NA],
                                                  const double qstar[DV_NA], const Flux& Fzm, const Flux& Fzp,
                                                  const Flux& Frm, const Flux& Frp, const Flux& Ftm, const Flux& Ftp,
-                                                 double f[DV_NV], double* fw, const Rec* rec) {
+                                                 double f[DV_NV], double* fw, const Rec* rec,
+                                                 const double* R_pre = nullptr) {
     const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
     const int64_t nc = (int64_t)Nr * Nth * Nz;
     const int64_t c0 = ((int64_t)i * Nth + j) * Nz + k;
@@ -106,7 +109,7 @@ static __device__ __forceinline__ void cell_tail(const dv_step_params& p, const 
         const int64_t wn = (int64_t)j * Nz + k;
         const double cov = aux.cov[wn];
         const double To = P0.T;
-        const double R_bed = wall_R_bed(p, P0);
+        const double R_bed = R_pre ? *R_pre : wall_R_bed(p, P0);
         double Q_jac, Q_amb, Q_wb;
         if (p.wall_on) {
             const double Tw = ld(off_w + wn);

@@ -2548,10 +2548,11 @@ int dv_model_set_krylov_fp32(dv_model* m, int32_t mask) {
 int dv_model_destroy(dv_model* m) {
     std::lock_guard<std::recursive_mutex> lk_(capture_mutex());
     if (!m) return DV_OK;
-    void* ptrs[] = {m->d_aux, m->d_rec, m->d_split, m->d_diag, m->d_acc, m->d_pc, m->d_pc32, m->d_J32, m->d_pc_work, m->d_pc_piv, m->d_pc_info, m->d_atol7,
+    void* ptrs[] = {m->d_aux, m->d_rec, m->d_split, m->d_jac, m->d_diag, m->d_acc, m->d_pc, m->d_pc32, m->d_J32, m->d_pc_work, m->d_pc_piv, m->d_pc_info, m->d_atol7,
                     m->d_err};
     cudaDeviceSynchronize();              // no work in flight still uses the buffers the pool keeps
     for (void* q : ptrs) pool_free(q);
+    if (m->jac_ev) cudaEventDestroy(m->jac_ev);
     if (m->W) {
         work_free(*m->W);
         delete m->W;
@@ -2602,6 +2603,7 @@ int dv_model_create(const dv_step_params* p, const double* feed_flux, const doub
     bool fail = pool_malloc((void**)&m->d_aux, sizeof(double) * (2 * nf + nwall)) != cudaSuccess ||
                 pool_malloc((void**)&m->d_rec, sizeof(double) * rec_n) != cudaSuccess ||
                 pool_malloc((void**)&m->d_split, sizeof(double) * split_doubles(*p)) != cudaSuccess ||
+                pool_malloc((void**)&m->d_jac, sizeof(double) * jac_scratch_doubles(*p)) != cudaSuccess ||
                 pool_malloc((void**)&m->d_diag, sizeof(double) * m->rl.total) != cudaSuccess ||
                 pool_malloc((void**)&m->d_acc, sizeof(double) * DV_NACC) != cudaSuccess ||
                 pool_malloc((void**)&m->d_pc, sizeof(double) * pc_need) != cudaSuccess ||
@@ -2611,7 +2613,8 @@ int dv_model_create(const dv_step_params* p, const double* feed_flux, const doub
                 pool_malloc((void**)&m->d_pc_piv, sizeof(int) * (size_t)m->pc_cap_parts * m->pc_cap_nb) != cudaSuccess ||
                 pool_malloc((void**)&m->d_pc_info, sizeof(int) * (size_t)m->pc_cap_parts) != cudaSuccess ||
                 pool_malloc((void**)&m->d_atol7, sizeof(double) * DV_NB) != cudaSuccess ||
-                pool_malloc((void**)&m->d_err, sizeof(int)) != cudaSuccess;
+                pool_malloc((void**)&m->d_err, sizeof(int)) != cudaSuccess ||
+                cudaEventCreateWithFlags(&m->jac_ev, cudaEventDisableTiming) != cudaSuccess;
     if (fail) {
         int rc = cuda_fail(cudaGetLastError(), "cudaMalloc(model workspace)");
         dv_model_destroy(m);
@@ -2619,6 +2622,7 @@ int dv_model_create(const dv_step_params* p, const double* feed_flux, const doub
     }
     debug_fill(m->d_rec, sizeof(double) * rec_n, 1);
     debug_fill(m->d_split, sizeof(double) * split_doubles(*p), 1);
+    debug_fill(m->d_jac, sizeof(double) * jac_scratch_doubles(*p), 1);
     debug_fill(m->d_diag, sizeof(double) * m->rl.total, 1);
     debug_fill(m->d_acc, sizeof(double) * DV_NACC, 1);
     debug_fill(m->d_pc, sizeof(double) * pc_need, 1);

@@ -1,7 +1,7 @@
 """FDJacobian on the GPU: drop-in for core/jacobian.py:21-91 of the reference.
 
 The colouring comes from the library's host code (bit-identical to numerics/sparsity.py:88-107);
-the values come from dv_fd_jacobian, which evaluates every colour perturbation in one launch into
+the values come from dv_fd_jacobian, which evaluates every colour perturbation in one call into
 the block layout J[slot][row 0..6][col 0..6][cell].  ``__call__`` returns the same scipy CSC matrix
 the reference does (pattern and entry order of build_pattern), ``block`` keeps J on the device.
 """

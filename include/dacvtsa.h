@@ -188,7 +188,7 @@ int dv_outlet_row(dv_model* m, double t, const double* y, double c_feed_co2, dou
  * n_core entries. */
 int dv_colour_columns(int32_t Nr, int32_t Nth, int32_t Nz, int32_t wall, int64_t* colour, int32_t* ncolours);
 /* Forward-difference Jacobian df/dy at (t, y) with f0 = f(t, y) (FDJacobian.__call__,
- * core/jacobian.py:71-86): every colour perturbation in one launch.  J is the block layout
+ * core/jacobian.py:71-86): every colour perturbation in one call.  J is the block layout
  * J[slot][row 0..6][col 0..6][cell] (jac_doubles): d f_row(cell) / d y_col(neighbour `slot`),
  * row/col 6 = the wall unknown of an outer-ring cell.  Same step rule h = 1.5e-8 max(|y|, typ). */
 int dv_fd_jacobian(dv_model* m, double t, const double* y, const double* f0, double* J, void* stream);
@@ -301,7 +301,8 @@ int dv_integrator_copy_y(const dv_integrator* g, double* dst, void* stream);
  * No reference counterpart.  Launch parameters of the hot kernels, per model: the Arnoldi steps the
  * GMRES graph runs ahead of its WHILE node (gmres_prefix, -1 = library default), the depth of the
  * preconditioner sweep's shared-memory ring of factor blocks (sweep_nbuf 2 or 3, 0 = deepest that
- * fits), the block sizes of the FP32 Jacobian product and of the FD Jacobian (0 = 128), and the Arnoldi
+ * fits), the block size of the FP32 Jacobian product, that of the FD Jacobian (accepted; its kernels now
+ * have one block shape each), and the Arnoldi
  * steps per pass through the WHILE node (gmres_body 1 or 2, 0 = library default: every pass costs a
  * device-side relaunch; a step after the stop returns at once).  None of them changes a result bit;
  * they only change the time. */

@@ -53,3 +53,36 @@ def test_jacobian_matches_dense_fd_and_colouring_is_valid():
     for r in range(Pr.shape[0]):
         cc = jac.color[Pr.indices[Pr.indptr[r]:Pr.indptr[r + 1]]]
         assert len(np.unique(cc)) == len(cc)
+
+
+@pytest.mark.parametrize("grid", [(1, 1, 1), (1, 1, 9), (1, 4, 2), (2, 3, 3), (3, 5, 5), (4, 1, 34)])
+@pytest.mark.parametrize("step", [0, 2])
+def test_jacobian_entries_are_the_quotients_of_the_residual(grid, step):
+    """Every entry equals the difference quotient of the whole residual with that one column perturbed,
+    to the bit (the same expressions on the same operands): columns, rings and sectors at the edges of
+    the grid, beds shorter than a slope's stencil, tiles with a remainder, feed / vent and vacuum ends."""
+    import torch
+    from dac_vtsa_b200 import host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.jacobian import FDJacobian
+    from dac_vtsa_b200.model import TVSAModel
+    cfg = load_config(override_dict={"grid.Nr": grid[0], "grid.Ntheta": grid[1], "grid.Nz": grid[2],
+                                     "wall.enabled": grid != (4, 1, 34)})
+    g = host.Grid.from_config(cfg)
+    props = host.get_backend(cfg)
+    st = host.seeded_state(cfg, g, props, seed=5, amplitude=0.02, P=101325.0 if step == 0 else 2.2e4)
+    st.q = st.q + np.random.default_rng(6).random(st.q.shape)
+    m = TVSAModel(cfg, g, props, cfg.cycle[step], st)
+    y = torch.from_numpy(m.pack(st)).to(m.device)
+    J = FDJacobian(m)(3.0, y).toarray()
+    f0, _ = m.rhs(3.0, y, want_acc=False)
+    typ = np.concatenate([np.full(g.ncell, a) for a in m.params.typ[:6]] + [np.full(m.n_w, m.params.typ[6])])
+    ref = np.zeros_like(J)
+    for col in range(m.n_core):
+        yv = float(y[col])
+        h = (yv + 1.5e-8 * max(abs(yv), typ[col])) - yv
+        yp = y.clone()
+        yp[col] = yv + h
+        # (divided by numpy: torch multiplies a CUDA tensor by a scalar's rounded reciprocal)
+        ref[:, col] = (m.rhs(3.0, yp, want_acc=False)[0] - f0).cpu().numpy() / h
+    assert np.array_equal(J, ref)
