@@ -982,7 +982,7 @@ static __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, 
 }
 
 // Self-test of the bounded wait: an mbarrier that nothing arrives at, waited on by one warp with
-// `polls` polls; the timeout sets bit 1 of *err exactly as in the sweep, and the kernel returns.
+// `polls` polls; the timeout sets bit 1 of *err, and the kernel returns.
 __global__ void k_selftest_mbar(int polls, int* err) {
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) {
@@ -1018,12 +1018,12 @@ struct PcFrame {
     __device__ __forceinline__ int gs(int sl) const { return rank == 0 ? sl : 4 - sl; }
 };
 
-// x = diag(1/sc) M^-1 diag(sc) b for all partitions: one CTA (256 threads; 8 lanes per group, two
-// rows per group) per partition, or per direction of a partition (TW).  The factor blocks of the
-// next planes stream into an NBUF-deep shared ring (cp.async.bulk with an mbarrier) while the
-// current plane is swept.  NJ = ld / 16: lane l reads the column pairs (2l + 16j, 2l + 16j + 1),
-// j < NJ, of a block row and of the solution plane with 16-byte loads (8-byte for FP32 blocks),
-// a fixed, fully unrolled batch; padding columns hold zeros.
+// x = diag(1/sc) M^-1 diag(sc) b for all partitions: one CTA per partition, or per direction of a
+// partition (TW).  Eight lanes take two rows of a plane's blocks; NJ = ld / 16: lane l holds the column
+// pairs (2l + 16j, 2l + 16j + 1), j < NJ, of its rows.  The factors go from global memory (L2) straight
+// into registers, two stages ahead of their use, and only the solution planes live in shared memory:
+// nothing of a stage but its newest plane is read after the barrier, and the plane before it stays in
+// registers.  Padding columns hold zeros.
 // Stages of one CTA (local frame):
 //   F(t), t = 1..n-1:   z_t = b_t - L1_t z_{t-1} - L2_t z_{t-2}                  (slots 0, 1)
 //   TW only:
@@ -1034,112 +1034,159 @@ struct PcFrame {
 //                       x of local plane n + i = [Sinv blocks of that plane] [r_m; r_m1]
 //   B(t), t = n-1..0:   x_t = Uinv_t z_t + (-Uinv_t U1_t) x_{t+1} + (-Uinv_t U2_t) x_{t+2}  (slots 2..4)
 // Without TW the backward stages run t = Nz-1..0 (couplings beyond the last plane are absent).
-#define PA_THREADS 256
+// A row's sum runs over its blocks in the order written above, then over the lanes by a butterfly.
+// What bounds it: 8x8x32 (18 CTAs, 26.5 MB in L2) 19.3 us a launch, 0.46 us a stage: the stage's 37 to 55
+// KB come from L2 at 50 bytes a cycle and SM, 4.5 us are before the first stage and after the last.  A
+// three-deep ring of bulk copies in shared memory, whose blocks then crossed shared memory twice more,
+// took 30.6 us; one row per lane group (twice the shared-memory reads of the planes) 23.6 us.  8x8x12: 15.3
+// -> 10.0 us, 16x16x64: 57.3 -> 46.4 us (182 MB at 4.0 TB/s).
 #define PA_LANES 8
-#define PA_IO 8            // entries per thread whose loads the prologue / epilogue batch
-template <int NJ, int NBUF, typename TS, bool TW>
-__global__ void __launch_bounds__(PA_THREADS) k_pc_apply(PcGeom gin, const TS* __restrict__ A,
-                                                         const double* __restrict__ b, const double* __restrict__ sc,
-                                                         double* __restrict__ x, int* __restrict__ err, PaFuse F) {
+#define PA_DEPTH 2         // stages whose factors are in flight ahead of their use
+// Factors that do not stay in L2 (126 MB) from one sweep to the next are also prefetched into it, PA_AHEAD
+// stages ahead.  The line lies between 86 MB, where prefetching what is already there costs 4 % (12x12x48:
+// 27.4 -> 28.6 us), and 100 MB, where it gains 6 % (16x16x64 in FP32: 50.5 -> 47.4 us); at 117 MB 47.4 ->
+// 39.4 us, at 182 MB 57.8 -> 46.4 us (8 stages: 46.9, 16: 55.6).
+#define PA_AHEAD 4
+#define PA_L2_BYTES (90ll << 20)
+#define PA_IO 4            // entries per thread whose loads the prologue / epilogue batch
+#define PA_SUM 256         // the result's sum of squares is taken over this many strided parts, warp by warp
+constexpr int pa_threads(int NJ) { return NJ <= 2 ? 128 : 64 * NJ; }       // 8 NJ row pairs of 8 lanes
+
+// stages of a CTA that holds np planes, at most (both ranks)
+constexpr int pa_stages(int np, bool tw) { return tw ? 2 * np - 2 : 2 * np - 1; }
+
+template <int NJ, typename TS, bool TW, bool AH>
+__global__ void __launch_bounds__(pa_threads(NJ), 1) k_pc_apply(PcGeom gin, const TS* __restrict__ A,
+                                                                const double* __restrict__ b,
+                                                                const double* __restrict__ sc, double* __restrict__ x,
+                                                                PaFuse F) {
     pdl_wait();                                // (launched programmatically inside the GMRES graph)
     pdl_trigger();
-    if (F.stop && *F.stop) {                   // an Arnoldi step after the solve stopped: a zero direction
-        if (blockIdx.x == 0 && threadIdx.x == 0 && F.out) *F.out = 0.0;
-        return;                                // (every CTA of the grid returns here: no barrier is left open)
-    }
     extern __shared__ __align__(128) double dsm[];
-    __shared__ __align__(8) uint64_t bars[NBUF];
-    constexpr int LD = NJ * 2 * PA_LANES;
+    constexpr int LD = NJ * 2 * PA_LANES, NT = pa_threads(NJ), DEPTH = PA_DEPTH;
+    using TS2 = typename std::conditional<std::is_same<TS, float>::value, float2, double2>::type;
     const int rank = TW ? (int)(blockIdx.x & 1u) : 0;
     const int part = TW ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const PcGeom g = pc_part(gin, part);
     const int nb = g.nb, Nz = g.Nz;
     const int tid = threadIdx.x;
-    const int64_t bs = g.bs;
+    const int bs = (int)g.bs;
     const PcFrame fr{rank, TW ? (rank == 0 ? g.zs : Nz - g.zs - 2) : Nz, Nz};
     const int n = fr.n;
-    double* xs = dsm;                          // [Nz][LD] local planes: b, then z (forward, in place); r on the separator
-    double* xb = xs + (int64_t)Nz * LD;        // [Nz][LD]: x (backward sweep); padding columns zero
-    double* xch = xb + (int64_t)Nz * LD;       // [2][LD]: this rank's partial right-hand sides of the separator (TW)
-    TS* buf0 = reinterpret_cast<TS*>(xch + 2 * LD);   // NBUF ring buffers of [3 bs]
-    const TS* base = A + (int64_t)part * Nz * 5 * bs;
+    // local planes held (the same on both ranks: each reads the other's xch at its own address)
+    const int np = TW ? max(g.zs, Nz - g.zs - 2) + 2 : Nz;
     const int S = TW ? 2 * n + 2 : 2 * Nz - 1;
-    // local planes whose b this CTA reads and whose x it writes
-    const int nio = TW ? (rank == 0 ? n + 2 : n) : Nz;
-    auto blk = [&](int t, int sl) -> const TS* { return base + ((int64_t)fr.gp(t) * 5 + fr.gs(sl)) * bs; };
-    // the stage's copies: one contiguous run of slots, plus (TW stage X) one more block
-    auto issue = [&](int s, uint32_t dst, uint32_t bar) {
-        const uint32_t b1 = (uint32_t)(bs * sizeof(TS));
-        const TS* src;
-        uint32_t nblk;
-        const TS* src2 = nullptr;
-        if (s < n - 1) {                                   // F(t): slots 0, 1
-            src = (fr.rank == 0) ? blk(s + 1, 0) : blk(s + 1, 1);
-            nblk = 2;
-        } else if (TW && s == n - 1) {                     // X: plane n slots 0, 1; plane n+1 slot 0
-            src = (fr.rank == 0) ? blk(n, 0) : blk(n, 1);
-            nblk = 2;
-            src2 = blk(n + 1, 0);
-        } else if (TW && s <= n + 1) {                     // C(i): the separator plane's two Sinv blocks
-            const int P = fr.gp(n + (s - n));
-            src = base + ((int64_t)P * 5 + (P == g.zs ? 2 : 1)) * bs;
-            nblk = 2;
-        } else {                                           // B(t): slots 2..4
-            const int t = TW ? n - 1 - (s - (n + 2)) : Nz - 1 - (s - (Nz - 1));
-            src = (fr.rank == 0) ? blk(t, 2) : blk(t, 4);
-            nblk = 3;
-        }
-        const uint32_t tot = (nblk + (src2 ? 1u : 0u)) * b1;
-        // a copy from outside the factor storage is not issued (its stage then times out)
-        if (!pc_range_ok(g, (int64_t)(src - A), (int64_t)nblk * bs) || (src2 && !pc_range_ok(g, (int64_t)(src2 - A), bs)))
-            return;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tot) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(dst), "l"(src), "r"(nblk * b1), "r"(bar) : "memory");
-        if (src2)
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(dst + nblk * b1), "l"(src2), "r"(b1), "r"(bar) : "memory");
-    };
-    if (tid == 0) {
-        for (int q = 0; q < NBUF; ++q) mbar_init(smem_u32(&bars[q]), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    const int rh = (nb + 1) >> 1;              // rows per half: a group of 8 lanes takes rows r0 and r0 + rh
-    // the thread that issues the ring's copies and the warp that polls their mbarriers: the last warp
-    // when it has no rows (nb <= 56), so neither the copy issue nor the poll is on the row warps' path
-    // to the next barrier; that warp then takes no part in the prologue either
-    const int issuer = (rh <= PA_THREADS / PA_LANES - 32 / PA_LANES) ? PA_THREADS - 32 : 0;
-    const int pollw = issuer / 32;
-    const int nthr = issuer ? issuer : PA_THREADS;   // threads that load b and clear xb
-    if (tid == issuer)                           // the first NBUF stages are in flight from the start
-        for (int q = 0; q < NBUF && q < S; ++q) issue(q, smem_u32(buf0 + (int64_t)q * 3 * bs), smem_u32(&bars[q]));
+    double* xs = dsm;                          // [np][LD] local planes: b, then z (forward, in place); r on the separator
+    double* xb = xs + np * LD;                 // [np][LD]: x (backward sweep); padding columns zero
+    double* xch = xb + np * LD;                // [2][LD]: this rank's partial right-hand sides of the separator (TW)
+    int4* desc = reinterpret_cast<int4*>(xch + 2 * LD);     // [S + DEPTH]: offsets of a stage's blocks (-1: none)
+    int* gl = reinterpret_cast<int*>(desc + pa_stages(np, TW) + DEPTH);     // [LD]: state index of row l at plane 0
+    const int stopped = F.stop ? *F.stop : 0;
     const int fcol = F.V ? *F.col : 0;
     const double fscale = F.V ? *F.scale : 0.0;
-    const double* __restrict__ src = F.V ? ((fcol == 0) ? F.src0 : F.src1) : b;
+    // a geometry beyond the storage is recorded and x is left untouched (the same on every CTA of a partition)
+    if (!pc_range_ok(g, (int64_t)part * Nz * 5 * bs, (int64_t)Nz * 5 * bs)) return;
+    const TS* base = A + (int64_t)part * Nz * 5 * bs;
+    // the stages' blocks, in the order their products are added (one code path then fetches any stage)
+    for (int s = tid; s < S + DEPTH; s += NT) {
+        int o[3] = {-1, -1, -1};
+        auto blk = [&](int t, int sl) { return (fr.gp(t) * 5 + fr.gs(sl)) * bs; };
+        if (s >= S) {
+        } else if (s < n - 1) {                            // F(t), t = s + 1
+            o[0] = blk(s + 1, 1);
+            if (s >= 1) o[1] = blk(s + 1, 0);
+        } else if (TW && s == n - 1) {                     // X
+            o[0] = blk(n, 1);
+            o[1] = blk(n, 0);
+            o[2] = blk(n + 1, 0);
+        } else if (TW && s <= n + 1) {                     // C(i): the separator plane's two Sinv blocks
+            const int P = fr.gp(s);
+            o[0] = (P * 5 + (P == g.zs ? 2 : 1)) * bs;
+            o[1] = o[0] + bs;
+        } else {                                           // B(t)
+            const int t = TW ? 2 * n + 1 - s : 2 * Nz - 2 - s;
+            o[0] = blk(t, 2);
+            if (TW || t + 1 < Nz) o[1] = blk(t, 3);
+            if (TW || t + 2 < Nz) o[2] = blk(t, 4);
+        }
+        // (the blocks of a stage are one run of slots, but for X's third: the run's first and its blocks)
+        const bool x3 = TW && s == n - 1;
+        const int first = o[1] < 0 ? o[0] : (o[2] < 0 || x3) ? min(o[0], o[1]) : min(o[0], o[2]);
+        const int cnt = o[0] < 0 ? 0 : o[1] < 0 ? 1 : (o[2] < 0 || x3) ? 2 : 3;
+        desc[s] = make_int4(o[0], o[1], o[2], s < S ? (first / bs) * 4 + cnt : 0);
+    }
+    if (tid < LD) {
+        int64_t gi = -1;
+        if (tid < nb) {
+            gi = pc_glob(g, part, 0, tid);                 // (plane k of the row: gi + k)
+            if (gi < 0 || gi + Nz > g.nstate) {
+                if (g.err) atomicOr(g.err, PC_ERR_RANGE);
+                gi = -1;
+            }
+        }
+        gl[tid] = (int)gi;
+    }
+    __syncthreads();
+    const int lane = tid % PA_LANES, rh = (nb + 1) >> 1;
+    const int r0 = tid / PA_LANES, r1 = r0 + rh;            // rows of this group
+    const bool put0 = r0 < rh && lane == 0, put1 = put0 && r1 < nb;
+    // this lane's first pair of its rows in slot 0, plane 0 (a row beyond the plane reads row 0 and is not stored)
+    const TS* mine0 = base + (r0 < rh ? r0 : 0) * LD + 2 * lane;
+    const TS* mine1 = base + (r0 < rh && r1 < nb ? r1 : 0) * LD + 2 * lane;
+    struct Blk {
+        TS2 a[NJ], b[NJ];
+    };
+    Blk R[DEPTH][3];
+    auto load = [&](int s, Blk (&M)[3]) {
+        const int4 d = desc[s];
+        const int o[3] = {d.x, d.y, d.z};
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+            if (o[e] >= 0) {
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    M[e].a[j] = __ldg(reinterpret_cast<const TS2*>(mine0 + o[e]) + PA_LANES * j);
+                    M[e].b[j] = __ldg(reinterpret_cast<const TS2*>(mine1 + o[e]) + PA_LANES * j);
+                }
+            }
+    };
+    // stages beyond the ones in registers, into L2 (factors larger than L2)
+    auto prefetch = [&](int s) {
+        if (s >= S) return;
+        const int w = desc[s].w;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                     ::"l"(base + (int64_t)(w >> 2) * bs), "r"((uint32_t)((w & 3) * bs * (int)sizeof(TS))) : "memory");
+    };
+    if (AH && tid >= DEPTH && tid < PA_AHEAD) prefetch(tid);
+    // buffer u serves the stages congruent to rem + u, so that X (without TW the first backward stage) is 0's
+    const int nf = n - 1;                      // forward stages
+    const int rem = nf % DEPTH;
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u) load(min((rem + u) % DEPTH, S), R[u]);
+    // an Arnoldi step after the solve stopped: a zero direction (every CTA of the grid returns here)
+    if (stopped) {
+        if (blockIdx.x == 0 && tid == 0 && F.out) *F.out = 0.0;
+        return;
+    }
+    const double* __restrict__ src = F.V ? ((F.src0 == F.src1 || fcol != 0) ? F.src1 : F.src0) : b;
     // b (or the basis vector to normalise) into xs: PA_IO entries per thread at a time, all their
-    // loads issued before the first use
-    for (int q0 = (tid < nthr) ? tid : Nz * LD; q0 < Nz * LD; q0 += PA_IO * nthr) {
-        int64_t gi[PA_IO];
+    // loads issued before the first use; rank 1 leaves the separator's b to rank 0
+    const int nio = TW ? (rank == 0 ? n + 2 : n) : Nz;
+    for (int q0 = tid; q0 < np * LD; q0 += PA_IO * NT) {
+        int gi[PA_IO];
         double bv[PA_IO], sv[PA_IO];
 #pragma unroll
         for (int u = 0; u < PA_IO; ++u) {
-            const int q = q0 + u * nthr;
+            const int q = q0 + u * NT;
             const int t = q / LD, l = q - t * LD;
-            bool in = q < Nz * LD && l < nb && t < nio;
-            gi[u] = in ? pc_glob(g, part, fr.gp(t), l) : -1;
-            if (in && (gi[u] < 0 || gi[u] >= g.nstate)) {
-                if (g.err) atomicOr(g.err, PC_ERR_RANGE);
-                in = false;
-                gi[u] = -1;
-            }
-            bv[u] = in ? src[gi[u]] : 0.0;
-            sv[u] = (in && sc) ? sc[gi[u]] : 1.0;
+            gi[u] = (t < nio && gl[l] >= 0) ? gl[l] + fr.gp(t) : -1;
+            bv[u] = gi[u] >= 0 ? src[gi[u]] : 0.0;
+            sv[u] = (gi[u] >= 0 && sc) ? sc[gi[u]] : 1.0;
         }
 #pragma unroll
         for (int u = 0; u < PA_IO; ++u) {
-            const int q = q0 + u * nthr;
-            if (q >= Nz * LD) break;
+            const int q = q0 + u * NT;
+            if (q >= np * LD) break;
             double v = 0.0;
             if (gi[u] >= 0) {
                 double x0 = bv[u];
@@ -1150,196 +1197,174 @@ __global__ void __launch_bounds__(PA_THREADS) k_pc_apply(PcGeom gin, const TS* _
                 v = sc ? x0 * sv[u] : x0;
             }
             xs[q] = v;
+            xb[q] = 0.0;
         }
     }
-    for (int q = tid; q < Nz * LD && tid < nthr; q += nthr) xb[q] = 0.0;
     __syncthreads();
-    const int lane = tid % PA_LANES;
-    const int grp = tid / PA_LANES;
-    const int r0 = grp, r1 = grp + rh;
-    const bool act0 = r0 < rh, act1 = act0 && r1 < nb;
-    int issued = (S < NBUF) ? S : NBUF;        // stages whose copies have been issued
-    int bi = 0, pb = NBUF - 1;                 // this stage's ring buffer, the previous stage's
-    uint32_t par = 0;
-    // one block times one solution plane for both rows of the group (the vector loads are shared)
-    using TS2 = typename std::conditional<std::is_same<TS, float>::value, float2, double2>::type;
-    auto dot2 = [&](const TS* M, const double* v, double& acc0, double& acc1) {
-        const TS2* ma = reinterpret_cast<const TS2*>(M + r0 * LD) + lane;
-        const TS2* mb = reinterpret_cast<const TS2*>(M + (act1 ? r1 : r0) * LD) + lane;
-        const double2* vp = reinterpret_cast<const double2*>(v) + lane;
+    // a plane's entries at this lane's columns
+    struct Vec {
+        double2 v[NJ];
+    };
+    auto plane = [&](const double* p, Vec& o) {
+        const double2* vp = reinterpret_cast<const double2*>(p) + lane;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) o.v[j] = vp[PA_LANES * j];
+    };
+    auto dot = [&](const Blk& M, const Vec& o, double& a0, double& a1) {
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-            const double2 vv = vp[PA_LANES * j];
-            const TS2 a = ma[PA_LANES * j], c = mb[PA_LANES * j];
-            acc0 += (double)a.x * vv.x;
-            acc1 += (double)c.x * vv.x;
-            acc0 += (double)a.y * vv.y;
-            acc1 += (double)c.y * vv.y;
+            a0 += (double)M.a[j].x * o.v[j].x;
+            a1 += (double)M.b[j].x * o.v[j].x;
+            a0 += (double)M.a[j].y * o.v[j].y;
+            a1 += (double)M.b[j].y * o.v[j].y;
         }
     };
-    auto reduce = [&](double& acc0, double& acc1) {
+    auto reduce = [&](double& a0, double& a1) {
 #pragma unroll
         for (int off = PA_LANES / 2; off > 0; off >>= 1) {
-            acc0 += __shfl_xor_sync(0xffffffffu, acc0, off, PA_LANES);
-            acc1 += __shfl_xor_sync(0xffffffffu, acc1, off, PA_LANES);
+            a0 += __shfl_xor_sync(0xffffffffu, a0, off, PA_LANES);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, off, PA_LANES);
         }
     };
-    auto put = [&](double* row, double a0, double a1) {
-        if (lane == 0 && act0) {
-            row[r0] = a0;
-            if (act1) row[r1] = a1;
-        }
+    auto store = [&](double* p, double a0, double a1) {
+        if (put0) p[r0] = a0;
+        if (put1) p[r1] = a1;
     };
-    // One barrier per stage: it publishes the previous stage's rows and frees its buffer, which is
-    // refilled right after it.  Forward rows overwrite b_t by z_t in xs (each row reads and writes
-    // only its own entry of plane t); backward rows go to xb, as every row reads all of z_t.  Warp
-    // `pollw` alone polls the copy's mbarrier; the barrier carries its answer to the others.
-    auto stage = [&](int s) -> bool {
-        TS* buf = buf0 + (int64_t)bi * 3 * bs;
-        const bool arrived = ((tid >> 5) == pollw) ? mbar_wait(smem_u32(&bars[bi]), par) : true;
-        if (!__syncthreads_and(arrived)) {       // uniform decision: no thread is left at a barrier
-            if (tid == 0) atomicOr(err, 1);
-            return false;
+    // One barrier per stage: it publishes the previous stage's rows.  Forward rows overwrite b_t by z_t in
+    // xs (each row reads and writes only its own entry of plane t); backward rows go to xb.  V[u] takes the
+    // newest plane of a stage served by buffer u, so V[u ^ 1] still holds the one before it.  The code of
+    // both loops is kept small: a launch runs through it once, from a cold instruction cache.
+    static_assert(DEPTH == 2, "V alternates with the buffers");
+    Vec V[2];
+#pragma unroll 1
+    for (int s0 = rem ? rem - DEPTH : 0; s0 < nf; s0 += DEPTH) {
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+            const int s = s0 + u;
+            if (s < 0) continue;
+            double* o = xs + (s + 1) * LD;
+            const double b0 = put0 ? o[r0] : 0.0, b1 = put1 ? o[r1] : 0.0;
+            __syncthreads();
+            plane(xs + s * LD, V[u]);
+            double a0 = 0.0, a1 = 0.0;
+            dot(R[u][0], V[u], a0, a1);
+            if (s >= 1) dot(R[u][1], V[u ^ 1], a0, a1);
+            load(s + DEPTH, R[u]);
+            if (AH && tid == 0) prefetch(s + PA_AHEAD);
+            reduce(a0, a1);
+            store(o, b0 - a0, b1 - a1);
         }
-        if (s >= 1 && s - 1 + NBUF < S) {        // the previous stage's buffer is free: refill it
-            if (tid == issuer) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                issue(s - 1 + NBUF, smem_u32(buf0 + (int64_t)pb * 3 * bs), smem_u32(&bars[pb]));
-            }
-            issued = s + NBUF;
-        }
-        const int64_t oL2 = (fr.rank == 0) ? 0 : bs, oL1 = (fr.rank == 0) ? bs : 0;
-        double a0 = 0.0, a1 = 0.0;
-        if (s < n - 1) {                                       // F(t)
-            const int t = s + 1;
-            double* row = xs + (int64_t)t * LD;
-            double b0 = 0.0, b1 = 0.0;                         // this plane's b, read ahead of the products
-            if (lane == 0 && act0) {
-                b0 = row[r0];
-                if (act1) b1 = row[r1];
-            }
-            if (act0) {
-                dot2(buf + oL1, xs + (int64_t)(t - 1) * LD, a0, a1);
-                if (t >= 2) dot2(buf + oL2, xs + (int64_t)(t - 2) * LD, a0, a1);
-            }
-            reduce(a0, a1);
-            if (lane == 0 && act0) {
-                row[r0] = b0 - a0;
-                if (act1) row[r1] = b1 - a1;
-            }
-        } else if (TW && s == n - 1) {                         // X: partial right-hand sides of the separator
-            if (act0) {
-                dot2(buf + oL1, xs + (int64_t)(n - 1) * LD, a0, a1);
-                dot2(buf + oL2, xs + (int64_t)(n - 2) * LD, a0, a1);
-            }
-            reduce(a0, a1);
-            if (lane == 0 && act0) {
-                xch[r0] = xs[(int64_t)n * LD + r0] - a0;
-                if (act1) xch[r1] = xs[(int64_t)n * LD + r1] - a1;
-            }
-            a0 = a1 = 0.0;
-            if (act0) dot2(buf + 2 * bs, xs + (int64_t)(n - 1) * LD, a0, a1);
-            reduce(a0, a1);
-            if (lane == 0 && act0) {
-                xch[LD + r0] = xs[(int64_t)(n + 1) * LD + r0] - a0;
-                if (act1) xch[LD + r1] = xs[(int64_t)(n + 1) * LD + r1] - a1;
-            }
-        } else if (TW && s <= n + 1) {                         // C(i): both ranks solve the separator
-            const int t = n + (s - n);
-            const int lz0 = (fr.rank == 0) ? n : n + 1;        // local plane of global zs
-            if (act0) {
-                dot2(buf, xs + (int64_t)lz0 * LD, a0, a1);
-                dot2(buf + bs, xs + (int64_t)(2 * n + 1 - lz0) * LD, a0, a1);
-            }
-            reduce(a0, a1);
-            put(xb + (int64_t)t * LD, a0, a1);
-        } else {                                               // B(t)
-            const int t = TW ? n - 1 - (s - (n + 2)) : Nz - 1 - (s - (Nz - 1));
-            const int lim = TW ? n + 2 : Nz;
-            const int64_t oU = (fr.rank == 0) ? 0 : 2 * bs, oW2 = (fr.rank == 0) ? 2 * bs : 0;
-            if (act0) {
-                dot2(buf + oU, xs + (int64_t)t * LD, a0, a1);
-                if (t + 1 < lim) dot2(buf + bs, xb + (int64_t)(t + 1) * LD, a0, a1);
-                if (t + 2 < lim) dot2(buf + oW2, xb + (int64_t)(t + 2) * LD, a0, a1);
-            }
-            reduce(a0, a1);
-            put(xb + (int64_t)t * LD, a0, a1);
-        }
-        pb = bi;
-        if (++bi == NBUF) {
-            bi = 0;
-            par ^= 1u;
-        }
-        return true;
-    };
-    bool ok = true;
-    int s = 0;
-    const int s_x = TW ? n : S;                  // stages before the exchange
-    for (; s < s_x && ok; ++s) ok = stage(s);
+    }
     if constexpr (TW) {
-        __syncthreads();                         // this rank's partials are in xch
-        cluster_sync_all();                      // ... and the other rank's (both ranks always arrive)
-        if (ok) {
-            const uint32_t other = (uint32_t)(fr.rank ^ 1);
-            for (int q = tid; q < 2 * LD; q += blockDim.x) {
-                const int c = q / LD, l = q - c * LD;   // separator plane zs + c, row l
-                if (l >= nb) continue;
-                // plane zs + c is slot c of rank 0's xch and slot 1 - c of rank 1's; the sum is
-                // taken in the same order on both ranks, so both hold the same r
-                const double* q0 = xch + c * LD + l;
-                const double* q1 = xch + (1 - c) * LD + l;
-                const double p0 = (fr.rank == 0) ? *q0 : ld_peer_cta(q0, other);
-                const double p1 = (fr.rank == 0) ? ld_peer_cta(q1, other) : *q1;
-                xs[(int64_t)(n + ((fr.rank == 0) ? c : 1 - c)) * LD + l] = p0 + p1;
-            }
+        {                                        // X: partial right-hand sides of the separator
+            __syncthreads();
+            plane(xs + (n - 1) * LD, V[0]);
+            double a0 = 0.0, a1 = 0.0, c0 = 0.0, c1 = 0.0;
+            dot(R[0][0], V[0], a0, a1);
+            dot(R[0][1], V[1], a0, a1);
+            dot(R[0][2], V[0], c0, c1);
+            load(n - 1 + DEPTH, R[0]);
+            if (AH && tid < 3) prefetch(n - 1 + tid + PA_AHEAD);      // (and C0's and C1's)
+            reduce(a0, a1);
+            reduce(c0, c1);
+            const double* p = xs + n * LD;
+            store(xch, (put0 ? p[r0] : 0.0) - a0, (put1 ? p[r1] : 0.0) - a1);
+            store(xch + LD, (put0 ? p[LD + r0] : 0.0) - c0, (put1 ? p[LD + r1] : 0.0) - c1);
+        }
+        cluster_sync_all();                      // both ranks' partials are in xch (both always arrive)
+        const uint32_t other = (uint32_t)(fr.rank ^ 1);
+        for (int q = tid; q < 2 * LD; q += NT) {
+            const int c = q / LD, l = q - c * LD;       // separator plane zs + c, row l
+            if (l >= nb) continue;
+            // plane zs + c is slot c of rank 0's xch and slot 1 - c of rank 1's; the sum is
+            // taken in the same order on both ranks, so both hold the same r
+            const double* q0 = xch + c * LD + l;
+            const double* q1 = xch + (1 - c) * LD + l;
+            const double p0 = (fr.rank == 0) ? *q0 : ld_peer_cta(q0, other);
+            const double p1 = (fr.rank == 0) ? ld_peer_cta(q1, other) : *q1;
+            xs[(n + ((fr.rank == 0) ? c : 1 - c)) * LD + l] = p0 + p1;
         }
         __syncthreads();
+        {                                        // C0, C1: both ranks solve the separator
+            const int lz0 = (fr.rank == 0) ? n : n + 1;     // local plane of global zs
+            plane(xs + lz0 * LD, V[0]);
+            plane(xs + (2 * n + 1 - lz0) * LD, V[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                Blk (&M)[3] = R[(1 + e) % DEPTH];
+                double a0 = 0.0, a1 = 0.0;
+                dot(M[0], V[0], a0, a1);
+                dot(M[1], V[1], a0, a1);
+                load(n + e + DEPTH, M);
+                reduce(a0, a1);
+                store(xb + (n + e) * LD, a0, a1);
+            }
+        }
     }
-    for (; s < S && ok; ++s) ok = stage(s);
-    const int s_fail = ok ? S : s - 1;           // first stage whose data was not consumed
+    __syncthreads();                             // planes read ahead of the first barrier below
+    if (TW) plane(xb + (n + 1) * LD, V[1]);
+    constexpr int B0 = TW ? 3 : 0;               // buffer of the first backward stage
+    const int lim = TW ? n + 2 : Nz;
+#pragma unroll 1
+    for (int s0 = TW ? n + 2 : Nz - 1; s0 < S; s0 += DEPTH) {
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+            const int s = s0 + u;
+            if (s >= S) break;
+            Blk (&M)[3] = R[(B0 + u) % DEPTH];
+            const int t = TW ? 2 * n + 1 - s : 2 * Nz - 2 - s;
+            Vec zt;
+            plane(xs + t * LD, zt);
+            double a0 = 0.0, a1 = 0.0;
+            dot(M[0], zt, a0, a1);
+            __syncthreads();
+            if (TW || t + 1 < lim) {
+                plane(xb + (t + 1) * LD, V[u]);
+                dot(M[1], V[u], a0, a1);
+            }
+            if (TW || t + 2 < lim) dot(M[2], V[u ^ 1], a0, a1);
+            load(s + DEPTH, M);
+            if (AH && tid == 0) prefetch(s + PA_AHEAD);
+            reduce(a0, a1);
+            store(xb + t * LD, a0, a1);
+        }
+    }
     __syncthreads();                             // the last stage's rows
-    double ss = 0.0;
-    if (!ok) {                                   // drain copies still in flight (bounded) and leave x untouched
-        if (tid == 0)
-            for (int s2 = s_fail; s2 < issued; ++s2)
-                mbar_wait(smem_u32(&bars[s2 % NBUF]), (uint32_t)((s2 / NBUF) & 1));
-    } else {                                     // x out, PA_IO entries per thread at a time
-        for (int q0 = tid; q0 < Nz * LD; q0 += PA_IO * PA_THREADS) {
-            int64_t gi[PA_IO];
+    // x out, and its sum of squares: part vt takes the entries congruent to vt, in order
+    __shared__ double wsum[PA_SUM / 32];
+    for (int vt = tid; vt < PA_SUM; vt += NT) {
+        double ss = 0.0;
+        for (int q0 = vt; q0 < nio * LD; q0 += PA_IO * PA_SUM) {     // PA_IO entries at a time
+            int gi[PA_IO];
             double sv[PA_IO];
 #pragma unroll
             for (int u = 0; u < PA_IO; ++u) {
-                const int q = q0 + u * PA_THREADS;
+                const int q = q0 + u * PA_SUM;
                 const int t = q / LD, l = q - t * LD;
-                bool in = q < Nz * LD && l < nb && t < nio;
-                gi[u] = in ? pc_glob(g, part, fr.gp(t), l) : -1;
-                if (in && (gi[u] < 0 || gi[u] >= g.nstate)) {
-                    if (g.err) atomicOr(g.err, PC_ERR_RANGE);
-                    in = false;
-                    gi[u] = -1;
-                }
-                sv[u] = (in && sc) ? sc[gi[u]] : 1.0;
+                gi[u] = (t < nio && gl[l] >= 0) ? gl[l] + fr.gp(t) : -1;
+                sv[u] = (gi[u] >= 0 && sc) ? sc[gi[u]] : 1.0;
             }
 #pragma unroll
             for (int u = 0; u < PA_IO; ++u) {
                 if (gi[u] < 0) continue;
-                const int q = q0 + u * PA_THREADS;
+                const int q = q0 + u * PA_SUM;
                 const double xv = sc ? xb[q] / sv[u] : xb[q];
                 x[gi[u]] = xv;
                 ss += xv * xv;
             }
         }
+        if (F.out) {                             // (vt's warp is whole: PA_SUM and NT are multiples of 32)
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            if ((vt & 31) == 0) wsum[vt >> 5] = ss;
+        }
     }
     if (F.out) {                                 // rms of the result: per-CTA partial, last CTA finishes
-        __shared__ double wsum[PA_THREADS / 32];
         __shared__ bool last;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-        if ((tid & 31) == 0) wsum[tid >> 5] = ss;
         __syncthreads();
         if (tid == 0) {
             double t = 0.0;
-            for (int w = 0; w < PA_THREADS / 32; ++w) t += wsum[w];
+            for (int w = 0; w < PA_SUM / 32; ++w) t += wsum[w];
             F.part[blockIdx.x] = t;
             __threadfence();
             last = (atomicAdd(F.ticket, 1u) == gridDim.x - 1);
@@ -1591,7 +1616,6 @@ static cudaError_t launch_pair(void (*kern)(KArgs...), unsigned grid, unsigned b
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-static size_t apply_smem(const PcGeom& g, int nbuf, size_t tsize);
 static bool apply_fusable(const PcGeom& g, size_t tsize);
 static size_t pc_tsize(const dv_model* m);
 
@@ -1658,49 +1682,47 @@ int precond_factor(dv_model* m, const double* J, double dh, int mode, cudaStream
     return DV_OK;
 }
 
-// shared memory of the sweep with an NBUF-deep ring: solution planes, one plane of scratch, buffers
-// shared memory of the sweep with an NBUF-deep ring of factor blocks stored as `tsize`-byte values
-static size_t apply_smem(const PcGeom& g, int nbuf, size_t tsize) {
-    return sizeof(double) * (size_t)(2 * (int64_t)g.Nz * g.ld + 2 * g.ld) + tsize * (size_t)((int64_t)nbuf * 3 * g.bs);
+// The rule for the register-streamed sweep, and with it for the twisted factorisation: two sets of
+// solution planes, the exchange planes and 2 x 3 factor blocks of `tsize`-byte values within the shared
+// memory of a CTA.  (The sweep itself needs the planes only; the line stays where it was because moving
+// it would change which shapes are factorised from both ends, and so their results.)
+static size_t apply_smem(const PcGeom& g, size_t tsize) {
+    return sizeof(double) * (size_t)(2 * (int64_t)g.Nz * g.ld + 2 * g.ld) + tsize * (size_t)(2 * 3 * g.bs);
 }
 
 static size_t pc_tsize(const dv_model* m) { return m->pc_fp32 ? sizeof(float) : sizeof(double); }
 
-// ring depth: three stages in flight when they fit in shared memory, else two
-static int apply_nbuf(const PcGeom& g, size_t tsize, int want = 0) {
-    const bool three = apply_smem(g, 3, tsize) <= (size_t)smem_optin();
-    return (three && want != 2) ? 3 : 2;
-}
-
-template <int NJ, int NBUF, typename TS, bool TW>
+template <int NJ, typename TS, bool TW>
 static void launch_apply_tw(const PcGeom& g, dv_model* m, const TS* A, const double* b, const double* sc, double* x,
                             cudaStream_t s, const PaFuse& F, bool count) {
-    const size_t dyn = apply_smem(g, NBUF, sizeof(TS));
-    auto kern = k_pc_apply<NJ, NBUF, TS, TW>;
+    const int np = TW ? std::max(g.zs, g.Nz - g.zs - 2) + 2 : g.Nz;
+    const size_t dyn = sizeof(double) * (size_t)(2 * np + 2) * g.ld + sizeof(int4) * (size_t)(pa_stages(np, TW) + PA_DEPTH) +
+                       sizeof(int) * (size_t)g.ld;
+    const int64_t bytes = (int64_t)sizeof(TS) * g.nparts * g.Nz * 5 * g.bs;
+    bool ah = m->tune.sweep_nbuf == 3 || (m->tune.sweep_nbuf != 2 && bytes > PA_L2_BYTES);
+    auto kern = k_pc_apply<NJ, TS, TW, false>;
+    if constexpr (TW && NJ >= 3) {              // (smaller blocks add up to PA_L2_BYTES on no supported cross-section)
+        if (ah) kern = k_pc_apply<NJ, TS, TW, true>;
+    }
     if (dyn > 48 * 1024) allow_dyn_smem((const void*)kern);
     if (count) prof_begin(dv::K_PC_APPLY, s);
-    if (TW) launch_pair(kern, 2u * g.nparts, PA_THREADS, dyn, s, F.pdl, g, A, b, sc, x, m->d_err, F);
-    else kern<<<g.nparts, PA_THREADS, dyn, s>>>(g, A, b, sc, x, m->d_err, F);
+    if (TW) launch_pair(kern, 2u * g.nparts, pa_threads(NJ), dyn, s, F.pdl, g, A, b, sc, x, F);
+    else kern<<<g.nparts, pa_threads(NJ), dyn, s>>>(g, A, b, sc, x, F);
     if (count) prof_end(dv::K_PC_APPLY, s);
 }
 
-template <int NJ, int NBUF, typename TS>
+template <int NJ, typename TS>
 static void launch_apply_k(const PcGeom& g, dv_model* m, const TS* A, const double* b, const double* sc, double* x,
                            cudaStream_t s, const PaFuse& F, bool count) {
-    if (g.zs > 0) launch_apply_tw<NJ, NBUF, TS, true>(g, m, A, b, sc, x, s, F, count);
-    else launch_apply_tw<NJ, NBUF, TS, false>(g, m, A, b, sc, x, s, F, count);
+    if (g.zs > 0) launch_apply_tw<NJ, TS, true>(g, m, A, b, sc, x, s, F, count);
+    else launch_apply_tw<NJ, TS, false>(g, m, A, b, sc, x, s, F, count);
 }
 
 template <int NJ>
 static void launch_apply_nj(const PcGeom& g, dv_model* m, const double* b, const double* sc, double* x, cudaStream_t s,
                             const PaFuse& F, bool count) {
-    if (m->pc_fp32) {               // factors stored in FP32 (mixed-precision Krylov), products in FP64
-        if (apply_nbuf(g, sizeof(float), m->tune.sweep_nbuf) == 3) launch_apply_k<NJ, 3, float>(g, m, m->d_pc32, b, sc, x, s, F, count);
-        else launch_apply_k<NJ, 2, float>(g, m, m->d_pc32, b, sc, x, s, F, count);
-    } else {
-        if (apply_nbuf(g, sizeof(double), m->tune.sweep_nbuf) == 3) launch_apply_k<NJ, 3, double>(g, m, m->d_pc, b, sc, x, s, F, count);
-        else launch_apply_k<NJ, 2, double>(g, m, m->d_pc, b, sc, x, s, F, count);
-    }
+    if (m->pc_fp32) launch_apply_k<NJ, float>(g, m, m->d_pc32, b, sc, x, s, F, count);   // FP32 factors, products in FP64
+    else launch_apply_k<NJ, double>(g, m, m->d_pc, b, sc, x, s, F, count);
 }
 
 static void launch_apply(const PcGeom& g, dv_model* m, const double* b, const double* sc, double* x, cudaStream_t s,
@@ -1733,7 +1755,7 @@ int precond_apply(dv_model* m, const double* b, const double* sc, double* x, cud
 }
 
 static bool apply_fusable(const PcGeom& g, size_t tsize) {
-    return g.nb <= 64 && g.ld % (2 * PA_LANES) == 0 && apply_smem(g, 2, tsize) <= (size_t)smem_optin();
+    return g.nb <= 64 && g.ld % (2 * PA_LANES) == 0 && apply_smem(g, tsize) <= (size_t)smem_optin();
 }
 
 bool precond_apply_fusable(dv_model* m) { return apply_fusable(geom_factored(m), pc_tsize(m)); }

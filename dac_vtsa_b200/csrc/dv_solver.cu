@@ -792,7 +792,7 @@ static int gmres(Work& W, const Op& op, const double* b, double rtol, double ato
 static int check_device_error(dv_model* m);
 static void clear_device_error(dv_model* m);
 
-// the model's device error word: bit 1 a preconditioner sweep's bulk-copy wait timed out, bit 4 a
+// the model's device error word: bit 1 a bulk-copy wait timed out, bit 4 a
 // grid barrier of a cooperative kernel (Gram-Schmidt, the FD matvec) timed out
 static const char* device_error_text(int e) {
     if (e & 32) return "a preconditioner index fell outside its storage (the access was skipped)";
@@ -2384,7 +2384,7 @@ int dv_autotune(dv_model* m, double t, const double* y, double dh, int32_t reps,
     }
     m->tune.fdjac_block = tu.fdjac_block;
     DV_TRY(precond_factor(m, W.J, dh, mode, st));
-    // sweep ring depth (the shared-memory sweep only)
+    // prefetch of the sweep's factors into L2 (the register-streamed sweep only)
     DV_CUDA(cudaMemcpyAsync(W.b, W.f, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
     if (precond_apply_fusable(m)) {
         bestv = INFINITY;

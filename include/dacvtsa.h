@@ -299,11 +299,10 @@ int dv_integrator_copy_y(const dv_integrator* g, double* dst, void* stream);
 
 /* ------------------------------------------------------------------ launch tuning
  * No reference counterpart.  Launch parameters of the hot kernels, per model: the Arnoldi steps the
- * GMRES graph runs ahead of its WHILE node (gmres_prefix, -1 = library default), the depth of the
- * preconditioner sweep's shared-memory ring of factor blocks (sweep_nbuf 2 or 3, 0 = deepest that
- * fits), the block size of the FP32 Jacobian product, that of the FD Jacobian (accepted; its kernels now
- * have one block shape each), and the Arnoldi
- * steps per pass through the WHILE node (gmres_body 1 or 2, 0 = library default: every pass costs a
+ * GMRES graph runs ahead of its WHILE node (gmres_prefix, -1 = library default), whether the
+ * preconditioner sweep prefetches its factors into L2 (sweep_nbuf 3: yes, 2: no, 0 = by their size),
+ * the block size of the FP32 Jacobian product, that of the FD Jacobian (accepted; its kernels have one
+ * block shape each), and the Arnoldi steps per pass through the WHILE node (gmres_body 1 or 2, 0 = library default: every pass costs a
  * device-side relaunch; a step after the stop returns at once).  None of them changes a result bit;
  * they only change the time. */
 typedef struct dv_tuning {

@@ -130,6 +130,36 @@ def test_split_partitions_exact_on_dominant_system(Nr, Nth, Nz):
     _check_dominant("theta_block", Nz, Nr, Nth)
 
 
+# block sizes at the edges of the sweep's 16-column groups and of its row pairs: nb 7 and 13 (one group),
+# 19 / 18 (two), 31, 48 without a padding column, 49 and 54 (four groups); odd and even halves of the
+# shortest twisted columns, and one-directional ones down to a single plane
+@pytest.mark.parametrize("Nr,Nth,Nz,mode", [(1, 3, 9, "sector"), (2, 3, 8, "sector"), (3, 3, 10, "sector"),
+                                            (4, 3, 11, "theta_block"), (5, 3, 9, "sector"), (4, 8, 13, "theta_block"),
+                                            (8, 3, 8, "sector"), (9, 9, 9, "theta_block"), (8, 8, 1, "theta_block"),
+                                            (2, 4, 2, "sector"), (8, 8, 7, "theta_block")])
+def test_sweep_block_sizes_and_prefetch(Nr, Nth, Nz, mode):
+    """The sweep equals the sparse LU solve at every block width it is built for, and gives the same bits
+    with and without prefetching the factors into L2 (tuning sweep_nbuf 3 / 2), in both storages."""
+    import ctypes
+    from dac_vtsa_b200._lib import DvTuning
+    m, _ = _pc_model(Nz, Nr, Nth)
+    Jd, Jc = _dominant_jacobian(m, 90 + Nz)
+    b = np.random.default_rng(8).standard_normal(m.n_core)
+    x_ref = spla.spsolve(_restricted(m, Jc, mode, 1.0), b)
+    for precision, tol in (("fp64", 1e-12), ("fp32_factors", 1e-5)):
+        m.set_krylov_precision(precision)
+        m.precond_factor(Jd, 1.0, mode)
+        xs = []
+        for nbuf in (2, 3):
+            t = DvTuning()
+            assert m.lib.dv_model_get_tuning(m.handle, ctypes.byref(t)) == 0
+            t.sweep_nbuf = nbuf
+            assert m.lib.dv_model_set_tuning(m.handle, ctypes.byref(t)) == 0
+            xs.append(m.precond_solve(b))
+        assert np.abs(xs[0] - x_ref).max() <= tol * np.abs(x_ref).max()
+        assert np.array_equal(xs[0], xs[1])
+
+
 def _check_dominant(mode, Nz, Nr, Nth=4):
     m, _ = _pc_model(Nz, Nr, Nth)
     Jd, Jc = _dominant_jacobian(m, 40 + Nz)
