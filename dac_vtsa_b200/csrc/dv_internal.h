@@ -81,6 +81,7 @@ struct Work {
     // device-driven GMRES: one CUDA graph per workspace (built at first use), its device state
     double *vin = nullptr, *wout = nullptr;   // normalised basis vector in / operator output
     unsigned* tickets = nullptr;              // ticket counters of the fused reductions (zeroed)
+    void* cgx = nullptr;                      // exchange buffer of the cooperative Gram-Schmidt kernel (zeroed)
     double* apart = nullptr;                  // per-CTA partials of the fused sweep's reduction
     void* gm = nullptr;                       // device GMRES state
     void* gm_host = nullptr;                  // pinned host mirror of it

@@ -547,6 +547,7 @@ struct GmDev {
     double H[GM_KMAX * (GM_KMAX + 1)], S[GM_KMAX + 1], gc[GM_KMAX], gs[GM_KMAX], y[GM_KMAX + 1];
 };
 static size_t gm_state_bytes() { return sizeof(GmDev); }
+static size_t cg_exchange_bytes();          // the Gram-Schmidt kernel's exchange buffer
 
 // ---------------------------------------------------------------- workspace
 // Test aid: with DVTSA_FILL=<byte>[,<mask>] in the environment, newly allocated workspaces are
@@ -572,7 +573,8 @@ int work_alloc(Work& W, int64_t n, int kdim, int64_t jac_doubles) {
         A(&W.Rt, n) || A(&W.tmp, n) || A(&W.best, n) || A(&W.part, (int64_t)W.nparts * (kdim + 2)) ||
         A(&W.scal, 32) || A(&W.hbuf, 4 * (kdim + 2)) || A(&W.ybuf, kdim + 2) || A(&W.J, jac_doubles) ||
         A(&W.vin, n) || A(&W.wout, n) || A(&W.apart, 4096) || pool_malloc(&W.gm, gm_state_bytes()) != cudaSuccess ||
-        pool_malloc((void**)&W.tickets, 16 * sizeof(unsigned)) != cudaSuccess)
+        pool_malloc((void**)&W.tickets, 16 * sizeof(unsigned)) != cudaSuccess ||
+        pool_malloc(&W.cgx, cg_exchange_bytes()) != cudaSuccess)
         return cuda_fail(cudaGetLastError(), "cudaMalloc(Krylov workspace)");
     if (pool_malloc_host(&W.gm_host, 256) != cudaSuccess) return cuda_fail(cudaGetLastError(), "cudaMallocHost");
     if (pool_malloc_host((void**)&W.hpin, sizeof(double) * 4 * (kdim + 8)) != cudaSuccess)
@@ -593,6 +595,8 @@ int work_alloc(Work& W, int64_t n, int kdim, int64_t jac_doubles) {
     }
     if (cudaMemset(W.tickets, 0, 16 * sizeof(unsigned)) != cudaSuccess)   // ticket counters start at zero
         return cuda_fail(cudaGetLastError(), "cudaMemset(tickets)");
+    if (cudaMemset(W.cgx, 0, cg_exchange_bytes()) != cudaSuccess)         // no epoch has been exchanged yet
+        return cuda_fail(cudaGetLastError(), "cudaMemset(exchange)");
     return DV_OK;
 }
 
@@ -605,6 +609,7 @@ void work_free(Work& W) {
     for (double* p : ptrs) pool_free(p);
     pool_free(W.gm);
     pool_free(W.tickets);
+    pool_free(W.cgx);
     pool_free_host(W.hpin);
     pool_free_host(W.gm_host);
     W = Work();
@@ -837,12 +842,7 @@ __device__ void lartg_d(double f, double g, double& c, double& s, double& r) {
     }
 }
 
-__global__ void k_gm_init(GmDev* st, const double* __restrict__ scal, int kdim, cudaGraphConditionalHandle hnd,
-                          unsigned* bar) {
-    if (threadIdx.x == 0 && bar) {              // barrier words of k_cgs_fused: no arrivals pending
-        bar[0] = 0u;
-        bar[2] = 0u;
-    }
+__global__ void k_gm_init(GmDev* st, const double* __restrict__ scal, int kdim, cudaGraphConditionalHandle hnd) {
     for (int q = threadIdx.x; q < kdim * (kdim + 1); q += blockDim.x) st->H[q] = 0.0;
     for (int q = threadIdx.x; q <= kdim; q += blockDim.x) st->S[q] = 0.0;
     __syncthreads();
@@ -933,31 +933,20 @@ __global__ void k_orth_update_gm(int64_t n, const GmDev* __restrict__ st, const 
     }
 }
 
-// Hessenberg column, Givens rotations, residual estimate and the stopping test of gmres().  One
-// thread.  The rotated entry k + 1 of the new column is carried to the next rotation in a register
-// and the loads (hh, the stored rotations) go through restrict pointers, so they run ahead of the
-// chain of rotations instead of each waiting behind the previous entry's store.
-__device__ void gm_givens(GmDev* st, const double* __restrict__ hh, int kdim, cudaGraphConditionalHandle hnd) {
+// Hessenberg column, Givens rotations, residual estimate and the stopping test of gmres().  One thread.
+// gm_givens_end: the part behind the stored rotations, from ||w||^2 before (hm) and ||w|| after (h1) the
+// orthogonalisation and the column's last entry rotated so far (carry).
+__device__ __forceinline__ void gm_givens_end(GmDev* st, double hm, double h1, double carry, int kdim,
+                                              cudaGraphConditionalHandle hnd) {
     const double eps = 2.220446049250313e-16;                 // double epsilon
     const int col = st->col;
-    const int m = col + 1;
     double* __restrict__ Hc = st->H + (int64_t)col * (kdim + 1);      // column col of H
-    const double* __restrict__ gcs = st->gc;
-    const double* __restrict__ gss = st->gs;
-    const double h0 = sqrt(hh[m]);
-    const double h1 = hh[2 * (kdim + 2)];
-    const double S_col = st->S[col], ptol = st->ptol;         // loaded with the column, ahead of their use
+    const double S_col = st->S[col], ptol = st->ptol;         // loaded ahead of their use
     const int iters = st->iters;
+    const double h0 = sqrt(hm);
     bool breakdown = false;
     if (h1 <= eps * h0 || !(h1 == h1)) breakdown = true;      // the subdiagonal entry is taken as 0
     else st->scale = 1.0 / h1;
-    double carry = hh[0] + hh[(kdim + 2)];                     // entry k of the column, rotated by 0..k-1
-    for (int k = 0; k < col; ++k) {
-        const double c = gcs[k], s2 = gss[k];
-        const double n0 = carry, n1 = hh[k + 1] + hh[(kdim + 2) + k + 1];
-        Hc[k] = c * n0 + s2 * n1;
-        carry = -s2 * n0 + c * n1;
-    }
     double c, s2, mag;
     lartg_d(carry, breakdown ? 0.0 : h1, c, s2, mag);
     st->gc[col] = c;
@@ -975,32 +964,62 @@ __device__ void gm_givens(GmDev* st, const double* __restrict__ hh, int kdim, cu
     st->done = stop;
     cudaGraphSetConditional(hnd, stop ? 0u : 1u);
 }
+// The whole update: the rotated entry k + 1 of the new column is carried to the next rotation in a
+// register and the loads (hh, the stored rotations) go through restrict pointers, so they run ahead of the
+// chain of rotations instead of each waiting behind the previous entry's store.
+__device__ void gm_givens(GmDev* st, const double* __restrict__ hh, int kdim, cudaGraphConditionalHandle hnd) {
+    const int col = st->col;
+    double* __restrict__ Hc = st->H + (int64_t)col * (kdim + 1);
+    const double* __restrict__ gcs = st->gc;
+    const double* __restrict__ gss = st->gs;
+    double carry = hh[0] + hh[(kdim + 2)];                     // entry k of the column, rotated by 0..k-1
+    for (int k = 0; k < col; ++k) {
+        const double c = gcs[k], s2 = gss[k];
+        const double n0 = carry, n1 = hh[k + 1] + hh[(kdim + 2) + k + 1];
+        Hc[k] = c * n0 + s2 * n1;
+        carry = -s2 * n0 + c * n1;
+    }
+    gm_givens_end(st, hh[col + 1], hh[2 * (kdim + 2)], carry, kdim, hnd);
+}
 
 __global__ void k_gm_givens(GmDev* st, const double* __restrict__ hh, int kdim, cudaGraphConditionalHandle hnd) {
     if (threadIdx.x == 0) gm_givens(st, hh, kdim, hnd);
 }
 
 // ---- fused classical Gram-Schmidt of the graph body (three kernels per Arnoldi step)
-// Warp sums of the first cnt entries of acc into out[q] (lane 0).  Each entry is the same butterfly
-// over the 32 lanes; they run eight at a time, side by side (one uniform branch per eight), so the
-// sums wait on about five shuffle latencies per eight entries instead of five per entry.
-__device__ __forceinline__ void warp_sums(const double (&acc)[GM_KMAX + 1], int cnt, int lane, double* out) {
+// Warp sums of the first cnt entries of acc into out[q].  Each entry's sum is the butterfly over the lane
+// distances 16, 8, 4, 2, 1; while more than one entry is left a lane keeps only half of its entries at
+// each distance and sends the other half to its partner (the same additions: a sum taken at the lane that
+// keeps the entry), so N entries cost about N shuffles instead of 5 N.
+template <int N>
+__device__ __forceinline__ void warp_sums_n(const double (&acc)[GM_KMAX + 1], int cnt, int lane, double* out) {
+    double v[N];
 #pragma unroll
-    for (int q0 = 0; q0 <= GM_KMAX; q0 += 8) {
-        if (q0 < cnt) {
-            double v[8];
+    for (int q = 0; q < N; ++q) v[q] = q <= GM_KMAX ? acc[q] : 0.0;
+    int left = N;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = (q0 + u <= GM_KMAX) ? acc[q0 + u] : 0.0;
+    for (int off = 16; off > 0; off >>= 1) {
+        if (left > 1) {
+            left >>= 1;
+            const bool up = lane & off;
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] += __shfl_xor_sync(0xffffffffu, v[u], off);
-            if (lane == 0)
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (q0 + u < cnt) out[q0 + u] = v[u];
+            for (int i = 0; i < N / 2; ++i)
+                if (i < left) {
+                    const double keep = up ? v[i + left] : v[i], send = up ? v[i] : v[i + left];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
         }
     }
+    constexpr int REP = 32 / N;                // lanes that hold the same entry
+    if (lane % REP == 0 && lane / REP < cnt) out[lane / REP] = v[0];
+}
+__device__ __forceinline__ void warp_sums(const double (&acc)[GM_KMAX + 1], int cnt, int lane, double* out) {
+    if (cnt <= 1) warp_sums_n<1>(acc, cnt, lane, out);
+    else if (cnt <= 8) warp_sums_n<8>(acc, cnt, lane, out);
+    else if (cnt <= 16) warp_sums_n<16>(acc, cnt, lane, out);
+    else warp_sums_n<32>(acc, cnt, lane, out);
 }
 
 // Block sums of the first cnt entries of acc (VB threads) into part[blockIdx.x * GM_PS + q];
@@ -1104,126 +1123,284 @@ __global__ void __launch_bounds__(VB) k_cgs_orth_norm(int64_t n, GmDev* st, cons
     }
 }
 
-// ---- CGS2 of one Arnoldi step in a single cooperative launch (grid_sync_bounded: dv_internal.h)
+// ---- CGS2 of one Arnoldi step in a single cooperative launch
+// k_cgs_dots + k_cgs_orth_dots + k_cgs_orth_norm in one launch, with the same block partition and the
+// same summation order (so the same results).  Between the passes every block needs every block's
+// partial sums: each is one 16-byte word of the exchange buffer, the sum beside the step's epoch, written
+// and read whole, so a block polls for the sums themselves (one trip through L2) instead of passing a
+// barrier and then reading them.  The epoch is one more than the last step's (*seq, set by block 0 when
+// it has received every block's last sums, so after all have read it); the buffer starts zeroed.
+// Block 0's ninth warp applies the stored Givens rotations to the new column while the others take the
+// third pass, and ends with the norm, the new rotation and the stopping test.
+// What bounds it: the trip through L2 of each of the three exchanges and the fixed-order sums behind
+// them.  8x8x32 (49 blocks) 19.5 -> 9.0 us a step, 16x16x64 (148 blocks, 3 elements a thread) 38.3 -> 17.7
+// us, against grid barriers, five shuffles per sum and warp, and the rotations behind the norm.
+struct __align__(16) CgWord {
+    double v;
+    unsigned long long e;
+};
+constexpr int CG_MAXB = 160;               // blocks at most (one per SM)
+constexpr int CG_T = VB + 32;              // 256 threads take the elements, the ninth warp the rotations
+constexpr size_t CG_WORDS = 3 * (size_t)CG_MAXB * GM_PS;
+static size_t cg_exchange_bytes() { return CG_WORDS * sizeof(CgWord) + sizeof(unsigned long long); }     // words, then seq
 
-// this block's sums of the first cnt entries of acc into part[blockIdx.x * GM_PS + q]
-__device__ __forceinline__ void gm_store_partials(const double (&acc)[GM_KMAX + 1], int cnt, double* part) {
-    __shared__ double sm[VB / 32][GM_PS];
+__device__ __forceinline__ void cg_store(CgWord* p, double v, unsigned long long e) {
+    asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}"
+                 ::"l"(p), "l"(__double_as_longlong(v)), "l"(e) : "memory");
+}
+__device__ __forceinline__ unsigned long long cg_load(const CgWord* p, double& v) {
+    long long b;
+    unsigned long long e;
+    asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(b), "=l"(e) : "l"(p) : "memory");
+    v = __longlong_as_double(b);
+    return e;
+}
+// barrier of the 256 element threads (the ninth warp is elsewhere)
+__device__ __forceinline__ void cg_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+// this block's sums of the first cnt entries of acc into its exchange words
+__device__ __forceinline__ void cg_publish(const double (&acc)[GM_KMAX + 1], int cnt, double (*sm)[GM_PS], CgWord* x,
+                                           unsigned long long e) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     warp_sums(acc, cnt, lane, sm[wid]);
-    __syncthreads();
+    cg_bar();
     if ((int)threadIdx.x < cnt) {
         double t = 0.0;
+#pragma unroll
         for (int w2 = 0; w2 < VB / 32; ++w2) t += sm[w2][threadIdx.x];
-        part[(int64_t)blockIdx.x * GM_PS + threadIdx.x] = t;
+        cg_store(x + (int64_t)blockIdx.x * GM_PS + threadIdx.x, t, e);
     }
 }
-
-// The grid's per-block partials of entries q < cnt, copied into this block's shared memory by all
-// its threads at once (one round of L2 loads), for a finish that then adds them in block order from
-// shared memory: the same additions in the same order as sum_partials, without one L2 round trip
-// per block.  Grids of more than CG_MAXB blocks finish with sum_partials.
-constexpr int CG_MAXB = 160;
-__device__ __forceinline__ void stage_partials(const double* part, int cnt, double (*ps)[GM_PS]) {
-    const int nb = (int)gridDim.x;
-    for (int i = threadIdx.x; i < nb * cnt; i += blockDim.x) {
-        const int b = i / cnt, q = i - b * cnt;
-        ps[b][q] = __ldcg(part + (int64_t)b * GM_PS + q);
+// every block's words of this epoch into ps (bounded polls; bit 4 of *err when a block's sums never came)
+__device__ __forceinline__ void cg_collect(const CgWord* x, int cnt, unsigned long long e, double (*ps)[GM_PS], int* err) {
+    const int items = (int)gridDim.x * cnt;
+    for (int i0 = threadIdx.x; i0 < items; i0 += 4 * VB) {
+        bool need[4];
+        int b[4], q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * VB;
+            need[u] = i < items;
+            b[u] = i / cnt;
+            q[u] = i - b[u] * cnt;
+        }
+        for (int it = 0; need[0] || need[1] || need[2] || need[3]; ++it) {
+            double v[4];
+            unsigned long long got[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) got[u] = need[u] ? cg_load(x + (int64_t)b[u] * GM_PS + q[u], v[u]) : 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (need[u] && got[u] == e) {
+                    ps[b[u]][q[u]] = v[u];
+                    need[u] = false;
+                }
+            if (it > (1 << 22)) {
+                atomicOr(err, 4);
+                break;
+            }
+        }
     }
-    __syncthreads();
 }
-__device__ __forceinline__ double finish_partials(const double* part, int q, double (*ps)[GM_PS]) {
-    if (gridDim.x > CG_MAXB) return sum_partials(part + q, (int)gridDim.x, GM_PS);
+// the sum over the blocks of entry q, in block order
+__device__ __forceinline__ double cg_sum(double (*ps)[GM_PS], int q) {
     double t = 0.0;
+#pragma unroll 8
     for (int b = 0; b < (int)gridDim.x; ++b) t += ps[b][q];
     return t;
 }
 
-// k_cgs_dots + k_cgs_orth_dots + k_cgs_orth_norm in one launch, with the same block partition and
-// the same summation order (so the same results): the two global sums between the passes are
-// grid barriers instead of kernel boundaries, and every block sums the partials itself in block
-// order.  Each pass has its own partials (a fast block never overwrites what a slow one reads).
-// hh receives h (pass 1, with w.w at hh[m]), h2 (pass 2) and ||w|| (pass 3); the last block of
-// pass 3 runs the Givens update and the stopping test.  bar: [0] arrivals, [1] generation,
-// [2] pass-3 ticket.
-__global__ void __launch_bounds__(VB) k_cgs_fused(int64_t n, GmDev* st, const double* __restrict__ V, int64_t ldv,
-                                                  double* __restrict__ hh, double* __restrict__ w,
-                                                  double* __restrict__ part, unsigned* bar, int kdim,
-                                                  cudaGraphConditionalHandle hnd, int* err) {
+// E: elements a thread has at most (0: any number, w then stays in memory between the passes).  E = 1: its
+// basis entries stay in registers over the passes; E > 1: they are fetched eight entries of every element at
+// a time (from L1 after the first pass).
+template <int E>
+__global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const double* __restrict__ V, int64_t ldv,
+                                                    double* __restrict__ w, CgWord* xw, int kdim,
+                                                    cudaGraphConditionalHandle hnd, int* err) {
     if (st->done) return;                  // a step after the solve stopped (uniform over the grid)
-    const int m = st->col + 1;
-    __shared__ double hs[GM_KMAX + 1];
+    __shared__ double sm[VB / 32][GM_PS], h1[GM_PS], h2[GM_PS], rot[2][GM_PS];
     __shared__ double ps[CG_MAXB][GM_PS];
-    __shared__ bool last;
-    const bool staged = gridDim.x <= CG_MAXB;     // grid-uniform
-    const int64_t pstride = (int64_t)gridDim.x * GM_PS;
-    double* part1 = part;
-    double* part2 = part + pstride;
-    double* part3 = part + 2 * pstride;
-    double acc[GM_KMAX + 1];
+    const int col = st->col, m = col + 1;
+    unsigned long long* seq = reinterpret_cast<unsigned long long*>(xw + CG_WORDS);
+    const unsigned long long e = *seq + 1;
+    CgWord *x1 = xw, *x2 = xw + (size_t)CG_MAXB * GM_PS, *x3 = xw + 2 * (size_t)CG_MAXB * GM_PS;
+    if (threadIdx.x >= VB) {
+        const int lane = threadIdx.x - VB;
+        if (blockIdx.x == 0 && lane < col) {
+            rot[0][lane] = st->gc[lane];
+            rot[1][lane] = st->gs[lane];
+        }
+        __syncthreads();                   // h1, h2
+        if (blockIdx.x != 0) return;
+        double carry = 0.0;
+        if (lane == 0) {
+            // entry k of the column, rotated by 0..k-1
+            double* Hc = st->H + (int64_t)col * (kdim + 1);
+            carry = h1[0] + h2[0];
+            for (int k = 0; k < col; ++k) {
+                const double c = rot[0][k], s2 = rot[1][k];
+                const double n0 = carry, n1 = h1[k + 1] + h2[k + 1];
+                Hc[k] = c * n0 + s2 * n1;
+                carry = -s2 * n0 + c * n1;
+            }
+        }
+        __syncthreads();                   // the third pass's sums
+        if (lane == 0) {
+            gm_givens_end(st, h1[m], sqrt(cg_sum(ps, 0)), carry, kdim, hnd);
+            *seq = e;
+        }
+        return;
+    }
+    const int64_t i0 = (int64_t)blockIdx.x * VB + threadIdx.x, step = (int64_t)gridDim.x * VB;
+    constexpr int EE = E > 0 ? E : 1;
+    double acc[GM_KMAX + 1], v[E == 1 ? GM_KMAX : 1], wi[EE], o[EE];
+    // entries c .. c + 7 of this thread's elements (zero beyond the basis or the vector)
+    auto fetch = [&](int c, double (&t)[EE][8]) {
+#pragma unroll
+        for (int x = 0; x < EE; ++x)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) t[x][u] = (c + u < m && i0 + x * step < n) ? V[(c + u) * ldv + i0 + x * step] : 0.0;
+    };
     // pass 1: V_q . w (q < m) and w . w
 #pragma unroll
     for (int q = 0; q <= GM_KMAX; ++q) acc[q] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double wi = w[i];
+    if constexpr (E > 0) {
 #pragma unroll
-        for (int q = 0; q <= GM_KMAX; ++q) {
-            if (q < m) acc[q] += V[q * ldv + i] * wi;
-            else if (q == m) acc[q] += wi * wi;
+        for (int x = 0; x < EE; ++x) wi[x] = i0 + x * step < n ? w[i0 + x * step] : 0.0;
+    }
+    if constexpr (E == 1) {
+#pragma unroll
+        for (int q = 0; q < GM_KMAX; ++q) v[q] = (q < m && i0 < n) ? V[q * ldv + i0] : 0.0;
+        if (i0 < n) {
+#pragma unroll
+            for (int q = 0; q <= GM_KMAX; ++q) {
+                if (q < GM_KMAX && q < m) acc[q] += v[q < GM_KMAX ? q : 0] * wi[0];
+                else if (q == m) acc[q] += wi[0] * wi[0];
+            }
+        }
+    } else if constexpr (E > 1) {
+#pragma unroll
+        for (int c = 0; c <= GM_KMAX; c += 8)
+            if (c <= m) {
+                double t[EE][8];
+                fetch(c, t);
+#pragma unroll
+                for (int x = 0; x < EE; ++x)
+                    if (i0 + x * step < n) {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const int q = c + u;
+                            if (q > GM_KMAX) continue;
+                            if (q < m) acc[q] += t[x][u] * wi[x];
+                            else if (q == m) acc[q] += wi[x] * wi[x];
+                        }
+                    }
+            }
+    } else {
+        for (int64_t i = i0; i < n; i += step) {
+            const double y = w[i];
+#pragma unroll
+            for (int q = 0; q <= GM_KMAX; ++q) {
+                if (q < m) acc[q] += V[q * ldv + i] * y;
+                else if (q == m) acc[q] += y * y;
+            }
         }
     }
-    gm_store_partials(acc, m + 1, part1);
-    grid_sync_bounded(bar, bar + 1, err);
-    if (staged) stage_partials(part1, m + 1, ps);
-    if ((int)threadIdx.x <= m) {
-        const double t = finish_partials(part1, threadIdx.x, ps);
-        hs[threadIdx.x] = t;
-        if (blockIdx.x == 0) hh[threadIdx.x] = t;
-    }
-    __syncthreads();
-    // pass 2: w -= sum_q h[q] V_q, then V_q . w
+    cg_publish(acc, m + 1, sm, x1, e);
+    cg_collect(x1, m + 1, e, ps, err);
+    cg_bar();
+    if ((int)threadIdx.x <= m) h1[threadIdx.x] = cg_sum(ps, threadIdx.x);
+    cg_bar();
+    // w -= sum_q h[q] V_q on the elements held in registers
+    auto orth = [&](const double* h) {
+#pragma unroll
+        for (int x = 0; x < EE; ++x) o[x] = 0.0;
+        if constexpr (E == 1) {
+#pragma unroll
+            for (int q = 0; q < GM_KMAX; ++q)
+                if (q < m) o[0] += h[q] * v[q];
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < m; c += 8) {
+                double t[EE][8];
+                fetch(c, t);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (c + u < m) {
+#pragma unroll
+                        for (int x = 0; x < EE; ++x) o[x] += h[c + u] * t[x][u];
+                    }
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < EE; ++x) wi[x] = wi[x] - o[x];
+    };
+    auto orth_at = [&](const double* h, int64_t i) {      // the same from memory (E = 0)
+        double s = 0.0;
+        for (int q = 0; q < m; ++q) s += h[q] * V[q * ldv + i];
+        return w[i] - s;
+    };
+    // pass 2: the first projection off, then V_q . w
 #pragma unroll
     for (int q = 0; q <= GM_KMAX; ++q) acc[q] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double o = 0.0;
-        for (int q = 0; q < m; ++q) o += hs[q] * V[q * ldv + i];
-        const double wi = w[i] - o;
-        w[i] = wi;
+    if constexpr (E == 1) {
+        if (i0 < n) {
+            orth(h1);
 #pragma unroll
-        for (int q = 0; q < GM_KMAX; ++q)
-            if (q < m) acc[q] += V[q * ldv + i] * wi;
-    }
-    gm_store_partials(acc, m, part2);
-    grid_sync_bounded(bar, bar + 1, err);
-    if (staged) stage_partials(part2, m, ps);
-    if ((int)threadIdx.x < m) {
-        const double t = finish_partials(part2, threadIdx.x, ps);
-        hs[threadIdx.x] = t;
-        if (blockIdx.x == 0) hh[(kdim + 2) + threadIdx.x] = t;
-    }
-    __syncthreads();
-    // pass 3: w -= sum_q h2[q] V_q, ||w||
-    acc[0] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double o = 0.0;
-        for (int q = 0; q < m; ++q) o += hs[q] * V[q * ldv + i];
-        const double wi = w[i] - o;
-        w[i] = wi;
-        acc[0] += wi * wi;
-    }
-    gm_store_partials(acc, 1, part3);
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(bar + 2, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (last) {                                 // block-uniform
-        __threadfence();
-        if (staged) stage_partials(part3, 1, ps);
-        if (threadIdx.x == 0) {
-            hh[2 * (kdim + 2)] = sqrt(finish_partials(part3, 0, ps));
-            bar[2] = 0u;
-            gm_givens(st, hh, kdim, hnd);
+            for (int q = 0; q < GM_KMAX; ++q)
+                if (q < m) acc[q] += v[q] * wi[0];
         }
+    } else if constexpr (E > 1) {
+        orth(h1);
+#pragma unroll
+        for (int c = 0; c < GM_KMAX; c += 8)
+            if (c < m) {
+                double t[EE][8];
+                fetch(c, t);
+#pragma unroll
+                for (int x = 0; x < EE; ++x)
+                    if (i0 + x * step < n) {
+#pragma unroll
+                        for (int u = 0; u < 8; ++u)
+                            if (c + u < GM_KMAX && c + u < m) acc[c + u < GM_KMAX ? c + u : 0] += t[x][u] * wi[x];
+                    }
+            }
+    } else {
+        for (int64_t i = i0; i < n; i += step) {
+            const double y = orth_at(h1, i);
+            w[i] = y;
+#pragma unroll
+            for (int q = 0; q < GM_KMAX; ++q)
+                if (q < m) acc[q] += V[q * ldv + i] * y;
+        }
+    }
+    cg_publish(acc, m, sm, x2, e);
+    cg_collect(x2, m, e, ps, err);
+    cg_bar();
+    if ((int)threadIdx.x < m) h2[threadIdx.x] = cg_sum(ps, threadIdx.x);
+    __syncthreads();
+    // pass 3: the second projection off, ||w||
+    acc[0] = 0.0;
+    if constexpr (E > 0) {
+        orth(h2);
+#pragma unroll
+        for (int x = 0; x < EE; ++x)
+            if (i0 + x * step < n) {
+                w[i0 + x * step] = wi[x];
+                acc[0] += wi[x] * wi[x];
+            }
+    } else {
+        for (int64_t i = i0; i < n; i += step) {
+            const double y = orth_at(h2, i);
+            w[i] = y;
+            acc[0] += y * y;
+        }
+    }
+    cg_publish(acc, 1, sm, x3, e);
+    if (blockIdx.x == 0) {                 // block-uniform
+        cg_collect(x3, 1, e, ps, err);
+        __syncthreads();
     }
 }
 
@@ -1235,38 +1412,57 @@ __global__ void k_selftest_grid(int polls, unsigned* bar, int* err) {
     grid_sync_bounded(bar, bar + 1, err, polls);
 }
 
-// least squares by back substitution (as in gmres()); ybuf = y, ncomb = its length
-__global__ void k_gm_solve(GmDev* st, double* __restrict__ ybuf, int kdim) {
-    if (threadIdx.x != 0) return;
+// least squares by back substitution (as in gmres()); ybuf = y, ncomb = its length.  One warp: H in
+// shared memory, lane q holds y[q] and takes its own update at every k (each entry's operations in the
+// order of the single loop over k, so the same bits).  One thread reading H from global memory took 11 us
+// at 10 columns and 46 us at 30; this takes 4 and 7 us.
+__global__ void __launch_bounds__(VB) k_gm_solve(GmDev* st, double* __restrict__ ybuf, int kdim) {
+    __shared__ double Hs[GM_KMAX * (GM_KMAX + 1)];
+    const int col = st->col;
     if (st->skip) {
-        st->ncomb = 0;
+        if (threadIdx.x == 0) st->ncomb = 0;
         return;
     }
-    const int col = st->col;
-    double* H = st->H;
-    auto h = [&](int c, int k) -> double& { return H[c * (kdim + 1) + k]; };
-    double* S = st->S;
-    if (h(col, col) == 0.0) S[col] = 0.0;
-    double* y = st->y;
-    for (int k = 0; k <= col; ++k) y[k] = S[k];
+    for (int q = threadIdx.x; q < (col + 1) * (kdim + 1); q += blockDim.x) Hs[q] = st->H[q];
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    auto h = [&](int c, int k) { return Hs[c * (kdim + 1) + k]; };
+    if (lane == 0 && h(col, col) == 0.0) st->S[col] = 0.0;
+    double y = lane <= col ? ((lane == col && h(col, col) == 0.0) ? 0.0 : st->S[lane]) : 0.0;
     for (int k = col; k > 0; --k) {
-        if (y[k] != 0.0) {
-            y[k] /= h(k, k);
-            double tmp = y[k];
-            for (int q = 0; q < k; ++q) y[q] -= tmp * h(k, q);
+        double yk = __shfl_sync(0xffffffffu, y, k);
+        if (yk != 0.0) {
+            yk /= h(k, k);
+            if (lane == k) y = yk;
+            if (lane < k) y -= yk * h(k, lane);
         }
     }
-    if (y[0] != 0.0) y[0] /= h(0, 0);
-    for (int k = 0; k <= col; ++k) ybuf[k] = y[k];
-    st->ncomb = col + 1;
+    if (lane == 0 && y != 0.0) y /= h(0, 0);
+    if (lane <= col) {
+        st->y[lane] = y;
+        ybuf[lane] = y;
+    }
+    if (lane == 0) st->ncomb = col + 1;
 }
 
-__global__ void k_combine_gm(int64_t n, const GmDev* __restrict__ st, const double* __restrict__ V, int64_t ldv,
-                             const double* __restrict__ y, double* __restrict__ x) {
+// x = sum_q y[q] V_q, in the order of q; eight basis entries in flight per thread
+__global__ void __launch_bounds__(VB) k_combine_gm(int64_t n, const GmDev* __restrict__ st, const double* __restrict__ V,
+                                                   int64_t ldv, const double* __restrict__ y, double* __restrict__ x) {
+    __shared__ double ys[GM_KMAX + 1];
     const int m = st->ncomb;
+    if ((int)threadIdx.x < m) ys[threadIdx.x] = y[threadIdx.x];
+    __syncthreads();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
-        for (int q = 0; q < m; ++q) acc += y[q] * V[q * ldv + i];
+        for (int q0 = 0; q0 < m; q0 += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = q0 + u < m ? V[(q0 + u) * ldv + i] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (q0 + u < m) acc += ys[q0 + u] * v[u];
+        }
         x[i] = acc;
     }
 }
@@ -1311,14 +1507,15 @@ static int gmres_body(const dv_model* m) {
     return v;
 }
 
-// DVTSA_GMRES_COOP=0 keeps the three-kernel CGS2 in the GMRES graph (read once per process)
-static bool gmres_coop_enabled() {
+// DVTSA_GMRES_COOP=0 keeps the three-kernel CGS2 in the GMRES graph, 2 the cooperative one's form that
+// leaves its elements in memory (read once per process; 1 by default)
+static int gmres_coop() {
     static int v = -1;
     if (v < 0) {
         const char* e = getenv("DVTSA_GMRES_COOP");
-        v = (e && e[0] == '0') ? 0 : 1;
+        v = (e && (e[0] == '0' || e[0] == '2')) ? e[0] - '0' : 1;
     }
-    return v == 1;
+    return v;
 }
 
 // The GMRES operator's launches inside the graph: the FP64 finite-difference matvec (three residual
@@ -1359,7 +1556,7 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
     if (e == cudaSuccess) {
         // pre: ||b||, loop state
         k_sumsq_finish<<<g, VB, 0, cs>>>(n, W.b, nullptr, W.part, W.tickets + 6, 2, W.scal + 9);
-        k_gm_init<<<1, VB, 0, cs>>>(st, W.scal, kdim, hnd, W.tickets + 8);
+        k_gm_init<<<1, VB, 0, cs>>>(st, W.scal, kdim, hnd);
         fixed[K_VECTOR] += 2;
     }
     const bool fused = precond_apply_fusable(m);
@@ -1368,8 +1565,8 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
     int nsm = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned gc = std::min<unsigned>(g, (unsigned)std::max(nsm, 1));
-    const bool coop = coop_ok && gmres_coop_enabled();
+    const unsigned gc = std::min<unsigned>(g, (unsigned)std::min(std::max(nsm, 1), CG_MAXB));
+    const bool coop = coop_ok && gmres_coop() != 0;
     bool coop_failed = false;
     // One Arnoldi step of the fused form: sweep with normalisation prologue and rms epilogue,
     // matvec, CGS2 in three kernels; every kernel returns at once when st->done is set.
@@ -1392,15 +1589,18 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
         if (coop) {                          // CGS2 as one cooperative launch (co-resident blocks)
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(gc);
-            cfg.blockDim = dim3(VB);
+            cfg.blockDim = dim3(CG_T);
             cfg.stream = c;
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeCooperative;
             at[0].val.cooperative = 1;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            if (cudaLaunchKernelEx(&cfg, k_cgs_fused, n, st, (const double*)W.V, ldv, W.hbuf, W.wout, W.part,
-                                   W.tickets + 8, kdim, hnd, m->d_err) != cudaSuccess)
+            const int64_t per = (n + (int64_t)gc * VB - 1) / ((int64_t)gc * VB);      // elements per thread
+            auto kern = k_cgs_fused<0>;
+            if (gmres_coop() == 1 && per <= 3) kern = per == 1 ? k_cgs_fused<1> : per == 2 ? k_cgs_fused<2> : k_cgs_fused<3>;
+            if (cudaLaunchKernelEx(&cfg, kern, n, st, (const double*)W.V, ldv, W.wout, (CgWord*)W.cgx, kdim, hnd,
+                                   m->d_err) != cudaSuccess)
                 coop_failed = true;
         } else {
             k_cgs_dots<<<g, VB, 0, c>>>(n, st, W.V, ldv, W.wout, W.part, W.tickets + 1, W.hbuf);
@@ -1475,7 +1675,7 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
     if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(cs, &cnode, 1, cudaStreamSetCaptureDependencies);
     if (e == cudaSuccess) {
         // post: y, x = V y, true residual r = b - AP x
-        k_gm_solve<<<1, 32, 0, cs>>>(st, W.ybuf, kdim);
+        k_gm_solve<<<1, VB, 0, cs>>>(st, W.ybuf, kdim);
         k_combine_gm<<<g, VB, 0, cs>>>(n, st, W.V, ldv, W.ybuf, W.x);
         fixed[K_VECTOR] += 2;
         int rc;
@@ -2274,6 +2474,7 @@ static int solve_stage(dv_integrator* g, const dv_newton_opts& no, double ts, co
 static void clear_device_error(dv_model* m) {
     cudaMemset(m->d_err, 0, sizeof(int));
     if (m->W && m->W->tickets) cudaMemset(m->W->tickets, 0, 16 * sizeof(unsigned));
+    if (m->W && m->W->cgx) cudaMemset(m->W->cgx, 0, cg_exchange_bytes());
     cudaDeviceSynchronize();
 }
 

@@ -465,3 +465,51 @@ def test_gmres_graph_forms_give_identical_results():
         assert r.returncode == 0, r.stderr[-2000:]
         out[name] = json.loads(r.stdout.strip().splitlines()[-1])
     assert out["default"] == out["three_kernel_cgs"] == out["no_prefix"] == out["one_step_body"] == out["pdl"] == out["coop_matvec"], out
+
+
+_CGS_RUN = r"""
+import sys
+import numpy as np
+sys.path.insert(0, {tests!r})
+from test_gpu_solver import CGS_GRIDS, _cgs_stage
+np.savez(sys.argv[1], **{{"%d_%d_%d" % g: np.concatenate([[it], z]) for g in CGS_GRIDS for it, z in [_cgs_stage(*g)]}})
+"""
+# elements per thread of the cooperative Gram-Schmidt kernel (148 blocks of 256): 1 (one block, several
+# blocks with a remainder), 2, 3 and 4 (the form that keeps them in memory)
+CGS_GRIDS = [(1, 1, 9), (5, 6, 31), (12, 12, 48), (16, 16, 64), (16, 16, 80)]
+
+
+def _cgs_stage(Nr, Nth, Nz):
+    """One Newton iteration of an implicit stage: (GMRES steps, the iterate in error scales from the start)."""
+    import torch
+    from dac_vtsa_b200.jacobian import FDJacobian
+    m, y = _pc_model(Nz, Nr, Nth)
+    yd = torch.from_numpy(np.ascontiguousarray(y)).to(m.device)
+    m.precond_factor(FDJacobian(m).block(0.0, yd), 0.3)
+    z, _, _, _, stats = m.newton_stage(0.3, yd, yd, 0.3, max_iter=1, cons_tol=0.0)
+    return stats["gmres_iters"], (z.cpu().numpy() - y) / (m.atol + m.cfg.solver.rtol * np.abs(y))
+
+
+def test_cooperative_gram_schmidt_at_every_element_count(tmp_path):
+    """The one-launch Gram-Schmidt gives the same bits whether a thread's elements stay in registers (one to
+    three of them) or in memory (DVTSA_GMRES_COOP=2), and, where the block partition is the same (one element
+    per thread), as the three-kernel form (DVTSA_GMRES_COOP=0)."""
+    import os
+    import subprocess
+    import sys
+    tests = os.path.dirname(os.path.abspath(__file__))
+    ref = {}
+    for form in ("0", "2"):
+        out = str(tmp_path / f"form{form}.npz")
+        r = subprocess.run([sys.executable, "-c", _CGS_RUN.format(tests=tests), out],
+                           env=dict(os.environ, DVTSA_GMRES_COOP=form), capture_output=True, text=True, timeout=600,
+                           cwd=os.path.dirname(tests))
+        assert r.returncode == 0, r.stderr[-2000:]
+        ref[form] = np.load(out)
+    for g in CGS_GRIDS:
+        it, z = _cgs_stage(*g)
+        assert it >= 2
+        a = np.concatenate([[it], z])
+        assert np.array_equal(a, ref["2"]["%d_%d_%d" % g]), g
+        if len(z) <= 148 * 256:
+            assert np.array_equal(a, ref["0"]["%d_%d_%d" % g]), g
