@@ -257,6 +257,6 @@ int precond_apply_capture(dv_model* m, const double* b, const double* sc, double
 // With `bar` (two zeroed barrier words) the three phases run as one cooperative launch.
 int matvec_capture(dv_model* m, const double* dargs, const double* z, const double* u, const double* sc,
                    const double* f0, const double* scal, double* out, cudaStream_t s, unsigned* bar = nullptr);
-// Kernels one matvec_capture with `bar` launched (1 cooperative, or the 3 of the split residual).
-int matvec_capture_kernels();
+// Kernels one matvec_capture with `bar` launched (1 of tiles or cooperative, or the 3 of the split residual).
+int matvec_capture_kernels(const dv_model* m);
 }  // namespace dv

@@ -919,15 +919,441 @@ __global__ void __launch_bounds__(DV_NB * 32, 3) k_jac_rows(dv_step_params p, Au
         (TJ)(outer_wall ? jac_quot(fw - f0[(int64_t)DV_NV * nc + (int64_t)j * Nz + k], h) : 0.0);
 }
 
+// ---------------------------------------------------------------- residual of a tile in one launch
+// The residual of a tile of TL_R x TL_T x TL_Z cells in one block, everything in between in shared memory.
+// The block evaluates the transport properties of its cells and of the neighbours their faces need; the
+// halo's properties (and the faces between tiles) are evaluated by each of the tiles that need them -- 56
+// property evaluations for 16 cells -- so no block waits for another.  The same expressions on the same
+// operands as the split residual, so the same bits.
+// The work is cut into many small items per phase, so that the warps of a phase run the same short code:
+// what bounds a tile is the chain of its phases, and in them the latency of FP64 operations (23 cycles) and
+// of fetching code that runs once (the first form, a role per warp and whole faces per thread, spent 28 000
+// cycles, half of its instruction fetches missing the SM's cache).  Phases, a barrier between each:
+//   load     the six unknowns of the tile's cells, the r / theta / z neighbours and the next z neighbours
+//   state    temperature, pressure, concentration of a cell
+//   terms    every power of the properties (cell, term); mole fractions and viscosities (cell, gas); the two
+//            Toth terms and the water loading of the own cells
+//   mix      Wilke's quotients (cell, gas); diffusivities; slopes (cell, variable); loadings and LDF rates
+//   flux     velocities, species fluxes and the enthalpy they carry (z, r, theta faces, column ends);
+//            stagnant conductivity (cell); the wall's Nusselt number
+//   heat     conduction through a face; wall resistance
+//   rows     the balances (row, cell)
+// 8x8x32 (128 tiles): 12.5 us, against 21.6 us for properties, faces and assembly in three launches.
+constexpr int TL_R = 2, TL_T = 2, TL_Z = 4, TL_COL = TL_R * TL_T, TL_OWN = TL_COL * TL_Z, TL_PROP = 56, TL_ALL = 64;
+constexpr int TL_WARPS = 14, TL_THREADS = 32 * TL_WARPS;
+static_assert(TL_PROP == TL_OWN + 2 * TL_T * TL_Z + 2 * TL_R * TL_Z + 2 * TL_COL && TL_ALL == TL_PROP + 2 * TL_COL,
+              "tile, r / theta / z neighbours, next z neighbours");
+constexpr int TL_ZF = TL_COL * (TL_Z + 1), TL_RF = (TL_R + 1) * TL_T * TL_Z, TL_TF = (TL_T + 1) * TL_R * TL_Z;
+constexpr int TL_F = TL_ZF + TL_RF + TL_TF;            // faces: z (column, face), r (face, 8), theta (face, 8)
+
+// Local cells: the own ones id = (ii TL_T + jj) TL_Z + kk, then the neighbours: 16, 24 below / above in r
+// (jj TL_Z + kk), 32, 40 in theta (ii TL_Z + kk), 48, 52 in z and 56, 60 two away in z (ii TL_T + jj).
+// Along z of own column cl = ii TL_T + jj, kk = -2 .. TL_Z + 1:
+static __device__ __forceinline__ int tl_zid(int cl, int kk) {
+    const int own = cl * TL_Z + kk, near = 48 + (kk > 0 ? 4 : 0) + cl, far = 56 + (kk > 0 ? 4 : 0) + cl;
+    return (unsigned)kk < TL_Z ? own : (kk == -1 || kk == TL_Z) ? near : far;
+}
+static __device__ __forceinline__ void tl_cell(int id, int& ii, int& jj, int& kk) {
+    const int g = id >> 3, e = id & 7;
+    if (id < 16) { ii = id >> 3; jj = (id >> 2) & 1; kk = id & 3; }
+    else if (id < 32) { ii = g == 2 ? -1 : TL_R; jj = e >> 2; kk = e & 3; }
+    else if (id < 48) { jj = g == 4 ? -1 : TL_T; ii = e >> 2; kk = e & 3; }
+    else { ii = (e >> 1) & 1; jj = e & 1; kk = id < 52 ? -1 : id < 56 ? TL_Z : id < 60 ? -2 : TL_Z + 1; }
+}
+
+struct TileShared {
+    double c[DV_NV][TL_ALL];                               // the unknowns
+    double T[TL_ALL], Tp[TL_ALL], P[TL_ALL], Cpos[TL_ALL];
+    double y[DV_NG][TL_PROP], mu[DV_NG][TL_PROP], sq[DV_NG][TL_PROP];
+    double pw[7][TL_PROP];                                 // powers: gas 0, 1, 2 first terms, gas 2's second, T^1.75, the others
+    double mt[DV_NG][TL_PROP], kt[DV_NG][TL_PROP];         // Wilke's quotients
+    double Dm[TL_PROP], lam0[TL_PROP];
+    double sl[4][TL_COL][TL_Z + 2];                        // slopes of cells -1 .. TL_Z of a column
+    double qw[TL_OWN], qt[2][TL_OWN], rate[DV_NA][TL_OWN], qs[DV_NA][TL_OWN], dyn[TL_OWN], Rb[TL_OWN];
+    double F[DV_NG + 1][TL_F], lx[TL_F], dist[TL_F], area[TL_F];      // species fluxes, enthalpy; conduction's inputs
+    int ida[TL_F], idb[TL_F];                              // cells of the face (-1: no conduction, H is final)
+};
+
+template <int MODE, bool REC, class L>
+static __device__ __forceinline__ void tile_residual(const dv_step_params& p, const Aux& aux, const Rec& rec, double t,
+                                                     const L& ld, const double* __restrict__ y,
+                                                     const double* __restrict__ u, const double* __restrict__ sc,
+                                                     const double* __restrict__ f0, double sig, double gh,
+                                                     double* __restrict__ out, TileShared& X) {
+    const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
+    const int64_t nc = (int64_t)Nr * Nth * Nz;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int w = tid >> 5;
+    const int nzt = (Nz + TL_Z - 1) / TL_Z, ntt = (Nth + TL_T - 1) / TL_T;
+    const int k0 = (int)(blockIdx.x % nzt) * TL_Z;
+    const int rt = blockIdx.x / nzt;
+    const int j0 = (rt % ntt) * TL_T, i0 = (rt / ntt) * TL_R;
+    // theta wraps (a slot beyond the last sector holds the first one)
+    auto sector = [&](int jj) {
+        int j = j0 + jj;
+        if (j < 0) j += Nth;
+        while (j >= Nth) j -= Nth;
+        return j;
+    };
+    auto own = [&](int ii, int jj, int kk) { return i0 + ii < Nr && j0 + jj < Nth && (unsigned)kk < TL_Z && k0 + kk < Nz; };
+    auto get = [&](int id, Cell& s) {
+#pragma unroll
+        for (int q = 0; q < DV_NG; ++q) s.c[q] = X.c[q][id];
+        s.q[0] = X.c[3][id];
+        s.q[1] = X.c[4][id];
+        s.e = X.c[5][id];
+    };
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    const bool muscl = (Nz >= 3 && p.limiter != DV_LIM_UPWIND);
+    // ---- load
+    for (int q = tid; q < DV_NV * TL_ALL; q += TL_THREADS) {
+        const int v = q / TL_ALL, id = q - v * TL_ALL;
+        int ii, jj, kk;
+        tl_cell(id, ii, jj, kk);
+        // (a neighbour outside the grid is never read; the nearest cell inside stands in for it)
+        const int i = min(max(i0 + ii, 0), Nr - 1), k = min(max(k0 + kk, 0), Nz - 1);
+        X.c[v][id] = ld(v * nc + ((int64_t)i * Nth + sector(jj)) * Nz + k);
+    }
+    __syncthreads();
+    // ---- state (as props_state)
+    if (tid < TL_ALL) {
+        Cell s;
+        get(tid, s);
+        const double Ctot = s.c[0] + s.c[1] + s.c[2];
+        const double T = cell_T(p, s);
+        X.T[tid] = T;
+        X.P[tid] = Ctot * DV_R * T;
+        X.Tp[tid] = npclip(T, 150.0, 1500.0);
+        X.Cpos[tid] = npmax(Ctot, 1e-9);
+    }
+    __syncthreads();
+    // ---- terms
+    if (w < 9) {                               // powers: slots of X.pw
+        for (int it = tid; it < 7 * TL_PROP; it += 9 * 32) {
+            const int slot = it / TL_PROP, id = it - slot * TL_PROP;
+            const int gas = slot < 3 ? slot : slot == 3 ? 2 : slot == 4 ? -1 : slot - 5, e = slot < 3 ? 0 : 1;
+            if (gas >= 0 && e == 1 && p.k_nt[gas] == 1) continue;
+            const double Tp = X.Tp[id];
+            X.pw[slot][id] = pow(gas >= 0 ? Tp / 300.0 : Tp, gas >= 0 ? p.k_n[gas][e] : 1.75);
+        }
+    } else if (w == 9) {                       // the two Toth terms of the own cells, side by side
+        const int id = lane & 15;
+        const bool wet = lane >= 16;
+        const double Tp = X.Tp[id], pp = npmax(X.c[0][id] * DV_R * Tp, 0.0);
+        double v = nan;
+        if (wet ? p.coads == DV_COADS_WADST : !co2_needs_qw(p)) {
+            const double qi = wet ? p.wadst_q_inf0 : p.co2_q_inf0, chi = wet ? p.wadst_chi : p.co2_chi;
+            const double b0 = wet ? p.wadst_b0 : p.co2_b0, dH = wet ? p.wadst_dH : p.co2_dH0;
+            const double tau = wet ? p.wadst_tau0 : p.co2_tau0, al = wet ? p.wadst_alpha : p.co2_alpha;
+            v = toth(pp, Tp, qi, chi, b0, dH, tau, al, p.co2_T0);
+        }
+        X.qt[wet ? 1 : 0][id] = v;
+    } else if (w == 10) {                      // water: saturation and GAB
+        if (lane < TL_OWN) {
+            const double Tp = X.Tp[lane], pw = X.c[1][lane] * DV_R * Tp;
+            X.qw[lane] = q_h2o(p, pw, Tp, psat_h2o(Tp));
+        }
+    } else {                                   // mole fractions, viscosities and their roots
+        for (int it = tid - 11 * 32; it < DV_NG * TL_PROP; it += 3 * 32) {
+            const int q = it / TL_PROP, id = it - q * TL_PROP;
+            const double mu = gas_mu(p, q, X.Tp[id]);
+            X.y[q][id] = X.c[q][id] / X.Cpos[id];
+            X.sq[q][id] = sqrt(mu);
+            X.mu[q][id] = mu;
+        }
+    }
+    __syncthreads();
+    // ---- mix
+    if (w < 6) {                               // Wilke & Mason-Saxena, gas q of a cell (as wilke_mix)
+        if (tid < DV_NG * TL_PROP) {
+            const int q = tid / TL_PROP, id = tid - q * TL_PROP;
+            const double sqi = X.sq[q][id];
+            const double pk = p.k_nt[q] == 1 ? p.k_0[q][0] * X.pw[q][id]
+                                             : p.k_w[q][0] * p.k_0[q][0] * X.pw[q][id] +
+                                                   p.k_w[q][1] * p.k_0[q][1] * X.pw[q == 2 ? 3 : q + 5][id];
+            const double yq = npclip(X.y[q][id], 0.0, 1.0), mu = X.mu[q][id];
+            double den = 0.0;
+#pragma unroll 1
+            for (int j = 0; j < DV_NG; ++j) {
+                const double yj = npclip(X.y[j][id], 0.0, 1.0);
+                const double t1 = 1.0 + sqi / X.sq[j][id] * p.mass_q[q][j];
+                const double m = t1 * t1 / p.wilke_den[q][j];
+                den = den + (j == q ? yj : yj * m);
+            }
+            den = npmax(den, 1e-30);
+            X.mt[q][id] = yq * mu / den;
+            X.kt[q][id] = yq * pk / den;
+        }
+    } else if (w < 8) {
+        const int id = tid - 6 * 32;
+        if (id < TL_PROP) {
+            double ycl[DV_NG];
+#pragma unroll
+            for (int q = 0; q < DV_NG; ++q) ycl[q] = npclip(X.y[q][id], 0.0, 1.0);
+            const double tp = 1.43e-7 * X.pw[4][id], Pc = npmax(X.P[id], 1.0);
+            X.Dm[id] = blanc_Dm(ycl, fuller_of(p, 0, tp, Pc), fuller_of(p, 1, tp, Pc));
+        }
+    } else if (w < 11) {                       // slopes of the cells next to the tile's z faces (as sp_slope)
+        const int it = tid - 8 * 32, v = it / (TL_COL * (TL_Z + 2)), r = it - v * (TL_COL * (TL_Z + 2));
+        const int cl = r / (TL_Z + 2), kk = r - cl * (TL_Z + 2) - 1, k = k0 + kk;
+        const double* a = v < DV_NG ? X.c[v] : X.T;
+        double s = 0.0;
+        if (muscl && k >= 1 && k <= Nz - 2) {
+            const double x = a[tl_zid(cl, kk)], dm = x - a[tl_zid(cl, kk - 1)], dp = a[tl_zid(cl, kk + 1)] - x;
+            s = limited_slope(p.limiter, dm, dp);
+        }
+        X.sl[v][cl][kk + 1] = s;
+    } else if (w == 11 && lane < TL_OWN) {     // loadings and LDF rates
+        Cell s;
+        get(lane, s);
+        const double Tp = X.Tp[lane], pp = npmax(s.c[0] * DV_R * Tp, 0.0), qw_eq = X.qw[lane];
+        const double dry = X.qt[0][lane], wet = X.qt[1][lane];
+        double rate[DV_NA], qstar[DV_NA];
+        qstar[0] = q_co2_raw(p, pp, Tp, p.basis_state ? s.q[1] : qw_eq, dry, wet) * (pp / (pp + p.p_reg));
+        qstar[1] = qw_eq;
+        ldf_rates(p, s, Tp, qstar, rate);
+#pragma unroll
+        for (int q = 0; q < DV_NA; ++q) {
+            X.rate[q][lane] = rate[q];
+            X.qs[q][lane] = qstar[q];
+        }
+    }
+    __syncthreads();
+    static_assert(4 * TL_COL * (TL_Z + 2) == 3 * 32, "slopes fill three warps");
+    // ---- flux
+    auto props = [&](int id, Cell& s, Props& o) {          // all but lam0
+        double ycl[DV_NG];
+        o.mu = o.kg = 0.0;
+#pragma unroll
+        for (int q = 0; q < DV_NG; ++q) {
+            s.c[q] = X.c[q][id];
+            o.y[q] = X.y[q][id];
+            ycl[q] = npclip(o.y[q], 0.0, 1.0);
+            o.mu = o.mu + X.mt[q][id];
+            o.kg = o.kg + X.kt[q][id];
+        }
+        s.q[0] = s.q[1] = s.e = 0.0;
+        o.T = X.T[id];
+        o.P = X.P[id];
+        o.Tp = 0.0;
+        o.Cpos = X.Cpos[id];
+        o.rho = o.Cpos * wsum3(p.M, ycl);
+        o.cpm = wsum3(p.cpg, ycl);
+        o.Dm = X.Dm[id];
+        o.lam0 = 0.0;
+    };
+    auto put = [&](int f, const FluxPart& F, int a, int b, double dist, double area) {
+#pragma unroll
+        for (int q = 0; q < DV_NG; ++q) X.F[q][f] = F.F[q];
+        X.F[DV_NG][f] = F.He;
+        X.lx[f] = F.lx;
+        X.ida[f] = a;
+        X.idb[f] = b;
+        X.dist[f] = dist;
+        X.area[f] = area;
+    };
+    if (w == 0) {                              // z faces between k0 + kf - 1 and k0 + kf
+        const int cl = lane / (TL_Z + 1), kf = lane - cl * (TL_Z + 1), ii = cl >> 1, jj = cl & 1, K = k0 + kf;
+        if (lane < TL_ZF && i0 + ii < Nr && j0 + jj < Nth && K > 0 && K < Nz) {
+            const int a = tl_zid(cl, kf - 1), b = tl_zid(cl, kf);
+            Cell ca, cb;
+            Props Lp, Rp;
+            props(a, ca, Lp);
+            props(b, cb, Rp);
+            double sL[4], sR[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                sL[v] = X.sl[v][cl][kf];
+                sR[v] = X.sl[v][cl][kf + 1];
+            }
+            const int64_t col = (int64_t)(i0 + ii) * Nth + j0 + jj;
+            const double nn = aux.n_nom[col];
+            FluxPart F;
+            double uz;
+            zface_part(p, i0 + ii, Lp, Rp, ca, cb, sL, sR, muscl, nn, F, &uz);
+            put(lane, F, a, b, p.dz, p.Az[i0 + ii]);
+            if (REC && kf > 0) rec.uz[col * (Nz - 1) + K - 1] = uz;      // (the tile of the lower cell)
+        }
+    } else if (w < 3) {                        // r faces between rings ii - 1, ii; theta faces between jj - 1, jj (periodic)
+        const bool th = w == 2;
+        const int n = lane >> 3, e = lane & 7, kk = e & 3;           // n: the face along r (theta)
+        const int ii = th ? e >> 2 : n, jj = th ? n : e >> 2, i = i0 + ii, j = j0 + jj;
+        const bool ok = lane < 24 && k0 + kk < Nz && i < Nr && (th ? Nth > 1 && j <= Nth : j < Nth && i > 0);
+        if (ok) {
+            const int a = th ? (n == 0 ? 32 + e : ii * 8 + (n - 1) * 4 + kk) : (n == 0 ? 16 + e : (n - 1) * 8 + e);
+            const int b = th ? (n == TL_T ? 40 + e : ii * 8 + n * 4 + kk) : (n == TL_R ? 24 + e : n * 8 + e);
+            Cell ca, cb;
+            Props A, B;
+            props(a, ca, A);
+            props(b, cb, B);
+            const double dist = th ? p.arc[i] : p.drc[i - 1], area = th ? p.Ath[i] : p.Ar[i - 1];
+            FluxPart F;
+            double ut;
+            tface_part(p, A, B, ca, cb, dist, area, F, &ut);
+            put(TL_ZF + (th ? TL_RF : 0) + lane, F, a, b, dist, area);
+            if (REC && n > 0) {       // (the tile of the lower cell)
+                if (th) rec.uth[((int64_t)i * Nth + j - 1) * Nz + k0 + kk] = ut;
+                else rec.ur[((int64_t)(i - 1) * Nth + j) * Nz + k0 + kk] = ut;
+            }
+        }
+    } else if (w == 3) {                       // the column ends
+        const int e = lane >> 2, cl = lane & 3, ii = cl >> 1, jj = cl & 1, kk = e == 0 ? 0 : Nz - 1 - k0;
+        if (lane < 2 * TL_COL && own(ii, jj, kk) && (e == 1 || k0 == 0)) {
+            const int64_t col = (int64_t)(i0 + ii) * Nth + j0 + jj;
+            Cell s;
+            Props o;
+            props(cl * TL_Z + kk, s, o);
+            double F_in[DV_NG], H_in;
+            const double ff = aux.feed_flux[col];
+            end_face(p, p.ends[e], t, i0 + ii, s, o, ff, F_in, H_in,
+                     REC ? rec.bnd + (int64_t)e * BR_N * Nr * Nth + col : nullptr, (int64_t)Nr * Nth);
+            FluxPart F;                        // stored as the +z flux through the face
+#pragma unroll
+            for (int q = 0; q < DV_NG; ++q) F.F[q] = (e == 0) ? F_in[q] : -F_in[q];
+            F.He = (e == 0) ? H_in : -H_in;
+            F.lx = 0.0;
+            put(cl * (TL_Z + 1) + (e == 0 ? 0 : kk + 1), F, -1, -1, 1.0, 0.0);
+        }
+    } else if (w < 6) {                        // stagnant conductivity
+        const int id = tid - 4 * 32;
+        if (id < TL_PROP) {
+            double kg = 0.0;
+#pragma unroll
+            for (int q = 0; q < DV_NG; ++q) kg = kg + X.kt[q][id];
+            X.lam0[id] = stagnant(p, kg);
+        }
+    } else if (w == 6) {                       // wall: the flow part of the Nusselt number
+        if (lane < TL_OWN && i0 + (lane >> 3) == Nr - 1) {
+            Cell s;
+            Props o;
+            props(lane, s, o);
+            X.dyn[lane] = wall_dyn(p, o);
+        }
+    }
+    __syncthreads();
+    // ---- heat
+    if (w < 3) {
+        // (the faces put above: the same conditions)
+        bool ok = false;
+        int f = 0;
+        if (w == 0) {
+            const int cl = lane / (TL_Z + 1), K = k0 + lane - cl * (TL_Z + 1);
+            ok = lane < TL_ZF && i0 + (cl >> 1) < Nr && j0 + (cl & 1) < Nth && K > 0 && K < Nz;
+            f = lane;
+        } else {
+            const bool th = w == 2;
+            const int n = lane >> 3, e = lane & 7, i = i0 + (th ? e >> 2 : n), j = j0 + (th ? n : e >> 2);
+            ok = lane < 24 && k0 + (e & 3) < Nz && i < Nr && (th ? Nth > 1 && j <= Nth : j < Nth && i > 0);
+            f = TL_ZF + (th ? TL_RF : 0) + lane;
+        }
+        if (ok) {
+            const int a = X.ida[f], b = X.idb[f];
+            const double He = X.F[DV_NG][f];
+            X.F[DV_NG][f] = face_H(He, X.lx[f], X.lam0[a], X.lam0[b], X.T[a], X.T[b], X.dist[f], X.area[f]);
+        }
+    } else if (w == 3) {
+        if (lane < TL_OWN && i0 + (lane >> 3) == Nr - 1) {
+            Cell s;
+            Props o;
+            props(lane, s, o);
+            o.lam0 = X.lam0[lane];
+            const double dyn = X.dyn[lane];
+            X.Rb[lane] = wall_R_rest(p, o, dyn);
+        }
+    }
+    __syncthreads();
+    // ---- rows: (row, own cell)
+    if (tid < DV_NB * TL_OWN) {
+        const int v = tid >> 4, id = tid & 15, ii = id >> 3, jj = (id >> 2) & 1, kk = id & 3;
+        const int i = i0 + ii, j = j0 + jj, k = k0 + kk;
+        if (own(ii, jj, kk) && (v < DV_NV || (i == Nr - 1 && p.wall_on))) {
+            const int64_t c0 = ((int64_t)i * Nth + j) * Nz + k;
+            const int64_t ix = v < DV_NV ? v * nc + c0 : (int64_t)DV_NV * nc + (int64_t)j * Nz + k;
+            const int cl = ii * TL_T + jj, zf = cl * (TL_Z + 1) + kk, rf = TL_ZF + ii * 8 + jj * TL_Z + kk;
+            const int tf = TL_ZF + TL_RF + jj * 8 + ii * TL_Z + kk;
+            const double T = X.T[id], Rb = X.Rb[id];
+            double r = 0.0;
+            const double yo = MODE == M_STAGE ? y[ix] : 0.0, uo = MODE != M_RHS ? u[ix] : 0.0;
+            const double so = MODE == M_MATVEC ? sc[ix] : 0.0, fo = MODE == M_MATVEC ? f0[ix] : 0.0;
+            double f;
+            if (v == 3 || v == 4) {
+                f = X.rate[v - 3][id];
+            } else if (v == DV_NV) {
+                wall_terms(p, aux, ld, jacket_T(p, t), j, k, T, Rb, &f);
+            } else {
+                const double* F = X.F[v < DV_NG ? v : DV_NG];
+                const double div = face_div(p, i, F[zf], F[zf + 1], F[rf], F[rf + 8], F[tf], F[tf + 8]);
+                f = v < DV_NG ? row_mass(p, i, div, (v < DV_NA) ? X.rate[v][id] : 0.0)
+                              : row_energy(p, aux, ld, t, i, j, k, T, Rb, div, nullptr, REC ? &rec : nullptr);
+            }
+            if (MODE == M_RHS) r = f;
+            else if (MODE == M_STAGE) r = yo - gh * f - uo;
+            else r = (uo * so - (gh * (f - fo) / sig)) / so;
+            out[ix] = r;
+            if (REC && v == 3) {
+                rec.T[c0] = T;
+                rec.P[c0] = X.P[id];
+#pragma unroll
+                for (int q = 0; q < DV_NG; ++q) rec.y[q * nc + c0] = X.y[q][id];
+                rec.qstar[c0] = X.qs[0][id];
+                rec.qstar[nc + c0] = X.qs[1][id];
+            }
+        }
+    }
+}
+
+template <int MODE, bool REC>
+__global__ void __launch_bounds__(TL_THREADS, 1) k_tile(dv_step_params p, Aux aux, Rec rec, double t,
+                                                     const double* __restrict__ y, const double* __restrict__ u,
+                                                     const double* __restrict__ sc, const double* __restrict__ f0,
+                                                     const double* __restrict__ scal, double gh,
+                                                     double* __restrict__ out, const double* __restrict__ dargs) {
+    __shared__ TileShared X;
+    pdl_wait();                   // (launched programmatically inside the GMRES graph)
+    if (dargs) {                  // launched from a CUDA graph: time and step factor live on the device
+        t = dargs[0];
+        gh = dargs[1];
+    }
+    if (MODE == M_MATVEC) {
+        if (scal[0] == 0.0) {     // matvec of a zero direction is zero
+            const int64_t n = (int64_t)DV_NV * p.Nr * p.Nth * p.Nz + (p.wall_on ? (int64_t)p.Nth * p.Nz : 0);
+            for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+                out[i] = 0.0;
+            return;
+        }
+        const double sig = matvec_sig(scal);
+        tile_residual<MODE, REC>(p, aux, rec, t, LoadDir{y, u, sc, sig}, y, u, sc, f0, sig, gh, out, X);
+    } else {
+        tile_residual<MODE, REC>(p, aux, rec, t, LoadPlain{y}, y, u, sc, f0, 0.0, gh, out, X);
+    }
+}
+
+static int64_t tile_blocks(const dv_step_params& p) {
+    return (int64_t)((p.Nr + TL_R - 1) / TL_R) * ((p.Nth + TL_T - 1) / TL_T) * ((p.Nz + TL_Z - 1) / TL_Z);
+}
+
 static Aux aux_of(const dv_model* m) { return Aux{m->aux.feed_flux, m->aux.n_nom, m->aux.cov}; }
 
 static unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
-// The split residual: properties, faces, assembly (three launches counted under `kind`).
+// Tiles up to two waves of blocks (one block per SM): up to there a tile launch is the shorter path --
+// residual of 8x8x12 (48 tiles) 21.5 -> 10.2 us, 8x8x32 (128) 21.6 -> 12.5, 12x8x32 (192) 22.9 -> 18.6, 9x9x33
+// (225) 22.7 -> 19.9 -- and beyond it the halo work repeats: 12x12x48 (432) 25.8 against 30.0, 16x16x64
+// (1024) 25.9 against 60.7.
+static bool use_tiles(const dv_step_params& p) { return tile_blocks(p) <= 296; }
+
+// The residual: tiles, or properties, faces and assembly (one or three launches counted under `kind`).
 template <int MODE, bool REC>
 static int split_residual(dv_model* m, const Rec& rec, double t, const double* y, const double* u, const double* sc,
                           const double* f0, const double* scal, double gh, double* out, cudaStream_t s, int kind) {
     const dv_step_params& p = m->p;
+    if (use_tiles(p) && out != y && out != u && out != sc) {      // (a tile reads its neighbours' inputs)
+        DV_LAUNCH(kind, s, k_tile<MODE, REC><<<(unsigned)tile_blocks(p), TL_THREADS, 0, s>>>(p, aux_of(m), rec, t, y, u, sc, f0,
+                                                                                            scal, gh, out, nullptr));
+        m->nfev += 1;
+        DV_CUDA(cudaGetLastError());
+        return DV_OK;
+    }
     const Split S = split_of(p, m->d_split);
     const int64_t ncol = (int64_t)p.Nr * p.Nth;
     const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol;
@@ -1004,7 +1430,9 @@ static bool matvec_coop_enabled() {
     return v == 1;
 }
 
-int matvec_capture_kernels() { return (g_matvec_coop_cap > 0 && matvec_coop_enabled()) ? 1 : 3; }
+int matvec_capture_kernels(const dv_model* m) {
+    return ((g_matvec_coop_cap > 0 && matvec_coop_enabled()) || use_tiles(m->p)) ? 1 : 3;
+}
 
 int matvec_capture(dv_model* m, const double* dargs, const double* z, const double* u, const double* sc,
                    const double* f0, const double* scal, double* out, cudaStream_t s, unsigned* bar) {
@@ -1039,6 +1467,16 @@ int matvec_capture(dv_model* m, const double* dargs, const double* z, const doub
             return DV_OK;
         cudaGetLastError();                   // a driver that refuses the cooperative node: three kernels
         coop_cap = 0;
+    }
+    if (use_tiles(p)) {
+        if (pdl_enabled())
+            DV_CUDA(launch_pdl(k_tile<M_MATVEC, false>, (unsigned)tile_blocks(p), TL_THREADS, s, p, aux_of(m), rec, 0.0, z, u,
+                               sc, f0, scal, 0.0, out, dargs));
+        else
+            k_tile<M_MATVEC, false><<<(unsigned)tile_blocks(p), TL_THREADS, 0, s>>>(p, aux_of(m), rec, 0.0, z, u, sc, f0, scal,
+                                                                                 0.0, out, dargs);
+        DV_CUDA(cudaGetLastError());
+        return DV_OK;
     }
     if (pdl_enabled()) {       // each kernel may start while its predecessor drains (pdl_wait in the kernel)
         DV_CUDA(launch_pdl(k_cprops<M_MATVEC>, nblk(m->nc, 32), CP_WARPS * 32, s, p, S, z, u, sc, scal));

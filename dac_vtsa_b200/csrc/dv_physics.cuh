@@ -69,9 +69,13 @@ static __device__ __forceinline__ double cell_T(const dv_step_params& p, const C
     return (s.e - Hq + A * p.T_ref) / (A - B);
 }
 
-static __device__ __forceinline__ double fuller(const dv_step_params& p, int pair, double T, double P) {
+// tp = 1.43e-7 T^1.75
+static __device__ __forceinline__ double fuller_of(const dv_step_params& p, int pair, double tp, double P) {
     P = npmax(P, 1.0);
-    return 1.43e-7 * pow(T, 1.75) / ((P / 1e5) * p.fuller_sqrtM[pair] * p.fuller_s[pair] * p.fuller_s[pair]);
+    return tp / ((P / 1e5) * p.fuller_sqrtM[pair] * p.fuller_s[pair] * p.fuller_s[pair]);
+}
+static __device__ __forceinline__ double fuller(const dv_step_params& p, int pair, double T, double P) {
+    return fuller_of(p, pair, 1.43e-7 * pow(T, 1.75), P);
 }
 
 static __device__ __forceinline__ double stagnant(const dv_step_params& p, double lam_g) {   // heat_transfer.py:23-56
@@ -293,10 +297,20 @@ static __device__ __forceinline__ double enth(const dv_step_params& p, const dou
 
 struct Flux { double F[DV_NG]; double H; };
 
+// A face's flux before its heat conduction: species fluxes, the enthalpy they carry and the dispersion part
+// of the conductivity.  face_H adds the conduction between cells A and B (dist and area of the face).
+struct FluxPart { double F[DV_NG], He, lx; };
+static __device__ __forceinline__ double face_H(double He, double lx, double lamA, double lamB, double TA, double TB,
+                                                double dist, double area) {
+    const double lam = 0.5 * (lamB + lamA) + lx;
+    return He - (lam * (TB - TA) / dist) * area;
+}
+
 // Interior z-face between cells L (k) and R (k+1) of column (i, j).
 // phiL/phiR limited slopes sL/sR (index 0..2 species, 3 = T); N_nom: nominal column flux.
-static __device__ void zface(const dv_step_params& p, int i, const Props& L, const Props& R, const Cell& cL, const Cell& cR,
-                      const double sL[4], const double sR[4], bool muscl, double N_nom, Flux& out, double* uz_out) {
+static __device__ __forceinline__ void zface_part(const dv_step_params& p, int i, const Props& L, const Props& R,
+                                                  const Cell& cL, const Cell& cR, const double sL[4], const double sR[4],
+                                                  bool muscl, double N_nom, FluxPart& out, double* uz_out) {
     double mu_z = 0.5 * (R.mu + L.mu), rho_z = 0.5 * (R.rho + L.rho);
     double uz = ergun_u((R.P - L.P) / p.dz, p.ka * mu_z, p.kb * rho_z);
     if (uz_out) *uz_out = uz;
@@ -327,14 +341,14 @@ static __device__ void zface(const dv_step_params& p, int i, const Props& L, con
     }
     double Tf = muscl ? (w * (L.T + 0.5 * sL[3]) + (1.0 - w) * (R.T - 0.5 * sR[3])) : (w * L.T + (1.0 - w) * R.T);
     double cpz = 0.5 * (R.cpm + L.cpm);
-    double lam_z = 0.5 * (R.lam0 + L.lam0) + Cz * cpz * fabs(u_disp) * p.dp / p.Pe_z;
-    out.H = enth(p, Fconv, Tf) + enth(p, J, 0.5 * (R.T + L.T)) - lam_z * (R.T - L.T) / p.dz * Az;
+    out.lx = Cz * cpz * fabs(u_disp) * p.dp / p.Pe_z;
+    out.He = enth(p, Fconv, Tf) + enth(p, J, 0.5 * (R.T + L.T));
 }
 
 // Transverse (r or theta) face between cells A (minus side) and B (plus side):
 // dist = drc (r) or arc (theta), area = Ar or Ath.
-static __device__ void tface(const dv_step_params& p, const Props& A, const Props& B, const Cell& cA, const Cell& cB,
-                      double dist, double area, Flux& out, double* u_out) {
+static __device__ __forceinline__ void tface_part(const dv_step_params& p, const Props& A, const Props& B, const Cell& cA,
+                                                  const Cell& cB, double dist, double area, FluxPart& out, double* u_out) {
     double mu_f = 0.5 * (B.mu + A.mu), rho_f = 0.5 * (B.rho + A.rho);
     double u = ergun_u((B.P - A.P) / dist, p.ka * mu_f, p.kb * rho_f);
     if (u_out) *u_out = u;
@@ -349,8 +363,26 @@ static __device__ void tface(const dv_step_params& p, const Props& A, const Prop
         J[k] = -p.eps_b * Df * Cf * (B.y[k] - A.y[k]) / dist * area;
         out.F[k] = Fconv[k] + J[k];
     }
-    double lam = 0.5 * (A.lam0 + B.lam0) + Cf * (0.5 * (A.cpm + B.cpm)) * fabs(p.u_nom) * p.dp / p.Pe_r;
-    out.H = enth(p, Fconv, w * A.T + (1.0 - w) * B.T) + enth(p, J, 0.5 * (A.T + B.T)) - lam * (B.T - A.T) / dist * area;
+    out.lx = Cf * (0.5 * (A.cpm + B.cpm)) * fabs(p.u_nom) * p.dp / p.Pe_r;
+    out.He = enth(p, Fconv, w * A.T + (1.0 - w) * B.T) + enth(p, J, 0.5 * (A.T + B.T));
+}
+
+static __device__ __forceinline__ void zface(const dv_step_params& p, int i, const Props& L, const Props& R, const Cell& cL,
+                                             const Cell& cR, const double sL[4], const double sR[4], bool muscl,
+                                             double N_nom, Flux& out, double* uz_out) {
+    FluxPart f;
+    zface_part(p, i, L, R, cL, cR, sL, sR, muscl, N_nom, f, uz_out);
+#pragma unroll
+    for (int k = 0; k < DV_NG; ++k) out.F[k] = f.F[k];
+    out.H = face_H(f.He, f.lx, L.lam0, R.lam0, L.T, R.T, p.dz, p.Az[i]);
+}
+static __device__ __forceinline__ void tface(const dv_step_params& p, const Props& A, const Props& B, const Cell& cA,
+                                             const Cell& cB, double dist, double area, Flux& out, double* u_out) {
+    FluxPart f;
+    tface_part(p, A, B, cA, cB, dist, area, f, u_out);
+#pragma unroll
+    for (int k = 0; k < DV_NG; ++k) out.F[k] = f.F[k];
+    out.H = face_H(f.He, f.lx, A.lam0, B.lam0, A.T, B.T, dist, area);
 }
 
 // Boundary record of one end face (accumulators / diagnostics), 16 doubles.
@@ -450,28 +482,33 @@ static __device__ void end_face(const dv_step_params& p, const dv_end& e, double
     }
 }
 
-// Bed-side wall resistance of an outer-ring cell (core/residual.py:329-335)
-static __device__ __forceinline__ double wall_R_bed(const dv_step_params& p, const Props& o) {
+// Bed-side wall resistance of an outer-ring cell (core/residual.py:329-335): the flow part of the wall
+// Nusselt number, which needs the viscosity and conductivity, then the rest, which needs lam0 too.
+static __device__ __forceinline__ double wall_dyn(const dv_step_params& p, const Props& o) {
+    // reference: np.all(Re <= 0) -> 0 (Re = 0 exactly when u_nom = 0)
+    if (p.lumped || p.htc_model == DV_HTC_CONSTANT || p.u_nom == 0.0) return 0.0;
+    double cp_mass = o.cpm / npmax(o.rho / o.Cpos, 1e-6);
+    double Re = o.rho * fabs(p.u_nom) * p.dp / o.mu;
+    double Pr = cp_mass * o.mu / o.kg;
+    double Rm = npmax(Re, 1e-12);
+    double a = 0.3 * pow(Pr, 1.0 / 3.0) * pow(Rm, 0.75);
+    double b = 0.054 * Pr * Rm;
+    return 1.0 / (1.0 / a + 1.0 / b);
+}
+static __device__ __forceinline__ double wall_R_rest(const dv_step_params& p, const Props& o, double dyn) {
     if (p.lumped) return 1.0 / p.U_lumped;
     double lam_out = o.lam0 + o.Cpos * o.cpm * fabs(p.u_nom) * p.dp / p.Pe_r;
     double aw;
     if (p.htc_model == DV_HTC_CONSTANT) {
         aw = p.alpha_const * 1.0;
     } else {
-        double cp_mass = o.cpm / npmax(o.rho / o.Cpos, 1e-6);
-        double Re = o.rho * fabs(p.u_nom) * p.dp / o.mu;
-        double Pr = cp_mass * o.mu / o.kg;
         double nu0 = (1.3 + 5.0 / p.N_ratio) * o.lam0 / o.kg;
-        double dyn = 0.0;
-        if (p.u_nom != 0.0) {     // reference: np.all(Re <= 0) -> 0 (Re = 0 exactly when u_nom = 0)
-            double Rm = npmax(Re, 1e-12);
-            double a = 0.3 * pow(Pr, 1.0 / 3.0) * pow(Rm, 0.75);
-            double b = 0.054 * Pr * Rm;
-            dyn = 1.0 / (1.0 / a + 1.0 / b);
-        }
         aw = (nu0 + dyn) * o.kg / p.dp;
     }
     return 1.0 / aw + p.half_dr_outer / lam_out;
+}
+static __device__ __forceinline__ double wall_R_bed(const dv_step_params& p, const Props& o) {
+    return wall_R_rest(p, o, wall_dyn(p, o));
 }
 
 static __device__ __forceinline__ double jacket_T(const dv_step_params& p, double t) {   // core/residual.py:199-202

@@ -65,11 +65,96 @@ static __device__ __forceinline__ void slope4(int lim, const Cell& m, const doub
     s[3] = limited_slope(lim, To - Tm, Tp - To);
 }
 
-// Divergence of the face fluxes, sorption sinks, wall / jacket / exchanger terms and records of
-// cell (i,j,k) (core/residual.py:298-365): f[0..5]; *fw = dTw/dt of its wall node.  Shared by the
-// thread-per-cell residual, the split residual's assembly and the Jacobian's rows, so all add in the
-// same order.  R_pre: the outer-ring cell's wall resistance where it has been evaluated already (the
-// same expression on the same properties), else null.
+// Balances of cell (i, j, k) from its face fluxes (core/residual.py:298-365), a row at a time; cell_tail
+// below takes them all.  Every caller adds in the same order.
+// divergence of one flux component (physics/mass.py:61-74); faces a one-ring or one-sector grid lacks are absent
+static __device__ __forceinline__ double face_div(const dv_step_params& p, int i, double zm, double zp, double rm, double rp,
+                                                  double tm, double tp) {
+    double d = zp - zm;
+    if (p.Nr > 1) {
+        if (i < p.Nr - 1) d = d + rp;
+        if (i > 0) d = d - rm;
+    }
+    if (p.Nth > 1) d = d + (tp - tm);
+    return d;
+}
+// species balance from the divergence and the uptake
+static __device__ __forceinline__ double row_mass(const dv_step_params& p, int i, double div, double sink) {
+    return -div / (p.eps_t * p.V[i]) - (p.rho_b / p.eps_t) * sink;
+}
+// Wall / jacket terms of the outer-ring cell at (j, k) (core/residual.py:328-359); *fw = dTw/dt of its node.
+struct WallQ { double jac, amb, wb; };
+template <class L>
+static __device__ __forceinline__ WallQ wall_terms(const dv_step_params& p, const Aux& aux, const L& ld, double Tj, int j,
+                                                   int k, double To, double R_bed, double* fw) {
+    const int Nth = p.Nth, Nz = p.Nz;
+    const int64_t off_w = (int64_t)DV_NV * p.Nr * Nth * Nz, wn = (int64_t)j * Nz + k;
+    const double cov = aux.cov[wn];
+    WallQ Q;
+    if (p.wall_on) {
+        const double Tw = ld(off_w + wn);
+        Q.jac = p.jacket_on ? cov * p.h_jac * p.A_wall_out * (Tj - Tw) : 0.0;
+        Q.amb = (1.0 - cov) * p.h_amb * p.A_wall_out * (p.T_amb - Tw);
+        Q.wb = p.A_wall_in * (Tw - To) / R_bed;
+        double cond = 0.0;
+        if (Nz > 1) {
+            if (k < Nz - 1) cond = cond + p.wall_kz * (ld(off_w + wn + 1) - Tw);
+            if (k > 0) cond = cond - p.wall_kz * (Tw - ld(off_w + wn - 1));
+        }
+        if (Nth > 1) {
+            const int jm = (j == 0) ? Nth - 1 : j - 1;
+            const int jp = (j == Nth - 1) ? 0 : j + 1;
+            const double Twp = ld(off_w + (int64_t)jp * Nz + k);
+            const double Twm = ld(off_w + (int64_t)jm * Nz + k);
+            cond = cond + p.wall_kt * (Twp - Tw);
+            cond = cond - p.wall_kt * (Tw - Twm);
+        }
+        if (fw) *fw = (Q.jac + Q.amb - Q.wb + cond) / p.wall_C;
+    } else {
+        if (p.jacket_on && p.h_jac > 0.0) {
+            double R_j = p.lumped ? R_bed : R_bed + 1.0 / p.h_jac;
+            Q.jac = cov * p.A_wall_in * (Tj - To) / R_j;
+        } else {
+            Q.jac = 0.0;
+        }
+        Q.amb = (p.h_amb > 0.0) ? (1.0 - cov) * p.A_wall_in * (p.T_amb - To) / (R_bed + 1.0 / p.h_amb) : 0.0;
+        Q.wb = Q.jac + Q.amb;
+    }
+    return Q;
+}
+// energy balance of cell (i, j, k) from the divergence of its enthalpy fluxes, with the wall, jacket and
+// exchanger terms and their records; *fw as above
+template <class L>
+static __device__ __forceinline__ double row_energy(const dv_step_params& p, const Aux& aux, const L& ld, double t, int i,
+                                                    int j, int k, double T, double R_bed, double de, double* fw,
+                                                    const Rec* rec) {
+    const double V = p.V[i];
+    double src = 0.0;
+    const double Tj = jacket_T(p, t);
+    if (i == p.Nr - 1) {
+        const WallQ Q = wall_terms(p, aux, ld, Tj, j, k, T, R_bed, fw);
+        src = src + Q.wb;
+        if (rec) {
+            const int64_t wn = (int64_t)j * p.Nz + k;
+            rec->Qj[wn] = Q.jac;
+            rec->Qa[wn] = Q.amb;
+            rec->Qw[wn] = Q.wb;
+            rec->Rb[wn] = R_bed;
+        }
+    }
+    double Q_hx = 0.0;
+    if (p.hx_on) {
+        Q_hx = p.hA_v * V * (Tj - T);
+        src = src + Q_hx;
+    }
+    if (rec) rec->Qhx[((int64_t)i * p.Nth + j) * p.Nz + k] = Q_hx;
+    return (-de + src) / V;
+}
+
+// All rows of cell (i,j,k): f[0..5]; *fw = dTw/dt of its wall node; and its records.  Shared by the
+// thread-per-cell residual, the split residual's assembly and the Jacobian's rows.  R_pre: the outer-ring
+// cell's wall resistance where it has been evaluated already (the same expression on the same properties),
+// else null.
 template <class L>
 static __device__ __forceinline__ void cell_tail(const dv_step_params& p, const Aux& aux, const L& ld, double t, int i,
                                                  int j, int k, const Props& P0, const double rate[DV_NA],
@@ -77,85 +162,19 @@ static __device__ __forceinline__ void cell_tail(const dv_step_params& p, const 
                                                  const Flux& Frm, const Flux& Frp, const Flux& Ftm, const Flux& Ftp,
                                                  double f[DV_NV], double* fw, const Rec* rec,
                                                  const double* R_pre = nullptr) {
-    const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
-    const int64_t nc = (int64_t)Nr * Nth * Nz;
-    const int64_t c0 = ((int64_t)i * Nth + j) * Nz + k;
-    const int64_t off_w = (int64_t)DV_NV * nc;
-    // ---------------- divergence (physics/mass.py:61-74) and species balance
-    const double V = p.V[i];
+    const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz;
+    const int64_t c0 = ((int64_t)i * p.Nth + j) * p.Nz + k;
 #pragma unroll
     for (int q = 0; q < DV_NG; ++q) {
-        double d = Fzp.F[q] - Fzm.F[q];
-        if (Nr > 1) {
-            if (i < Nr - 1) d = d + Frp.F[q];
-            if (i > 0) d = d - Frm.F[q];
-        }
-        if (Nth > 1) d = d + (Ftp.F[q] - Ftm.F[q]);
-        double sink = (q < DV_NA) ? rate[q] : 0.0;
-        f[q] = -d / (p.eps_t * V) - (p.rho_b / p.eps_t) * sink;
+        const double div = face_div(p, i, Fzm.F[q], Fzp.F[q], Frm.F[q], Frp.F[q], Ftm.F[q], Ftp.F[q]);
+        f[q] = row_mass(p, i, div, (q < DV_NA) ? rate[q] : 0.0);
     }
     f[3] = rate[0];
     f[4] = rate[1];
-    double de = Fzp.H - Fzm.H;
-    if (Nr > 1) {
-        if (i < Nr - 1) de = de + Frp.H;
-        if (i > 0) de = de - Frm.H;
-    }
-    if (Nth > 1) de = de + (Ftp.H - Ftm.H);
-    // ---------------- wall / jacket / exchanger (core/residual.py:328-359)
-    double src = 0.0;
-    const double Tj = jacket_T(p, t);
-    if (i == Nr - 1) {
-        const int64_t wn = (int64_t)j * Nz + k;
-        const double cov = aux.cov[wn];
-        const double To = P0.T;
-        const double R_bed = R_pre ? *R_pre : wall_R_bed(p, P0);
-        double Q_jac, Q_amb, Q_wb;
-        if (p.wall_on) {
-            const double Tw = ld(off_w + wn);
-            Q_jac = p.jacket_on ? cov * p.h_jac * p.A_wall_out * (Tj - Tw) : 0.0;
-            Q_amb = (1.0 - cov) * p.h_amb * p.A_wall_out * (p.T_amb - Tw);
-            Q_wb = p.A_wall_in * (Tw - To) / R_bed;
-            double cond = 0.0;
-            if (Nz > 1) {
-                if (k < Nz - 1) cond = cond + p.wall_kz * (ld(off_w + wn + 1) - Tw);
-                if (k > 0) cond = cond - p.wall_kz * (Tw - ld(off_w + wn - 1));
-            }
-            if (Nth > 1) {
-                const int jm = (j == 0) ? Nth - 1 : j - 1;
-                const int jp = (j == Nth - 1) ? 0 : j + 1;
-                const double Twp = ld(off_w + (int64_t)jp * Nz + k);
-                const double Twm = ld(off_w + (int64_t)jm * Nz + k);
-                cond = cond + p.wall_kt * (Twp - Tw);
-                cond = cond - p.wall_kt * (Tw - Twm);
-            }
-            if (fw) *fw = (Q_jac + Q_amb - Q_wb + cond) / p.wall_C;
-        } else {
-            if (p.jacket_on && p.h_jac > 0.0) {
-                double R_j = p.lumped ? R_bed : R_bed + 1.0 / p.h_jac;
-                Q_jac = cov * p.A_wall_in * (Tj - To) / R_j;
-            } else {
-                Q_jac = 0.0;
-            }
-            Q_amb = (p.h_amb > 0.0) ? (1.0 - cov) * p.A_wall_in * (p.T_amb - To) / (R_bed + 1.0 / p.h_amb) : 0.0;
-            Q_wb = Q_jac + Q_amb;
-        }
-        src = src + Q_wb;
-        if (rec) {
-            rec->Qj[wn] = Q_jac;
-            rec->Qa[wn] = Q_amb;
-            rec->Qw[wn] = Q_wb;
-            rec->Rb[wn] = R_bed;
-        }
-    }
-    double Q_hx = 0.0;
-    if (p.hx_on) {
-        Q_hx = p.hA_v * V * (Tj - P0.T);
-        src = src + Q_hx;
-    }
-    f[5] = (-de + src) / V;
+    const double de = face_div(p, i, Fzm.H, Fzp.H, Frm.H, Frp.H, Ftm.H, Ftp.H);
+    const double R_bed = (i == p.Nr - 1) ? (R_pre ? *R_pre : wall_R_bed(p, P0)) : 0.0;
+    f[5] = row_energy(p, aux, ld, t, i, j, k, P0.T, R_bed, de, fw, rec);
     if (rec) {
-        rec->Qhx[c0] = Q_hx;
         rec->T[c0] = P0.T;
         rec->P[c0] = P0.P;
 #pragma unroll

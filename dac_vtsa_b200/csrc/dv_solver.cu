@@ -1526,7 +1526,7 @@ static int op_capture(dv_model* m, Work& W, const double* dargs, double* out, cu
 }
 static void op_count(const dv_model* m, int64_t* cnt) {
     if (m->op32) cnt[K_SPMV] += 1;
-    else cnt[K_MATVEC] += matvec_capture_kernels();
+    else cnt[K_MATVEC] += matvec_capture_kernels(m);
 }
 
 // A capture that another host thread invalidated (for instance by the first launch of a kernel,

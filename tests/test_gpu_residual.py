@@ -152,3 +152,45 @@ def test_split_residual_is_bit_identical_to_the_thread_per_cell_evaluation():
         torch.cuda.synchronize()
         assert np.array_equal(f, f2.cpu().numpy()), meta["name"]
         assert np.array_equal(acc, acc2.cpu().numpy()), meta["name"]
+
+
+@pytest.mark.parametrize("grid,step,wall", [((1, 1, 1), 0, True), ((1, 1, 2), 2, True), ((2, 3, 2), 1, True),
+                                            ((1, 5, 3), 0, True), ((3, 5, 7), 2, True), ((5, 4, 9), 1, False),
+                                            ((2, 1, 6), 0, False), ((9, 9, 33), 1, True), ((12, 12, 48), 0, True)])
+def test_tile_residual_at_ragged_grids_is_bit_identical_to_the_other_evaluations(grid, step, wall):
+    """Tiles cut by every edge of the grid, single rings and sectors, columns shorter than a slope's
+    stencil, and a grid past the tile limit: f and the rates against the thread-per-cell kernel, the
+    stage residual against the split evaluation (taken when the result replaces its right-hand side),
+    with a cell of NaN as well.  Bits, as the expressions are the same."""
+    import ctypes as C
+    from dac_vtsa_b200 import _lib, host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.model import TVSAModel
+    from dac_vtsa_b200.params import build_params
+    lib = _lib.load()
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    cfg = load_config(override_dict={"grid.Nr": grid[0], "grid.Ntheta": grid[1], "grid.Nz": grid[2],
+                                     "wall.enabled": wall})
+    g = host.Grid.from_config(cfg)
+    props = host.get_backend(cfg)
+    st = host.seeded_state(cfg, g, props, seed=8, amplitude=0.02, P=101325.0 if step == 0 else 2.2e4)
+    st.q = st.q + np.random.default_rng(9).random(st.q.shape)
+    m = TVSAModel(cfg, g, props, cfg.cycle[step], st)
+    params, *aux, _ = build_params(m.cfg, m.grid, m.props, m.step, m.P_start, None)
+    feed, nnom, cov = (torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64)).to(m.device) for a in aux)
+    y = torch.from_numpy(m.pack(st)).to(m.device)
+    bad = y.clone()
+    bad[g.ncell // 2] = float("nan")
+    for s in (y, bad):
+        f, acc = m.rhs(3.0, s)
+        f2, acc2 = torch.empty_like(s), torch.empty_like(acc)
+        rc = lib.dv_rhs_acc_noalloc(C.byref(params), feed.data_ptr(), nnom.data_ptr(), cov.data_ptr(), 3.0,
+                                    s.data_ptr(), f2.data_ptr(), acc2.data_ptr(), stream)
+        assert rc == 0, lib.dv_last_error()
+        assert np.array_equal(f.cpu().numpy(), f2.cpu().numpy(), equal_nan=True)
+        assert np.array_equal(acc.cpu().numpy(), acc2.cpu().numpy(), equal_nan=True)
+        known = s * 1.001
+        R = m.stage_residual(3.0, s, 0.7, known)
+        rc = lib.dv_stage_residual(m.handle, 3.0, s.data_ptr(), 0.7, known.data_ptr(), known.data_ptr(), stream)
+        assert rc == 0, lib.dv_last_error()
+        assert np.array_equal(R.cpu().numpy(), known.cpu().numpy(), equal_nan=True)
