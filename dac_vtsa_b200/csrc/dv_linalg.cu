@@ -248,10 +248,18 @@ __global__ void k_pc_scatter(PcGeom g, const double* __restrict__ J, double dh, 
 }
 
 // ---------------------------------------------------------------- shared-memory dense kernels (row-major)
-// 256 threads as a 16 x 16 grid; thread (ty, tx) owns rows ty + 16a and columns tx + 16b (a, b < 4),
-// i.e. a 4 x 4 register tile of any nb <= 64 matrix.  No integer division in the inner loops.
-#define SM_T 16
-#define SM_R 4
+// Each works with a team of whole warps of the block, so that teams can work side by side.  Functions of
+// their own, not inlined: the factorisation calls them from many places, and its code then stays in the
+// instruction cache while two teams run different parts of it.
+struct Team {
+    int tid, n, bar;                              // thread of the team, its threads, its barrier
+    __device__ __forceinline__ int lane() const { return tid & 31; }
+    __device__ __forceinline__ int warp() const { return tid >> 5; }
+    __device__ __forceinline__ int warps() const { return n >> 5; }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory");
+    }
+};
 
 // D = A B + D on the FP64 tensor cores: one 8x8x4 product per warp instruction.  Fragments
 // (lane = 4 g + t): a = A[g][t], b = B[t][g], d = D[g][2t .. 2t+1].
@@ -261,99 +269,175 @@ static __device__ __forceinline__ void dmma_884(double& d0, double& d1, double a
                  : "d"(a), "d"(b));
 }
 
-// C = beta C + alpha A B (row-major in shared memory, leading dimension ld, nb <= 64, alpha = +-1):
-// 8x8 output tiles spread over the warps, each accumulated by DMMA over k in steps of 4; entries
-// beyond nb read as zero and are not written.  (Accumulating all of a warp's tiles together
-// measured slower on B200: 5.8 us against 3.7 us for nb = 48.)
-static __device__ void sm_gemm(int nb, int ld, double alpha, const double* A, const double* B, double beta,
-                               double* C) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int nt = (nb + 7) >> 3;
-    for (int tile = warp; tile < nt * nt; tile += nw) {
-        const int ti = tile / nt, tj = tile - ti * nt;
-        const int r = 8 * ti + g;                 // row of A and C held by this lane
-        const int cb = 8 * tj + g;                // column of B in the b fragment
-        const int c0 = 8 * tj + 2 * t4;           // columns of C in the d fragment
-        double d0 = 0.0, d1 = 0.0;
-        for (int kk = 0; kk < nb; kk += 4) {
-            const int ka = kk + t4;
-            const double a = (r < nb && ka < nb) ? alpha * A[r * ld + ka] : 0.0;
-            const double b = (ka < nb && cb < nb) ? B[ka * ld + cb] : 0.0;
-            dmma_884(d0, d1, a, b);
-        }
-        if (r < nb) {
-            double* cp = C + r * ld + c0;
-            if (c0 < nb) cp[0] = (beta == 0.0) ? d0 : beta * cp[0] + d0;
-            if (c0 + 1 < nb) cp[1] = (beta == 0.0) ? d1 : beta * cp[1] + d1;
-        }
-    }
-    __syncthreads();
-}
-
-// C = beta C + alpha Bd X with Bd block diagonal (cell blocks); all three in shared memory with
-// leading dimension ld.
-static __device__ void sm_bd_left(const PcGeom& g, int ld, double alpha, const double* Bd, const double* X,
-                                  double beta, double* C) {
-    const int nb = g.nb;
-    const int tx = threadIdx.x % SM_T, ty = threadIdx.x / SM_T;
+// C = Cin + S A B, S = +-1 (Cin null: C = S A B); A and B in shared memory (row-major, leading
+// dimension ld), Cin and C in any space (ldi, ldc).  8x8 output tiles spread over the warps, each
+// accumulated by DMMA over k in steps of 4, three tiles of a warp at a time (a dependent DMMA takes 29
+// cycles, three independent ones 10 each).  Rows and columns past nb read the last one (they enter no
+// entry that is written); past k = nb both operands are zero.
+static __device__ __noinline__ void tm_gemm(Team T, int nb, int ld, int S, const double* A, const double* B,
+                                            const double* Cin, int ldi, double* C, int ldc) {
+    __builtin_assume(__isShared(A));
+    __builtin_assume(__isShared(B));
+    constexpr int U = 4;
+    const int lane = T.lane(), g = lane >> 2, t4 = lane & 3;
+    const int nt = (nb + 7) >> 3, nt2 = nt * nt, full = nb & ~3;
+    for (int t0 = T.warp(); t0 < nt2; t0 += U * T.warps()) {
+        const double *ap[U], *bp[U];
+        double d0[U], d1[U], e0[U], e1[U];
+        int r[U], c0[U];
 #pragma unroll
-    for (int a = 0; a < SM_R; ++a) {
-        const int r = ty + SM_T * a;
-        if (r >= nb) continue;
-        int b0, bsz;
-        pc_cellblock(g, r, b0, bsz);
+        for (int u = 0; u < U; ++u) {
+            const int tile = t0 + u * T.warps(), ti = tile / nt, tj = tile - ti * nt;
+            r[u] = tile < nt2 ? 8 * ti + g : nb;  // row of A and C held by this lane (nb: no tile)
+            c0[u] = 8 * tj + 2 * t4;              // columns of C in the d fragment
+            ap[u] = A + min(r[u], nb - 1) * ld + t4;
+            bp[u] = B + t4 * ld + min(8 * tj + g, nb - 1);
+            d0[u] = d1[u] = e0[u] = e1[u] = 0.0;
+            if (Cin && r[u] < nb) {
+                if (c0[u] < nb) e0[u] = Cin[r[u] * ldi + c0[u]];
+                if (c0[u] + 1 < nb) e1[u] = Cin[r[u] * ldi + c0[u] + 1];
+            }
+        }
+#pragma unroll 2
+        for (int kk = 0; kk < full; kk += 4) {
 #pragma unroll
-        for (int b = 0; b < SM_R; ++b) {
-            const int c = tx + SM_T * b;
-            if (c >= nb) continue;
-            double acc = 0.0;
-            for (int q = b0; q < b0 + bsz; ++q) acc += Bd[r * ld + q] * X[q * ld + c];
-            double* cp = C + r * ld + c;
-            *cp = (beta == 0.0) ? alpha * acc : beta * (*cp) + alpha * acc;
+            for (int u = 0; u < U; ++u) dmma_884(d0[u], d1[u], ap[u][kk], bp[u][kk * ld]);
+        }
+        if (full < nb) {
+            const bool in = full + t4 < nb;
+#pragma unroll
+            for (int u = 0; u < U; ++u) dmma_884(d0[u], d1[u], in ? ap[u][full] : 0.0, in ? bp[u][full * ld] : 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (r[u] >= nb) continue;
+            const double f0 = S < 0 ? 0.0 - d0[u] : d0[u], f1 = S < 0 ? 0.0 - d1[u] : d1[u];
+            if (c0[u] < nb) C[r[u] * ldc + c0[u]] = Cin ? e0[u] + f0 : f0;
+            if (c0[u] + 1 < nb) C[r[u] * ldc + c0[u] + 1] = Cin ? e1[u] + f1 : f1;
         }
     }
-    __syncthreads();
 }
 
-// C = beta C + alpha X Bd with Bd block diagonal (any memory space, leading dimension ldb); X and C
-// in shared memory with leading dimension ld.
-static __device__ void sm_bd_right(const PcGeom& g, int ld, double alpha, const double* X, const double* Bd,
-                                   int ldb, double beta, double* C) {
-    const int nb = g.nb;
-    const int tx = threadIdx.x % SM_T, ty = threadIdx.x / SM_T;
+// C = Bd X with Bd block diagonal (cell blocks; any space, leading dimension ldb): a cell per warp
+static __device__ __noinline__ void tm_bd_left(Team T, int nb, int ncv, int ld, const double* Bd, int ldb,
+                                               const double* X, double* C) {
+    __builtin_assume(__isShared(X));
+    __builtin_assume(__isShared(C));
+    const int lane = T.lane();
+    const int ncell = ncv / DV_NV, nblk = ncell + (nb - ncv);
+    for (int cell = T.warp(); cell < nblk; cell += T.warps()) {
+        const int b0 = cell < ncell ? cell * DV_NV : ncv + cell - ncell, bsz = cell < ncell ? DV_NV : 1;
+        double x[2][DV_NV];
 #pragma unroll
-    for (int b = 0; b < SM_R; ++b) {
-        const int c = tx + SM_T * b;
-        if (c >= nb) continue;
-        int b0, bsz;
-        pc_cellblock(g, c, b0, bsz);
+        for (int q = 0; q < DV_NV; ++q) {
+            x[0][q] = (q < bsz && lane < nb) ? X[(b0 + q) * ld + lane] : 0.0;
+            x[1][q] = (q < bsz && lane + 32 < nb) ? X[(b0 + q) * ld + lane + 32] : 0.0;
+        }
+        for (int r = b0; r < b0 + bsz; ++r) {
+            double acc[2] = {0.0, 0.0};
 #pragma unroll
-        for (int a = 0; a < SM_R; ++a) {
-            const int r = ty + SM_T * a;
-            if (r >= nb) continue;
-            double acc = 0.0;
-            for (int q = b0; q < b0 + bsz; ++q) acc += X[r * ld + q] * Bd[q * ldb + c];
-            double* cp = C + r * ld + c;
-            *cp = (beta == 0.0) ? alpha * acc : beta * (*cp) + alpha * acc;
+            for (int q = 0; q < DV_NV; ++q) {
+                if (q < bsz) {
+                    const double v = Bd[r * ldb + b0 + q];
+                    acc[0] += v * x[0][q];
+                    acc[1] += v * x[1][q];
+                }
+            }
+            if (lane < nb) C[r * ld + lane] = acc[0];
+            if (lane + 32 < nb) C[r * ld + lane + 32] = acc[1];
         }
     }
-    __syncthreads();
 }
 
-// In-place Gauss-Jordan inverse (row-major, nb <= 64) with partial pivoting; returns 1 on a zero /
-// non-finite pivot (replaced by 1 so the factors stay finite; reported through the info flag).
-// In-place Gauss-Jordan inverse with partial pivoting of the nb x nb block *A (shared memory, nb <=
-// 64, 256 threads), ping-ponging between *A and *B (same size).  Thread t updates column t % 64 on
-// the rows congruent to t / 64 modulo 4 (coalesced row accesses, broadcast column-k reads); the
+// Block-diagonal right factors in shared memory by columns: u2[q][c] is entry (first row of c's block + q, c),
+// zero past the block.  One entry per thread of a team of 64 DV_NV.
+constexpr int BD_LD = 64;
+static __device__ __forceinline__ double bd_entry(const PcGeom& g, int tid, const double* Bd, int ldb) {
+    const int q = tid / BD_LD, c = tid - q * BD_LD;
+    int b0, bsz;
+    pc_cellblock(g, c, b0, bsz);
+    return (c < g.nb && q < bsz) ? Bd[(b0 + q) * ldb + c] : 0.0;
+}
+
+// C = Cin - X Bd (Cin null: C = -X Bd), Bd block diagonal as above; X in shared memory, Cin and C in any space
+static __device__ __noinline__ void tm_bd_right(Team T, int nb, int ncv, int ld, const double* X, const double* u2,
+                                                const double* Cin, int ldi, double* C, int ldc) {
+    __builtin_assume(__isShared(X));
+    __builtin_assume(__isShared(u2));
+    const int lane = T.lane();
+    const int ca = lane, cb = lane + 32;
+    const int ba = ca < ncv ? ca / DV_NV * DV_NV : ca, bb = cb < ncv ? cb / DV_NV * DV_NV : cb;
+    const int na = ca >= nb ? 0 : ca < ncv ? DV_NV : 1, nbb = cb >= nb ? 0 : cb < ncv ? DV_NV : 1;
+    double va[DV_NV], vb[DV_NV];
+#pragma unroll
+    for (int q = 0; q < DV_NV; ++q) {
+        va[q] = u2[q * BD_LD + ca];
+        vb[q] = u2[q * BD_LD + cb];
+    }
+    constexpr int U = 4;                          // rows together, their inputs loaded first
+    for (int r0 = T.warp(); r0 < nb; r0 += U * T.warps()) {
+        double ia[U], ib[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * T.warps();
+            ia[u] = (Cin && r < nb && na) ? Cin[r * ldi + ca] : 0.0;
+            ib[u] = (Cin && r < nb && nbb) ? Cin[r * ldi + cb] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * T.warps();
+            if (r >= nb) break;
+            double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll
+            for (int q = 0; q < DV_NV; ++q) {
+                if (q < na) acc0 += X[r * ld + ba + q] * va[q];
+                if (q < nbb) acc1 += X[r * ld + bb + q] * vb[q];
+            }
+            if (na) C[r * ldc + ca] = Cin ? ia[u] - acc0 : -acc0;
+            if (nbb) C[r * ldc + cb] = Cin ? ib[u] - acc1 : -acc1;
+        }
+    }
+}
+
+// D = S, entries of nb x nb, any spaces
+static __device__ __noinline__ void tm_copy(Team T, int nb, const double* S, int lds, double* D, int ldd) {
+    const int lane = T.lane();
+    constexpr int U = 4;
+    for (int r0 = T.warp(); r0 < nb; r0 += U * T.warps()) {
+        double v0[U], v1[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * T.warps();
+            v0[u] = (r < nb && lane < nb) ? S[r * lds + lane] : 0.0;
+            v1[u] = (r < nb && lane + 32 < nb) ? S[r * lds + lane + 32] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * T.warps();
+            if (r < nb && lane < nb) D[r * ldd + lane] = v0[u];
+            if (r < nb && lane + 32 < nb) D[r * ldd + lane + 32] = v1[u];
+        }
+    }
+}
+
+// Gauss-Jordan inverse with partial pivoting of the nb x nb block *A (shared memory, nb <= 32, a team
+// of 128 threads), ping-ponging between *A and *B (same size).  Thread t updates column t % 32 on
+// the rows congruent to t / 32 modulo 4 (coalesced row accesses, broadcast column-k reads); the
 // threads of column k+1 also keep the running maxima of its new entries (rows > k), so the next
 // pivot is known after the one barrier of the step.  The pivot is the largest |entry|, the
 // smallest row index among equal ones.  The row interchanges are undone at the end by a single
 // column gather.  On return *A holds the inverse (the pointers may have been exchanged).
-static __device__ int sm_inverse_unb(int nb, int ld, double*& A, double*& B, int* perm, int* idx, double* pv, int* pi) {
-    const int tid = threadIdx.x;
-    const int cc = tid & 63, rq = tid >> 6;
-    constexpr int RPT = 16;                       // rows per thread for nb <= 64
+static __device__ __noinline__ int tm_inverse_unb(Team T, int nb, int ld, double* A, double* B, int* perm, int* idx,
+                                                  double* pv, int* pi) {
+    __builtin_assume(__isShared(A));
+    __builtin_assume(__isShared(B));
+    __builtin_assume(__isShared(perm));
+    __builtin_assume(__isShared(idx));
+    __builtin_assume(__isShared(pv));
+    __builtin_assume(__isShared(pi));
+    const int tid = T.tid;
+    const int cc = tid & 31, rq = tid >> 5;
+    constexpr int RPT = 8;                        // rows per thread for nb <= 32
     int bad = 0;
     if (cc == 0) {                                // column 0: partial maxima per row group
         double best = -1.0;
@@ -365,7 +449,7 @@ static __device__ int sm_inverse_unb(int nb, int ld, double*& A, double*& B, int
         pv[rq] = best;
         pi[rq] = bi;
     }
-    __syncthreads();
+    T.sync();
     for (int k = 0; k < nb; ++k) {
         const double* cpv = pv + 4 * (k & 1);
         const int* cpi = pi + 4 * (k & 1);
@@ -374,6 +458,7 @@ static __device__ int sm_inverse_unb(int nb, int ld, double*& A, double*& B, int
 #pragma unroll
         for (int q = 1; q < 4; ++q)
             if (cpv[q] > best || (cpv[q] == best && cpi[q] < p)) { best = cpv[q]; p = cpi[q]; }
+        if (p >= nb) p = k;                       // (a column of NaN has no largest entry)
         if (tid == 0) perm[k] = p;
         double piv = A[p * ld + k];
         if (!(fabs(piv) > 0.0) || !isfinite(piv)) { bad = 1; piv = 1.0; }
@@ -406,7 +491,7 @@ static __device__ int sm_inverse_unb(int nb, int ld, double*& A, double*& B, int
                 pi[4 * ((k + 1) & 1) + rq] = nbi;
             }
         }
-        __syncthreads();
+        T.sync();
         double* t = A; A = B; B = t;
     }
     if (tid == 0) {                               // the row interchanges, undone as column interchanges
@@ -417,199 +502,255 @@ static __device__ int sm_inverse_unb(int nb, int ld, double*& A, double*& B, int
             idx[q] = t;
         }
     }
-    __syncthreads();
+    T.sync();
     if (cc < nb)
         for (int i = rq; i < nb; i += 4) B[i * ld + cc] = A[i * ld + idx[cc]];
-    __syncthreads();
+    T.sync();
     double* t = A; A = B; B = t;
     return bad;
 }
 
-// Blocked Gauss-Jordan inverse with partial pivoting of the nb x nb block *A (shared memory, nb <=
-// 64, 256 threads, leading dimension ld); *B (same size) is scratch.  Columns are processed in
-// panels of 8: the pivot steps of a panel run on a small column-major copy of its columns (one
-// barrier per step, the next pivot found by the warp that updates its column), then the panel's
-// row interchanges are applied to the other columns, the panel's pivot rows are set aside and the
-// other columns receive the panel's combined transformation as one rank-8 DMMA update:
-//   x <- [x with the pivot rows zeroed] + Panel * x(pivot rows).
-// The pivot is the largest |entry|, the smallest row index among equal ones.  The row
-// interchanges are undone at the end by one column gather.  On return *A holds the inverse (the
-// pointers may have been exchanged).
-static __device__ int sm_inverse_blk(int nb, int ld, double*& A, double*& B, int* perm, int* idx, int* pi) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double* P0 = B;                               // panel copies: [8][nb] column-major, ping-pong
-    double* P1 = B + nb * 8;
-    double* Bs = B + 2 * nb * 8;                  // the panel's pivot rows: [8][ld] (fits: see sm_inverse)
+// One panel of the blocked inverse: Gauss-Jordan steps on columns j0 .. j0 + jb - 1 of A by one warp, the
+// panel in its registers (rows lane and lane + 32).  Rows keep their place in memory; pos0 / pos1 are
+// the positions that row interchanges give them, which decide ties: the pivot is the largest |entry| of the rows
+// that are no pivot yet (done0 / done1), at the smallest position among equal ones.  Returns 1 on a zero or
+// non-finite pivot (replaced by 1 so the factors stay finite).  Pan: the panel again, [row][PAN_LD]; prow: its
+// pivots' rows in memory, pmask: the same as bits.
+// A step works on x[0], and the columns move down by one with it, so that the loop need not be unrolled (its code
+// is fetched once).  A step's chain is the search and the quotient, the next column's update and again: the
+// lanes divide by their own larger entry, magnitudes are ordered by their upper words (integers; FP64 comparisons
+// took half of a step), and the other columns' updates (pivot row q, factors g) follow while the next
+// division runs.  All lanes take the same branches; one lane storing by itself would leave the warp in two
+// parts, each of which issues the rest of the step.
+constexpr int PAN_LD = 12;                        // (a DMMA fragment's 8 rows on different banks)
+static __device__ __forceinline__ int inv_panel(int nb, int ld, double* A, int j0, int jb, int lane, int& pos0, int& pos1,
+                                                bool& done0, bool& done1, double* Pan, int* prow, unsigned* pmask) {
+    const unsigned all = 0xffffffffu;
+    const int r0 = min(lane, nb - 1), r1 = min(lane + 32, nb - 1);
+    double x0[9], x1[9];                          // from the second on shifted: see the updates below
+    if (jb == 8) {                                // (rows of 16-byte pairs: ld and j0 are even)
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+            const double2 a = *reinterpret_cast<const double2*>(A + r0 * ld + j0 + c);
+            const double2 b = *reinterpret_cast<const double2*>(A + r1 * ld + j0 + c);
+            x0[c ? c + 1 : 0] = a.x;
+            x0[c + 2] = a.y;
+            x1[c ? c + 1 : 0] = b.x;
+            x1[c + 2] = b.y;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int cc = j0 + min(c, jb - 1);
+            x0[c ? c + 1 : 0] = (c < jb) ? A[r0 * ld + cc] : 0.0;
+            x1[c ? c + 1 : 0] = (c < jb) ? A[r1 * ld + cc] : 0.0;
+        }
+    }
     int bad = 0;
-    for (int j0 = 0; j0 < nb; j0 += 8) {
-        const int jb = min(8, nb - j0);
-        for (int q = tid; q < nb * 8; q += blockDim.x) {       // panel copy
-            const int cq = q / nb, i = q - cq * nb;
-            P0[q] = (cq < jb) ? A[i * ld + j0 + cq] : 0.0;
-        }
-        if (warp == 0) {                          // pivot of the panel's first column
-            double best = -1.0;
-            int bi = nb;
-            for (int i = j0 + lane; i < nb; i += 32) {
-                const double v = fabs(A[i * ld + j0]);
-                if (v > best) { best = v; bi = i; }
-            }
+    unsigned m0 = 0u, m1 = 0u;
+    double q[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, g0 = 0.0, g1 = 0.0;
+    bool w0 = false, w1 = false;                  // this lane's row is the last step's pivot row
+#pragma unroll 1
+    for (int kq = 0; kq < jb; ++kq) {
+        const double f0 = x0[0], f1 = x1[0];
+        const unsigned h0 = done0 ? 0u : ((unsigned)__double2hiint(f0) & 0x7fffffffu) + 1u;      // 0: no candidate
+        const unsigned h1 = done1 ? 0u : ((unsigned)__double2hiint(f1) & 0x7fffffffu) + 1u;
+        const bool up = h1 > h0;                  // the lane's larger entry: row lane + 32
+        const unsigned hm = up ? h1 : h0;
+        const unsigned best = __reduce_max_sync(all, hm);
+        double xc = (hm > 0x100000u && hm <= 0x7ff00000u) ? (up ? f1 : f0) : 1.0;   // (normal numbers: no branch in the quotient)
+        asm("" : "+d"(xc));                       // (or the quotient of a zero is taken, and not used: 150 cycles)
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const double ov = __shfl_down_sync(0xffffffffu, best, off);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-            }
-            if (lane == 0) pi[0] = bi;
+        for (int c = 1; c < 8; ++c) {
+            x0[c] = w0 ? q[c] : __fma_rn(-g0, q[c], x0[c + 1]);
+            x1[c] = w1 ? q[c] : __fma_rn(-g1, q[c], x1[c + 1]);
         }
-        __syncthreads();
-        double* Pc = P0;
-        double* Pn = P1;
-        for (int kq = 0; kq < jb; ++kq) {         // pivot steps of the panel: warp w updates column w
-            const int k = j0 + kq;
-            const int p = pi[kq & 1];
-            if (tid == 0) perm[k] = p;
-            double piv = Pc[kq * nb + p];
-            if (!(fabs(piv) > 0.0) || !isfinite(piv)) { bad = 1; piv = 1.0; }
-            const double inv = 1.0 / piv;
-            const int cq = warp;
-            double best = -1.0;
-            int bi = nb;
-            if (cq < jb) {
-                const double pr = ((cq == kq) ? 1.0 : Pc[cq * nb + p]) * inv;
-                for (int i = lane; i < nb; i += 32) {
-                    double val;
-                    if (i == k) {
-                        val = pr;
-                    } else {
-                        const int src = (i == p) ? k : i;
-                        val = ((cq == kq) ? 0.0 : Pc[cq * nb + src]) - Pc[kq * nb + src] * pr;
-                    }
-                    Pn[cq * nb + i] = val;
-                    if (cq == kq + 1 && i > k) {
-                        const double v = fabs(val);
-                        if (v > best) { best = v; bi = i; }
-                    }
-                }
+        const unsigned b0 = __ballot_sync(all, h0 == best), b1 = __ballot_sync(all, h1 == best);
+        int src = __ffs(b0 | b1) - 1;
+        bool srcup = b1 != 0u;
+        const bool odd = __popc(b0) + __popc(b1) != 1 || best <= 0x100000u || best > 0x7ff00000u;
+        double inv = 1.0 / xc;
+        if (odd) {
+            // equal upper words, zero, subnormal, infinite, NaN: whole magnitudes, then positions
+            constexpr unsigned long long INF = 0x7ff0000000000000ull, MAG = 0x7fffffffffffffffull;
+            const unsigned long long a0 = (unsigned long long)__double_as_longlong(f0) & MAG;
+            const unsigned long long a1 = (unsigned long long)__double_as_longlong(f1) & MAG;
+            const unsigned long long k0 = (!done0 && a0 <= INF) ? a0 + 1 : 0, k1 = (!done1 && a1 <= INF) ? a1 + 1 : 0;
+            bool u = k1 > k0 || (k1 == k0 && k1 != 0 && pos1 < pos0);
+            const unsigned long long kk = u ? k1 : k0;
+            unsigned pc = (unsigned)(u ? pos1 : pos0);
+            const unsigned mh = __reduce_max_sync(all, (unsigned)(kk >> 32));
+            const bool c1 = (unsigned)(kk >> 32) == mh;
+            const unsigned ml = __reduce_max_sync(all, c1 ? (unsigned)kk : 0u);
+            bool c2 = c1 && (unsigned)kk == ml;
+            if ((mh | ml) == 0u) {                // a column of NaN: the row in the smallest place
+                u = done0 || (!done1 && pos1 < pos0);
+                pc = (unsigned)(u ? pos1 : pos0);
+                c2 = !(done0 && done1);
             }
-            if (cq == kq + 1) {                   // the next pivot (warp-uniform branch)
+            const unsigned mp = __reduce_min_sync(all, c2 ? pc : all);
+            c2 = c2 && pc == mp;
+            src = __ffs(__ballot_sync(all, c2)) - 1;
+            srcup = (__ballot_sync(all, u) >> src) & 1u;
+            const bool ok = (__ballot_sync(all, kk > 1 && kk <= INF) >> src) & 1u;
+            inv = 1.0 / (ok ? (srcup ? f1 : f0) : 1.0);
+            if (!ok) bad = 1;
+        }
+        inv = __shfl_sync(all, inv, src);
+        const double p1 = __shfl_sync(all, srcup ? x1[1] : x0[1], src) * inv;
+        const int k = j0 + kq, pp = __shfl_sync(all, srcup ? pos1 : pos0, src);
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    const double ov = __shfl_down_sync(0xffffffffu, best, off);
-                    const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                    if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-                }
-                if (lane == 0) pi[(kq + 1) & 1] = bi;
-            }
-            __syncthreads();
-            double* t = Pc; Pc = Pn; Pn = t;
-        }
-        if (tid < nb && (tid < j0 || tid >= j0 + jb)) {    // the panel's row interchanges elsewhere
-            const int c = tid;
-            for (int kq = 0; kq < jb; ++kq) {
-                const int k = j0 + kq, p = perm[k];
-                if (p != k) {
-                    const double t = A[k * ld + c];
-                    A[k * ld + c] = A[p * ld + c];
-                    A[p * ld + c] = t;
-                }
-            }
-        }
-        __syncthreads();
-        for (int q = tid; q < 8 * ld; q += blockDim.x) {   // set the pivot rows aside
-            const int kq = q / ld, c = q - kq * ld;
-            double v = 0.0;
-            if (kq < jb && c < nb && (c < j0 || c >= j0 + jb)) {
-                v = A[(j0 + kq) * ld + c];
-                A[(j0 + kq) * ld + c] = 0.0;
-            }
-            Bs[q] = v;
-        }
-        __syncthreads();
-        {                                         // other columns += Panel * Bs; panel columns <- Panel
-            const int g = lane >> 2, t4 = lane & 3;
-            const int nt = (nb + 7) >> 3;
-            for (int tile = warp; tile < nt * nt; tile += (int)(blockDim.x >> 5)) {
-                const int ti = tile / nt, tj = tile - ti * nt;
-                const int r = 8 * ti + g, cb = 8 * tj + g, c0 = 8 * tj + 2 * t4;
-                double d0 = 0.0, d1 = 0.0;
-#pragma unroll
-                for (int kk = 0; kk < 8; kk += 4) {
-                    const double a = (r < nb && kk + t4 < jb) ? Pc[(kk + t4) * nb + r] : 0.0;
-                    const double b = (cb < nb) ? Bs[(kk + t4) * ld + cb] : 0.0;
-                    dmma_884(d0, d1, a, b);
-                }
-                if (r < nb) {
-                    double* cp = A + r * ld;
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int c = c0 + e;
-                        if (c >= nb) continue;
-                        if (c >= j0 && c < j0 + jb) cp[c] = Pc[(c - j0) * nb + r];
-                        else cp[c] += (e == 0) ? d0 : d1;
-                    }
-                }
-            }
-        }
-        __syncthreads();
+        for (int c = 2; c < 8; ++c) q[c - 1] = __shfl_sync(all, srcup ? x1[c] : x0[c], src) * inv;
+        q[7] = inv;
+        w0 = lane == src && !srcup;
+        w1 = lane == src && srcup;
+        x0[0] = w0 ? p1 : __fma_rn(-f0, p1, x0[1]);
+        x1[0] = w1 ? p1 : __fma_rn(-f1, p1, x1[1]);
+        x0[8] = x1[8] = 0.0;
+        g0 = f0;
+        g1 = f1;
+        pos0 = w0 ? k : pos0 == k ? pp : pos0;
+        pos1 = w1 ? k : pos1 == k ? pp : pos1;
+        done0 = done0 || w0;
+        done1 = done1 || w1;
+        if (srcup) m1 |= 1u << src;
+        else m0 |= 1u << src;
+        prow[kq] = src + (srcup ? 32 : 0);
     }
-    if (tid == 0) {                               // the row interchanges, undone as column interchanges
-        for (int c = 0; c < nb; ++c) idx[c] = c;
-        for (int k = nb - 1; k >= 0; --k) {
-            const int q = perm[k], t = idx[k];
-            idx[k] = idx[q];
-            idx[q] = t;
+#pragma unroll
+    for (int c = 1; c < 8; ++c) {
+        x0[c] = w0 ? q[c] : __fma_rn(-g0, q[c], x0[c + 1]);
+        x1[c] = w1 ? q[c] : __fma_rn(-g1, q[c], x1[c + 1]);
+    }
+    pmask[0] = m0;
+    pmask[1] = m1;
+    if (jb == 8) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int r = lane + 32 * e;
+            if (r < nb) {
+#pragma unroll
+                for (int c = 0; c < 8; c += 2) {
+                    const double2 v = make_double2(e ? x1[c] : x0[c], e ? x1[c + 1] : x0[c + 1]);
+                    *reinterpret_cast<double2*>(A + r * ld + j0 + c) = v;
+                    *reinterpret_cast<double2*>(Pan + r * PAN_LD + c) = v;
+                }
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = (i + jb) & 7;           // the column in x[i] now
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = lane + 32 * e;
+                const double v = e ? x1[i] : x0[i];
+                if (r < nb && c < jb) A[r * ld + j0 + c] = v;
+                if (r < nb) Pan[r * PAN_LD + c] = (c < jb) ? v : 0.0;
+            }
         }
     }
-    __syncthreads();
-    for (int q = tid; q < nb * nb; q += blockDim.x) {
-        const int i = q / nb, c = q - i * nb;
-        B[i * ld + c] = A[i * ld + idx[c]];
-    }
-    __syncthreads();
-    double* t = A; A = B; B = t;
+    __syncwarp();
     return bad;
 }
 
-// Inverse of the nb x nb block *A: blocked when *B can hold the panel copies and pivot rows.
-static __device__ int sm_inverse(int nb, int ld, double*& A, double*& B, int* perm, int* idx, double* pv, int* pi) {
-    if (16 * nb + 8 * ld <= nb * ld) return sm_inverse_blk(nb, ld, A, B, perm, idx, pi);
-    return sm_inverse_unb(nb, ld, A, B, perm, idx, pv, pi);
+// Columns 8 tb .. 8 tb + 7 of A after a panel of jb pivots,
+//   x <- [x with the pivot rows zeroed] + Panel * x(pivot rows), a rank-8 DMMA update:
+// by one warp, or (`shared`) by all of the team, each a part of the rows.
+static __device__ __forceinline__ void inv_update(const Team& T, bool shared, int nb, int ld, double* A, int tb, int jb,
+                                                  const double* Pan, const int* prow, const unsigned* pmask) {
+    const int lane = T.lane(), g = lane >> 2, t4 = lane & 3, nt = (nb + 7) >> 3;
+    const int cb = min(8 * tb + g, nb - 1), c0 = 8 * tb + 2 * t4;
+    const double b0 = (t4 < jb) ? A[prow[t4] * ld + cb] : 0.0, b1 = (t4 + 4 < jb) ? A[prow[t4 + 4] * ld + cb] : 0.0;
+    const unsigned m0 = pmask[0], m1 = pmask[1];
+    if (shared) T.sync();                         // (every pivot row has been read)
+    else __syncwarp();
+    const int first = shared ? T.warp() : 0, step = shared ? T.warps() : 1;
+#pragma unroll 1
+    for (int t0 = first; t0 < nt; t0 += 4 * step) {
+        double d0[4], d1[4], e0[4], e1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = 8 * (t0 + u * step) + g;
+            const double* pp = Pan + min(r, nb - 1) * PAN_LD + t4;
+            const bool live = r < nb && !(((r < 32 ? m0 : m1) >> (r & 31)) & 1u);      // (a pivot row counts as zero)
+            e0[u] = (live && c0 < nb) ? A[r * ld + c0] : 0.0;
+            e1[u] = (live && c0 + 1 < nb) ? A[r * ld + c0 + 1] : 0.0;
+            d0[u] = d1[u] = 0.0;
+            dmma_884(d0[u], d1[u], pp[0], b0);
+            dmma_884(d0[u], d1[u], pp[4], b1);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = 8 * (t0 + u * step) + g;
+            if (r >= nb) continue;
+            if (c0 < nb) A[r * ld + c0] = e0[u] + d0[u];
+            if (c0 + 1 < nb) A[r * ld + c0 + 1] = e1[u] + d1[u];
+        }
+    }
 }
 
-// rows x columns < nb of a block, global (leading dimension ld) <-> shared memory (lds); the
-// padding columns keep the zeros they were given.  256 threads, nb <= PC_SMEM_NB: thread t moves
-// the entries t + 256 i (row-major over nb x nb), i < CP_K, stepping (row, column) without a
-// division; cp_in issues all of its global loads before the first shared store, so one copy
-// costs one L2 round trip.
-#define CP_K 13                                  // 13 * 256 >= 56 * 56
-static __device__ void cp_in(int nb, int ld, int lds, const double* __restrict__ src, double* __restrict__ dst) {
-    const int dr = 256 / nb, dc = 256 - dr * nb;
-    int r = threadIdx.x / nb, c = threadIdx.x - r * nb;
-    double v[CP_K];
-    int off[CP_K];
-#pragma unroll
-    for (int i = 0; i < CP_K; ++i) {
-        off[i] = (r < nb) ? r * lds + c : -1;
-        v[i] = (r < nb) ? src[r * ld + c] : 0.0;
-        r += dr;
-        c += dc;
-        if (c >= nb) { c -= nb; ++r; }
+// Blocked Gauss-Jordan inverse with partial pivoting of the nb x nb block A (shared memory, nb <= 64) into
+// X, by a team of 4 warps; A is overwritten.  Panels of 8 columns: warp 0 takes a panel's pivot steps, the
+// others meanwhile update the columns that the next panel does not need with the panel before.  The pivot steps are a serial chain (a division and a search for the largest entry, 48 times
+// for nb = 48); with the panel in one warp's registers a step has no barrier and no trip through shared
+// memory: 79 000 -> 32 000 cycles an inverse (nb = 43; before, steps by eight warps with a barrier each).
+static __device__ __noinline__ int tm_inverse_blk(Team T, int nb, int ld, double* A, double* X, int* pos, int* prow,
+                                                  unsigned* pmask) {
+    __builtin_assume(__isShared(A));
+    __builtin_assume(__isShared(X));
+    __builtin_assume(__isShared(pos));
+    __builtin_assume(__isShared(prow));
+    __builtin_assume(__isShared(pmask));
+    const int lane = T.lane(), warp = T.warp(), nt = (nb + 7) >> 3;
+    int pos0 = lane, pos1 = lane + 32, bad = 0;
+    bool done0 = lane >= nb, done1 = lane + 32 >= nb;       // (rows past nb are never pivots)
+    for (int j = 0; j < nt; ++j) {
+        const int b = j & 1, jb = min(8, nb - 8 * j);
+        double* Pan = X + b * nb * PAN_LD;
+        if (warp == 0) {
+            bad |= inv_panel(nb, ld, A, 8 * j, jb, lane, pos0, pos1, done0, done1, Pan, prow + 8 * b, pmask + 2 * b);
+            if (j == nt - 1) {
+                if (lane < nb) pos[lane] = pos0;
+                if (lane + 32 < nb) pos[lane + 32] = pos1;
+            }
+        }
+        T.sync();
+        // the next panel's columns by all warps, the other columns by warps 1 to 3 (after the last panel by all)
+        const bool end = j == nt - 1;
+        if (!end) {
+            inv_update(T, true, nb, ld, A, j + 1, jb, Pan, prow + 8 * b, pmask + 2 * b);
+            T.sync();
+        }
+        for (int e = end ? warp : warp == 0 ? nt : warp - 1; e < (end ? nt - 1 : nt - 2); e += end ? 4 : 3)
+            inv_update(T, false, nb, ld, A, (end || e < j) ? e : e + 2, jb, Pan, prow + 8 * b, pmask + 2 * b);
+        __syncwarp();
     }
-#pragma unroll
-    for (int i = 0; i < CP_K; ++i)
-        if (off[i] >= 0) dst[off[i]] = v[i];
+    T.sync();
+    for (int r = warp; r < nb; r += 4) {          // the rows in their positions, the interchanges undone on the columns
+        double* xp = X + pos[r] * ld;
+        if (lane < nb) xp[lane] = A[r * ld + pos[lane]];
+        if (lane + 32 < nb) xp[lane + 32] = A[r * ld + pos[lane + 32]];
+    }
+    T.sync();
+    return bad;
 }
-static __device__ void cp_out(int nb, int ld, int lds, const double* __restrict__ src, double* __restrict__ dst) {
-    const int dr = 256 / nb, dc = 256 - dr * nb;
-    int r = threadIdx.x / nb, c = threadIdx.x - r * nb;
-#pragma unroll
-    for (int i = 0; i < CP_K; ++i) {
-        if (r < nb) dst[r * ld + c] = src[r * lds + c];
-        r += dr;
-        c += dc;
-        if (c >= nb) { c -= nb; ++r; }
-    }
+
+// Inverse of the block A into X, by a team of 4 warps (the pointers may have been exchanged in all
+// threads of the block: `odd`); blocked when X can hold two panels.
+struct InvWork {
+    double pv[8];
+    int pi[8], perm[64], idx[64], pos[64], prow[16];
+    unsigned pmask[4];
+};
+static __device__ __forceinline__ bool inv_blocked(int nb, int ld) { return 16 * nb + 8 * ld <= nb * ld; }
+static __device__ __forceinline__ int tm_inverse(const Team& T, int nb, int ld, double* A, double* X, InvWork& W) {
+    if (inv_blocked(nb, ld)) return tm_inverse_blk(T, nb, ld, A, X, W.pos, W.prow, W.pmask);
+    return tm_inverse_unb(T, nb, ld, A, X, W.perm, W.idx, W.pv, W.pi);
+}
+// after tm_inverse, in every thread: X the inverse, A free (an odd number of unblocked steps ends in A)
+static __device__ __forceinline__ void inv_swap(int nb, int ld, double*& A, double*& X) {
+    if (!inv_blocked(nb, ld) && (nb & 1)) { double* t = A; A = X; X = t; }
 }
 
 // ---------------------------------------------------------------- clusters of two CTAs
@@ -646,27 +787,43 @@ static __device__ __forceinline__ int ld_peer_cta(const int* p, uint32_t rank) {
 //   plane zs:   slot 2 Sinv11 = Dm + Dm S12 Dn S21 Dm,  slot 3 Sinv12 = -Dm S12 Dn
 //   plane zs+1: slot 1 Sinv21 = -Dn S21 Dm,             slot 2 Sinv22 = Dn
 // so that the sweep solves the separator in two independent stages.
+//
+// What bounds it is the chain through the planes: L1 = (..) Uinv_{k-1}, D -= L1 U1_{k-1}, the inverse of D
+// (a serial chain itself).  Four warps take the inverse; the other twelve do meanwhile what plane k's
+// inverse does not need -- U1_k, the products of plane k-1 that are only stored, and from plane k+1
+// L2 = A(k+1,k-1) Uinv_{k-1}, A(k+1,k) - L2 U1_{k-1}, A(k+1,k+1) - L2 U2_{k-1} -- with results that are only
+// stored written from registers, so that nine blocks are enough.  The warps that share the panel warp's scheduler
+// stay out of it: their DMMAs would keep its FP64 unit busy (514 us with them, 488 without).
+// 8x8x32 (18 CTAs): 1190 -> 449 us; 16x16x64 (68): 2440 -> 861.  Of a plane's 135 000 cycles before, 79 000 were
+// the inverse and the rest products and copies in turn with it; now the inverse is two thirds of 50 000.
+constexpr int FAC_T = 512, FAC_INV = 128, FAC_HELP = 288;
+static_assert(2 * FAC_HELP >= DV_NV * BD_LD, "two entries of U2 per thread");
+static __device__ __forceinline__ void pc_prefetch(const double* b, int64_t n, int tid, int nt) {
+    for (int64_t e = (int64_t)tid * 16; e < n; e += (int64_t)nt * 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(b + e));
+}
 template <bool TW>
-__global__ void __launch_bounds__(256) k_pc_factor_smem(PcGeom gin, double* __restrict__ A, int* __restrict__ info, int lds) {
+__global__ void __launch_bounds__(FAC_T) k_pc_factor_smem(PcGeom gin, double* __restrict__ Af, int* __restrict__ info, int lds) {
     const int rank = TW ? (int)(blockIdx.x & 1u) : 0;
     const int part = TW ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const PcGeom g = pc_part(gin, part);
     extern __shared__ __align__(128) double dsm[];
-    __shared__ int perm[64], idx[64];
-    __shared__ double pv[8];
-    __shared__ int pi[8];
+    __shared__ InvWork W;
+    __shared__ double u2[DV_NV * BD_LD];       // U2_{k-1} = A(k-1, k+1) during plane k
     __shared__ int qoff[4], sbad;
     const int nb = g.nb, ld = g.ld;
     const int n2 = nb * lds;                   // one shared-memory block
     const int Nz = g.Nz;
     const int n = TW ? (rank == 0 ? g.zs : Nz - g.zs - 2) : Nz;
-    double* buf[9];
-    for (int q = 0; q < 9; ++q) buf[q] = dsm + (int64_t)q * n2;
-    double *S0 = buf[0], *S1 = buf[1], *S2 = buf[2], *S3 = buf[3], *T = buf[4];
-    double *Ui1 = buf[5], *Ui2 = buf[6], *U11 = buf[7], *U12 = buf[8];
-    for (int64_t q = threadIdx.x; q < 9 * (int64_t)n2; q += blockDim.x) dsm[q] = 0.0;   // zero padding columns
-    __syncthreads();
-    double* base = A + (int64_t)part * Nz * 5 * g.bs;
+    const int tid = threadIdx.x;
+    const bool inverts = tid < FAC_INV;
+    const Team all{tid, FAC_T, 0};
+    const int hw = ((tid >> 7) - 1) * 3 + ((tid >> 5) & 3) - 1;          // helping warp
+    const bool helps = !inverts && ((tid >> 5) & 3) != 0;
+    const Team mine{inverts ? tid : hw * 32 + (tid & 31), inverts ? FAC_INV : FAC_HELP, inverts ? 1 : 2};
+    // D of the plane and of the next, (A(k,k-1) - ..), L1, L2 of the next, U1, Uinv_{k-1}, U1_{k-1}, Uinv
+    double *S2 = dsm, *S2n = dsm + n2, *S1 = dsm + 2 * n2, *L1 = dsm + 3 * n2, *S0 = dsm + 4 * n2, *S3 = dsm + 5 * n2;
+    double *Ui = dsm + 6 * n2, *U1 = dsm + 7 * n2, *X = dsm + 8 * n2;
+    double* base = Af + (int64_t)part * Nz * 5 * g.bs;
     // block (local plane t, local slot sl)
     auto B = [&](int t, int sl) -> double* {
         const int P = (rank == 0) ? t : Nz - 1 - t;
@@ -676,81 +833,78 @@ __global__ void __launch_bounds__(256) k_pc_factor_smem(PcGeom gin, double* __re
         if (P < 0 || P >= Nz || !pc_range_ok(g, (int64_t)part * Nz * 5 * g.bs + off, g.bs)) return base;
         return base + off;
     };
+    auto swap = [](double*& a, double*& b) { double* t = a; a = b; b = t; };
     int bad = 0;
+    tm_copy(all, nb, B(0, 2), ld, S2, lds);
+    all.sync();
     for (int k = 0; k < n; ++k) {
-        if (k >= 2) cp_in(nb, ld, lds, B(k, 0), S0);
-        if (k >= 1) cp_in(nb, ld, lds, B(k, 1), S1);
-        cp_in(nb, ld, lds, B(k, 2), S2);
-        cp_in(nb, ld, lds, B(k, 3), S3);
-        __syncthreads();
-        if (k >= 2) {
-            double* U2_2 = B(k - 2, 4);                                        // A(k-2, k), block diagonal
-            sm_bd_left(g, lds, 1.0, S0, Ui2, 0.0, T);                               // L2 = A(k,k-2) Uinv_{k-2}
-            double* t = S0; S0 = T; T = t;
-            sm_gemm(nb, lds, -1.0, S0, U12, 1.0, S1);                           // A(k,k-1) -= L2 U1_{k-2}
-            sm_bd_right(g, lds, -1.0, S0, U2_2, ld, 1.0, S2);                           // D -= L2 U2_{k-2}
-            sm_bd_right(g, lds, -1.0, Ui2, U2_2, ld, 0.0, T);                           // -Uinv_{k-2} U2_{k-2}
-            cp_out(nb, ld, lds, T, U2_2);                                             // (U2_{k-2} is not needed again)
-            __syncthreads();
-        }
         if (k >= 1) {
-            const double* U2_1 = B(k - 1, 4);                                  // A(k-1, k+1), block diagonal
-            if (k == 1) sm_bd_left(g, lds, 1.0, S1, Ui1, 0.0, T);                  // L1 = A(1,0) Uinv_0
-            else sm_gemm(nb, lds, 1.0, S1, Ui1, 0.0, T);                        // L1 = (...) Uinv_{k-1}
-            double* t = S1; S1 = T; T = t;
-            sm_gemm(nb, lds, -1.0, S1, U11, 1.0, S2);                           // D -= L1 U1_{k-1}
-            sm_bd_right(g, lds, -1.0, S1, U2_1, ld, 1.0, S3);                           // U1 = A(k,k+1) - L1 U2_{k-1}
+            if (k == 1) tm_bd_left(all, nb, g.ncv, lds, S1, lds, Ui, L1);                    // L1 = A(1,0) Uinv_0
+            else tm_gemm(all, nb, lds, 1, S1, Ui, nullptr, 0, L1, lds);              // L1 = (...) Uinv_{k-1}
+            all.sync();
+            tm_gemm(all, nb, lds, -1, L1, U1, S2, lds, S2, lds);                     // D -= L1 U1_{k-1}
+            all.sync();
         }
-        bad |= sm_inverse(nb, lds, S2, T, perm, idx, pv, pi);              // (T: ping-pong buffer)
-        sm_gemm(nb, lds, -1.0, S2, S3, 0.0, T);                                 // -Uinv_k U1_k
-        if (k >= 2) cp_out(nb, ld, lds, S0, B(k, 0));
-        if (k >= 1) cp_out(nb, ld, lds, S1, B(k, 1));
-        cp_out(nb, ld, lds, S2, B(k, 2));
-        cp_out(nb, ld, lds, T, B(k, 3));
-        __syncthreads();
-        // rotate: Uinv_{k-2} <- Uinv_{k-1} <- Uinv_k ; U1 likewise; freed blocks become S2 / S3
-        double* fi = Ui2; Ui2 = Ui1; Ui1 = S2; S2 = fi;
-        double* fu = U12; U12 = U11; U11 = S3; S3 = fu;
+        if (inverts) {
+            bad |= tm_inverse(mine, nb, lds, S2, X, W);
+            double *a = S2, *x = X;
+            inv_swap(nb, lds, a, x);
+            tm_copy(mine, nb, x, lds, B(k, 2), ld);
+        } else if (helps) {
+            const bool next = k + 1 < n || TW;
+            const double u2a = bd_entry(g, mine.tid, B(k, 4), ld);                   // U2_k, for the next plane
+            const double u2b = mine.tid + FAC_HELP < DV_NV * BD_LD ? bd_entry(g, mine.tid + FAC_HELP, B(k, 4), ld) : 0.0;
+            if (k + 2 < Nz) pc_prefetch(B(k + 2, rank == 0 ? 0 : 4), 5 * g.bs, mine.tid, mine.n);
+            if (k >= 1) {
+                if (next) tm_bd_left(mine, nb, g.ncv, lds, B(k + 1, 0), ld, Ui, S0);         // L2 = A(k+1,k-1) Uinv_{k-1}
+                tm_bd_right(mine, nb, g.ncv, lds, L1, u2, B(k, 3), ld, S3, lds);            // U1 = A(k,k+1) - L1 U2_{k-1}
+                tm_gemm(mine, nb, lds, -1, Ui, U1, nullptr, 0, B(k - 1, 3), ld);     // -Uinv_{k-1} U1_{k-1}
+                tm_copy(mine, nb, L1, lds, B(k, 1), ld);
+            } else {
+                tm_copy(mine, nb, B(0, 3), ld, S3, lds);
+                if (next) {
+                    tm_copy(mine, nb, B(1, 1), ld, S1, lds);
+                    tm_copy(mine, nb, B(1, 2), ld, S2n, lds);
+                }
+            }
+            if (next && k >= 1) {
+                mine.sync();                                                         // L2 complete, U2 and A(k+1,k-1) read
+                tm_gemm(mine, nb, lds, -1, S0, U1, B(k + 1, 1), ld, S1, lds);        // A(k+1,k) - L2 U1_{k-1}
+                // A(k+1,k+1) - L2 U2_{k-1}; of a separator plane the Schur contribution alone
+                tm_bd_right(mine, nb, g.ncv, lds, S0, u2, k + 1 < n ? B(k + 1, 2) : nullptr, ld, S2n, lds);
+                tm_copy(mine, nb, S0, lds, B(k + 1, 0), ld);
+                tm_bd_right(mine, nb, g.ncv, lds, Ui, u2, nullptr, 0, B(k - 1, 4), ld);     // -Uinv_{k-1} U2_{k-1}
+            }
+            mine.sync();
+            u2[mine.tid] = u2a;
+            if (mine.tid + FAC_HELP < DV_NV * BD_LD) u2[mine.tid + FAC_HELP] = u2b;
+        }
+        all.sync();
+        inv_swap(nb, lds, S2, X);
+        swap(Ui, X);
+        swap(U1, S3);
+        swap(S2, S2n);
     }
+    tm_gemm(all, nb, lds, -1, Ui, U1, nullptr, 0, B(n - 1, 3), ld);                  // -Uinv_{n-1} U1_{n-1}
     if constexpr (!TW) {
         // slot 4 of the last two planes: U2_k = A(k, k+2) = 0 for k >= Nz-2 (zeroed at assembly)
-        if (threadIdx.x == 0) info[part] = bad;
+        if (tid == 0) info[part] = bad;
     } else {
-        // separator plane n: coupled to planes n-2 and n-1
-        cp_in(nb, ld, lds, B(n, 0), S0);                                             // A(n, n-2)
-        cp_in(nb, ld, lds, B(n, 1), S1);                                             // A(n, n-1)
-        __syncthreads();
-        double* U2_2 = B(n - 2, 4);                                            // A(n-2, n)
-        double* U2_1 = B(n - 1, 4);                                            // A(n-1, n+1)
-        sm_bd_left(g, lds, 1.0, S0, Ui2, 0.0, T);                                   // L2_n = A(n,n-2) Uinv_{n-2}
-        { double* t = S0; S0 = T; T = t; }
-        sm_gemm(nb, lds, -1.0, S0, U12, 1.0, S1);                               // A(n,n-1) - L2 U1_{n-2}
-        sm_bd_right(g, lds, -1.0, S0, U2_2, ld, 0.0, S2);                               // Q(n,n) = -L2 U2_{n-2}
-        sm_bd_right(g, lds, -1.0, Ui2, U2_2, ld, 0.0, T);                               // -Uinv_{n-2} U2_{n-2}
-        cp_out(nb, ld, lds, T, U2_2);
-        __syncthreads();
-        sm_gemm(nb, lds, 1.0, S1, Ui1, 0.0, T);                                 // L1_n = (...) Uinv_{n-1}
-        { double* t = S1; S1 = T; T = t; }
-        sm_gemm(nb, lds, -1.0, S1, U11, 1.0, S2);                               // Q(n,n) -= L1 U1_{n-1}
-        sm_bd_right(g, lds, -1.0, S1, U2_1, ld, 0.0, S3);                               // Q(n,n+1) = -L1 U2_{n-1}
-        cp_out(nb, ld, lds, S0, B(n, 0));
-        cp_out(nb, ld, lds, S1, B(n, 1));
-        __syncthreads();
-        // separator plane n+1: coupled to plane n-1 only
-        cp_in(nb, ld, lds, B(n + 1, 0), S0);                                         // A(n+1, n-1)
-        __syncthreads();
-        sm_bd_left(g, lds, 1.0, S0, Ui1, 0.0, T);                                   // L2_{n+1} = A(n+1,n-1) Uinv_{n-1}
-        { double* t = S0; S0 = T; T = t; }
-        double* Q10 = Ui2;                                                     // (Uinv_{n-2}, U1_{n-2}: done)
-        double* Q11 = U12;
-        sm_gemm(nb, lds, -1.0, S0, U11, 0.0, Q10);                              // Q(n+1,n) = -L2 U1_{n-1}
-        sm_bd_right(g, lds, -1.0, S0, U2_1, ld, 0.0, Q11);                              // Q(n+1,n+1) = -L2 U2_{n-1}
-        sm_bd_right(g, lds, -1.0, Ui1, U2_1, ld, 0.0, T);                               // -Uinv_{n-1} U2_{n-1}
-        cp_out(nb, ld, lds, T, U2_1);
-        cp_out(nb, ld, lds, S0, B(n + 1, 0));
-        if (threadIdx.x == 0) {
-            qoff[0] = (int)(S2 - dsm);
-            qoff[1] = (int)(S3 - dsm);
+        // separator plane n (L2_n, A(n,n-1) - L2 U1_{n-2} and -L2 U2_{n-2} are there), plane n+1: coupled to n-1 only
+        tm_gemm(all, nb, lds, 1, S1, Ui, nullptr, 0, L1, lds);                       // L1_n = (...) Uinv_{n-1}
+        tm_bd_left(all, nb, g.ncv, lds, B(n + 1, 0), ld, Ui, S0);                            // L2_{n+1} = A(n+1,n-1) Uinv_{n-1}
+        all.sync();
+        double *Q00 = S2, *Q01 = S3, *Q10 = X, *Q11 = S2n;
+        tm_gemm(all, nb, lds, -1, L1, U1, Q00, lds, Q00, lds);                       // Q(n,n) -= L1 U1_{n-1}
+        tm_bd_right(all, nb, g.ncv, lds, L1, u2, nullptr, 0, Q01, lds);                     // Q(n,n+1) = -L1 U2_{n-1}
+        tm_gemm(all, nb, lds, -1, S0, U1, nullptr, 0, Q10, lds);                     // Q(n+1,n) = -L2 U1_{n-1}
+        tm_bd_right(all, nb, g.ncv, lds, S0, u2, nullptr, 0, Q11, lds);                     // Q(n+1,n+1) = -L2 U2_{n-1}
+        tm_bd_right(all, nb, g.ncv, lds, Ui, u2, nullptr, 0, B(n - 1, 4), ld);              // -Uinv_{n-1} U2_{n-1}
+        tm_copy(all, nb, L1, lds, B(n, 1), ld);
+        tm_copy(all, nb, S0, lds, B(n + 1, 0), ld);
+        if (tid == 0) {
+            qoff[0] = (int)(Q00 - dsm);
+            qoff[1] = (int)(Q01 - dsm);
             qoff[2] = (int)(Q10 - dsm);
             qoff[3] = (int)(Q11 - dsm);
             sbad = bad;
@@ -758,38 +912,47 @@ __global__ void __launch_bounds__(256) k_pc_factor_smem(PcGeom gin, double* __re
         __syncthreads();
         cluster_sync_all();                                                    // both ranks hold Q
         // rank 0: S = A_sep + Q(rank 0) + Q(rank 1); rank 1's local block (a, b) is separator (1-a, 1-b)
-        double* Sb[4] = {S2, S3, Q10, Q11};                                    // separator (0,0) (0,1) (1,0) (1,1)
+        double* Sb[4] = {Q00, Q01, Q10, Q11};                                  // separator (0,0) (0,1) (1,0) (1,1)
         if (rank == 0) {
-            int ro[4];
-            for (int q = 0; q < 4; ++q) ro[q] = ld_peer_cta(&qoff[3 - q], 1u);
             const double* Ab[4] = {B(n, 2), B(n, 3), B(n + 1, 1), B(n + 1, 2)};
-            for (int q = 0; q < 4; ++q)
-                for (int r = threadIdx.x >> 5; r < nb; r += blockDim.x >> 5)
-                    for (int c = threadIdx.x & 31; c < nb; c += 32) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int ro = ld_peer_cta(&qoff[3 - q], 1u);
+#pragma unroll 2
+                for (int r = tid >> 5; r < nb; r += FAC_T / 32)
+                    for (int c = tid & 31; c < nb; c += 32) {
                         const int es = r * lds + c;
-                        Sb[q][es] = (Ab[q][r * ld + c] + Sb[q][es]) + ld_peer_cta(dsm + ro[q] + es, 1u);
+                        Sb[q][es] = (Ab[q][r * ld + c] + Sb[q][es]) + ld_peer_cta(dsm + ro + es, 1u);
                     }
-            if (threadIdx.x == 0) bad |= ld_peer_cta(&sbad, 1u);
+            }
+            if (tid == 0) bad |= ld_peer_cta(&sbad, 1u);
         }
         __syncthreads();
         cluster_sync_all();                                                    // rank 1's blocks have been read
         if (rank == 0) {
             double *S11 = Sb[0], *S12 = Sb[1], *S21 = Sb[2], *S22 = Sb[3];
-            double* Xn = S0;                                                   // free: S0, S1, Ui1, U11 (+ T)
-            double* Y = S1;
-            bad |= sm_inverse(nb, lds, S11, T, perm, idx, pv, pi);             // Dm = S11^-1
-            sm_gemm(nb, lds, -1.0, S11, S12, 0.0, Xn);                          // Xn = -Dm S12
-            sm_gemm(nb, lds, 1.0, S21, S11, 0.0, Y);                            // Y = S21 Dm
-            sm_gemm(nb, lds, 1.0, S21, Xn, 1.0, S22);                           // S22 - S21 Dm S12
-            bad |= sm_inverse(nb, lds, S22, T, perm, idx, pv, pi);             // Dn = Sinv22
-            sm_gemm(nb, lds, 1.0, Xn, S22, 0.0, S12);                           // Sinv12 = Xn Dn
-            sm_gemm(nb, lds, -1.0, S22, Y, 0.0, S21);                           // Sinv21 = -Dn Y
-            sm_gemm(nb, lds, -1.0, S12, Y, 1.0, S11);                           // Sinv11 = Dm - Sinv12 Y
-            cp_out(nb, ld, lds, S11, B(n, 2));
-            cp_out(nb, ld, lds, S12, B(n, 3));
-            cp_out(nb, ld, lds, S21, B(n + 1, 1));
-            cp_out(nb, ld, lds, S22, B(n + 1, 2));
-            if (threadIdx.x == 0) info[part] = bad;
+            double *Xn = S0, *Y = S1, *T = L1;                                 // free: S0, S1, L1, Ui, U1
+            if (inverts) bad |= tm_inverse(mine, nb, lds, S11, T, W);          // Dm = S11^-1
+            all.sync();
+            inv_swap(nb, lds, S11, T);
+            swap(S11, T);
+            tm_gemm(all, nb, lds, -1, S11, S12, nullptr, 0, Xn, lds);          // Xn = -Dm S12
+            tm_gemm(all, nb, lds, 1, S21, S11, nullptr, 0, Y, lds);            // Y = S21 Dm
+            all.sync();
+            tm_gemm(all, nb, lds, 1, S21, Xn, S22, lds, S22, lds);             // S22 - S21 Dm S12
+            all.sync();
+            if (inverts) bad |= tm_inverse(mine, nb, lds, S22, T, W);          // Dn = Sinv22
+            all.sync();
+            inv_swap(nb, lds, S22, T);
+            swap(S22, T);
+            tm_gemm(all, nb, lds, 1, Xn, S22, nullptr, 0, S12, lds);           // Sinv12 = Xn Dn
+            tm_gemm(all, nb, lds, -1, S22, Y, nullptr, 0, S21, lds);           // Sinv21 = -Dn Y
+            all.sync();
+            tm_gemm(all, nb, lds, -1, S12, Y, S11, lds, B(n, 2), ld);          // Sinv11 = Dm - Sinv12 Y
+            tm_copy(all, nb, S12, lds, B(n, 3), ld);
+            tm_copy(all, nb, S21, lds, B(n + 1, 1), ld);
+            tm_copy(all, nb, S22, lds, B(n + 1, 2), ld);
+            if (tid == 0) info[part] = bad;
         }
     }
 }
@@ -1645,21 +1808,22 @@ int precond_factor(dv_model* m, const double* J, double dh, int mode, cudaStream
     dim3 grid((unsigned)((m->nc + 127) / 128), DV_NSLOT);
     DV_LAUNCH(dv::K_PC_FACTOR, s, k_pc_scatter<<<grid, 128, 0, s>>>(g, J, dh, m->d_pc));
     const int optin = smem_optin();
-    const size_t budget = (size_t)optin - 2048;             // static shared memory of the kernel
+    constexpr size_t own = 6144;                            // static shared memory of the kernel (at most)
+    const size_t budget = (size_t)optin - own;
     const int lds = pc_lds(g.nb, budget);
     const size_t dyn = (size_t)9 * g.nb * lds * sizeof(double);
     const bool factor_smem = g.nb <= PC_SMEM_NB && dyn <= budget;
     g.zs = pc_twist_zs(g, pc_tsize(m), factor_smem);
     if (factor_smem && g.zs > 0) {
-        if (dyn > 48 * 1024)
+        if (dyn + own > 48 * 1024)
             DV_CUDA(allow_dyn_smem((const void*)k_pc_factor_smem<true>));
         DV_LAUNCH(dv::K_PC_FACTOR, s,
-                  DV_CUDA(launch_pair(k_pc_factor_smem<true>, 2u * g.nparts, 256u, dyn, s, false, g, m->d_pc, m->d_pc_info,
+                  DV_CUDA(launch_pair(k_pc_factor_smem<true>, 2u * g.nparts, (unsigned)FAC_T, dyn, s, false, g, m->d_pc, m->d_pc_info,
                                       lds)));
     } else if (factor_smem) {
-        if (dyn > 48 * 1024)
+        if (dyn + own > 48 * 1024)
             DV_CUDA(allow_dyn_smem((const void*)k_pc_factor_smem<false>));
-        DV_LAUNCH(dv::K_PC_FACTOR, s, k_pc_factor_smem<false><<<g.nparts, 256, dyn, s>>>(g, m->d_pc, m->d_pc_info, lds));
+        DV_LAUNCH(dv::K_PC_FACTOR, s, k_pc_factor_smem<false><<<g.nparts, FAC_T, dyn, s>>>(g, m->d_pc, m->d_pc_info, lds));
     } else {
         const size_t static_smem = (2 * 1024 + 256) * sizeof(double) + 256 * sizeof(int);
         size_t need = (size_t)2 * g.nb * g.nb * sizeof(double);

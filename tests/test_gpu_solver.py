@@ -243,6 +243,37 @@ def test_twisted_separator_inverse_on_stiff_stage_matrix(Nz, dh, monkeypatch):
     assert berr(x_one) <= max(1e-12, 10 * ref), (berr(x_one), ref)
 
 
+@pytest.mark.parametrize("Nr,Nz,wall", [(1, 3, True), (3, 9, True), (4, 2, False), (4, 9, True), (5, 3, True),
+                                        (8, 9, False), (8, 8, True), (9, 9, False), (9, 12, True)])
+def test_factorisation_pivots_among_equal_entries(Nr, Nz, wall):
+    """Blocks of 7 to 55 unknowns (unblocked and blocked inverses, last panels of 1 to 8 columns, block
+    sizes that no step of 4 divides, one- and two-sided elimination) whose in-plane entries are 0 and
+    +-1/2 with a diagonal of 1/2, 1 or 3/2, so that pivots are found away from the diagonal and among
+    equal magnitudes.  Against a dense solve: with pivoting inside the blocks the error is that of a
+    backward stable elimination, eps times the condition number times a small multiple of the block size."""
+    import torch
+    from dac_vtsa_b200 import host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.jacobian import FDJacobian
+    from dac_vtsa_b200.model import TVSAModel
+    cfg = load_config(override_dict={"grid.Nr": Nr, "grid.Ntheta": 1, "grid.Nz": Nz, "wall.enabled": wall})
+    g = host.Grid.from_config(cfg)
+    props = host.get_backend(cfg)
+    m = TVSAModel(cfg, g, props, cfg.cycle[0], host.seeded_state(cfg, g, props, seed=1, amplitude=0.01))
+    jac = FDJacobian(m)
+    rng = np.random.default_rng(Nr * 100 + Nz)
+    slot = jac._blk // (7 * 7 * g.ncell)
+    val = np.where((slot >= 1) & (slot <= 4), 0.02 * rng.standard_normal(len(slot)), rng.integers(-1, 2, len(slot)))
+    Jb = np.zeros(m.jac_doubles)
+    Jb[jac._blk] = val
+    M = np.eye(m.n_core) - 0.5 * sp.csc_matrix((val, jac.indices, jac.indptr), shape=(m.n_core, m.n_core)).toarray()
+    b = rng.standard_normal(m.n_core)
+    m.precond_factor(torch.from_numpy(Jb).to(m.device), 0.5, "full")
+    x, ref = m.precond_solve(b), np.linalg.solve(M, b)
+    nb = 6 * Nr + (1 if wall else 0)
+    assert np.abs(x - ref).max() <= 10 * nb * np.finfo(float).eps * np.linalg.cond(M, np.inf) * np.abs(ref).max()
+
+
 def test_implicit_solver_matches_rk4_on_short_transient():
     """Reference integration test (tests/test_physics_and_numerics.py:182-200): SDIRK2 Newton-Krylov
     on the GPU vs classical RK4 (oracle) on a 2x1x4 blowdown, 2 ms, scaled RMS error < 1."""
