@@ -10,13 +10,13 @@
 // produced; the integrator starts Newton from whichever of the two guesses has the smaller scaled
 // residual, so the unchanged Newton tolerance decides the converged state in both cases.
 //
-// Products (all M = 128 rows per CTA, N <= 128 columns, K in chunks of 64 staged through a two-deep
-// shared-memory ring by cp.async, one elected thread issuing the MMAs and committing to an mbarrier):
+// Products (all M = 128 rows per CTA, N <= 128 columns, operands staged in shared memory by cp.async, one
+// elected thread issuing the MMAs and committing to an mbarrier):
 //   forward   H1 = tanh(X W1^T + b1), H2, H3 likewise, O = H3 W4^T + b4
 //   backward  D4 = dL/dO, D3 = (D4 W4) * (1 - H3^2), D2 = (D3 W3) * (1 - H2^2), D1 = (D2 W2) * (1 - H1^2)
 //             dW4^T = H3^T D4, dW3 = D3^T H2, dW2 = D2^T H1, dW1 = D1^T X (K = samples, split over CTAs)
-// Every activation and gradient is written in both panel layouts (rows = samples for the next forward /
-// backward product, rows = features for the weight-gradient product).
+// Forward and backward of 128 rows are one launch (k_chain): activations and gradients stay in shared memory
+// with rows = samples and are written with rows = features for the weight-gradient products (k_gemm).
 #include <cmath>
 #include <cstdio>
 #include <algorithm>
@@ -34,205 +34,326 @@ namespace mlp {
 
 using namespace dv::umma;
 
-enum { E_TANH = 0, E_OUT = 1, E_LOSS = 2, E_DTANH = 3, E_PART = 4 };
+__device__ __forceinline__ float bf2f(bf16 x) { return __bfloat162float(x); }
 
+constexpr int GT = 512;                        // threads of a product: the epilogue has 4 warps per 32 rows,
+                                               // each a quarter of the 16-column groups
+
+// ------------------------------------------------------------------------------------ products
+// D [128 nb][N] = A B^T, block x of nb its rows 128 x (split 0), or a part of K to an FP32 partial sum of its
+// own, D [x][128][N] (split 1: the weight gradients).  Up to four products in one launch, `per` blocks each.
 struct GemmP {
     const bf16* A;
     int64_t ra;           // rows of A's panel layout
     const bf16* B;
     int64_t rb;           // rows of B's panel layout (rows 0..N-1 used)
     int N;                // 16..128, multiple of 16
-    int kpanels;          // K / 8 handled by one CTA (even)
-    int split;            // 1: blockIdx.x selects a K range (weight gradients); 0: an M tile
-    int mode;
-    int64_t rows_valid;   // rows at or beyond this are written as zero and carry no loss
-    const float* bias;
-    bf16* orm;            // output, panel layout with rows = samples (orm_r rows)
-    int64_t orm_r;
-    bf16* ofm;            // output, panel layout with rows = features (ofm_r rows), K = samples
-    int64_t ofm_r;
-    float* of;            // fp32 output (E_OUT rows x ldf; E_PART partials)
-    int64_t ldf;
-    const bf16* hd;       // E_DTANH: activation (panel layout, rows = samples, hd_r rows)
-    int64_t hd_r;
-    const float* tgt;     // E_LOSS: targets [rows][8]
-    float dscale;         // E_LOSS: dL/dO = dscale * (O - target)
-    float* lossp;         // E_LOSS: per-CTA sum of squared errors
-    float* bsum;          // E_LOSS / E_DTANH: per-CTA column sums of the written gradient [grid][N]
+    float* of;
+};
+struct GemmBatch {
+    GemmP p[4];
+    int per;              // blocks of a product
+    int kpanels;          // K / 8 of a block (even)
+    int split;
     int* err;
 };
 
 constexpr int KCH = 8;                         // panels per staged K chunk (64 columns)
+constexpr int RING = 6;                        // staged chunks
 constexpr uint32_t STAGE_A = KCH * 128 * 16;   // 16 KB
 constexpr uint32_t STAGE_B = KCH * 128 * 16;   // 16 KB (N <= 128)
-constexpr uint32_t GEMM_SMEM = 2 * (STAGE_A + STAGE_B);
-// allocation with a guard band: a descriptor whose leading and stride offsets were read the other way
-// round (row groups 2 KB apart) still addresses only memory of this CTA
-constexpr uint32_t GEMM_SMEM_ALLOC = GEMM_SMEM + 65536;
+constexpr uint32_t GEMM_SMEM = RING * (STAGE_A + STAGE_B);
 
-__device__ __forceinline__ float bf2f(bf16 x) { return __bfloat162float(x); }
-
-__global__ void __launch_bounds__(128) k_gemm(GemmP g) {
+// Bound by latency: six of a block's chunks are in flight before its first product (two in flight and a
+// launch for each weight gradient: 74 us a training step; the four together now 11.6).
+__global__ void __launch_bounds__(GT) k_gemm(GemmBatch gb) {
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ __align__(8) uint64_t bars[RING];
     __shared__ uint32_t tmem_s;
-    __shared__ float red[4][16];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int which = blockIdx.x / gb.per, x = blockIdx.x - which * gb.per;
+    const GemmP g = gb.p[which];
     const int N = g.N;
-    const int64_t m0 = g.split ? 0 : (int64_t)blockIdx.x * 128;
-    const int64_t kp0 = g.split ? (int64_t)blockIdx.x * g.kpanels : 0;
-    const int nch = (g.kpanels + KCH - 1) / KCH;
+    const int64_t m0 = gb.split ? 0 : (int64_t)x * 128;
+    const int64_t kp0 = gb.split ? (int64_t)x * gb.kpanels : 0;
+    const int nch = (gb.kpanels + KCH - 1) / KCH;
     const uint32_t sb = smem_u32(smem);
-    const uint32_t sA[2] = {sb, sb + STAGE_A};
-    const uint32_t sB[2] = {sb + 2 * STAGE_A, sb + 2 * STAGE_A + STAGE_B};
     const uint32_t ncols = N <= 32 ? 32u : (N <= 64 ? 64u : 128u);
-    const uint32_t bar0 = smem_u32(&bars[0]), bar1 = smem_u32(&bars[1]);
     if (warp == 0) tmem_alloc(smem_u32(&tmem_s), ncols);
     if (tid == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar1, 1);
+        for (int q = 0; q < RING; ++q) mbar_init(smem_u32(&bars[q]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    auto load = [&](int c) {                   // a (possibly empty) group of copies per chunk
+        if (c < nch) {
+            const uint32_t sA = sb + (c % RING) * (STAGE_A + STAGE_B), sB = sA + STAGE_A;
+            const int pc = min(KCH, gb.kpanels - c * KCH);
+            const int64_t kp = kp0 + (int64_t)c * KCH;
+            for (int idx = tid; idx < pc * 128; idx += GT) {
+                const int p = idx >> 7, r = idx & 127;
+                cp_async16(sA + p * 2048 + r * 16, g.A + ((kp + p) * g.ra + m0 + r) * 8);
+            }
+            for (int idx = tid; idx < pc * N; idx += GT) {
+                const int p = idx / N, r = idx - p * N;
+                cp_async16(sB + p * (N * 16) + r * 16, g.B + ((kp + p) * g.rb + r) * 8);
+            }
+        }
+        cp_async_commit();
+    };
+    for (int c = 0; c < RING; ++c) load(c);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_s;
     const uint32_t idesc = idesc_bf16_m128(N);
-
-    auto load = [&](int c, int s) {
-        const int pc = min(KCH, g.kpanels - c * KCH);
-        const int64_t kp = kp0 + (int64_t)c * KCH;
-        for (int idx = tid; idx < pc * 128; idx += 128) {
-            const int p = idx >> 7, r = idx & 127;
-            cp_async16(sA[s] + p * 2048 + r * 16, g.A + ((kp + p) * g.ra + m0 + r) * 8);
-        }
-        for (int idx = tid; idx < pc * N; idx += 128) {
-            const int p = idx / N, r = idx - p * N;
-            cp_async16(sB[s] + p * (N * 16) + r * 16, g.B + ((kp + p) * g.rb + r) * 8);
-        }
-        cp_async_commit();
-    };
     bool ok = true;
-    load(0, 0);
     for (int c = 0; c < nch; ++c) {
-        const int s = c & 1;
-        if (c + 1 < nch) {
-            if (c >= 1 && !mbar_wait(s ? bar0 : bar1, (uint32_t)(((c - 1) >> 1) & 1))) ok = false;
-            load(c + 1, s ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
+        cp_async_wait<RING - 1>();
         fence_proxy_async();
         __syncthreads();
+        const uint32_t bar = smem_u32(&bars[c % RING]);
         if (tid == 0) {
             fence_after_sync();
-            const int pc = min(KCH, g.kpanels - c * KCH);
+            const uint32_t sA = sb + (c % RING) * (STAGE_A + STAGE_B), sB = sA + STAGE_A;
+            const int pc = min(KCH, gb.kpanels - c * KCH);
             for (int q = 0; q < pc / 2; ++q) {
-                const uint64_t da = sdesc(sA[s] + q * 2 * 2048, 2048, 128);
-                const uint64_t db = sdesc(sB[s] + q * 2 * (N * 16), N * 16, 128);
+                const uint64_t da = sdesc(sA + q * 2 * 2048, 2048, 128);
+                const uint64_t db = sdesc(sB + q * 2 * (N * 16), N * 16, 128);
                 mma_bf16(tmem, da, db, idesc, (c > 0 || q > 0) ? 1u : 0u);
             }
-            mma_commit(s ? bar1 : bar0);
+            mma_commit(bar);
         }
+        if (c + RING < nch && !mbar_wait(bar, (uint32_t)((c / RING) & 1))) ok = false;     // its buffer is free
+        load(c + RING);
     }
-    const int last = nch - 1;
-    if (!mbar_wait((last & 1) ? bar1 : bar0, (uint32_t)((last >> 1) & 1))) ok = false;
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;     // one verdict for the whole CTA (the epilogue has barriers)
+    const uint32_t bar = smem_u32(&bars[(nch - 1) % RING]);
+    const uint32_t par = (uint32_t)(((nch - 1) / RING) & 1);
+    if (!mbar_wait(bar, par)) ok = false;
+    cp_async_wait<0>();
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
     fence_after_sync();
     if (!ok) {
-        atomicOr(g.err, 8);
-        // the products may still run: give them one more bounded wait before the memory is released
-        mbar_wait((last & 1) ? bar1 : bar0, (uint32_t)((last >> 1) & 1));
+        atomicOr(gb.err, 8);
+        mbar_wait(bar, par);                   // the products may still run: one more bounded wait before the memory is released
     }
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-    const int64_t row = m0 + tid;
-    float lsum = 0.0f;
-    for (int c0 = 0; c0 < N && ok; c0 += 16) {
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    for (int c0 = (warp >> 2) * 16; c0 < N && ok; c0 += 64) {
         float v[16];
         tmem_ld16(trow + c0, v);
-        if (g.mode == E_PART) {
-            float* o = g.of + ((int64_t)blockIdx.x * 128 + tid) * N + c0;
+        float4* o = reinterpret_cast<float4*>(g.of + ((int64_t)x * 128 + row) * N + c0);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = v[i];
-            continue;
-        }
-        if (g.mode == E_OUT) {
-            if (row < g.rows_valid) {
-                float* o = g.of + row * g.ldf + c0;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) o[i] = v[i] + g.bias[c0 + i];
-            }
-            continue;
-        }
-        const bool live = row < g.rows_valid;
-        float w[16];
-        if (g.mode == E_TANH) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) w[i] = live ? tanhf(v[i] + g.bias[c0 + i]) : 0.0f;
-        } else if (g.mode == E_DTANH) {
-            const uint4* hp0 = reinterpret_cast<const uint4*>(g.hd + pidx(row, c0, g.hd_r));
-            const uint4* hp1 = reinterpret_cast<const uint4*>(g.hd + pidx(row, c0 + 8, g.hd_r));
-            uint4 hv[2] = {*hp0, *hp1};
-            const bf16* hb = reinterpret_cast<const bf16*>(hv);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float h = bf2f(hb[i]);
-                w[i] = live ? v[i] * (1.0f - h * h) : 0.0f;
-            }
-        } else {   // E_LOSS
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int n = c0 + i;
-                float d = 0.0f;
-                if (live && n < NOUT_USED) d = (v[i] + g.bias[n]) - g.tgt[row * 8 + n];
-                lsum += d * d;
-                w[i] = g.dscale * d;
-            }
-        }
-        bf16 wb[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) wb[i] = __float2bfloat16_rn(w[i]);
-        if (g.orm) {
-            *reinterpret_cast<uint4*>(g.orm + pidx(row, c0, g.orm_r)) = *reinterpret_cast<const uint4*>(wb);
-            *reinterpret_cast<uint4*>(g.orm + pidx(row, c0 + 8, g.orm_r)) = *reinterpret_cast<const uint4*>(wb + 8);
-        }
-        if (g.ofm) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) g.ofm[pidx(c0 + i, row, g.ofm_r)] = wb[i];
-        }
-        if (g.bsum) {   // column sums of the bf16-rounded gradient, in a fixed order
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float x = bf2f(wb[i]);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                if (lane == 0) red[warp][i] = x;
-            }
-            __syncthreads();
-            if (tid < 16)
-                g.bsum[(int64_t)blockIdx.x * N + c0 + tid] = ((red[0][tid] + red[1][tid]) + red[2][tid]) + red[3][tid];
-            __syncthreads();
-        }
-    }
-    if (g.mode == E_LOSS && g.lossp) {
-        float x = lsum;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        __syncthreads();
-        if (lane == 0) red[warp][0] = x;
-        __syncthreads();
-        if (tid == 0) g.lossp[blockIdx.x] = ((red[0][0] + red[1][0]) + red[2][0]) + red[3][0];
+        for (int i = 0; i < 4; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     }
     fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, ncols);
 }
 
-static int gemm(const GemmP& g, int grid, cudaStream_t s) {
+static int gemm(const GemmBatch& g, int products, cudaStream_t s) {
     DV_CUDA(dv::allow_dyn_smem((const void*)k_gemm));
-    DV_LAUNCH(dv::K_MLP, s, k_gemm<<<grid, 128, GEMM_SMEM_ALLOC, s>>>(g));
+    DV_LAUNCH(dv::K_MLP, s, k_gemm<<<products * g.per, GT, GEMM_SMEM, s>>>(g));
     return launch_ok("k_gemm");
+}
+
+// ------------------------------------------------------------------------------------ the chain of a row tile
+// The whole chain of 128 rows in one block: forward (TRAIN 0: X -> O), or forward, loss and backward down to D1.
+// Nothing in it crosses rows, so an activation stays in shared memory as the next product's operand
+// (and for 1 - H^2), weights arrive two products ahead, and a training step's products leave only what the weight
+// gradients read: H and D with rows = features, written 128 bytes at a time while the next product runs.
+// Bound by latency, seven times product, epilogue, barrier, on 32 SMs for 4096 rows: 31 us, where a launch for each
+// product with 128 threads and every activation through L2 in both layouts took 97.
+enum { E_TANH = 0, E_OUT = 1, E_LOSS = 2, E_DTANH = 3 };
+struct ChainP {
+    const bf16* X;        // rows x NIN, panel layout of xr rows
+    int64_t xr;
+    const bf16 *W1, *W2, *W3, *W4, *W4t, *W3t, *W2t;
+    const float* P;       // parameters (biases)
+    int64_t rows_valid;   // rows at or beyond this are zero in every output and carry no loss
+    float* out;           // O [rows][NOUT] (forward)
+    const float* tgt;     // targets [rows][8]
+    float dscale;         // dL/dO = dscale * (O - target)
+    float* lossp;         // per-block sum of squared errors
+    float* bsum;          // per-block column sums of D1, D2, D3, D4, each [blocks][its width], TB * 128 apart
+    bf16 *H1t, *H2t, *H3t, *D4t, *D3t, *D2t, *D1t;      // rows = features, K = samples
+    int* err;
+};
+constexpr uint32_t ACT = 16 * 128 * 16;        // an activation of 128 rows x 128 columns
+constexpr uint32_t D4_AT = 4 * ACT, WBUF_AT = D4_AT + 2 * 128 * 16, CHAIN_SMEM = WBUF_AT + 2 * ACT;
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(GT) k_chain(ChainP g) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bar_s;
+    __shared__ uint32_t tmem_s;
+    __shared__ float red[2][4][4][16];         // (group of columns, column group's warps, quarter of the rows, column)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int quarter = warp & 3, cg = warp >> 2;
+    constexpr int STAGES = TRAIN ? 7 : 4;
+    const int64_t m0 = (int64_t)blockIdx.x * 128;
+    const uint32_t sb = smem_u32(smem), bar = smem_u32(&bar_s);
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_s), 128);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // stage s: X W1^T, H1 W2^T, H2 W3^T, H3 W4^T, D4 W4, D3 W3, D2 W2.  Operand and result places (multiples of ACT; 4: D4):
+    // D3 takes X's, D2 H3's, D1 D3's
+    const uint32_t a_at = 0x3043210u, o_at = 0x0304321u;
+    auto place = [&](uint32_t code, int st) { return ((code >> (4 * st)) & 15u) * ACT; };
+    auto panels = [](int st) { return st == 0 ? NIN / 8 : st == 4 ? NOUT / 8 : NH / 8; };
+    auto width = [](int st) { return st == 3 ? NOUT : NH; };
+    auto load_w = [&](int st) {                // (a group of copies per stage, empty past the last)
+        if (st < STAGES) {
+            const bf16* w = st == 0 ? g.W1 : st == 1 ? g.W2 : st == 2 ? g.W3 : st == 3 ? g.W4 : st == 4 ? g.W4t : st == 5 ? g.W3t : g.W2t;
+            const uint32_t dst = sb + WBUF_AT + (st & 1) * ACT;
+            for (int q = tid; q < panels(st) * width(st); q += GT) cp_async16(dst + q * 16, w + (int64_t)q * 8);
+        }
+        cp_async_commit();
+    };
+    for (int q = tid; q < NIN / 8 * 128; q += GT) cp_async16(sb + q * 16, g.X + ((int64_t)(q >> 7) * g.xr + m0 + (q & 127)) * 8);
+    load_w(0);
+    load_w(1);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = tmem_s, trow = tmem + ((uint32_t)(quarter * 32) << 16);
+    const int64_t row = m0 + quarter * 32 + lane;
+    const bool live = row < g.rows_valid;
+    // columns of the result at `at` as rows: 8 x 8 blocks (panel, eight rows), transposed by the load, 128 bytes each
+    auto transpose_out = [&](uint32_t at, int np, bf16* dst) {
+        for (int b = warp * 4; b < np * 16; b += GT / 32 * 4) {
+            const int q = b + (lane >> 3);
+            uint32_t r[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                         : "r"(sb + at + (q >> 4) * 2048 + ((q & 15) * 8 + (lane & 7)) * 16)
+                         : "memory");
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int pe = (b + e) >> 4, ge = (b + e) & 15;
+                reinterpret_cast<uint32_t*>(dst + ((m0 >> 3) + ge) * (int64_t)(np * 64) + pe * 64)[lane] = r[e];
+            }
+        }
+    };
+    auto tdst = [&](int st) {
+        return st == 0 ? g.H1t : st == 1 ? g.H2t : st == 2 ? g.H3t : st == 3 ? g.D4t : st == 4 ? g.D3t : st == 5 ? g.D2t : g.D1t;
+    };
+    bool ok = true;
+#pragma unroll 1
+    for (int st = 0; st < STAGES; ++st) {
+        const int N = width(st), np = panels(st);
+        cp_async_wait<1>();                    // this stage's weights (the next stage's may be on their way)
+        fence_proxy_async();
+        __syncthreads();
+        if (tid == 0) {
+            fence_after_sync();
+            const uint32_t sA = sb + place(a_at, st), sB = sb + WBUF_AT + (st & 1) * ACT;
+            const uint32_t idesc = idesc_bf16_m128(N);
+            for (int q = 0; q < np / 2; ++q)
+                mma_bf16(tmem, sdesc(sA + q * 2 * 2048, 2048, 128), sdesc(sB + q * 2 * (N * 16), N * 16, 128), idesc, q > 0 ? 1u : 0u);
+            mma_commit(bar);
+        }
+        __syncwarp();
+        if (TRAIN && st > 0) transpose_out(place(o_at, st - 1), width(st - 1) / 8, tdst(st - 1));
+        if (!mbar_wait(bar, (uint32_t)(st & 1))) ok = false;
+        ok = __syncthreads_and(ok ? 1 : 0) != 0;
+        fence_after_sync();
+        if (!ok) {
+            if (tid == 0) atomicOr(g.err, 8);
+            mbar_wait(bar, (uint32_t)(st & 1));          // the product may still run: one more bounded wait
+            break;
+        }
+        load_w(st + 2);
+        const int mode = st < 3 ? E_TANH : st > 3 ? E_DTANH : TRAIN ? E_LOSS : E_OUT;
+        const float* bias = g.P + (st == 0 ? OFF_B1 : st == 1 ? OFF_B2 : st == 2 ? OFF_B3 : OFF_B4);
+        uint8_t* const orow = smem + place(o_at, st) + (quarter * 32 + lane) * 16;
+        const uint8_t* const hrow = smem + (7 - st) * ACT + (quarter * 32 + lane) * 16;      // (H3, H2, H1 of stages 4, 5, 6)
+        float lsum = 0.0f;
+        int half = 0;
+#pragma unroll 1
+        for (int c0 = cg * 16; c0 < N; c0 += 64, half ^= 1) {
+            float v[16], w[16];
+            tmem_ld16(trow + c0, v);
+            if (mode == E_OUT) {
+                if (live) {
+                    float* o = g.out + row * NOUT + c0;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = v[i] + bias[c0 + i];
+                }
+                continue;
+            }
+            if (mode == E_TANH) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i] = live ? tanhf(v[i] + bias[c0 + i]) : 0.0f;
+            } else if (mode == E_DTANH) {
+                const uint4 hv[2] = {*reinterpret_cast<const uint4*>(hrow + (c0 >> 3) * 2048),
+                                     *reinterpret_cast<const uint4*>(hrow + (c0 >> 3) * 2048 + 2048)};
+                const bf16* hb = reinterpret_cast<const bf16*>(hv);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float h = bf2f(hb[i]);
+                    w[i] = live ? v[i] * (1.0f - h * h) : 0.0f;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int n = c0 + i;
+                    float d = 0.0f;
+                    if (live && n < NOUT_USED) d = (v[i] + bias[n]) - g.tgt[row * 8 + n];
+                    lsum += d * d;
+                    w[i] = g.dscale * d;
+                }
+            }
+            bf16 wb[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) wb[i] = __float2bfloat16_rn(w[i]);
+            *reinterpret_cast<uint4*>(orow + (c0 >> 3) * 2048) = *reinterpret_cast<const uint4*>(wb);
+            *reinterpret_cast<uint4*>(orow + (c0 >> 3) * 2048 + 2048) = *reinterpret_cast<const uint4*>(wb + 8);
+            if (mode >= E_LOSS) {   // column sums of the bf16-rounded gradient, in a fixed order
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float x = bf2f(wb[i]);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+                    if (lane == 0) red[half][cg][quarter][i] = x;
+                }
+            }
+        }
+        if (mode == E_LOSS && cg == 0) {
+            float x = lsum;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == 0) red[1][0][quarter][0] = x;
+        }
+        fence_before_sync();
+        if (mode >= E_LOSS) {
+            __syncthreads();
+            float* bs = g.bsum + (int64_t)(6 - st) * gridDim.x * 128 + (int64_t)blockIdx.x * N;
+            if (tid < N) {
+                const float (*r)[16] = red[tid >> 6][(tid >> 4) & 3];
+                const int i = tid & 15;
+                bs[tid] = ((r[0][i] + r[1][i]) + r[2][i]) + r[3][i];
+            }
+            if (mode == E_LOSS && tid == 0)
+                g.lossp[blockIdx.x] = ((red[1][0][0][0] + red[1][0][1][0]) + red[1][0][2][0]) + red[1][0][3][0];
+        }
+    }
+    cp_async_wait<0>();
+    fence_before_sync();
+    __syncthreads();
+    if (TRAIN && ok) transpose_out(place(o_at, 6), NH / 8, g.D1t);
+    if (warp == 0) {
+        fence_after_sync();
+        tmem_dealloc(tmem, 128);
+    }
+}
+
+template <bool TRAIN>
+static int chain(const ChainP& g, int blocks, cudaStream_t s) {
+    DV_CUDA(dv::allow_dyn_smem((const void*)k_chain<TRAIN>));
+    DV_LAUNCH(dv::K_MLP, s, k_chain<TRAIN><<<blocks, GT, CHAIN_SMEM, s>>>(g));
+    return launch_ok("k_chain");
 }
 
 // ------------------------------------------------------------------------------------ features
@@ -409,121 +530,90 @@ __global__ void k_collect_grad(const float* __restrict__ part, const float* __re
     if (q < NPARAM) G[q] = param_grad(q, part, bsum);
 }
 
-__global__ void k_adam(float* __restrict__ P, const float* __restrict__ G, float* __restrict__ Mo, float* __restrict__ Vo,
-                       float lr, float b1, float b2, float eps, float c1, float c2) {
+// bf16 operand copies of parameter q: W (rows = outputs) and W^T (rows = inputs) panels
+struct Packed {
+    bf16 *W1, *W2, *W3, *W4, *W2t, *W3t, *W4t;
+};
+__device__ __forceinline__ void pack_param(const Packed& k, int64_t q, float p) {
+    const bf16 w = __float2bfloat16_rn(p);
+    if (q < OFF_B1) {
+        k.W1[pidx(q / NIN, q % NIN, NH)] = w;
+    } else if (q >= OFF_W2 && q < OFF_B2) {
+        const int m = (int)((q - OFF_W2) / NH), n = (int)((q - OFF_W2) % NH);
+        k.W2[pidx(m, n, NH)] = w;
+        k.W2t[pidx(n, m, NH)] = w;
+    } else if (q >= OFF_W3 && q < OFF_B3) {
+        const int m = (int)((q - OFF_W3) / NH), n = (int)((q - OFF_W3) % NH);
+        k.W3[pidx(m, n, NH)] = w;
+        k.W3t[pidx(n, m, NH)] = w;
+    } else if (q >= OFF_W4 && q < OFF_B4) {
+        const int o = (int)((q - OFF_W4) / NH), h = (int)((q - OFF_W4) % NH);
+        k.W4[pidx(o, h, NOUT)] = w;
+        k.W4t[pidx(h, o, NH)] = w;
+    }
+}
+
+// A training step's end: gradient, Adam and operand copies of each parameter.
+__global__ void k_update(const float* __restrict__ part, const float* __restrict__ bsum, float* __restrict__ P,
+                         float* __restrict__ Mo, float* __restrict__ Vo, float lr, float b1, float b2, float eps, float c1,
+                         float c2, Packed k) {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= NPARAM) return;
-    const float g = G[q];
+    const float g = param_grad(q, part, bsum);
     const float m = b1 * Mo[q] + (1.0f - b1) * g;
     const float v = b2 * Vo[q] + (1.0f - b2) * g * g;
     Mo[q] = m;
     Vo[q] = v;
-    P[q] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+    const float p = P[q] - lr * (m / c1) / (sqrtf(v / c2) + eps);
+    P[q] = p;
+    pack_param(k, q, p);
 }
 
-// bf16 operand copies of the fp32 parameters: W (rows = outputs) and W^T (rows = inputs) panels
-__global__ void k_pack_weights(const float* __restrict__ P, bf16* W1, bf16* W2, bf16* W3, bf16* W4, bf16* W2t, bf16* W3t,
-                               bf16* W4t) {
+__global__ void k_pack_weights(const float* __restrict__ P, Packed k) {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < (int64_t)NH * NIN) {
-        const int m = (int)(q / NIN), n = (int)(q % NIN);
-        W1[pidx(m, n, NH)] = __float2bfloat16_rn(P[OFF_W1 + q]);
-    }
-    if (q < (int64_t)NH * NH) {
-        const int m = (int)(q / NH), n = (int)(q % NH);
-        const bf16 a = __float2bfloat16_rn(P[OFF_W2 + q]), b = __float2bfloat16_rn(P[OFF_W3 + q]);
-        W2[pidx(m, n, NH)] = a;
-        W2t[pidx(n, m, NH)] = a;
-        W3[pidx(m, n, NH)] = b;
-        W3t[pidx(n, m, NH)] = b;
-    }
-    if (q < (int64_t)NOUT * NH) {
-        const int o = (int)(q / NH), h = (int)(q % NH);
-        const bf16 a = __float2bfloat16_rn(P[OFF_W4 + q]);
-        W4[pidx(o, h, NOUT)] = a;
-        W4t[pidx(h, o, NH)] = a;
-    }
+    if (q < NPARAM) pack_param(k, q, P[q]);
 }
 
 static unsigned g1(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
+static Packed packed(const dv_mlp* net) { return Packed{net->W1, net->W2, net->W3, net->W4, net->W2t, net->W3t, net->W4t}; }
+
 static int pack(dv_mlp* net, cudaStream_t s) {
-    // one thread per entry of the largest matrix (W2, W3: NH x NH)
-    const int64_t most = std::max<int64_t>((int64_t)NH * NIN, std::max<int64_t>((int64_t)NH * NH, (int64_t)NOUT * NH));
-    DV_LAUNCH(dv::K_MLP, s, k_pack_weights<<<g1(most), 256, 0, s>>>(net->P, net->W1, net->W2, net->W3, net->W4, net->W2t,
-                                                                     net->W3t, net->W4t));
+    DV_LAUNCH(dv::K_MLP, s, k_pack_weights<<<g1(NPARAM), 256, 0, s>>>(net->P, packed(net)));
     return launch_ok("k_pack_weights");
 }
 
-static GemmP base(dv_mlp* net) {
-    GemmP g;
+static ChainP chain_of(dv_mlp* net, const bf16* X, int64_t xr, int64_t rows_valid) {
+    ChainP g;
     memset(&g, 0, sizeof g);
-    g.err = net->d_err;
+    g.X = X; g.xr = xr; g.rows_valid = rows_valid; g.P = net->P; g.err = net->d_err;
+    g.W1 = net->W1; g.W2 = net->W2; g.W3 = net->W3; g.W4 = net->W4; g.W4t = net->W4t; g.W3t = net->W3t; g.W2t = net->W2t;
     return g;
 }
 
-// Forward + backward of one batch (rows of Xb/Xbt/Tb); leaves the gradient in net->G and the loss
-// partials in net->lossp.
-static int grad_batch(dv_mlp* net, int64_t rows_valid, cudaStream_t s) {
-    const int TB = NB / 128;
-    GemmP g = base(net);
-    g.rows_valid = rows_valid;
-    // H1 = tanh(X W1^T + b1)
-    g.A = net->Xb; g.ra = NB; g.B = net->W1; g.rb = NH; g.N = NH; g.kpanels = NIN / 8; g.mode = E_TANH;
-    g.bias = net->P + OFF_B1; g.orm = net->H1; g.orm_r = NB; g.ofm = net->H1t; g.ofm_r = NH;
-    DV_TRY(gemm(g, TB, s));
-    g.A = net->H1; g.B = net->W2; g.kpanels = NH / 8; g.bias = net->P + OFF_B2; g.orm = net->H2; g.ofm = net->H2t;
-    DV_TRY(gemm(g, TB, s));
-    g.A = net->H2; g.B = net->W3; g.bias = net->P + OFF_B3; g.orm = net->H3; g.ofm = net->H3t;
-    DV_TRY(gemm(g, TB, s));
-    // O = H3 W4^T + b4 ; D4 = dscale (O - T)
-    g.A = net->H3; g.B = net->W4; g.rb = NOUT; g.N = NOUT; g.mode = E_LOSS; g.bias = net->P + OFF_B4;
-    g.orm = net->D4; g.orm_r = NB; g.ofm = net->D4t; g.ofm_r = NOUT; g.tgt = net->Tb;
-    g.dscale = 2.0f / (float)((double)rows_valid * NOUT_USED);
-    g.lossp = net->lossp; g.bsum = net->bpart + 3 * TB * 128;
-    DV_TRY(gemm(g, TB, s));
-    // D3 = (D4 W4) (1 - H3^2) ; D2 ; D1
-    GemmP d = base(net);
-    d.rows_valid = rows_valid;
-    d.mode = E_DTANH; d.N = NH; d.orm_r = NB; d.ofm_r = NH; d.hd_r = NB;
-    d.A = net->D4; d.ra = NB; d.B = net->W4t; d.rb = NH; d.kpanels = NOUT / 8; d.hd = net->H3;
-    d.orm = net->D3; d.ofm = net->D3t; d.bsum = net->bpart + 2 * TB * 128;
-    DV_TRY(gemm(d, TB, s));
-    d.A = net->D3; d.B = net->W3t; d.kpanels = NH / 8; d.hd = net->H2; d.orm = net->D2; d.ofm = net->D2t;
-    d.bsum = net->bpart + 1 * TB * 128;
-    DV_TRY(gemm(d, TB, s));
-    d.A = net->D2; d.B = net->W2t; d.hd = net->H1; d.orm = net->D1; d.ofm = net->D1t; d.bsum = net->bpart;
-    DV_TRY(gemm(d, TB, s));
+// Forward + backward of one batch (rows of Xb/Xbt/Tb); leaves the weight-gradient partials in net->part, the
+// bias sums in net->bpart and the loss partials in lossp.
+static int grad_batch(dv_mlp* net, int64_t rows_valid, float* lossp, cudaStream_t s) {
+    ChainP g = chain_of(net, net->Xb, NB, rows_valid);
+    g.tgt = net->Tb; g.dscale = 2.0f / (float)((double)rows_valid * NOUT_USED);
+    g.lossp = lossp; g.bsum = net->bpart;
+    g.H1t = net->H1t; g.H2t = net->H2t; g.H3t = net->H3t; g.D4t = net->D4t; g.D3t = net->D3t; g.D2t = net->D2t; g.D1t = net->D1t;
+    DV_TRY(chain<true>(g, NB / 128, s));
     // weight gradients: K = samples split over NSPLIT CTAs each
     const int64_t PS = (int64_t)NSPLIT * 128 * 128;
-    GemmP w = base(net);
-    w.split = 1; w.mode = E_PART; w.kpanels = NB / 8 / NSPLIT;
-    w.A = net->D1t; w.ra = NH; w.B = net->Xbt; w.rb = NIN; w.N = NIN; w.of = net->part;
-    DV_TRY(gemm(w, NSPLIT, s));
-    w.A = net->D2t; w.B = net->H1t; w.rb = NH; w.N = NH; w.of = net->part + PS;
-    DV_TRY(gemm(w, NSPLIT, s));
-    w.A = net->D3t; w.B = net->H2t; w.of = net->part + 2 * PS;
-    DV_TRY(gemm(w, NSPLIT, s));
-    w.A = net->H3t; w.B = net->D4t; w.rb = NOUT; w.N = NOUT; w.of = net->part + 3 * PS;
-    DV_TRY(gemm(w, NSPLIT, s));
-    DV_LAUNCH(dv::K_MLP, s, k_collect_grad<<<g1(NPARAM), 256, 0, s>>>(net->part, net->bpart, net->G));
-    return launch_ok("k_collect_grad");
+    GemmBatch w;
+    w.per = NSPLIT; w.kpanels = NB / 8 / NSPLIT; w.split = 1; w.err = net->d_err;
+    w.p[0] = GemmP{net->D1t, NH, net->Xbt, NIN, NIN, net->part};
+    w.p[1] = GemmP{net->D2t, NH, net->H1t, NH, NH, net->part + PS};
+    w.p[2] = GemmP{net->D3t, NH, net->H2t, NH, NH, net->part + 2 * PS};
+    w.p[3] = GemmP{net->H3t, NH, net->D4t, NOUT, NOUT, net->part + 3 * PS};
+    return gemm(w, 4, s);
 }
 
 static int forward_rows(dv_mlp* net, const bf16* X, int64_t rows, int64_t rows_valid, float* out, cudaStream_t s) {
-    const int grid = (int)(rows / 128);
-    GemmP g = base(net);
-    g.rows_valid = rows_valid;
-    g.A = X; g.ra = rows; g.B = net->W1; g.rb = NH; g.N = NH; g.kpanels = NIN / 8; g.mode = E_TANH;
-    g.bias = net->P + OFF_B1; g.orm = net->Ha; g.orm_r = rows;
-    DV_TRY(gemm(g, grid, s));
-    g.A = net->Ha; g.B = net->W2; g.kpanels = NH / 8; g.bias = net->P + OFF_B2; g.orm = net->Hb;
-    DV_TRY(gemm(g, grid, s));
-    g.A = net->Hb; g.B = net->W3; g.bias = net->P + OFF_B3; g.orm = net->Ha;
-    DV_TRY(gemm(g, grid, s));
-    g.A = net->Ha; g.B = net->W4; g.rb = NOUT; g.N = NOUT; g.mode = E_OUT; g.bias = net->P + OFF_B4; g.orm = nullptr;
-    g.of = out; g.ldf = NOUT;
-    return gemm(g, grid, s);
+    ChainP g = chain_of(net, X, rows, rows_valid);
+    g.out = out;
+    return chain<false>(g, (int)(rows / 128), s);
 }
 
 int predict(dv_mlp* net, const StageInputs& in, const double* ytr, double* pred, cudaStream_t s) {
@@ -596,12 +686,12 @@ int dv_mlp_create(int64_t sample_capacity, uint64_t seed, dv_mlp** out) {
     A(&n->norm, NNORM);
     A(&n->Xs, std::max<int64_t>(n->cap, NB) * NIN); A(&n->Ts, std::max<int64_t>(n->cap, NB) * 8);
     A(&n->Xb, (int64_t)NB * NIN); A(&n->Xbt, (int64_t)NB * NIN); A(&n->Tb, (int64_t)NB * 8);
-    for (bf16** p : {&n->H1, &n->H2, &n->H3, &n->H1t, &n->H2t, &n->H3t, &n->D3, &n->D2, &n->D1, &n->D3t, &n->D2t, &n->D1t})
+    for (bf16** p : {&n->H1t, &n->H2t, &n->H3t, &n->D3t, &n->D2t, &n->D1t})
         A(p, (int64_t)NB * NH);
-    A(&n->D4, (int64_t)NB * NOUT); A(&n->D4t, (int64_t)NB * NOUT);
-    A(&n->part, 4LL * NSPLIT * 128 * 128); A(&n->bpart, 4LL * TB * 128); A(&n->lossp, TB);
+    A(&n->D4t, (int64_t)NB * NOUT);
+    A(&n->part, 4LL * NSPLIT * 128 * 128); A(&n->bpart, 4LL * TB * 128); A(&n->lossp, LOSS_KEEP * TB);
     A(&n->d_err, 1);
-    if (rc == DV_OK && cudaMallocHost((void**)&n->h_loss, sizeof(float) * TB) != cudaSuccess)
+    if (rc == DV_OK && cudaMallocHost((void**)&n->h_loss, sizeof(float) * LOSS_KEEP * TB) != cudaSuccess)
         rc = cuda_fail(cudaGetLastError(), "cudaMallocHost(mlp)");
     if (rc != DV_OK) { dv_mlp_destroy(n); return rc; }
     // initial parameters: uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) hidden weights, zero biases, zero output
@@ -631,8 +721,8 @@ int dv_mlp_destroy(dv_mlp* n) {
     std::lock_guard<std::recursive_mutex> lk_(dv::capture_mutex());
     if (!n) return DV_OK;
     void* ptrs[] = {n->P, n->G, n->Mo, n->Vo, n->W1, n->W2, n->W3, n->W4, n->W2t, n->W3t, n->W4t, n->norm, n->Xs, n->Ts,
-                    n->Xb, n->Xbt, n->H1, n->H2, n->H3, n->H1t, n->H2t, n->H3t, n->D4, n->D4t, n->D3, n->D2, n->D1,
-                    n->D3t, n->D2t, n->D1t, n->Tb, n->part, n->bpart, n->lossp, n->Xi, n->Ha, n->Hb, n->Oi, n->d_err};
+                    n->Xb, n->Xbt, n->H1t, n->H2t, n->H3t, n->D4t, n->D3t, n->D2t, n->D1t, n->Tb, n->part, n->bpart,
+                    n->lossp, n->Xi, n->Oi, n->d_err};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (n->h_loss) cudaFreeHost(n->h_loss);
@@ -644,14 +734,12 @@ int dv_mlp_reserve(dv_mlp* n, int64_t ncell) {
     if (!n || ncell <= 0) { set_error("dv_mlp_reserve: bad argument"); return DV_ERR_ARG; }
     const int64_t rows = (ncell + 127) / 128 * 128;
     if (rows <= n->inf_rows) return DV_OK;
-    for (void* p : {(void*)n->Xi, (void*)n->Ha, (void*)n->Hb, (void*)n->Oi})
+    for (void* p : {(void*)n->Xi, (void*)n->Oi})
         if (p) cudaFree(p);
-    n->Xi = n->Ha = n->Hb = nullptr;
+    n->Xi = nullptr;
     n->Oi = nullptr;
     n->inf_rows = 0;
     int rc = dalloc(&n->Xi, rows * NIN);
-    if (rc == DV_OK) rc = dalloc(&n->Ha, rows * NH);
-    if (rc == DV_OK) rc = dalloc(&n->Hb, rows * NH);
     if (rc == DV_OK) rc = dalloc(&n->Oi, rows * NOUT);
     if (rc == DV_OK) n->inf_rows = rows;
     return rc;
@@ -750,30 +838,28 @@ int dv_mlp_gemm_host(int32_t M, int32_t N, int32_t K, const float* A, const floa
     for (int64_t r = 0; r < N; ++r)
         for (int k = 0; k < K; ++k) bp[pidx(r, k, N)] = bb[r * K + k];
     bf16 *dA = nullptr, *dB = nullptr;
-    float *dD = nullptr, *dz = nullptr;
+    float* dD = nullptr;
     int* derr = nullptr;
     int rc = DV_OK;
     if (cudaMalloc((void**)&dA, ap.size() * 2) != cudaSuccess || cudaMalloc((void**)&dB, bp.size() * 2) != cudaSuccess ||
-        cudaMalloc((void**)&dD, sizeof(float) * (size_t)M * N) != cudaSuccess ||
-        cudaMalloc((void**)&dz, sizeof(float) * N) != cudaSuccess || cudaMalloc((void**)&derr, sizeof(int)) != cudaSuccess)
+        cudaMalloc((void**)&dD, sizeof(float) * (size_t)M * N) != cudaSuccess || cudaMalloc((void**)&derr, sizeof(int)) != cudaSuccess)
         rc = cuda_fail(cudaGetLastError(), "cudaMalloc(gemm check)");
     if (rc == DV_OK) {
         cudaMemcpy(dA, ap.data(), ap.size() * 2, cudaMemcpyHostToDevice);
         cudaMemcpy(dB, bp.data(), bp.size() * 2, cudaMemcpyHostToDevice);
-        cudaMemset(dz, 0, sizeof(float) * N);
         cudaMemset(derr, 0, sizeof(int));
-        GemmP g;
+        GemmBatch g;
         memset(&g, 0, sizeof g);
-        g.A = dA; g.ra = M; g.B = dB; g.rb = N; g.N = N; g.kpanels = K / 8; g.mode = E_OUT; g.rows_valid = M;
-        g.bias = dz; g.of = dD; g.ldf = N; g.err = derr;
-        rc = gemm(g, M / 128, 0);
+        g.p[0] = GemmP{dA, M, dB, N, N, dD};
+        g.per = M / 128; g.kpanels = K / 8; g.err = derr;
+        rc = gemm(g, 1, 0);
         if (rc == DV_OK && cudaDeviceSynchronize() != cudaSuccess) rc = cuda_fail(cudaGetLastError(), "k_gemm");
         int e = 0;
         if (rc == DV_OK) cudaMemcpy(&e, derr, sizeof(int), cudaMemcpyDeviceToHost);
         if (rc == DV_OK && e) { set_error("dv_mlp: a tensor-core product's completion wait timed out"); rc = DV_ERR_CUDA; }
         if (rc == DV_OK) cudaMemcpy(D, dD, sizeof(float) * (size_t)M * N, cudaMemcpyDeviceToHost);
     }
-    for (void* q : {(void*)dA, (void*)dB, (void*)dD, (void*)dz, (void*)derr})
+    for (void* q : {(void*)dA, (void*)dB, (void*)dD, (void*)derr})
         if (q) cudaFree(q);
     return rc;
 }
@@ -796,7 +882,9 @@ int dv_mlp_gradient_host(dv_mlp* n, const float* X, const float* T, int64_t rows
     DV_CUDA(cudaMemcpy(n->Xb, rm.data(), rm.size() * 2, cudaMemcpyHostToDevice));
     DV_CUDA(cudaMemcpy(n->Xbt, fm.data(), fm.size() * 2, cudaMemcpyHostToDevice));
     DV_CUDA(cudaMemcpy(n->Tb, tb.data(), tb.size() * 4, cudaMemcpyHostToDevice));
-    DV_TRY(grad_batch(n, rows, 0));
+    DV_TRY(grad_batch(n, rows, n->lossp, 0));
+    DV_LAUNCH(dv::K_MLP, 0, k_collect_grad<<<g1(NPARAM), 256, 0, 0>>>(n->part, n->bpart, n->G));
+    DV_TRY(launch_ok("k_collect_grad"));
     DV_CUDA(cudaMemcpy(grad, n->G, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
     std::vector<float> lp(NB / 128);
     DV_CUDA(cudaMemcpy(lp.data(), n->lossp, sizeof(float) * lp.size(), cudaMemcpyDeviceToHost));
@@ -834,19 +922,22 @@ int dv_mlp_train(dv_mlp* n, int32_t steps, float lr, uint64_t seed, int32_t keep
                                                                                     (int64_t)(seed & 0x7fffffffffffll),
                                                                                     n->adam_t, n->norm, n->Xb, n->Xbt, n->Tb));
         DV_CUDA(cudaGetLastError());
-        DV_TRY(grad_batch(n, NB, s));
+        const int slot = it % LOSS_KEEP;
+        DV_TRY(grad_batch(n, NB, n->lossp + slot * TB, s));
         n->adam_t += 1;
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.0f - std::pow(b1, (float)n->adam_t), c2 = 1.0f - std::pow(b2, (float)n->adam_t);
-        DV_LAUNCH(dv::K_MLP, s, k_adam<<<g1(NPARAM), 256, 0, s>>>(n->P, n->G, n->Mo, n->Vo, lr, b1, b2, 1e-8f, c1, c2));
+        DV_LAUNCH(dv::K_MLP, s, k_update<<<g1(NPARAM), 256, 0, s>>>(n->part, n->bpart, n->P, n->Mo, n->Vo, lr, b1, b2, 1e-8f, c1,
+                                                                   c2, packed(n)));
         DV_CUDA(cudaGetLastError());
-        DV_TRY(pack(n, s));
-        if (loss_hist) {
-            DV_CUDA(cudaMemcpyAsync(n->h_loss, n->lossp, sizeof(float) * TB, cudaMemcpyDeviceToHost, s));
+        if (loss_hist && (slot == LOSS_KEEP - 1 || it == steps - 1)) {      // the partial sums of up to LOSS_KEEP steps at once
+            DV_CUDA(cudaMemcpyAsync(n->h_loss, n->lossp, sizeof(float) * (slot + 1) * TB, cudaMemcpyDeviceToHost, s));
             DV_CUDA(cudaStreamSynchronize(s));
-            double t = 0.0;
-            for (int b = 0; b < TB; ++b) t += n->h_loss[b];
-            loss_hist[it] = (float)(t / ((double)NB * NOUT_USED));
+            for (int q = 0; q <= slot; ++q) {
+                double t = 0.0;
+                for (int b = 0; b < TB; ++b) t += n->h_loss[q * TB + b];
+                loss_hist[it - slot + q] = (float)(t / ((double)NB * NOUT_USED));
+            }
         }
     }
     DV_CUDA(cudaStreamSynchronize(s));

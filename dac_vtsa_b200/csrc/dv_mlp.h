@@ -12,6 +12,7 @@ namespace mlp {
 // used).  All widths are multiples of 16 (tcgen05 K and N granularity).
 constexpr int NIN = 112, NH = 128, NOUT = 16, NOUT_USED = 6, NFEAT = 97;
 constexpr int NB = 4096;       // training batch (samples)
+constexpr int LOSS_KEEP = 64;  // training steps whose loss partials are read back together
 constexpr int NSPLIT = 8;      // K splits of the weight-gradient products (NB / NSPLIT samples each)
 // parameter vector (fp32): W1 [NH x NIN], b1 [NH], W2 [NH x NH], b2, W3 [NH x NH], b3, W4 [NOUT x NH], b4 [NOUT]
 constexpr int64_t OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NIN, OFF_W2 = OFF_B1 + NH, OFF_B2 = OFF_W2 + NH * NH,
@@ -36,17 +37,16 @@ struct dv_mlp {
     float* Ts = nullptr;
     int64_t cap = 0, count = 0;
     // training batch buffers
-    __nv_bfloat16 *Xb = nullptr, *Xbt = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *H1t = nullptr,
-                  *H2t = nullptr, *H3t = nullptr, *D4 = nullptr, *D4t = nullptr, *D3 = nullptr, *D2 = nullptr,
-                  *D1 = nullptr, *D3t = nullptr, *D2t = nullptr, *D1t = nullptr;
+    __nv_bfloat16 *Xb = nullptr, *Xbt = nullptr, *H1t = nullptr, *H2t = nullptr, *H3t = nullptr, *D4t = nullptr,
+                  *D3t = nullptr, *D2t = nullptr, *D1t = nullptr;
     float *Tb = nullptr, *part = nullptr, *bpart = nullptr, *lossp = nullptr;
     // inference buffers (rows = cells rounded up to 128), sized by dv_mlp_reserve
     int64_t inf_rows = 0;
-    __nv_bfloat16 *Xi = nullptr, *Ha = nullptr, *Hb = nullptr;
+    __nv_bfloat16* Xi = nullptr;
     float* Oi = nullptr;
     int* d_err = nullptr;
     int64_t adam_t = 0;
-    float* h_loss = nullptr;                    // pinned: loss partials of the last step
+    float* h_loss = nullptr;                    // pinned: loss partials of the last LOSS_KEEP steps
 };
 
 namespace dv {

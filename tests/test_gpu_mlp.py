@@ -92,3 +92,21 @@ def test_training_reduces_the_loss_on_recorded_stage_solutions():
     assert np.all(np.isfinite(hist))
     first, last = float(np.mean(hist[:10])), float(np.mean(hist[-20:]))
     assert last < 0.5 * first, (first, last)
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 16, 16), (128, 112, 64), (256, 128, 400), (128, 48, 448), (384, 128, 1040)])
+def test_product_kernel_over_ring_and_remainders(M, N, K):
+    """The product kernel with fewer, as many and more 64-column chunks than it stages, and with a last chunk
+    of part of the columns: exact BF16 inputs, FP32 accumulation (error at most K steps of 2^-24 on the sum
+    of the magnitudes)."""
+    import ctypes as C
+    from dac_vtsa_b200 import _lib
+    rng = np.random.default_rng(M + N + K)
+    A, B = (rng.integers(-64, 65, s).astype(np.float32) / 64 for s in ((M, K), (N, K)))      # 7 bits: exact in BF16
+    A *= 2.0 ** rng.integers(-6, 7, (M, 1)).astype(np.float32)
+    D = np.full((M, N), np.nan, dtype=np.float32)
+    ptr = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    assert _lib.load().dv_mlp_gemm_host(M, N, K, ptr(A), ptr(B), ptr(D)) == 0
+    ref = A.astype(np.float64) @ B.astype(np.float64).T
+    bound = K * 2.0 ** -24 * (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T)
+    assert (np.abs(D - ref) <= bound + 2.0 ** -24 * np.abs(ref)).all()
