@@ -275,46 +275,173 @@ __global__ void k_sumsq(int64_t n, const double* __restrict__ a, const double* _
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// k_sumsq then k_finish in one launch: the block that finishes last (ticket) sums the partials
-// with k_finish's own strided loop and tree, so the result is the same to the bit
-__global__ void k_sumsq_finish(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
-                               double* __restrict__ part, unsigned* ticket, int mode, double* __restrict__ out) {
-    __shared__ double sh[VB];
-    __shared__ bool last;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double v = b ? a[i] / b[i] : a[i];
-        acc += v * v;
-    }
-    sh[threadIdx.x] = acc;
+// Sums over the VB threads of K values each, added like k_sumsq's tree (t + 128, 64, .. 1) but by a warp per
+// value, eight entries a lane and then the lanes: two barriers instead of nine a value.  Valid in every thread.
+template <int K>
+__device__ __forceinline__ void tree_sums(const double (&acc)[K], double (*sh)[VB], double* out) {
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < K; ++k) sh[k][t] = acc[k];
     __syncthreads();
-    for (int s = VB / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
+    if (t < 32 * K) {
+        const double* a = sh[t >> 5] + (t & 31);
+        double s = ((a[0] + a[128]) + (a[64] + a[192])) + ((a[32] + a[160]) + (a[96] + a[224]));
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, off);
+        if ((t & 31) == 0) out[t >> 5] = s;
     }
+    __syncthreads();
+}
+
+// k_sumsq and k_finish for K sums in one launch: the block that finishes last (ticket) sums the partials
+// with k_finish's own strided loop and tree, so the result is the same to the bit.  True in that block,
+// with the K totals in tot (shared).
+template <int K>
+__device__ __forceinline__ bool tree_finish(const double (&acc)[K], double* part, unsigned* ticket, double (*sh)[VB],
+                                            double* tot) {
+    __shared__ bool last;
+    tree_sums<K>(acc, sh, tot);
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = sh[0];
+#pragma unroll
+        for (int k = 0; k < K; ++k) part[(int64_t)k * gridDim.x + blockIdx.x] = tot[k];
         __threadfence();
         last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
-    if (!last) return;
+    if (!last) return false;
     __threadfence();
-    acc = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc += ((volatile const double*)part)[i];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = VB / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
+    double a[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        a[k] = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+            a[k] += ((volatile const double*)part)[(int64_t)k * gridDim.x + i];
     }
-    if (threadIdx.x == 0) {
-        double v = sh[0];
-        if (mode == 0) v = sqrt(v / (double)n);
-        else if (mode == 1) v = fmax(1.0, sqrt(v / (double)n));
-        else if (mode == 2) v = sqrt(v);
-        out[0] = v;
-        *ticket = 0u;
+    tree_sums<K>(a, sh, tot);
+    if (threadIdx.x == 0) *ticket = 0u;
+    return true;
+}
+__device__ __forceinline__ double finish_mode(double v, int64_t n, int mode) {
+    if (mode == 0) return sqrt(v / (double)n);
+    if (mode == 1) return fmax(1.0, sqrt(v / (double)n));
+    return mode == 2 ? sqrt(v) : v;
+}
+
+__global__ void __launch_bounds__(VB) k_sumsq_finish(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
+                                                     double* __restrict__ part, unsigned* ticket, int mode,
+                                                     double* __restrict__ out) {
+    __shared__ double sh[1][VB], tot[1];
+    double acc[1] = {0.0};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double v = b ? a[i] / b[i] : a[i];
+        acc[0] += v * v;
+    }
+    if (tree_finish<1>(acc, part, ticket, sh, tot) && threadIdx.x == 0) out[0] = finish_mode(tot[0], n, mode);
+}
+
+// ---- the vector work of a Newton iteration between its residuals and solves, one launch each time (the same
+// element-wise expressions and sums as a launch for each of them, which took 4 us apiece, most of it the
+// launches; with the solve that GMRES leaves, 200 -> 120 us of an iteration outside GMRES at 8x8x32)
+
+// The full step from the preconditioned solution u: dz = u s, zt = truncate(z + dz), rms(dz) and rms((zt - z) / s).
+__global__ void __launch_bounds__(VB) k_nk_step(int64_t n, int64_t npos, const double* __restrict__ u,
+                                                const double* __restrict__ s, const double* __restrict__ z,
+                                                double* __restrict__ dz, double* __restrict__ zt, double* __restrict__ part,
+                                                unsigned* ticket, double* __restrict__ o_dz, double* __restrict__ o_step) {
+    __shared__ double sh[2][VB], tot[2];
+    double acc[2] = {0.0, 0.0};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double si = s[i], zi = z[i], d = u[i] * si;
+        dz[i] = d;
+        acc[0] += d * d;
+        double v = zi + d;
+        if (i < npos) v = npmax(v, 0.1 * npmax(zi, 0.0));
+        zt[i] = v;
+        const double q = (v - zi) / si;
+        acc[1] += q * q;
+    }
+    if (tree_finish<2>(acc, part, ticket, sh, tot) && threadIdx.x == 0) {
+        *o_dz = finish_mode(tot[0], n, 0);
+        *o_step = finish_mode(tot[1], n, 0);
+    }
+}
+
+// Stage residual R = z - dh f - known.  A trial point: rms(R / s) and its own scale w.  FIRST, the start of
+// a stage solve: the scale s of z itself, rms(R / s), max(1, rms(z / s)) and GMRES's right-hand side b = -R / s.
+template <bool FIRST>
+__global__ void __launch_bounds__(VB) k_nk_residual(int64_t nc, int64_t n, const double* __restrict__ z,
+                                                    const double* __restrict__ f, const double* __restrict__ known,
+                                                    double dh, const double* __restrict__ atol7, double rtol,
+                                                    double* __restrict__ R, double* s, double* __restrict__ w,
+                                                    double* __restrict__ b, double* __restrict__ part, unsigned* ticket,
+                                                    double* __restrict__ o_res, double* __restrict__ o_zs) {
+    constexpr int K = FIRST ? 2 : 1;
+    __shared__ double sh[K][VB], tot[K];
+    double acc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double zi = z[i], r = (zi + -dh * f[i]) - known[i];
+        R[i] = r;
+        int v = (int)(i / nc);
+        if (v > DV_NV) v = DV_NV;
+        const double own = atol7[v] + rtol * fabs(zi);
+        double si;
+        if (FIRST) {
+            s[i] = si = own;
+            b[i] = -r / si;
+            const double q = zi / si;
+            acc[K - 1] += q * q;
+        } else {
+            si = s[i];
+            w[i] = own;
+        }
+        const double q = r / si;
+        acc[0] += q * q;
+    }
+    if (tree_finish<K>(acc, part, ticket, sh, tot) && threadIdx.x == 0) {
+        *o_res = finish_mode(tot[0], n, 0);
+        if (FIRST) *o_zs = finish_mode(tot[K - 1], n, 1);
+    }
+}
+
+// Accept the trial point (z, f, R <- zt, ft, Rt) and prepare the next iteration: s, b = -R / s, max(1, rms(z / s)).
+__global__ void __launch_bounds__(VB) k_nk_accept(int64_t nc, int64_t n, const double* __restrict__ zt,
+                                                  const double* __restrict__ ft, const double* __restrict__ Rt,
+                                                  const double* __restrict__ atol7, double rtol, double* __restrict__ z,
+                                                  double* __restrict__ f, double* __restrict__ R, double* __restrict__ s,
+                                                  double* __restrict__ b, double* __restrict__ part, unsigned* ticket,
+                                                  double* __restrict__ o_zs) {
+    __shared__ double sh[1][VB], tot[1];
+    double acc[1] = {0.0};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double zi = zt[i], r = Rt[i];
+        z[i] = zi;
+        f[i] = ft[i];
+        R[i] = r;
+        int v = (int)(i / nc);
+        if (v > DV_NV) v = DV_NV;
+        const double si = atol7[v] + rtol * fabs(zi);
+        s[i] = si;
+        b[i] = -r / si;
+        const double q = zi / si;
+        acc[0] += q * q;
+    }
+    if (tree_finish<1>(acc, part, ticket, sh, tot) && threadIdx.x == 0) *o_zs = finish_mode(tot[0], n, 1);
+}
+
+// Accept the trial point of a converged iteration; best and out (where given) take zt too.
+__global__ void __launch_bounds__(VB) k_nk_keep(int64_t n, const double* __restrict__ zt, const double* __restrict__ ft,
+                                                const double* __restrict__ Rt, double* __restrict__ z,
+                                                double* __restrict__ f, double* __restrict__ R, double* __restrict__ best,
+                                                double* __restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double v = zt[i];
+        z[i] = v;
+        f[i] = ft[i];
+        R[i] = Rt[i];
+        if (best) best[i] = v;
+        if (out) out[i] = v;
     }
 }
 
@@ -1962,19 +2089,18 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
     // Queue the evaluation of the full Newton step from the GMRES solution W.x: dz, the trial point
     // at lam = 1 with its stage residual, and the scalars the host tests (rms(dz), rms(R/s), the
     // preconditioned norm, the step length, the balance sums); copy them into W.hpin[16..47].
-    auto speculate = [&]() -> int {
-        DV_TRY(precond_apply(m, W.x, W.s, W.u, st));
-        DV_LAUNCH(dv::K_VECTOR, st, k_mul<<<g, VB, 0, st>>>(n, W.u, W.s, W.dz));
-        DV_TRY(rms_ratio_dev(W, n, W.dz, nullptr, 0, W.scal + 11, st));
-        DV_LAUNCH(dv::K_VECTOR, st, k_truncate<<<g, VB, 0, st>>>(n, C.npos, W.z, 1.0, W.dz, W.zt));
-        DV_TRY(stage(W.zt, W.ft, W.Rt));
-        DV_TRY(rms_ratio_dev(W, n, W.Rt, W.s, 0, W.scal + 12, st));
+    // have_u: W.u = P^-1 x is there (the GMRES graph's last solve, for its true residual).
+    auto speculate = [&](bool have_u) -> int {
+        if (!have_u) DV_TRY(precond_apply(m, W.x, W.s, W.u, st));
+        DV_LAUNCH(dv::K_VECTOR, st, k_nk_step<<<g, VB, 0, st>>>(n, C.npos, W.u, W.s, W.z, W.dz, W.zt, W.part, W.tickets + 6,
+                                                                W.scal + 11, W.scal + 14));
+        DV_TRY(launch_rhs(m, t, W.zt, W.ft, nullptr, st));
+        DV_LAUNCH(dv::K_VECTOR, st, k_nk_residual<false><<<g, VB, 0, st>>>(m->nc, n, W.zt, W.ft, rhs_known, dh, C.atol7, rtol,
+                                                                           W.Rt, W.s, W.w, nullptr, W.part, W.tickets + 6,
+                                                                           W.scal + 12, nullptr));
         DV_TRY(precond_apply(m, W.Rt, nullptr, W.tmp, st));
         DV_TRY(rms_ratio_dev(W, n, W.tmp, W.s, 0, W.scal + 13, st));
-        DV_LAUNCH(dv::K_VECTOR, st, k_axpby<<<g, VB, 0, st>>>(n, 1.0, W.zt, -1.0, W.z, W.r));
-        DV_TRY(rms_ratio_dev(W, n, W.r, W.s, 0, W.scal + 14, st));
         if (C.o.cons_tol > 0.0) {
-            scale(W.zt, W.w);
             // into scal[16..23]: scal[0..1] still feed the matvec of a GMRES rerun after a refresh
             DV_LAUNCH(dv::K_VECTOR, st, k_cons<<<cons_grid(m->nc), VB, 0, st>>>(m->p, W.Rt, W.w, W.apart, W.tickets + 5,
                                                                                   W.scal + 16));
@@ -1984,14 +2110,16 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
     };
 
     DV_TRY(copy(z0, W.z));
-    DV_TRY(stage(W.z, W.f, W.R));
-    scale(W.z, W.s);
-    // rms(R/s) and the preconditioned norm of R, queued into scal[24..25]: they come back with the
+    DV_TRY(launch_rhs(m, t, W.z, W.f, nullptr, st));
+    // R, and with it rms(R/s) and the preconditioned norm of R, queued into scal[24..25]: they come back with the
     // first iteration's speculated scalars (one synchronisation fewer per stage solve and per
     // norm); a non-finite rms then returns z0 as before, with the counters of that iteration undone
-    DV_TRY(rms_ratio_dev(W, n, W.R, W.s, 0, W.scal + 24, st));
+    DV_LAUNCH(dv::K_VECTOR, st, k_nk_residual<true><<<g, VB, 0, st>>>(m->nc, n, W.z, W.f, rhs_known, dh, C.atol7, rtol, W.R,
+                                                                      W.s, nullptr, W.b, W.part, W.tickets + 6, W.scal + 24,
+                                                                      W.scal + 1));
     DV_TRY(precond_apply(m, W.R, nullptr, W.tmp, st));
     DV_TRY(rms_ratio_dev(W, n, W.tmp, W.s, 0, W.scal + 25, st));
+    bool prepared = true;        // s, b and max(1, rms(z/s)) of the next iteration are there
     double rn = 0.0, pn = 0.0;
     const int64_t nfev0 = m->nfev;
     double step_prev = -1.0;     // < 0 : None
@@ -2004,9 +2132,12 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
     const double sqrt_n = std::sqrt((double)n);
     while (it + 1 < C.o.max_iter + polish) {
         ++it;
-        scale(W.z, W.s);
-        DV_LAUNCH(dv::K_VECTOR, st, k_div<<<g, VB, 0, st>>>(n, -1.0, W.R, W.s, W.b));                    // b = -R/s
-        DV_TRY(rms_ratio_dev(W, n, W.z, W.s, 1, W.scal + 1, st));           // zs = max(1, rms(z/s))
+        if (!prepared) {
+            scale(W.z, W.s);
+            DV_LAUNCH(dv::K_VECTOR, st, k_div<<<g, VB, 0, st>>>(n, -1.0, W.R, W.s, W.b));                // b = -R/s
+            DV_TRY(rms_ratio_dev(W, n, W.z, W.s, 1, W.scal + 1, st));       // zs = max(1, rms(z/s))
+        }
+        prepared = false;
         Op op{m, t, dh, W.z, W.f, W.s, n};
         const double floor_ = (polish ? 1e-4 : 0.1 * kappa) * sqrt_n;
         int info = 0;
@@ -2015,7 +2146,7 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
         DV_TRY(gmres_start(W, op, W.b, polish ? 1e-3 : C.o.eta, floor_, C.o.krylov_dim, &info, &inner, &pending, st));
         // the full step (lam = 1) and every norm the host tests next, queued behind GMRES, read
         // back with one synchronisation (same kernels and inputs as evaluating them one by one)
-        DV_TRY(speculate());
+        DV_TRY(speculate(pending));
         DV_CUDA(cudaStreamSynchronize(st));
         if (pending) DV_TRY(gmres_graph_collect(W, m, &info, &inner));
         if (it == 0) {                                       // the norms queued before the loop
@@ -2074,7 +2205,7 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
             DV_TRY(copy(W.tmp, W.b));
         }
         if (!spec_ok) {
-            DV_TRY(speculate());
+            DV_TRY(speculate(false));
             DV_CUDA(cudaStreamSynchronize(st));
         }
         const double* sv = W.hpin + 16;                      // speculated scalars (see speculate)
@@ -2116,10 +2247,6 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
             DV_TRY(rms_ratio(W, n, W.tmp, W.s, &step, st));
         }
         const bool cons_spec = (lam == 1.0);
-        // accept the trial point (copies, not pointer swaps: the GMRES graph is built on these addresses)
-        DV_TRY(copy(W.zt, W.z));
-        DV_TRY(copy(W.ft, W.f));
-        DV_TRY(copy(W.Rt, W.R));
         rn = rn_try;
         pn = pn_try;
         const double rate = (step_prev < 0.0) ? 0.0 : step / std::max(step_prev, 1e-300);
@@ -2127,17 +2254,23 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
         const bool converged = (lam == 1.0 && step <= kappa && (info == 0 || sp)) ||
                                (sp && lam == 1.0 && info == 0 && rate < 1.0 && rate / (1.0 - rate) * step <= kappa) ||
                                pn <= kappa;
+        // accept the trial point (copies, not pointer swaps: the GMRES graph is built on these addresses)
+        auto keep = [&](double* best, double* out) {
+            DV_LAUNCH(dv::K_VECTOR, st, k_nk_keep<<<g, VB, 0, st>>>(n, W.zt, W.ft, W.Rt, W.z, W.f, W.R, best, out));
+        };
         if (converged) {
-            if (!have_best || rn < best_rn) {
+            const bool better = !have_best || rn < best_rn;
+            if (better) {
                 have_best = true;
                 best_rn = rn;
-                DV_TRY(copy(W.z, W.best));
             }
-            bool ok;
-            if (cons_spec) ok = cons_eval(sv + 16);
-            else DV_TRY(cons_ok(W.R, W.z, &ok));
+            bool ok = cons_spec && cons_eval(sv + 16);
+            keep(better ? W.best : nullptr, ok ? zout : nullptr);
+            if (!cons_spec) {
+                DV_TRY(cons_ok(W.R, W.z, &ok));
+                if (ok) DV_TRY(copy(W.z, zout));
+            }
             if (ok) {
-                DV_TRY(copy(W.z, zout));
                 r.ok = 1; r.iters = it + 1; r.rate = rate;
                 return DV_OK;
             }
@@ -2167,11 +2300,15 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
             return DV_OK;
         }
         if (have_best) {
+            keep(nullptr, nullptr);
             r.balance_unclosed += 1;
             DV_TRY(return_best());
             r.ok = 1; r.iters = it + 1; r.rate = rate;
             return DV_OK;
         }
+        DV_LAUNCH(dv::K_VECTOR, st, k_nk_accept<<<g, VB, 0, st>>>(m->nc, n, W.zt, W.ft, W.Rt, C.atol7, rtol, W.z, W.f, W.R, W.s,
+                                                                  W.b, W.part, W.tickets + 6, W.scal + 1));
+        prepared = true;
         if (sp && lam == 1.0 && info == 0) {
             const int left = C.o.max_iter - it - 1;
             if (it >= 2 && (rate >= 1.0 || std::pow(rate, left) / (1.0 - rate) * step > kappa * 1e3)) {

@@ -521,6 +521,28 @@ def _cgs_stage(Nr, Nth, Nz):
     return stats["gmres_iters"], (z.cpu().numpy() - y) / (m.atol + m.cfg.solver.rtol * np.abs(y))
 
 
+@pytest.mark.parametrize("Nr,Nth,Nz,dh", [(1, 1, 3, 0.01), (2, 3, 5, 0.01), (3, 5, 7, 0.01), (4, 4, 16, 1e-4),
+                                          (8, 8, 33, 1e-4)])
+def test_newton_iterations_at_sizes_off_the_block_size(Nr, Nth, Nz, dh):
+    """Stage solves of fewer unknowns than one block of the vector kernels, and of counts that no block size
+    divides: the returned state solves the stage.  A converged iteration's step is at most kappa in error
+    scales, and the error left after it, measured as the preconditioned residual, is smaller than the step."""
+    import torch
+    from dac_vtsa_b200.jacobian import FDJacobian
+    m, y = _pc_model(Nz, Nr, Nth)
+    yd = torch.from_numpy(np.ascontiguousarray(y)).to(m.device)
+    kappa = 0.01
+    m.precond_factor(FDJacobian(m).block(0.0, yd), dh)
+    z, ok, iters, rate, _ = m.newton_stage(dh, yd, yd, dh, kappa=kappa, cons_tol=0.0)
+    assert ok and iters >= 1
+    R = m.stage_residual(dh, z, dh, yd)
+    s = torch.from_numpy(m.atol).to(m.device) + m.cfg.solver.rtol * z.abs()
+    pn = float(((m.precond_solve(R) / s) ** 2).mean().sqrt())
+    assert pn <= kappa, pn
+    npos = 5 * m.grid.ncell
+    assert bool((z[:npos] >= 0.1 ** iters * yd[:npos].clamp(min=0.0)).all())
+
+
 def test_cooperative_gram_schmidt_at_every_element_count(tmp_path):
     """The one-launch Gram-Schmidt gives the same bits whether a thread's elements stay in registers (one to
     three of them) or in memory (DVTSA_GMRES_COOP=2), and, where the block partition is the same (one element
