@@ -524,7 +524,8 @@ __global__ void k_combine(int64_t n, int m, const double* __restrict__ V, int64_
 // block sums in block order (deterministic) and resets the ticket.
 __global__ void __launch_bounds__(VB) k_cons(dv_step_params p, const double* __restrict__ R,
                                              const double* __restrict__ s, double* __restrict__ part,
-                                             unsigned* ticket, double* __restrict__ out) {
+                                             unsigned* ticket, double* out, const double* all = nullptr,
+                                             double* host = nullptr) {
     __shared__ double sh[VB / 32][8];
     __shared__ bool last;
     const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz, nw = p.wall_on ? (int64_t)p.Nth * p.Nz : 0;
@@ -571,6 +572,10 @@ __global__ void __launch_bounds__(VB) k_cons(dv_step_params p, const double* __r
     if (last && threadIdx.x < 8) {
         __threadfence();
         out[threadIdx.x] = sum_partials(part + threadIdx.x, (int)gridDim.x, 8);
+    }
+    if (last && host && threadIdx.x < 32) {      // 32 scalars, these eight among them, to pinned memory
+        __syncwarp();
+        host[threadIdx.x] = ((volatile const double*)all)[threadIdx.x];
     }
     if (last && threadIdx.x == 0) *ticket = 0u;
 }
@@ -1594,19 +1599,25 @@ __global__ void __launch_bounds__(VB) k_combine_gm(int64_t n, const GmDev* __res
     }
 }
 
-__global__ void k_gm_info(GmDev* st, const double* __restrict__ scal) {
-    if (threadIdx.x != 0) return;
-    const double rnorm = scal[10];
-    st->rnorm = rnorm;
-    st->info = st->skip ? 0 : ((rnorm <= st->atol_eff) ? 0 : 1);
-}
-
-// Host view of the results read back after a graph run.
+// Host view of the results of a graph run (pinned; written by k_gm_info itself: as two copies behind
+// the graph they took 14 us of an iteration).
 struct GmHost {
     double args[4];               // t, dh, rtol, atol
     int res[6];                   // col, done, skip, iters, info, ncomb
     int err;                      // the model's device error word, read back with the results
 };
+
+__global__ void k_gm_info(GmDev* st, const double* __restrict__ scal, const int* __restrict__ err, GmHost* host) {
+    if (threadIdx.x != 0) return;
+    const double rnorm = scal[10];
+    st->rnorm = rnorm;
+    const int info = st->skip ? 0 : ((rnorm <= st->atol_eff) ? 0 : 1);
+    st->info = info;
+    const int res[6] = {st->col, st->done, st->skip, st->iters, info, st->ncomb};
+#pragma unroll
+    for (int q = 0; q < 6; ++q) host->res[q] = res[q];
+    host->err = *err;
+}
 
 // Arnoldi steps captured ahead of the WHILE node: GM_PREFIX, or DVTSA_GMRES_PREFIX=<0..8> from the
 // environment (read once per process; a tuning knob: more steps save WHILE relaunches of long
@@ -1825,7 +1836,7 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
         op_count(m, fixed);
         k_axpby<<<g, VB, 0, cs>>>(n, 1.0, W.b, -1.0, W.r, W.r);
         k_sumsq_finish<<<g, VB, 0, cs>>>(n, W.r, nullptr, W.part, W.tickets + 6, 2, W.scal + 10);
-        k_gm_info<<<1, 32, 0, cs>>>(st, W.scal);
+        k_gm_info<<<1, 32, 0, cs>>>(st, W.scal, m->d_err, (GmHost*)W.gm_host);
         fixed[K_VECTOR] += 3;
         if (rc != DV_OK) e = cudaErrorUnknown;
     }
@@ -1892,8 +1903,6 @@ static int gmres_graph(Work& W, const Op& op, const double* b, double rtol, doub
     GmDev* dev = (GmDev*)W.gm;
     DV_CUDA(cudaMemcpyAsync(dev, hst->args, sizeof(hst->args), cudaMemcpyHostToDevice, st));
     DV_CUDA(cudaGraphLaunch(W.gm_exec, st));
-    DV_CUDA(cudaMemcpyAsync(hst->res, &dev->col, sizeof(hst->res), cudaMemcpyDeviceToHost, st));
-    DV_CUDA(cudaMemcpyAsync(&hst->err, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     return DV_OK;
 }
 
@@ -2088,7 +2097,7 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
     };
     // Queue the evaluation of the full Newton step from the GMRES solution W.x: dz, the trial point
     // at lam = 1 with its stage residual, and the scalars the host tests (rms(dz), rms(R/s), the
-    // preconditioned norm, the step length, the balance sums); copy them into W.hpin[16..47].
+    // preconditioned norm, the step length, the balance sums), which end up in W.hpin[16..47].
     // have_u: W.u = P^-1 x is there (the GMRES graph's last solve, for its true residual).
     auto speculate = [&](bool have_u) -> int {
         if (!have_u) DV_TRY(precond_apply(m, W.x, W.s, W.u, st));
@@ -2103,9 +2112,10 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
         if (C.o.cons_tol > 0.0) {
             // into scal[16..23]: scal[0..1] still feed the matvec of a GMRES rerun after a refresh
             DV_LAUNCH(dv::K_VECTOR, st, k_cons<<<cons_grid(m->nc), VB, 0, st>>>(m->p, W.Rt, W.w, W.apart, W.tickets + 5,
-                                                                                  W.scal + 16));
+                                                                                  W.scal + 16, W.scal, W.hpin + 16));
+        } else {
+            DV_CUDA(cudaMemcpyAsync(W.hpin + 16, W.scal, sizeof(double) * 32, cudaMemcpyDeviceToHost, st));
         }
-        DV_CUDA(cudaMemcpyAsync(W.hpin + 16, W.scal, sizeof(double) * 32, cudaMemcpyDeviceToHost, st));
         return DV_OK;
     };
 
