@@ -156,17 +156,33 @@ static int gemm(const GemmBatch& g, int products, cudaStream_t s) {
     return launch_ok("k_gemm");
 }
 
+__device__ __forceinline__ uint64_t mix64(uint64_t x) {
+    x ^= x >> 30;
+    x *= 0xbf58476d1ce4e5b9ull;
+    x ^= x >> 27;
+    x *= 0x94d049bb133111ebull;
+    x ^= x >> 31;
+    return x;
+}
+
 // ------------------------------------------------------------------------------------ the chain of a row tile
 // The whole chain of 128 rows in one block: forward (TRAIN 0: X -> O), or forward, loss and backward down to D1.
 // Nothing in it crosses rows, so an activation stays in shared memory as the next product's operand
 // (and for 1 - H^2), weights arrive two products ahead, and a training step's products leave only what the weight
 // gradients read: H and D with rows = features, written 128 bytes at a time while the next product runs.
-// Bound by latency, seven times product, epilogue, barrier, on 32 SMs for 4096 rows: 31 us, where a launch for each
-// product with 128 threads and every activation through L2 in both layouts took 97.
+// Bound by latency, seven times product, epilogue, barrier, on 32 SMs for 4096 rows: 34 us with the drawing of the
+// batch, where a launch for each product with 128 threads and every activation through L2 in both layouts took 97
+// and the drawing another 6.
 enum { E_TANH = 0, E_OUT = 1, E_LOSS = 2, E_DTANH = 3 };
 struct ChainP {
     const bf16* X;        // rows x NIN, panel layout of xr rows
     int64_t xr;
+    // a batch drawn from the recorded samples (else null): row j is sample hash(seed, step, j) mod count of X, its
+    // targets Ts scaled and clipped by nrm, X^T written for the first weight gradient
+    const float* Ts;
+    const double* nrm;
+    int64_t count, seed, step;
+    bf16* Xbt;
     const bf16 *W1, *W2, *W3, *W4, *W4t, *W3t, *W2t;
     const float* P;       // parameters (biases)
     int64_t rows_valid;   // rows at or beyond this are zero in every output and carry no loss
@@ -186,6 +202,7 @@ __global__ void __launch_bounds__(GT) k_chain(ChainP g) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar_s;
     __shared__ uint32_t tmem_s;
+    __shared__ int64_t sample[128];
     __shared__ float red[2][4][4][16];         // (group of columns, column group's warps, quarter of the rows, column)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quarter = warp & 3, cg = warp >> 2;
@@ -211,7 +228,15 @@ __global__ void __launch_bounds__(GT) k_chain(ChainP g) {
         }
         cp_async_commit();
     };
-    for (int q = tid; q < NIN / 8 * 128; q += GT) cp_async16(sb + q * 16, g.X + ((int64_t)(q >> 7) * g.xr + m0 + (q & 127)) * 8);
+    const bool drawn = TRAIN && g.Ts != nullptr;
+    if (drawn) {
+        if (tid < 128)
+            sample[tid] = (int64_t)(mix64((uint64_t)g.seed * 0x9e3779b97f4a7c15ull + (uint64_t)g.step * 1000003ull +
+                                          (uint64_t)(m0 + tid)) % (uint64_t)g.count);
+        __syncthreads();
+    }
+    for (int q = tid; q < NIN / 8 * 128; q += GT)
+        cp_async16(sb + q * 16, g.X + ((int64_t)(q >> 7) * g.xr + (drawn ? sample[q & 127] : m0 + (q & 127))) * 8);
     load_w(0);
     load_w(1);
     fence_before_sync();
@@ -255,6 +280,7 @@ __global__ void __launch_bounds__(GT) k_chain(ChainP g) {
             mma_commit(bar);
         }
         __syncwarp();
+        if (drawn && st == 0) transpose_out(0, NIN / 8, g.Xbt);
         if (TRAIN && st > 0) transpose_out(place(o_at, st - 1), width(st - 1) / 8, tdst(st - 1));
         if (!mbar_wait(bar, (uint32_t)(st & 1))) ok = false;
         ok = __syncthreads_and(ok ? 1 : 0) != 0;
@@ -296,11 +322,17 @@ __global__ void __launch_bounds__(GT) k_chain(ChainP g) {
                     w[i] = live ? v[i] * (1.0f - h * h) : 0.0f;
                 }
             } else {
+                const int64_t sj = drawn ? sample[quarter * 32 + lane] : row;
+                const double clip = drawn ? g.nrm[19] : 0.0;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const int n = c0 + i;
                     float d = 0.0f;
-                    if (live && n < NOUT_USED) d = (v[i] + bias[n]) - g.tgt[row * 8 + n];
+                    if (live && n < NOUT_USED) {
+                        const float tgt = drawn ? (float)fmax(-clip, fmin(clip, (double)g.Ts[sj * 8 + n] / g.nrm[13 + n]))
+                                                : g.tgt[row * 8 + n];
+                        d = (v[i] + bias[n]) - tgt;
+                    }
                     lsum += d * d;
                     w[i] = g.dscale * d;
                 }
@@ -463,41 +495,6 @@ __global__ void k_targets(StageInputs in, const double* __restrict__ zs, const d
 }
 
 // ------------------------------------------------------------------------------------ training
-__device__ __forceinline__ uint64_t mix64(uint64_t x) {
-    x ^= x >> 30;
-    x *= 0xbf58476d1ce4e5b9ull;
-    x ^= x >> 27;
-    x *= 0x94d049bb133111ebull;
-    x ^= x >> 31;
-    return x;
-}
-
-// Batch rows j < NB: sample idx(j) (a hash of seed, step and j, or j itself when seed < 0) copied in
-// both layouts, targets scaled by the output scales and clipped.
-__global__ void k_gather(const bf16* __restrict__ Xs, int64_t cap, const float* __restrict__ Ts, int64_t count,
-                         int64_t seed, int64_t step, const double* __restrict__ nrm, bf16* __restrict__ Xb,
-                         bf16* __restrict__ Xbt, float* __restrict__ Tb) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)NB * (NIN / 8)) return;
-    const int64_t j = t / (NIN / 8);
-    const int p = (int)(t - j * (NIN / 8));
-    const int64_t s = seed < 0 ? j : (int64_t)(mix64((uint64_t)seed * 0x9e3779b97f4a7c15ull + (uint64_t)step * 1000003ull +
-                                                     (uint64_t)j) % (uint64_t)count);
-    const uint4 v = *reinterpret_cast<const uint4*>(Xs + pidx(s, p * 8, cap));
-    *reinterpret_cast<uint4*>(Xb + pidx(j, p * 8, NB)) = v;
-    const bf16* e = reinterpret_cast<const bf16*>(&v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) Xbt[pidx(p * 8 + q, j, NIN)] = e[q];
-    if (p == 0) {
-        const double clip = nrm[19];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            float x = q < NOUT_USED ? (float)fmax(-clip, fmin(clip, (double)Ts[s * 8 + q] / nrm[13 + q])) : 0.0f;
-            Tb[j * 8 + q] = x;
-        }
-    }
-}
-
 // Gradient of parameter q: the weight-gradient partials (or the bias column sums) summed in CTA order.
 __device__ float param_grad(int64_t q, const float* __restrict__ part, const float* __restrict__ bsum) {
     // part: [4 products][NSPLIT][128][128] ; bsum: [4 layers][NB/128][128]
@@ -591,11 +588,15 @@ static ChainP chain_of(dv_mlp* net, const bf16* X, int64_t xr, int64_t rows_vali
     return g;
 }
 
-// Forward + backward of one batch (rows of Xb/Xbt/Tb); leaves the weight-gradient partials in net->part, the
-// bias sums in net->bpart and the loss partials in lossp.
-static int grad_batch(dv_mlp* net, int64_t rows_valid, float* lossp, cudaStream_t s) {
-    ChainP g = chain_of(net, net->Xb, NB, rows_valid);
-    g.tgt = net->Tb; g.dscale = 2.0f / (float)((double)rows_valid * NOUT_USED);
+// Forward + backward of one batch (draw < 0: the rows of Xb/Xbt/Tb; else step `draw` of the batches drawn from
+// the recorded samples with `seed`); leaves the weight-gradient partials in net->part, the bias sums in
+// net->bpart and the loss partials in lossp.
+static int grad_batch(dv_mlp* net, int64_t rows_valid, int64_t seed, int64_t draw, float* lossp, cudaStream_t s) {
+    ChainP g = draw < 0 ? chain_of(net, net->Xb, NB, rows_valid) : chain_of(net, net->Xs, net->cap, rows_valid);
+    if (draw >= 0) {
+        g.Ts = net->Ts; g.nrm = net->norm; g.count = net->count; g.seed = seed; g.step = draw;
+    }
+    g.Xbt = net->Xbt; g.tgt = net->Tb; g.dscale = 2.0f / (float)((double)rows_valid * NOUT_USED);
     g.lossp = lossp; g.bsum = net->bpart;
     g.H1t = net->H1t; g.H2t = net->H2t; g.H3t = net->H3t; g.D4t = net->D4t; g.D3t = net->D3t; g.D2t = net->D2t; g.D1t = net->D1t;
     DV_TRY(chain<true>(g, NB / 128, s));
@@ -882,7 +883,7 @@ int dv_mlp_gradient_host(dv_mlp* n, const float* X, const float* T, int64_t rows
     DV_CUDA(cudaMemcpy(n->Xb, rm.data(), rm.size() * 2, cudaMemcpyHostToDevice));
     DV_CUDA(cudaMemcpy(n->Xbt, fm.data(), fm.size() * 2, cudaMemcpyHostToDevice));
     DV_CUDA(cudaMemcpy(n->Tb, tb.data(), tb.size() * 4, cudaMemcpyHostToDevice));
-    DV_TRY(grad_batch(n, rows, n->lossp, 0));
+    DV_TRY(grad_batch(n, rows, 0, -1, n->lossp, 0));
     DV_LAUNCH(dv::K_MLP, 0, k_collect_grad<<<g1(NPARAM), 256, 0, 0>>>(n->part, n->bpart, n->G));
     DV_TRY(launch_ok("k_collect_grad"));
     DV_CUDA(cudaMemcpy(grad, n->G, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
@@ -918,12 +919,8 @@ int dv_mlp_train(dv_mlp* n, int32_t steps, float lr, uint64_t seed, int32_t keep
     }
     const int TB = NB / 128;
     for (int it = 0; it < steps; ++it) {
-        DV_LAUNCH(dv::K_MLP, s, k_gather<<<g1((int64_t)NB * (NIN / 8)), 256, 0, s>>>(n->Xs, n->cap, n->Ts, n->count,
-                                                                                    (int64_t)(seed & 0x7fffffffffffll),
-                                                                                    n->adam_t, n->norm, n->Xb, n->Xbt, n->Tb));
-        DV_CUDA(cudaGetLastError());
         const int slot = it % LOSS_KEEP;
-        DV_TRY(grad_batch(n, NB, n->lossp + slot * TB, s));
+        DV_TRY(grad_batch(n, NB, (int64_t)(seed & 0x7fffffffffffll), n->adam_t, n->lossp + slot * TB, s));
         n->adam_t += 1;
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.0f - std::pow(b1, (float)n->adam_t), c2 = 1.0f - std::pow(b2, (float)n->adam_t);
