@@ -457,8 +457,9 @@ static __device__ __forceinline__ void sp_slope(const dv_step_params& p, const S
     s[3] = limited_slope(p.limiter, T[c] - T[c - 1], T[c + 1] - T[c]);
 }
 
-// One thread per face: interior z faces, r faces, theta faces, then the two end faces of every
-// column (kept last so the warps of each range run one kind of face).
+// One thread per face: interior z faces, r faces, theta faces, the two end faces of every column
+// (kept last so the warps of each range run one kind of face); then the wall resistance of each outer-ring
+// cell, into rec.Rb (the longest chain of a cell's balances, two powers: here beside the faces).
 // The face of index g (all kinds in the order above).
 template <bool REC>
 __device__ __forceinline__ void faces_at(const dv_step_params& p, const Aux& aux, const Split& S, const Rec& rec,
@@ -540,6 +541,14 @@ __device__ __forceinline__ void faces_at(const dv_step_params& p, const Aux& aux
         for (int q = 0; q < DV_NG; ++q) F.F[q] = (e == 0) ? F_in[q] : -F_in[q];
         F.H = (e == 0) ? H_in : -H_in;
         flux_put(S.zf, S.nzf, col * (Nz + 1) + (e == 0 ? 0 : Nz), F);
+        return;
+    }
+    g -= 2 * ncol;
+    if (g < (int64_t)Nth * Nz) {
+        Cell s;
+        Props o;
+        sp_get(S, (int64_t)(Nr - 1) * Nth * Nz + g, s, o);
+        rec.Rb[g] = wall_R_bed(p, o);
     }
 }
 
@@ -551,101 +560,95 @@ __global__ void __launch_bounds__(64) k_faces(dv_step_params p, Aux aux, Split S
     faces_at<REC>(p, aux, S, rec, t, scal, dargs, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// The assembly of cell c.
-template <int MODE, bool REC>
-__device__ __forceinline__ void assemble_at(const dv_step_params& p, const Aux& aux, const Split& S, const Rec& rec,
-                                            double t, const double* __restrict__ y, const double* __restrict__ u,
-                                            const double* __restrict__ sc, const double* __restrict__ f0,
-                                            const double* __restrict__ scal, double gh, double* __restrict__ out,
-                                            const double* __restrict__ dargs, int64_t c) {
+// Row v (0..5, or 6: the wall node) of cell c: true, its index and value where the cell has one.
+template <int MODE, bool REC, class L>
+__device__ __forceinline__ bool assemble_row(const dv_step_params& p, const Aux& aux, const Split& S, const Rec& rec,
+                                             double t, const L& ld, const double* __restrict__ y,
+                                             const double* __restrict__ u, const double* __restrict__ sc,
+                                             const double* __restrict__ f0, double sig, double gh, int64_t c, int v,
+                                             int64_t& ix, double& r) {
     const int64_t nc = S.nc;
-    if (c >= nc) return;
-    if (dargs) {                  // launched from a CUDA graph: time and step factor live on the device
-        t = dargs[0];
-        gh = dargs[1];
-    }
+    if (c >= nc) return false;
     int i, j, k;
     cell_ijk(p, c, i, j, k);
     const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
-    const bool outer_wall = (i == Nr - 1) && p.wall_on;
-    const int64_t iw = (int64_t)DV_NV * nc + (int64_t)j * Nz + k;
-    if (MODE == M_MATVEC && scal[0] == 0.0) {      // matvec of a zero direction is zero
-#pragma unroll
-        for (int v = 0; v < DV_NV; ++v) out[v * nc + c] = 0.0;
-        if (outer_wall) out[iw] = 0.0;
-        return;
-    }
-    Cell s0;
-    Props P0;
-    sp_get(S, c, s0, P0);
-    double rate[DV_NA], qstar[DV_NA];
-#pragma unroll
-    for (int q = 0; q < DV_NA; ++q) {
-        rate[q] = S.cell[(SP_RATE0 + q) * nc + c];
-        qstar[q] = S.cell[(SP_QS0 + q) * nc + c];
-    }
-    const int64_t col = (int64_t)i * Nth + j;
-    Flux Fzm, Fzp, Frm, Frp, Ftm, Ftp;
-    flux_get(S.zf, S.nzf, col * (Nz + 1) + k, Fzm);
-    flux_get(S.zf, S.nzf, col * (Nz + 1) + k + 1, Fzp);
-    if (Nr > 1) {
-        if (i > 0) flux_get(S.rf, S.nrf, c - (int64_t)Nth * Nz, Frm);
-        if (i < Nr - 1) flux_get(S.rf, S.nrf, c, Frp);
-    }
-    if (Nth > 1) {
-        const int jm = (j == 0) ? Nth - 1 : j - 1;
-        flux_get(S.tf, S.ntf, ((int64_t)i * Nth + jm) * Nz + k, Ftm);
-        flux_get(S.tf, S.ntf, c, Ftp);
-    }
-    double f[DV_NV], fw = 0.0;
-    if (MODE == M_MATVEC) {
-        const double sig = matvec_sig(scal);
-        LoadDir ld{y, u, sc, sig};
-        cell_tail(p, aux, ld, t, i, j, k, P0, rate, qstar, Fzm, Fzp, Frm, Frp, Ftm, Ftp, f,
-                  outer_wall ? &fw : nullptr, REC ? &rec : nullptr);
-#pragma unroll
-        for (int v = 0; v < DV_NV; ++v) {
-            const int64_t ix = v * nc + c;
-            const double vv = u[ix] * sc[ix];
-            out[ix] = (vv - gh * (f[v] - f0[ix]) / sig) / sc[ix];
-        }
-        if (outer_wall) {
-            const double vv = u[iw] * sc[iw];
-            out[iw] = (vv - gh * (fw - f0[iw]) / sig) / sc[iw];
-        }
-        return;
-    }
-    LoadPlain ld{y};
-    cell_tail(p, aux, ld, t, i, j, k, P0, rate, qstar, Fzm, Fzp, Frm, Frp, Ftm, Ftp, f,
-              outer_wall ? &fw : nullptr, REC ? &rec : nullptr);
-    if (MODE == M_RHS) {
-#pragma unroll
-        for (int v = 0; v < DV_NV; ++v) out[v * nc + c] = f[v];
-        if (outer_wall) out[iw] = fw;
+    const int64_t wn = (int64_t)j * Nz + k;
+    if (v == DV_NV && !(i == Nr - 1 && p.wall_on)) return false;
+    ix = v < DV_NV ? v * nc + c : (int64_t)DV_NV * nc + wn;
+    double f;
+    if (v == 3 || v == 4) {
+        f = S.cell[(SP_RATE0 + v - 3) * nc + c];
+    } else if (v == DV_NV) {
+        wall_terms(p, aux, ld, jacket_T(p, t), j, k, S.cell[SP_T * nc + c], rec.Rb[wn], &f);
     } else {
-#pragma unroll
-        for (int v = 0; v < DV_NV; ++v) {
-            const int64_t ix = v * nc + c;
-            out[ix] = y[ix] - gh * f[v] - u[ix];
+        const int q = v < DV_NG ? v : DV_NG;
+        const double* z = S.zf + q * S.nzf + ((int64_t)i * Nth + j) * (Nz + 1) + k;
+        double rm = 0.0, rp = 0.0, tm = 0.0, tp = 0.0;
+        if (Nr > 1) {
+            if (i > 0) rm = S.rf[q * S.nrf + c - (int64_t)Nth * Nz];
+            if (i < Nr - 1) rp = S.rf[q * S.nrf + c];
         }
-        if (outer_wall) out[iw] = y[iw] - gh * fw - u[iw];
+        if (Nth > 1) {
+            tm = S.tf[q * S.ntf + ((int64_t)i * Nth + (j == 0 ? Nth - 1 : j - 1)) * Nz + k];
+            tp = S.tf[q * S.ntf + c];
+        }
+        const double div = face_div(p, i, z[0], z[1], rm, rp, tm, tp);
+        f = v < DV_NG ? row_mass(p, i, div, (v < DV_NA) ? S.cell[(SP_RATE0 + v) * nc + c] : 0.0)
+                      : row_energy(p, aux, ld, t, i, j, k, S.cell[SP_T * nc + c], i == Nr - 1 ? rec.Rb[wn] : 0.0, div,
+                                   nullptr, REC ? &rec : nullptr);
     }
+    if (MODE == M_RHS) {
+        r = f;
+    } else if (MODE == M_STAGE) {
+        r = y[ix] - gh * f - u[ix];
+    } else {
+        const double vv = u[ix] * sc[ix];
+        r = (vv - gh * (f - f0[ix]) / sig) / sc[ix];
+    }
+    if (REC && v == 3) {
+        rec.T[c] = S.cell[SP_T * nc + c];
+        rec.P[c] = S.cell[SP_P * nc + c];
+#pragma unroll
+        for (int q = 0; q < DV_NG; ++q) rec.y[q * nc + c] = S.cell[(SP_Y0 + q) * nc + c];
+        rec.qstar[c] = S.cell[SP_QS0 * nc + c];
+        rec.qstar[nc + c] = S.cell[(SP_QS0 + 1) * nc + c];
+    }
+    return true;
 }
 
+// A warp per row, 32 cells per block.  Bound by latency: a balance is two divisions, three more in a matvec, and a
+// thread with a whole cell took them and the wall's resistance in turn with 3.5 warps an SM (16x16x64:
+// 5.4 -> 3.7 us, in a matvec 9.4 -> 4.5).  The rows are stored when all have been read, so out may be an input of its own rows.
+constexpr int AS_CELLS = 32;
 template <int MODE, bool REC>
-__global__ void __launch_bounds__(64) k_assemble(dv_step_params p, Aux aux, Split S, Rec rec, double t,
+__global__ void __launch_bounds__(DV_NB * AS_CELLS) k_assemble(dv_step_params p, Aux aux, Split S, Rec rec, double t,
                                                  const double* __restrict__ y, const double* __restrict__ u,
                                                  const double* __restrict__ sc, const double* __restrict__ f0,
                                                  const double* __restrict__ scal, double gh,
                                                  double* __restrict__ out, const double* __restrict__ dargs) {
     pdl_wait();
-    assemble_at<MODE, REC>(p, aux, S, rec, t, y, u, sc, f0, scal, gh, out, dargs,
-                           (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const int64_t c = (int64_t)blockIdx.x * AS_CELLS + (threadIdx.x & 31);
+    const int v = threadIdx.x >> 5;
+    if (dargs) {                  // launched from a CUDA graph: time and step factor live on the device
+        t = dargs[0];
+        gh = dargs[1];
+    }
+    int64_t ix = 0;
+    double r = 0.0;
+    bool has;
+    if (MODE == M_MATVEC) {
+        const double sig = matvec_sig(scal);
+        has = assemble_row<MODE, REC>(p, aux, S, rec, t, LoadDir{y, u, sc, sig}, y, u, sc, f0, sig, gh, c, v, ix, r);
+        if (scal[0] == 0.0) r = 0.0;      // matvec of a zero direction is zero
+    } else {
+        has = assemble_row<MODE, REC>(p, aux, S, rec, t, LoadPlain{y}, y, u, sc, f0, 0.0, gh, c, v, ix, r);
+    }
+    __syncthreads();
+    if (has) out[ix] = r;
 }
 
 // The FD matvec of the GMRES graph in one cooperative launch: the blocks of k_cprops, k_faces and
-// k_assemble (the same per-block / per-index code, in the same 64-thread blocks) taken in grid-
-// stride order, the three phases separated by two bounded grid barriers (bar[0..1]; bit 4 of *err
+// k_assemble (the same per-index code, in 64-thread blocks) taken in grid-stride order, the three phases separated by two bounded grid barriers (bar[0..1]; bit 4 of *err
 // on a timeout).  Saves two kernel boundaries per Arnoldi step; results are bit-identical.
 __global__ void __launch_bounds__(64) k_matvec_coop(dv_step_params p, Aux aux, Split S, Rec rec,
                                                     const double* __restrict__ z, const double* __restrict__ u,
@@ -660,7 +663,14 @@ __global__ void __launch_bounds__(64) k_matvec_coop(dv_step_params p, Aux aux, S
         faces_at<false>(p, aux, S, rec, 0.0, scal, dargs, vb * 64 + threadIdx.x);
     grid_sync_bounded(bar, bar + 1, err);
     for (int64_t vb = blockIdx.x; vb < nb_cells; vb += gridDim.x)
-        assemble_at<M_MATVEC, false>(p, aux, S, rec, 0.0, z, u, sc, f0, scal, 0.0, out, dargs, vb * 64 + threadIdx.x);
+        for (int v = 0; v < DV_NB; ++v) {
+            const double sig = matvec_sig(scal);
+            int64_t ix;
+            double r;
+            if (assemble_row<M_MATVEC, false>(p, aux, S, rec, dargs ? dargs[0] : 0.0, LoadDir{z, u, sc, sig}, z, u, sc, f0, sig,
+                                              dargs ? dargs[1] : 0.0, vb * 64 + threadIdx.x, v, ix, r))
+                out[ix] = scal[0] == 0.0 ? 0.0 : r;
+        }
 }
 
 // ---------------------------------------------------------------- finite-difference Jacobian
@@ -1354,11 +1364,11 @@ static int split_residual(dv_model* m, const Rec& rec, double t, const double* y
     }
     const Split S = split_of(p, m->d_split);
     const int64_t ncol = (int64_t)p.Nr * p.Nth;
-    const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol;
+    const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol + p.Nth * p.Nz;
     DV_LAUNCH(kind, s, k_cprops<MODE><<<nblk(m->nc, 32), CP_WARPS * 32, 0, s>>>(p, S, y, u, sc, scal));
     DV_LAUNCH(kind, s, k_faces<REC><<<nblk(nfaces, 64), 64, 0, s>>>(p, aux_of(m), S, rec, t,
                                                                   MODE == M_MATVEC ? scal : nullptr, nullptr));
-    DV_LAUNCH(kind, s, k_assemble<MODE, REC><<<nblk(m->nc, 64), 64, 0, s>>>(p, aux_of(m), S, rec, t, y, u, sc, f0,
+    DV_LAUNCH(kind, s, k_assemble<MODE, REC><<<nblk(m->nc, AS_CELLS), DV_NB * AS_CELLS, 0, s>>>(p, aux_of(m), S, rec, t, y, u, sc, f0,
                                                                            scal, gh, out, nullptr));
     m->nfev += 1;
     DV_CUDA(cudaGetLastError());
@@ -1438,7 +1448,7 @@ int matvec_capture(dv_model* m, const double* dargs, const double* z, const doub
     const Split S = split_of(p, m->d_split);
     const Rec rec = make_rec(m->rl, m->d_rec);
     const int64_t ncol = (int64_t)p.Nr * p.Nth;
-    const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol;
+    const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol + p.Nth * p.Nz;
     int& coop_cap = g_matvec_coop_cap;
     if (coop_cap < 0) {
         int dev = 0, nsm = 0, bps = 0;
@@ -1479,13 +1489,13 @@ int matvec_capture(dv_model* m, const double* dargs, const double* z, const doub
     if (pdl_enabled()) {       // each kernel may start while its predecessor drains (pdl_wait in the kernel)
         DV_CUDA(launch_pdl(k_cprops<M_MATVEC>, nblk(m->nc, 32), CP_WARPS * 32, s, p, S, z, u, sc, scal));
         DV_CUDA(launch_pdl(k_faces<false>, nblk(nfaces, 64), 64, s, p, aux_of(m), S, rec, 0.0, scal, dargs));
-        DV_CUDA(launch_pdl(k_assemble<M_MATVEC, false>, nblk(m->nc, 64), 64, s, p, aux_of(m), S, rec, 0.0, z, u, sc, f0,
+        DV_CUDA(launch_pdl(k_assemble<M_MATVEC, false>, nblk(m->nc, AS_CELLS), DV_NB * AS_CELLS, s, p, aux_of(m), S, rec, 0.0, z, u, sc, f0,
                            scal, 0.0, out, dargs));
         return DV_OK;
     }
     k_cprops<M_MATVEC><<<nblk(m->nc, 32), CP_WARPS * 32, 0, s>>>(p, S, z, u, sc, scal);
     k_faces<false><<<nblk(nfaces, 64), 64, 0, s>>>(p, aux_of(m), S, rec, 0.0, scal, dargs);
-    k_assemble<M_MATVEC, false><<<nblk(m->nc, 64), 64, 0, s>>>(p, aux_of(m), S, rec, 0.0, z, u, sc, f0, scal, 0.0,
+    k_assemble<M_MATVEC, false><<<nblk(m->nc, AS_CELLS), DV_NB * AS_CELLS, 0, s>>>(p, aux_of(m), S, rec, 0.0, z, u, sc, f0, scal, 0.0,
                                                              out, dargs);
     DV_CUDA(cudaGetLastError());
     return DV_OK;
