@@ -1,7 +1,8 @@
 """Launch-parameter autotuner: picks the hot kernels' launch parameters per grid shape and caches them.
 
 ``tune(model, y, dh)`` runs the library's timer (dv_autotune) on the model at state y: every candidate
-of the FD-Jacobian block size, the preconditioner sweep's ring depth, the FP32 Jacobian product's
+of the preconditioner sweep's L2 prefetch (and of the FD Jacobian's block size, which its kernels no
+longer have), the FP32 Jacobian product's
 block size and the GMRES graph's prefix of unrolled Arnoldi steps, timed with CUDA events on the
 model's own matrices; the fastest of each is kept in the model.  ``cached(model)`` applies an earlier
 result for the same grid, preconditioner, precision and GPU from the cache file (``$DVTSA_TUNE_CACHE``,

@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(ACC_T) k_accumulators(dv_step_params p, const 
 
 // ---------------------------------------------------------------- split residual
 // The residual as three launches with short per-thread chains: per-cell properties and uptake
-// (k_cprops), the flux through every face once (k_faces), per-cell divergence and sources
-// (k_assemble, through cell_tail).  Each step evaluates the same expressions on the same inputs
+// (k_cprops), the flux through every face once (k_faces), divergence and sources of each row
+// (k_assemble).  Each step evaluates the same expressions on the same inputs
 // as cell_eval, so the results are the same bits; the thread-per-cell kernel computes the
 // properties of every cell seven times and every face twice.
 enum { SP_C0 = 0, SP_T = 3, SP_P, SP_CPOS, SP_Y0, SP_MU = SP_Y0 + 3, SP_KG, SP_RHO, SP_CPM, SP_DM, SP_LAM0,
@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(DV_NB * AS_CELLS) k_assemble(dv_step_params p,
         has = assemble_row<MODE, REC>(p, aux, S, rec, t, LoadDir{y, u, sc, sig}, y, u, sc, f0, sig, gh, c, v, ix, r);
         if (scal[0] == 0.0) r = 0.0;      // matvec of a zero direction is zero
     } else {
-        has = assemble_row<MODE, REC>(p, aux, S, rec, t, LoadPlain{y}, y, u, sc, f0, 0.0, gh, c, v, ix, r);
+        has = assemble_row<MODE, REC>(p, aux, S, rec, t, LoadPlain{y}, y, u, sc, f0, 1.0, gh, c, v, ix, r);
     }
     __syncthreads();
     if (has) out[ix] = r;
@@ -1332,7 +1332,7 @@ __global__ void __launch_bounds__(TL_THREADS, 1) k_tile(dv_step_params p, Aux au
         const double sig = matvec_sig(scal);
         tile_residual<MODE, REC>(p, aux, rec, t, LoadDir{y, u, sc, sig}, y, u, sc, f0, sig, gh, out, X);
     } else {
-        tile_residual<MODE, REC>(p, aux, rec, t, LoadPlain{y}, y, u, sc, f0, 0.0, gh, out, X);
+        tile_residual<MODE, REC>(p, aux, rec, t, LoadPlain{y}, y, u, sc, f0, 1.0, gh, out, X);
     }
 }
 

@@ -152,7 +152,7 @@ static __device__ __forceinline__ double row_energy(const dv_step_params& p, con
 }
 
 // All rows of cell (i,j,k): f[0..5]; *fw = dTw/dt of its wall node; and its records.  Shared by the
-// thread-per-cell residual, the split residual's assembly and the Jacobian's rows.  R_pre: the outer-ring
+// thread-per-cell residual and the Jacobian's rows.  R_pre: the outer-ring
 // cell's wall resistance where it has been evaluated already (the same expression on the same properties),
 // else null.
 template <class L>
