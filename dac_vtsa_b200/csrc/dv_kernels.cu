@@ -224,12 +224,14 @@ struct Split {
     double* zf;            // [4][ncol (Nz+1)]: +z flux through face kf of a column (kf 0 = top end, Nz = bottom end)
     double* rf;            // [4][(Nr-1) Nth Nz]: +r flux between rings i and i+1 at (j, k)
     double* tf;            // [4][Nr Nth Nz]: +theta flux between sectors j and j+1 (periodic) at (i, k)
+    double* wall;          // [Nth Nz]: wall rows of a call whose result replaces its state
     int64_t nc, nzf, nrf, ntf;
 };
 
 int64_t split_doubles(const dv_step_params& p) {
     const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz, ncol = (int64_t)p.Nr * p.Nth;
-    return SP_NCELL * nc + 4 * (ncol * (p.Nz + 1) + (int64_t)(p.Nr - 1) * p.Nth * p.Nz + nc);
+    return SP_NCELL * nc + 4 * (ncol * (p.Nz + 1) + (int64_t)(p.Nr - 1) * p.Nth * p.Nz + nc) +
+           (int64_t)p.Nth * p.Nz;
 }
 
 static Split split_of(const dv_step_params& p, double* base) {
@@ -242,6 +244,7 @@ static Split split_of(const dv_step_params& p, double* base) {
     S.zf = S.cell + SP_NCELL * S.nc;
     S.rf = S.zf + 4 * S.nzf;
     S.tf = S.rf + 4 * S.nrf;
+    S.wall = S.tf + 4 * S.ntf;
     return S;
 }
 
@@ -618,14 +621,16 @@ __device__ __forceinline__ bool assemble_row(const dv_step_params& p, const Aux&
 
 // A warp per row, 32 cells per block.  Bound by latency: a balance is two divisions, three more in a matvec, and a
 // thread with a whole cell took them and the wall's resistance in turn with 3.5 warps an SM (16x16x64:
-// 5.4 -> 3.7 us, in a matvec 9.4 -> 4.5).  The rows are stored when all have been read, so out may be an input of its own rows.
+// 5.4 -> 3.7 us, in a matvec 9.4 -> 4.5).  A block stores its rows when all of them have been read, so out may be
+// an input that is read by its own rows alone.  The wall rows also read the wall temperatures of other blocks, so
+// they go to `wall`: their place in out, or scratch where out holds those temperatures.
 constexpr int AS_CELLS = 32;
 template <int MODE, bool REC>
 __global__ void __launch_bounds__(DV_NB * AS_CELLS) k_assemble(dv_step_params p, Aux aux, Split S, Rec rec, double t,
                                                  const double* __restrict__ y, const double* __restrict__ u,
                                                  const double* __restrict__ sc, const double* __restrict__ f0,
-                                                 const double* __restrict__ scal, double gh,
-                                                 double* __restrict__ out, const double* __restrict__ dargs) {
+                                                 const double* __restrict__ scal, double gh, double* __restrict__ out,
+                                                 double* __restrict__ wall, const double* __restrict__ dargs) {
     pdl_wait();
     const int64_t c = (int64_t)blockIdx.x * AS_CELLS + (threadIdx.x & 31);
     const int v = threadIdx.x >> 5;
@@ -644,7 +649,7 @@ __global__ void __launch_bounds__(DV_NB * AS_CELLS) k_assemble(dv_step_params p,
         has = assemble_row<MODE, REC>(p, aux, S, rec, t, LoadPlain{y}, y, u, sc, f0, 1.0, gh, c, v, ix, r);
     }
     __syncthreads();
-    if (has) out[ix] = r;
+    if (has) (v < DV_NV ? out[ix] : wall[ix - (int64_t)DV_NV * S.nc]) = r;
 }
 
 // The FD matvec of the GMRES graph in one cooperative launch: the blocks of k_cprops, k_faces and
@@ -1355,7 +1360,10 @@ template <int MODE, bool REC>
 static int split_residual(dv_model* m, const Rec& rec, double t, const double* y, const double* u, const double* sc,
                           const double* f0, const double* scal, double gh, double* out, cudaStream_t s, int kind) {
     const dv_step_params& p = m->p;
-    if (use_tiles(p) && out != y && out != u && out != sc) {      // (a tile reads its neighbours' inputs)
+    // out is one of the inputs that LoadPlain / LoadDir read: a tile reads its neighbours' (the right-hand side of
+    // a stage residual, M_STAGE's u, is read by its own rows alone, but keeps the split path it has always taken)
+    const bool over = out == y || (MODE == M_MATVEC && (out == u || out == sc));
+    if (use_tiles(p) && !over && out != u) {
         DV_LAUNCH(kind, s, k_tile<MODE, REC><<<(unsigned)tile_blocks(p), TL_THREADS, 0, s>>>(p, aux_of(m), rec, t, y, u, sc, f0,
                                                                                             scal, gh, out, nullptr));
         m->nfev += 1;
@@ -1363,13 +1371,16 @@ static int split_residual(dv_model* m, const Rec& rec, double t, const double* y
         return DV_OK;
     }
     const Split S = split_of(p, m->d_split);
+    double* const wall = out + (int64_t)DV_NV * m->nc;
     const int64_t ncol = (int64_t)p.Nr * p.Nth;
     const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol + p.Nth * p.Nz;
     DV_LAUNCH(kind, s, k_cprops<MODE><<<nblk(m->nc, 32), CP_WARPS * 32, 0, s>>>(p, S, y, u, sc, scal));
     DV_LAUNCH(kind, s, k_faces<REC><<<nblk(nfaces, 64), 64, 0, s>>>(p, aux_of(m), S, rec, t,
                                                                   MODE == M_MATVEC ? scal : nullptr, nullptr));
     DV_LAUNCH(kind, s, k_assemble<MODE, REC><<<nblk(m->nc, AS_CELLS), DV_NB * AS_CELLS, 0, s>>>(p, aux_of(m), S, rec, t, y, u, sc, f0,
-                                                                           scal, gh, out, nullptr));
+                                                                           scal, gh, out, over ? S.wall : wall, nullptr));
+    if (over && p.wall_on)
+        DV_CUDA(cudaMemcpyAsync(wall, S.wall, sizeof(double) * p.Nth * p.Nz, cudaMemcpyDeviceToDevice, s));
     m->nfev += 1;
     DV_CUDA(cudaGetLastError());
     return DV_OK;
@@ -1490,13 +1501,13 @@ int matvec_capture(dv_model* m, const double* dargs, const double* z, const doub
         DV_CUDA(launch_pdl(k_cprops<M_MATVEC>, nblk(m->nc, 32), CP_WARPS * 32, s, p, S, z, u, sc, scal));
         DV_CUDA(launch_pdl(k_faces<false>, nblk(nfaces, 64), 64, s, p, aux_of(m), S, rec, 0.0, scal, dargs));
         DV_CUDA(launch_pdl(k_assemble<M_MATVEC, false>, nblk(m->nc, AS_CELLS), DV_NB * AS_CELLS, s, p, aux_of(m), S, rec, 0.0, z, u, sc, f0,
-                           scal, 0.0, out, dargs));
+                           scal, 0.0, out, out + (int64_t)DV_NV * m->nc, dargs));
         return DV_OK;
     }
     k_cprops<M_MATVEC><<<nblk(m->nc, 32), CP_WARPS * 32, 0, s>>>(p, S, z, u, sc, scal);
     k_faces<false><<<nblk(nfaces, 64), 64, 0, s>>>(p, aux_of(m), S, rec, 0.0, scal, dargs);
     k_assemble<M_MATVEC, false><<<nblk(m->nc, AS_CELLS), DV_NB * AS_CELLS, 0, s>>>(p, aux_of(m), S, rec, 0.0, z, u, sc, f0, scal, 0.0,
-                                                             out, dargs);
+                                                             out, out + (int64_t)DV_NV * m->nc, dargs);
     DV_CUDA(cudaGetLastError());
     return DV_OK;
 }

@@ -160,9 +160,10 @@ int dv_model_sizes(const dv_model* m, int64_t* n_core, int64_t* ncell, int64_t* 
 int64_t dv_model_nfev(const dv_model* m);
 
 /* f = dy/dt (TVSAModel.rhs, core/residual.py:211-365); acc (36 accumulator rates,
- * core/residual.py:371-417) is written when non-NULL. */
+ * core/residual.py:371-417) is written when non-NULL.  f may be y itself. */
 int dv_rhs(dv_model* m, double t, const double* y, double* f, double* acc, void* stream);
-/* R = y - gamma_h f(t, y) - rhs_known (TVSAModel.stage_residual, core/residual.py:420-423) */
+/* R = y - gamma_h f(t, y) - rhs_known (TVSAModel.stage_residual, core/residual.py:420-423); R may be y
+ * or rhs_known itself. */
 int dv_stage_residual(dv_model* m, double t, const double* y, double gamma_h, const double* rhs_known,
                       double* R, void* stream);
 /* Diagnostics of TVSAModel.rhs(diag=True) (core/residual.py:366-368) into `diag` (diag_doubles):

@@ -194,3 +194,34 @@ def test_tile_residual_at_ragged_grids_is_bit_identical_to_the_other_evaluations
         rc = lib.dv_stage_residual(m.handle, 3.0, s.data_ptr(), 0.7, known.data_ptr(), known.data_ptr(), stream)
         assert rc == 0, lib.dv_last_error()
         assert np.array_equal(R.cpu().numpy(), known.cpu().numpy(), equal_nan=True)
+
+
+@pytest.mark.parametrize("grid,wall", [((1, 1, 30), True), ((3, 5, 7), True), ((3, 5, 7), False), ((12, 12, 48), True)])
+def test_results_may_replace_the_state(grid, wall):
+    """f, and a stage residual, written over the state they are evaluated at: the same bits as apart from it
+    (the wall rows read the temperatures of neighbouring wall nodes, which other blocks replace)."""
+    import ctypes as C
+    from dac_vtsa_b200 import _lib, host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.model import TVSAModel
+    lib = _lib.load()
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    cfg = load_config(override_dict={"grid.Nr": grid[0], "grid.Ntheta": grid[1], "grid.Nz": grid[2],
+                                     "wall.enabled": wall})
+    g = host.Grid.from_config(cfg)
+    st = host.seeded_state(cfg, g, host.get_backend(cfg), seed=4, amplitude=0.02)
+    st.Tw = st.Tw + np.random.default_rng(5).random(st.Tw.shape)
+    m = TVSAModel(cfg, g, host.get_backend(cfg), cfg.cycle[0], st)
+    y = torch.from_numpy(m.pack(st)).to(m.device)
+    known = y * 1.001
+    f, acc = m.rhs(3.0, y)
+    R = m.stage_residual(3.0, y, 0.7, known)
+    for a in (None, torch.empty_like(acc)):
+        s = y.clone()
+        assert lib.dv_rhs(m.handle, 3.0, s.data_ptr(), s.data_ptr(), a.data_ptr() if a is not None else None,
+                          stream) == 0, lib.dv_last_error()
+        assert np.array_equal(s.cpu().numpy(), f.cpu().numpy())
+        assert a is None or np.array_equal(a.cpu().numpy(), acc.cpu().numpy())
+    s = y.clone()
+    assert lib.dv_stage_residual(m.handle, 3.0, s.data_ptr(), 0.7, known.data_ptr(), s.data_ptr(), stream) == 0
+    assert np.array_equal(s.cpu().numpy(), R.cpu().numpy())
