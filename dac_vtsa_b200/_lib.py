@@ -150,6 +150,7 @@ SIGNATURES = [
     ("dv_integrator_copy_y", C.c_int, [P, P, P]),
     ("dv_rhs_acc_noalloc", C.c_int, [C.POINTER(DvStepParams), P, P, P, D, P, P, P, P]),
     ("dv_selftest_wait_timeout", C.c_int, [I32, C.POINTER(I32)]),
+    ("dv_selftest_exchange_timeout", C.c_int, [I32, I32, C.POINTER(D), C.POINTER(I32)]),
     ("dv_model_flag_wait_timeout", C.c_int, [P, I32]),
     ("dv_model_set_tuning", C.c_int, [P, C.POINTER(DvTuning)]),
     ("dv_model_get_tuning", C.c_int, [P, C.POINTER(DvTuning)]),

@@ -247,7 +247,7 @@ struct PaFuse {
 // measured 2 % slower on the 8x8x32 heating window, bit-identical results).
 bool pdl_enabled();
 bool precond_apply_fusable(dv_model* m);
-// bounded-wait self-test: one sweep-style mbarrier wait that nothing completes (bit 1 of *err)
+// self-test of the tensor-core products' bounded wait: an mbarrier that nothing completes (bit 1 of *err)
 int selftest_mbar_timeout(int polls, int* err, cudaStream_t s);
 // The same launches without launch accounting or attribute changes, for stream capture (the
 // attributes are set by an earlier precond_apply).  Returns the number of kernels launched.

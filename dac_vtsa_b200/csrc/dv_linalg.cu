@@ -1128,45 +1128,6 @@ __global__ void __launch_bounds__(256) k_pc_factor_glob(PcGeom gin, double* __re
 }
 
 // ---------------------------------------------------------------- sweeps
-static __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-static __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// bounded wait: false after `limit` polls (~2^22 by default; each poll may itself suspend briefly)
-static __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int limit = 1 << 22) {
-    for (int it = 0; it < limit; ++it)
-        if (mbar_try(bar, parity)) return true;
-    return false;
-}
-
-// Self-test of the bounded wait: an mbarrier that nothing arrives at, waited on by one warp with
-// `polls` polls; the timeout sets bit 1 of *err, and the kernel returns.
-__global__ void k_selftest_mbar(int polls, int* err) {
-    __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&bar), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
-    const bool arrived = mbar_wait(smem_u32(&bar), 0u, polls);
-    __syncwarp();
-    if (threadIdx.x == 0) {
-        if (!arrived) atomicOr(err, 1);
-        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&bar)) : "memory");
-    }
-}
-
-int selftest_mbar_timeout(int polls, int* err, cudaStream_t s) {
-    k_selftest_mbar<<<1, 32, 0, s>>>(polls, err);
-    DV_CUDA(cudaGetLastError());
-    return DV_OK;
-}
-
 // Plane frame of one elimination direction.  TW = false: planes 0..Nz-1 top-down (the whole
 // partition).  TW = true (twisted factorisation, a cluster of two CTAs per partition): rank 0
 // eliminates planes 0..zs-1 top-down, rank 1 planes Nz-1..zs+2 bottom-up, and the separator

@@ -150,6 +150,23 @@ __global__ void __launch_bounds__(GT) k_gemm(GemmBatch gb) {
     if (warp == 0) tmem_dealloc(tmem, ncols);
 }
 
+// Self-test of the products' bounded wait: an mbarrier that nothing arrives at, waited on by one warp with
+// `polls` polls; the timeout sets bit 1 of *err, and the kernel returns.
+__global__ void k_selftest_mbar(int polls, int* err) {
+    __shared__ __align__(8) uint64_t bar;
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&bar), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    const bool arrived = mbar_wait(smem_u32(&bar), 0u, polls);
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        if (!arrived) atomicOr(err, 1);
+        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&bar)) : "memory");
+    }
+}
+
 static int gemm(const GemmBatch& g, int products, cudaStream_t s) {
     DV_CUDA(dv::allow_dyn_smem((const void*)k_gemm));
     DV_LAUNCH(dv::K_MLP, s, k_gemm<<<products * g.per, GT, GEMM_SMEM, s>>>(g));
@@ -647,6 +664,12 @@ int record_targets(dv_mlp* net, const StageInputs& in, const double* zstar, cons
 }
 
 }  // namespace mlp
+
+int selftest_mbar_timeout(int polls, int* err, cudaStream_t s) {
+    mlp::k_selftest_mbar<<<1, 32, 0, s>>>(polls, err);
+    DV_CUDA(cudaGetLastError());
+    return DV_OK;
+}
 }  // namespace dv
 
 using namespace dv;

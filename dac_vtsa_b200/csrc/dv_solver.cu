@@ -929,12 +929,11 @@ static int gmres(Work& W, const Op& op, const double* b, double rtol, double ato
 static int check_device_error(dv_model* m);
 static void clear_device_error(dv_model* m);
 
-// the model's device error word: bit 1 a bulk-copy wait timed out, bit 4 a
-// grid barrier of a cooperative kernel (Gram-Schmidt, the FD matvec) timed out
+// the model's device error word: bit 4 the Gram-Schmidt kernel's exchange or the grid barrier of the
+// cooperative FD matvec timed out
 static const char* device_error_text(int e) {
     if (e & 32) return "a preconditioner index fell outside its storage (the access was skipped)";
-    if (e & 1) return "a bounded device wait (preconditioner bulk copy) timed out";
-    if (e & 4) return "a bounded device wait (GMRES grid barrier) timed out";
+    if (e & 4) return "a bounded device wait (GMRES exchange or grid barrier) timed out";
     return "a bounded device wait timed out";
 }
 
@@ -1304,9 +1303,13 @@ __device__ __forceinline__ void cg_publish(const double (&acc)[GM_KMAX + 1], int
         cg_store(x + (int64_t)blockIdx.x * GM_PS + threadIdx.x, t, e);
     }
 }
-// every block's words of this epoch into ps (bounded polls; bit 4 of *err when a block's sums never came)
-__device__ __forceinline__ void cg_collect(const CgWord* x, int cnt, unsigned long long e, double (*ps)[GM_PS], int* err) {
+// every block's words of this epoch into ps: false, and bit 4 of *err, when a block's sums had not come within
+// `limit` polls of this thread (1 << 22: about three seconds)
+constexpr int CG_POLLS = 1 << 22;
+__device__ __forceinline__ bool cg_collect(const CgWord* x, int cnt, unsigned long long e, double (*ps)[GM_PS], int* err,
+                                           int limit = CG_POLLS) {
     const int items = (int)gridDim.x * cnt;
+    int polls = 0;
     for (int i0 = threadIdx.x; i0 < items; i0 += 4 * VB) {
         bool need[4];
         int b[4], q[4];
@@ -1317,7 +1320,7 @@ __device__ __forceinline__ void cg_collect(const CgWord* x, int cnt, unsigned lo
             b[u] = i / cnt;
             q[u] = i - b[u] * cnt;
         }
-        for (int it = 0; need[0] || need[1] || need[2] || need[3]; ++it) {
+        for (; need[0] || need[1] || need[2] || need[3]; ++polls) {
             double v[4];
             unsigned long long got[4];
 #pragma unroll
@@ -1328,12 +1331,13 @@ __device__ __forceinline__ void cg_collect(const CgWord* x, int cnt, unsigned lo
                     ps[b[u]][q[u]] = v[u];
                     need[u] = false;
                 }
-            if (it > (1 << 22)) {
+            if (polls > limit) {
                 atomicOr(err, 4);
-                break;
+                return false;
             }
         }
     }
+    return true;
 }
 // the sum over the blocks of entry q, in block order
 __device__ __forceinline__ double cg_sum(double (*ps)[GM_PS], int q) {
@@ -1377,9 +1381,13 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
                 carry = -s2 * n0 + c * n1;
             }
         }
-        __syncthreads();                   // the third pass's sums
+        const int gave_up = __syncthreads_or(0);       // the third pass's sums
         if (lane == 0) {
             gm_givens_end(st, h1[m], sqrt(cg_sum(ps, 0)), carry, kdim, hnd);
+            if (gave_up) {                 // the solve ends here, instead of another wait in every step to come
+                st->done = 1;
+                cudaGraphSetConditional(hnd, 0u);
+            }
             *seq = e;
         }
         return;
@@ -1440,7 +1448,7 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
         }
     }
     cg_publish(acc, m + 1, sm, x1, e);
-    cg_collect(x1, m + 1, e, ps, err);
+    bool ok = cg_collect(x1, m + 1, e, ps, err);
     cg_bar();
     if ((int)threadIdx.x <= m) h1[threadIdx.x] = cg_sum(ps, threadIdx.x);
     cg_bar();
@@ -1508,7 +1516,7 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
         }
     }
     cg_publish(acc, m, sm, x2, e);
-    cg_collect(x2, m, e, ps, err);
+    ok = cg_collect(x2, m, e, ps, err) && ok;
     cg_bar();
     if ((int)threadIdx.x < m) h2[threadIdx.x] = cg_sum(ps, threadIdx.x);
     __syncthreads();
@@ -1531,9 +1539,23 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
     }
     cg_publish(acc, 1, sm, x3, e);
     if (blockIdx.x == 0) {                 // block-uniform
-        cg_collect(x3, 1, e, ps, err);
-        __syncthreads();
+        ok = cg_collect(x3, 1, e, ps, err) && ok;
+        __syncthreads_or(ok ? 0 : 1);
     }
+}
+
+// Self-test of the exchange: two blocks, block b publishing the sum of 256 times b + 1; block 1 only where `publish`
+// (else block 0 gives up after `polls` polls and sets bit 4 of *err).  *sum: both blocks' sums, added by block 0.
+__global__ void __launch_bounds__(VB) k_selftest_exchange(int polls, int publish, CgWord* x, double* sum, int* err) {
+    __shared__ double sm[VB / 32][GM_PS], ps[2][GM_PS];
+    if (blockIdx.x == 1 && !publish) return;
+    double acc[GM_KMAX + 1];
+#pragma unroll
+    for (int q = 0; q <= GM_KMAX; ++q) acc[q] = blockIdx.x + 1.0;
+    cg_publish(acc, 1, sm, x, 1ull);
+    if (blockIdx.x == 1) return;
+    const int gave_up = __syncthreads_or(cg_collect(x, 1, 1ull, ps, err, polls) ? 0 : 1);
+    if (threadIdx.x == 0 && !gave_up) *sum = cg_sum(ps, 0);
 }
 
 // Self-test of the bounded grid barrier: a cooperative pair of blocks of which block 1 returns
@@ -2688,6 +2710,30 @@ int dv_selftest_wait_timeout(int32_t polls, int32_t* bits) {
     if (rc != DV_OK) return rc;
     if (e != cudaSuccess) return cuda_fail(e, "dv_selftest_wait_timeout");
     *bits = h;
+    return DV_OK;
+}
+
+int dv_selftest_exchange_timeout(int32_t polls, int32_t publish, double* sum, int32_t* bits) {
+    if (!sum || !bits || polls < 1) { set_error("dv_selftest_exchange_timeout: null argument or polls < 1"); return DV_ERR_ARG; }
+    struct Buf { CgWord x[2 * GM_PS]; double sum; int err; };
+    Buf* d = nullptr;
+    DV_CUDA(cudaMalloc((void**)&d, sizeof(Buf)));
+    cudaError_t e = cudaMemset(d, 0, sizeof(Buf));
+    if (e == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2);
+        cfg.blockDim = dim3(VB);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, k_selftest_exchange, (int)polls, (int)publish, d->x, &d->sum, &d->err);
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(sum, &d->sum, sizeof(double), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(bits, &d->err, sizeof(int), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return cuda_fail(e, "dv_selftest_exchange_timeout");
     return DV_OK;
 }
 

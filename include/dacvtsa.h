@@ -397,13 +397,17 @@ int dv_integrator_set_predictor(dv_integrator* g, dv_mlp* net, int32_t predict, 
 int dv_rhs_acc_noalloc(const dv_step_params* p, const double* feed_flux, const double* n_nom,
                        const double* coverage, double t, const double* y, double* f, double* acc, void* stream);
 
-/* Failure-detection self-test (no reference counterpart): runs the library's two bounded device
- * waits against events that never happen -- an mbarrier wait on a barrier nothing arrives
- * at, and the cooperative Gram-Schmidt kernel's grid barrier with one block that never arrives --
- * each giving up after `polls` polls.  *bits receives the device error word they set (1: the
- * mbarrier wait, 4: the grid barrier; 5 when both timed out as they must).  The waits return,
- * so the CUDA context stays usable.  Synchronous; allocates 16 bytes of device memory. */
+/* Failure-detection self-tests (no reference counterpart): the library's bounded device waits run
+ * against events that never happen, each giving up after `polls` polls.  The waits return, so the CUDA
+ * context stays usable.  Synchronous; each allocates at most 2 KB of device memory.
+ * dv_selftest_wait_timeout: the tensor-core products' mbarrier wait on a barrier nothing arrives at, and
+ * the cooperative FD matvec's grid barrier with one block that never arrives.  *bits receives the error
+ * word they set (1: the mbarrier wait, 4: the grid barrier; 5 when both timed out as they must).
+ * dv_selftest_exchange_timeout: the Gram-Schmidt kernel's exchange between two blocks, of which the second
+ * publishes its sums only when publish != 0.  publish: *bits = 0 and *sum = 768 (256 times 1 and 2);
+ * else *bits = 4, the bit on which a solve reports the timeout, and *sum = 0. */
 int dv_selftest_wait_timeout(int32_t polls, int32_t* bits);
+int dv_selftest_exchange_timeout(int32_t polls, int32_t publish, double* sum, int32_t* bits);
 /* Failure-injection hook on the host (no reference counterpart): sets the model's device error word
  * to `bits` as a bounded wait that gave up would.  The model's next synchronising call reports
  * DV_ERR_CUDA with the wait named, then clears the word and the reduction tickets the abandoned wait

@@ -47,3 +47,16 @@ def test_model_recovers_after_a_reported_timeout():
         TRBDF2(m, cfg, h_max=0.5).integrate(d["y"], 2.0, [2.0])
     res = TRBDF2(m, cfg, h_max=0.5).integrate(d["y"], 2.0, [2.0])
     assert res.t == pytest.approx(2.0) and np.all(np.isfinite(res.y))
+
+
+@pytest.mark.parametrize("polls", [1, 1000])
+def test_gram_schmidt_exchange_gives_up_and_reports(polls):
+    """The exchange every Arnoldi step waits in: with a block that never publishes its sums it gives up after
+    `polls` polls and sets the bit that a solve reports; with both blocks it delivers their sums."""
+    from dac_vtsa_b200 import _lib
+    lib = _lib.load()
+    total, bits = C.c_double(-1.0), C.c_int32(-1)
+    assert lib.dv_selftest_exchange_timeout(polls, 0, C.byref(total), C.byref(bits)) == 0, lib.dv_last_error()
+    assert (bits.value, total.value) == (4, 0.0)
+    assert lib.dv_selftest_exchange_timeout(1 << 22, 1, C.byref(total), C.byref(bits)) == 0, lib.dv_last_error()
+    assert (bits.value, total.value) == (0, 768.0)
