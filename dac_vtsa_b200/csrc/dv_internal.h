@@ -88,7 +88,8 @@ struct Work {
     cudaGraph_t gm_graph = nullptr;
     cudaGraphExec_t gm_exec = nullptr;
     cudaStream_t gm_cs = nullptr;             // capture stream
-    int gm_kdim = 0, gm_mode = -1, gm_nb = 0, gm_nparts = 0, gm_fp32 = -1, gm_zs = -1, gm_op32 = -1, gm_tuned = -2;
+    int gm_kdim = 0, gm_mode = -1, gm_nb = 0, gm_nparts = 0, gm_fp32 = -1, gm_zs = -1, gm_op32 = -1;
+    dv_tuning gm_tune = {};                   // the model's tuning the graph was captured with
     int gm_prefix = 0;                        // Arnoldi steps captured ahead of the WHILE node
     int gm_body = 1;                          // Arnoldi steps per pass through the WHILE body
     int64_t gm_fixed[K_NKIND] = {}, gm_iter[K_NKIND] = {};   // launches per graph run: fixed + per iteration

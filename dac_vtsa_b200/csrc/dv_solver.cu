@@ -1888,7 +1888,7 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
     W.gm_prefix = prefix;
     W.gm_fp32 = m->pc_fp32;
     W.gm_op32 = m->op32;
-    W.gm_tuned = m->tune.gmres_prefix;
+    W.gm_tune = m->tune;
     W.gm_body = body_steps;
     for (int k = 0; k < K_NKIND; ++k) {
         W.gm_fixed[k] = fixed[k];
@@ -1914,7 +1914,8 @@ static int gmres_graph(Work& W, const Op& op, const double* b, double rtol, doub
     dv_model* m = op.m;
     if (!W.gm_exec || W.gm_kdim != kdim || W.gm_mode != m->pc_mode || W.gm_nb != m->pc_nb ||
         W.gm_nparts != m->pc_nparts || W.gm_fp32 != m->pc_fp32 || W.gm_zs != m->pc_zs ||
-        W.gm_op32 != m->op32 || W.gm_tuned != m->tune.gmres_prefix ||
+        W.gm_op32 != m->op32 || W.gm_tune.gmres_prefix != m->tune.gmres_prefix ||
+        W.gm_tune.sweep_nbuf != m->tune.sweep_nbuf || W.gm_tune.spmv_block != m->tune.spmv_block ||
         (precond_apply_fusable(m) && W.gm_body != gmres_body(m)))
         DV_TRY(gm_build(m, W, kdim));
     GmHost* hst = (GmHost*)W.gm_host;

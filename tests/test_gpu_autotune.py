@@ -54,3 +54,37 @@ def test_tuned_parameters_do_not_change_results(tmp_path, monkeypatch):
     assert list(table.values())[0]["params"] == chosen
     d, m2, _, _ = _c0()
     assert autotune.cached(m2, d["s0_y0"], dh=0.5) == chosen and autotune.get(m2) == chosen
+
+
+def test_gmres_graph_follows_the_sweep_prefetch():
+    """A sweep_nbuf set after a solve takes effect in the GMRES graph too (the sweep kernel's variant is fixed at
+    capture), with the same bits."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from dac_vtsa_b200 import autotune, host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.jacobian import FDJacobian
+    from dac_vtsa_b200.model import TVSAModel
+    cfg = load_config(override_dict={"grid.Nr": 7, "grid.Ntheta": 3, "grid.Nz": 9})
+    g = host.Grid.from_config(cfg)
+    st = host.seeded_state(cfg, g, host.get_backend(cfg), seed=2)
+    m = TVSAModel(cfg, g, host.get_backend(cfg), cfg.cycle[0], st)
+    y = torch.from_numpy(m.pack(st)).to(m.device)
+    m.precond_factor(FDJacobian(m).block(1.0, y), 0.05)
+
+    def solve(nbuf):
+        autotune.apply(m, {"sweep_nbuf": nbuf})
+        z = m.newton_stage(1.05, y, y, 0.05)[0]
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            m.newton_stage(1.05, y, y, 0.05)
+            torch.cuda.synchronize()
+        names = {e.name.split("(dv::")[0] for e in p.events() if "k_pc_apply<" in e.name}
+        if not names:
+            pytest.skip("the profiler delivered no kernel names")
+        return z, names
+
+    z2, without = solve(2)
+    z3, with_prefetch = solve(3)
+    assert torch.equal(z2, z3)
+    assert not without & with_prefetch, (without, with_prefetch)
