@@ -1,13 +1,12 @@
 """Launch-parameter autotuner: picks the hot kernels' launch parameters per grid shape and caches them.
 
 ``tune(model, y, dh)`` runs the library's timer (dv_autotune) on the model at state y: every candidate
-of the preconditioner sweep's L2 prefetch (and of the FD Jacobian's block size, which its kernels no
-longer have), the FP32 Jacobian product's
-block size and the GMRES graph's prefix of unrolled Arnoldi steps, timed with CUDA events on the
-model's own matrices; the fastest of each is kept in the model.  ``cached(model)`` applies an earlier
-result for the same grid, preconditioner, precision and GPU from the cache file (``$DVTSA_TUNE_CACHE``,
-default ``~/.cache/dac_vtsa_b200/tune.json``) and tunes on a miss.  The parameters never change a result
-bit, only the time.
+of the preconditioner sweep's L2 prefetch, the FP32 Jacobian product's block size and the GMRES graph's
+prefix and body of unrolled Arnoldi steps, timed with CUDA events on the model's own matrices; the fastest
+of each is kept in the model.  (fdjac_block is accepted and unused: the FD Jacobian's kernels have one block
+shape each.)  ``cached(model)`` applies an earlier result for the same grid, preconditioner, precision and
+GPU from the cache file (``$DVTSA_TUNE_CACHE``, default ``~/.cache/dac_vtsa_b200/tune.json``) and tunes on a
+miss.  The parameters never change a result bit, only the time.
 """
 from __future__ import annotations
 
@@ -25,6 +24,9 @@ FIELDS = ("gmres_prefix", "sweep_nbuf", "spmv_block", "fdjac_block", "gmres_body
 TIMES = ("fdjac_64", "fdjac_128", "sweep_nbuf2", "sweep_nbuf3", "spmv_64", "spmv_128", "spmv_256",
          "stage_prefix0", "stage_prefix2", "stage_prefix4", "stage_prefix6", "stage_prefix8",
          "stage_body1", "stage_body2")
+# What the fields mean; entries of another version are measured again.  1 (no suffix): sweep_nbuf was the depth of
+# the sweep's shared-memory ring; 2: it says whether the sweep prefetches its factors into L2.
+VERSION = 2
 
 
 def cache_path() -> str:
@@ -35,7 +37,8 @@ def cache_path() -> str:
 def key(model, precision: str = "fp64") -> str:
     g = model.grid
     name = torch.cuda.get_device_name(model.device).replace(" ", "_")
-    return f"{name}/{g.Nr}x{g.Nth}x{g.Nz}/wall{int(model.n_w > 0)}/{model.cfg.solver.preconditioner}/{precision}"
+    return (f"{name}/{g.Nr}x{g.Nth}x{g.Nz}/wall{int(model.n_w > 0)}/{model.cfg.solver.preconditioner}/{precision}"
+            f"/v{VERSION}")
 
 
 def get(model) -> Dict[str, int]:
