@@ -2769,20 +2769,15 @@ int dv_autotune(dv_model* m, double t, const double* y, double dh, int32_t reps,
     dv_tuning tu = m->tune;
     const int mode = m->pc_ready ? m->pc_mode : 2;
     DV_TRY(launch_rhs(m, t, y, W.f, nullptr, st));
-    // FD Jacobian block size
-    const int fj[2] = {64, 128};
+    // FD Jacobian: its kernels have one block shape each, so one time stands in both slots
+    DV_TRY(time_us(st, reps, [&] { return launch_fd_jacobian(m, t, y, W.f, W.J, st); }, &tm[0]));
+    tm[1] = tm[0];
+    if (tu.fdjac_block == 0) tu.fdjac_block = 128;
     double bestv = INFINITY;
-    for (int q = 0; q < 2; ++q) {
-        m->tune.fdjac_block = fj[q];
-        DV_TRY(time_us(st, reps, [&] { return launch_fd_jacobian(m, t, y, W.f, W.J, st); }, &tm[q]));
-        if (tm[q] < bestv) { bestv = tm[q]; tu.fdjac_block = fj[q]; }
-    }
-    m->tune.fdjac_block = tu.fdjac_block;
     DV_TRY(precond_factor(m, W.J, dh, mode, st));
     // prefetch of the sweep's factors into L2 (the register-streamed sweep only)
     DV_CUDA(cudaMemcpyAsync(W.b, W.f, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
     if (precond_apply_fusable(m)) {
-        bestv = INFINITY;
         for (int q = 0; q < 2; ++q) {
             m->tune.sweep_nbuf = 2 + q;
             DV_TRY(time_us(st, reps, [&] { return precond_apply(m, W.b, nullptr, W.x, st); }, &tm[2 + q]));

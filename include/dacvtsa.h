@@ -315,8 +315,8 @@ int dv_model_get_tuning(const dv_model* m, dv_tuning* t);
 /* Autotuner: at state y (time t) and stage coefficient dh, factorise I - dh J, then time every
  * candidate of each parameter (`reps` launches each; the GMRES prefix by whole Newton stage solves)
  * with CUDA events on `stream`, keep the fastest in the model and return it in *best.  times_us
- * (optional, ntimes entries) receives the measured per-launch times in the order: fdjac 64, 128;
- * sweep nbuf 2, 3; spmv 64, 128, 256; stage solve with prefix 0, 2, 4, 6, 8; stage solve with the
+ * (optional, ntimes entries) receives the measured per-launch times in the order: fdjac 64, 128 (one
+ * measurement: the value is not used, and stays or becomes 128); sweep nbuf 2, 3; spmv 64, 128, 256; stage solve with prefix 0, 2, 4, 6, 8; stage solve with the
  * chosen prefix and body 1, 2 (0 where a candidate does not apply).  Synchronises. */
 #define DV_TUNE_NTIMES 14
 int dv_autotune(dv_model* m, double t, const double* y, double dh, int32_t reps, dv_tuning* best, double* times_us,
