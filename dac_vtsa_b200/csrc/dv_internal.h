@@ -167,7 +167,7 @@ struct dv_model {
     dv::RecLayout rl;
     double* d_rec;                  // internal record scratch (accumulators)
     double* d_split;                // per-cell properties and per-face fluxes of the split residual
-    double* d_jac;                  // scratch of the finite-difference Jacobian
+    double* d_jac;                  // scratch of the finite-difference Jacobian (null: it did not fit)
     cudaEvent_t jac_ev;             // end of the last Jacobian (its scratch is free for another stream)
     int jac_used;                   // jac_ev has been recorded
     double* d_diag;                 // diagnostics record of the outlet summary (dv_outlet_row)

@@ -854,6 +854,26 @@ static __device__ __forceinline__ double jac_quot(double d, double h) {
     return (d == 0.0 && h > 0.0 && h < 1e300) ? d : d / h;
 }
 
+// Cell (ni, nj, nk) in neighbour slot `slot` of row cell (i, j, k); false where the grid has none, or where
+// column variable cv is a wall temperature and that cell has no wall node.
+static __device__ __forceinline__ bool jac_neighbour(const dv_step_params& p, int slot, int cv, int i, int j, int k,
+                                                     int& ni, int& nj, int& nk) {
+    ni = i, nj = j, nk = k;
+    bool ok = true;
+    switch (slot) {
+        case 0: break;
+        case 1: nk = k - 1; ok = nk >= 0; break;
+        case 2: nk = k + 1; ok = nk < p.Nz; break;
+        case 3: nk = k - 2; ok = nk >= 0; break;
+        case 4: nk = k + 2; ok = nk < p.Nz; break;
+        case 5: ni = i - 1; ok = ni >= 0; break;
+        case 6: ni = i + 1; ok = ni < p.Nr; break;
+        case 7: ok = p.Nth > 1; nj = (j == 0) ? p.Nth - 1 : j - 1; break;
+        default: ok = p.Nth > 1; nj = (j == p.Nth - 1) ? 0 : j + 1; break;
+    }
+    return cv == DV_NV ? ok && p.wall_on && ni == p.Nr - 1 : ok;
+}
+
 // One warp per column variable cv (0..6) of a tile of 32 row cells, blockIdx.y = neighbour slot: the
 // seven warps read the same unperturbed fluxes and properties (one of them from L2, the others from L1)
 // and each (row, column) plane of J is written coalesced.
@@ -870,22 +890,9 @@ __global__ void __launch_bounds__(DV_NB * 32, 3) k_jac_rows(dv_step_params p, Au
     cell_ijk(p, c, i, j, k);
     const int Nr = p.Nr, Nth = p.Nth, Nz = p.Nz;
     const int jm = (j == 0) ? Nth - 1 : j - 1;
-    int ni = i, nj = j, nk = k;
-    bool ok = true;
-    switch (slot) {
-        case 0: break;
-        case 1: nk = k - 1; ok = nk >= 0; break;
-        case 2: nk = k + 1; ok = nk < Nz; break;
-        case 3: nk = k - 2; ok = nk >= 0; break;
-        case 4: nk = k + 2; ok = nk < Nz; break;
-        case 5: ni = i - 1; ok = ni >= 0; break;
-        case 6: ni = i + 1; ok = ni < Nr; break;
-        case 7: ok = Nth > 1; nj = jm; break;
-        default: ok = Nth > 1; nj = (j == Nth - 1) ? 0 : j + 1; break;
-    }
-    if (cv == DV_NV) ok = ok && p.wall_on && (ni == Nr - 1);
+    int ni, nj, nk;
     TJ* Jb = J + ((int64_t)slot * DV_NB * DV_NB + cv) * nc + c;         // row stride DV_NB*nc
-    if (!ok) {
+    if (!jac_neighbour(p, slot, cv, i, j, k, ni, nj, nk)) {
 #pragma unroll
         for (int rv = 0; rv < DV_NB; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)0.0;
         return;
@@ -930,6 +937,36 @@ __global__ void __launch_bounds__(DV_NB * 32, 3) k_jac_rows(dv_step_params p, Au
     for (int rv = 0; rv < DV_NV; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)jac_quot(f[rv] - f0[rv * nc + c], h);
     Jb[(int64_t)DV_NV * DV_NB * nc] =
         (TJ)(outer_wall ? jac_quot(fw - f0[(int64_t)DV_NV * nc + (int64_t)j * Nz + k], h) : 0.0);
+}
+
+// The same entries without scratch: a thread evaluates its whole row for one (neighbour slot, column) pair,
+// blockIdx.y = slot * 7 + cv.  155 us at 8x8x32, 1270 at 16x16x64 (above: 34, 172): for calls that may not use
+// the model's scratch.
+template <class TJ>
+__global__ void __launch_bounds__(128) k_jac_cells(dv_step_params p, Aux aux, double t, const double* __restrict__ y,
+                                                   const double* __restrict__ f0, TJ* __restrict__ J) {
+    const int64_t nc = (int64_t)p.Nr * p.Nth * p.Nz;
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nc) return;
+    const int slot = blockIdx.y / DV_NB, cv = blockIdx.y % DV_NB;
+    int i, j, k, ni, nj, nk;
+    cell_ijk(p, c, i, j, k);
+    TJ* Jb = J + ((int64_t)slot * DV_NB * DV_NB + cv) * nc + c;         // row stride DV_NB*nc
+    if (!jac_neighbour(p, slot, cv, i, j, k, ni, nj, nk)) {
+#pragma unroll
+        for (int rv = 0; rv < DV_NB; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)0.0;
+        return;
+    }
+    const int64_t n = ((int64_t)ni * p.Nth + nj) * p.Nz + nk;           // the column's cell
+    const int64_t col = (cv < DV_NV) ? (int64_t)cv * nc + n : (int64_t)DV_NV * nc + (int64_t)nj * p.Nz + nk;
+    const double h = fd_step(p, y[col], cv);
+    const bool outer_wall = (i == p.Nr - 1) && p.wall_on;
+    double f[DV_NV], fw = 0.0;
+    cell_eval(p, aux, LoadPert{y, col, h}, t, i, j, k, f, outer_wall ? &fw : nullptr, (const Rec*)nullptr);
+#pragma unroll
+    for (int rv = 0; rv < DV_NV; ++rv) Jb[(int64_t)rv * DV_NB * nc] = (TJ)jac_quot(f[rv] - f0[rv * nc + c], h);
+    Jb[(int64_t)DV_NV * DV_NB * nc] =
+        (TJ)(outer_wall ? jac_quot(fw - f0[(int64_t)DV_NV * nc + (int64_t)j * p.Nz + k], h) : 0.0);
 }
 
 // ---------------------------------------------------------------- residual of a tile in one launch
@@ -1515,15 +1552,22 @@ int matvec_capture(dv_model* m, const double* dargs, const double* z, const doub
 template <class TJ>
 static int fd_jacobian(dv_model* m, double t, const double* y, const double* f0, TJ* J, cudaStream_t s) {
     const dv_step_params& p = m->p;
+    // The scratch belongs to one Jacobian at a time: a call on another stream waits for the last one (jac_ev).  A
+    // captured call cannot: its graph runs later, and nothing orders it against other calls.  So it takes the
+    // form without scratch, as does a model whose scratch did not fit on the device.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    DV_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone || !m->d_jac) {
+        DV_LAUNCH(dv::K_FDJAC, s, k_jac_cells<TJ><<<dim3(nblk(m->nc, 128), DV_NSLOT * DV_NB), 128, 0, s>>>(p, aux_of(m), t, y,
+                                                                                                         f0, J));
+        DV_CUDA(cudaGetLastError());
+        return DV_OK;
+    }
     const JacScratch X = jac_scratch_of(p, m->d_jac);
     const Split& S = X.S;
     const int64_t ncol = (int64_t)p.Nr * p.Nth, nw = (int64_t)p.Nth * p.Nz;
     const int64_t nfaces = ncol * (p.Nz - 1) + (p.Nr > 1 ? S.nrf : 0) + (p.Nth > 1 ? S.ntf : 0) + 2 * ncol;
-    // the scratch belongs to one Jacobian at a time: a call on another stream waits for the last one
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    DV_CUDA(cudaStreamIsCapturing(s, &cap));
-    const bool order = cap == cudaStreamCaptureStatusNone;
-    if (order && m->jac_used) DV_CUDA(cudaStreamWaitEvent(s, m->jac_ev, 0));
+    if (m->jac_used) DV_CUDA(cudaStreamWaitEvent(s, m->jac_ev, 0));
     DV_LAUNCH(dv::K_FDJAC, s, k_jac_props<<<dim3(nblk(m->nc, 32), JAC_VAR), CP_WARPS * 32, 0, s>>>(p, S, y));
     // x covers the z faces (the most of the perturbed kinds) and the unperturbed index space
     const unsigned gx = std::max(nblk(S.nzf, 32), nblk(nfaces + JAC_VAR * nw, JF_THREADS));
@@ -1531,10 +1575,8 @@ static int fd_jacobian(dv_model* m, double t, const double* y, const double* f0,
     DV_LAUNCH(dv::K_FDJAC, s, k_jac_rows<TJ><<<dim3(nblk(m->nc, 32), DV_NSLOT), DV_NB * 32, 0, s>>>(p, aux_of(m), X, t, y,
                                                                                                  f0, J));
     DV_CUDA(cudaGetLastError());
-    if (order) {
-        DV_CUDA(cudaEventRecord(m->jac_ev, s));
-        m->jac_used = 1;
-    }
+    DV_CUDA(cudaEventRecord(m->jac_ev, s));
+    m->jac_used = 1;
     return DV_OK;
 }
 

@@ -2993,7 +2993,6 @@ int dv_model_create(const dv_step_params* p, const double* feed_flux, const doub
     bool fail = pool_malloc((void**)&m->d_aux, sizeof(double) * (2 * nf + nwall)) != cudaSuccess ||
                 pool_malloc((void**)&m->d_rec, sizeof(double) * rec_n) != cudaSuccess ||
                 pool_malloc((void**)&m->d_split, sizeof(double) * split_doubles(*p)) != cudaSuccess ||
-                pool_malloc((void**)&m->d_jac, sizeof(double) * jac_scratch_doubles(*p)) != cudaSuccess ||
                 pool_malloc((void**)&m->d_diag, sizeof(double) * m->rl.total) != cudaSuccess ||
                 pool_malloc((void**)&m->d_acc, sizeof(double) * DV_NACC) != cudaSuccess ||
                 pool_malloc((void**)&m->d_pc, sizeof(double) * pc_need) != cudaSuccess ||
@@ -3012,7 +3011,6 @@ int dv_model_create(const dv_step_params* p, const double* feed_flux, const doub
     }
     debug_fill(m->d_rec, sizeof(double) * rec_n, 1);
     debug_fill(m->d_split, sizeof(double) * split_doubles(*p), 1);
-    debug_fill(m->d_jac, sizeof(double) * jac_scratch_doubles(*p), 1);
     debug_fill(m->d_diag, sizeof(double) * m->rl.total, 1);
     debug_fill(m->d_acc, sizeof(double) * DV_NACC, 1);
     debug_fill(m->d_pc, sizeof(double) * pc_need, 1);
@@ -3027,6 +3025,11 @@ int dv_model_create(const dv_step_params* p, const double* feed_flux, const doub
         dv_model_destroy(m);
         return rc;
     }
+    // last, and no failure when it does not fit: the Jacobian then runs without it
+    const char* js = getenv("DVTSA_JAC_SCRATCH");
+    if (js && js[0] == '0') m->d_jac = nullptr;
+    else if (pool_malloc((void**)&m->d_jac, sizeof(double) * jac_scratch_doubles(*p)) != cudaSuccess) cudaGetLastError();
+    else debug_fill(m->d_jac, sizeof(double) * jac_scratch_doubles(*p), 1);
     cudaMemcpy(m->d_aux, feed_flux, sizeof(double) * nf, cudaMemcpyHostToDevice);
     cudaMemcpy(m->d_aux + nf, n_nom, sizeof(double) * nf, cudaMemcpyHostToDevice);
     cudaMemcpy(m->d_aux + 2 * nf, coverage, sizeof(double) * nwall, cudaMemcpyHostToDevice);

@@ -191,7 +191,9 @@ int dv_colour_columns(int32_t Nr, int32_t Nth, int32_t Nz, int32_t wall, int64_t
 /* Forward-difference Jacobian df/dy at (t, y) with f0 = f(t, y) (FDJacobian.__call__,
  * core/jacobian.py:71-86): every colour perturbation in one call.  J is the block layout
  * J[slot][row 0..6][col 0..6][cell] (jac_doubles): d f_row(cell) / d y_col(neighbour `slot`),
- * row/col 6 = the wall unknown of an outer-ring cell.  Same step rule h = 1.5e-8 max(|y|, typ). */
+ * row/col 6 = the wall unknown of an outer-ring cell.  Same step rule h = 1.5e-8 max(|y|, typ).  Uses
+ * scratch of the model (about 340 doubles a cell, allocated with it where it fits; calls on different
+ * streams wait for one another); in a stream capture a slower form that needs none, same bits. */
 int dv_fd_jacobian(dv_model* m, double t, const double* y, const double* f0, double* J, void* stream);
 
 /* ------------------------------------------------------------------ preconditioner

@@ -86,3 +86,45 @@ def test_jacobian_entries_are_the_quotients_of_the_residual(grid, step):
         # (divided by numpy: torch multiplies a CUDA tensor by a scalar's rounded reciprocal)
         ref[:, col] = (m.rhs(3.0, yp, want_acc=False)[0] - f0).cpu().numpy() / h
     assert np.array_equal(J, ref)
+
+
+@pytest.mark.parametrize("grid", [(1, 1, 9), (3, 5, 7), (8, 8, 12)])
+def test_jacobian_without_scratch_and_in_a_captured_graph(grid, monkeypatch):
+    """A model without the Jacobian's scratch, and a captured call, give the same bits; replays of the captured
+    call run beside direct calls at another state on another stream (no order between them, no shared scratch)."""
+    import ctypes as C
+    import torch
+    from dac_vtsa_b200 import host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.jacobian import FDJacobian
+    from dac_vtsa_b200.model import TVSAModel
+    cfg = load_config(override_dict={"grid.Nr": grid[0], "grid.Ntheta": grid[1], "grid.Nz": grid[2]})
+    g = host.Grid.from_config(cfg)
+    props = host.get_backend(cfg)
+    st = host.seeded_state(cfg, g, props, seed=5, amplitude=0.02)
+    m = TVSAModel(cfg, g, props, cfg.cycle[0], st)
+    y1 = torch.from_numpy(m.pack(st)).to(m.device)
+    y2 = y1 * 1.001
+    f1, f2 = m.rhs(3.0, y1, want_acc=False)[0], m.rhs(3.0, y2, want_acc=False)[0]
+    J1, J2 = FDJacobian(m).block(3.0, y1, f1), FDJacobian(m).block(3.0, y2, f2)
+    monkeypatch.setenv("DVTSA_JAC_SCRATCH", "0")
+    bare = TVSAModel(cfg, g, props, cfg.cycle[0], st)
+    assert torch.equal(FDJacobian(bare).block(3.0, y1, f1), J1)
+
+    def call(y, f, J, stream):
+        assert m.lib.dv_fd_jacobian(m.handle, 3.0, y.data_ptr(), f.data_ptr(), J.data_ptr(),
+                                    C.c_void_p(stream.cuda_stream)) == 0, m.lib.dv_last_error()
+
+    out1 = torch.full_like(J1, np.nan)
+    out2 = [torch.full_like(J2, np.nan) for _ in range(20)]
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        call(y1, f1, out1, torch.cuda.current_stream())
+    for o in out2:
+        graph.replay()
+        call(y2, f2, o, side)
+    torch.cuda.synchronize()
+    assert torch.equal(out1, J1)
+    assert all(torch.equal(o, J2) for o in out2)
