@@ -1178,8 +1178,12 @@ constexpr int pa_threads(int NJ) { return NJ <= 2 ? 128 : 64 * NJ; }       // 8 
 
 // stages of a CTA that holds np planes, at most (both ranks)
 constexpr int pa_stages(int np, bool tw) { return tw ? 2 * np - 2 : 2 * np - 1; }
+// The kernel's last parameter ALT.  Twisted: prefetch into L2 as above.  Top-down: a stage's blocks are worked out
+// when they are fetched, instead of looked up in a table in shared memory -- only where small blocks in a long
+// column leave no room for the table beside the planes (1x1x806 in FP64 and beyond), as it is slower (1x1x700:
+// 324 -> 368 us, 4x1x200: 143 -> 154).
 
-template <int NJ, typename TS, bool TW, bool AH>
+template <int NJ, typename TS, bool TW, bool ALT>
 __global__ void __launch_bounds__(pa_threads(NJ), 1) k_pc_apply(PcGeom gin, const TS* __restrict__ A,
                                                                 const double* __restrict__ b,
                                                                 const double* __restrict__ sc, double* __restrict__ x,
@@ -1188,6 +1192,7 @@ __global__ void __launch_bounds__(pa_threads(NJ), 1) k_pc_apply(PcGeom gin, cons
     pdl_trigger();
     extern __shared__ __align__(128) double dsm[];
     constexpr int LD = NJ * 2 * PA_LANES, NT = pa_threads(NJ), DEPTH = PA_DEPTH;
+    constexpr bool AH = TW && ALT, TABLE = TW || !ALT;
     using TS2 = typename std::conditional<std::is_same<TS, float>::value, float2, double2>::type;
     const int rank = TW ? (int)(blockIdx.x & 1u) : 0;
     const int part = TW ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -1203,17 +1208,17 @@ __global__ void __launch_bounds__(pa_threads(NJ), 1) k_pc_apply(PcGeom gin, cons
     double* xs = dsm;                          // [np][LD] local planes: b, then z (forward, in place); r on the separator
     double* xb = xs + np * LD;                 // [np][LD]: x (backward sweep); padding columns zero
     double* xch = xb + np * LD;                // [2][LD]: this rank's partial right-hand sides of the separator (TW)
-    int4* desc = reinterpret_cast<int4*>(xch + 2 * LD);     // [S + DEPTH]: offsets of a stage's blocks (-1: none)
-    int* gl = reinterpret_cast<int*>(desc + pa_stages(np, TW) + DEPTH);     // [LD]: state index of row l at plane 0
+    int4* desc = reinterpret_cast<int4*>(xch + 2 * LD);     // [S + DEPTH] (table): offsets of a stage's blocks (-1: none)
+    int* gl = reinterpret_cast<int*>(desc + (TABLE ? pa_stages(np, TW) + DEPTH : 0));     // [LD]: state index of row l at plane 0
     const int stopped = F.stop ? *F.stop : 0;
     const int fcol = F.V ? *F.col : 0;
     const double fscale = F.V ? *F.scale : 0.0;
     // a geometry beyond the storage is recorded and x is left untouched (the same on every CTA of a partition)
     if (!pc_range_ok(g, (int64_t)part * Nz * 5 * bs, (int64_t)Nz * 5 * bs)) return;
     const TS* base = A + (int64_t)part * Nz * 5 * bs;
-    // the stages' blocks, in the order their products are added (one code path then fetches any stage)
-    for (int s = tid; s < S + DEPTH; s += NT) {
-        int o[3] = {-1, -1, -1};
+    // a stage's blocks, in the order their products are added
+    auto blocks = [&](int s, int (&o)[3]) {
+        o[0] = o[1] = o[2] = -1;
         auto blk = [&](int t, int sl) { return (fr.gp(t) * 5 + fr.gs(sl)) * bs; };
         if (s >= S) {
         } else if (s < n - 1) {                            // F(t), t = s + 1
@@ -1233,6 +1238,10 @@ __global__ void __launch_bounds__(pa_threads(NJ), 1) k_pc_apply(PcGeom gin, cons
             if (TW || t + 1 < Nz) o[1] = blk(t, 3);
             if (TW || t + 2 < Nz) o[2] = blk(t, 4);
         }
+    };
+    for (int s = TABLE ? tid : S + DEPTH; s < S + DEPTH; s += NT) {
+        int o[3];
+        blocks(s, o);
         // (the blocks of a stage are one run of slots, but for X's third: the run's first and its blocks)
         const bool x3 = TW && s == n - 1;
         const int first = o[1] < 0 ? o[0] : (o[2] < 0 || x3) ? min(o[0], o[1]) : min(o[0], o[2]);
@@ -1262,8 +1271,13 @@ __global__ void __launch_bounds__(pa_threads(NJ), 1) k_pc_apply(PcGeom gin, cons
     };
     Blk R[DEPTH][3];
     auto load = [&](int s, Blk (&M)[3]) {
-        const int4 d = desc[s];
-        const int o[3] = {d.x, d.y, d.z};
+        int o[3];
+        if constexpr (TABLE) {
+            const int4 d = desc[s];
+            o[0] = d.x, o[1] = d.y, o[2] = d.z;
+        } else {
+            blocks(s, o);
+        }
 #pragma unroll
         for (int e = 0; e < 3; ++e)
             if (o[e] >= 0) {
@@ -1821,13 +1835,20 @@ template <int NJ, typename TS, bool TW>
 static void launch_apply_tw(const PcGeom& g, dv_model* m, const TS* A, const double* b, const double* sc, double* x,
                             cudaStream_t s, const PaFuse& F, bool count) {
     const int np = TW ? std::max(g.zs, g.Nz - g.zs - 2) + 2 : g.Nz;
-    const size_t dyn = sizeof(double) * (size_t)(2 * np + 2) * g.ld + sizeof(int4) * (size_t)(pa_stages(np, TW) + PA_DEPTH) +
-                       sizeof(int) * (size_t)g.ld;
-    const int64_t bytes = (int64_t)sizeof(TS) * g.nparts * g.Nz * 5 * g.bs;
-    bool ah = m->tune.sweep_nbuf == 3 || (m->tune.sweep_nbuf != 2 && bytes > PA_L2_BYTES);
+    const size_t planes = sizeof(double) * (size_t)(2 * np + 2) * g.ld + sizeof(int) * (size_t)g.ld;
+    const size_t table = sizeof(int4) * (size_t)(pa_stages(np, TW) + PA_DEPTH);
+    size_t dyn = planes + table;
     auto kern = k_pc_apply<NJ, TS, TW, false>;
     if constexpr (TW && NJ >= 3) {              // (smaller blocks add up to PA_L2_BYTES on no supported cross-section)
-        if (ah) kern = k_pc_apply<NJ, TS, TW, true>;
+        const int64_t bytes = (int64_t)sizeof(TS) * g.nparts * g.Nz * 5 * g.bs;
+        if (m->tune.sweep_nbuf == 3 || (m->tune.sweep_nbuf != 2 && bytes > PA_L2_BYTES)) kern = k_pc_apply<NJ, TS, TW, true>;
+    }
+    if constexpr (!TW && NJ <= 2) {             // (larger blocks: the rule's six are more than a table for its planes)
+        constexpr size_t own = 256;             // static shared memory of the kernel (at most)
+        if (dyn + own > (size_t)smem_optin()) {
+            kern = k_pc_apply<NJ, TS, TW, true>;
+            dyn = planes;
+        }
     }
     if (dyn > 48 * 1024) allow_dyn_smem((const void*)kern);
     if (count) prof_begin(dv::K_PC_APPLY, s);

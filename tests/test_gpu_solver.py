@@ -212,6 +212,21 @@ def test_twisted_factorisation_matches_one_directional(Nz, mode, monkeypatch):
     assert 0.0 < rel < 1e-13, rel
 
 
+@pytest.mark.parametrize("Nz", [805, 806, 886, 887])
+def test_top_down_sweep_at_the_limits_of_shared_memory(Nz, monkeypatch):
+    """1-D columns at the last and first number of planes whose stage descriptors, and whose planes by the sweep's
+    rule, fit in shared memory: the top-down solve agrees with the twisted one (dominant system, rounding)."""
+    m, _ = _pc_model(Nz, 1, 1)
+    Jd, _ = _dominant_jacobian(m, 3)
+    b = np.random.default_rng(5).standard_normal(m.n_core)
+    m.precond_factor(Jd, 1.0, "theta_block")
+    x_tw = m.precond_solve(b)
+    monkeypatch.setenv("DVTSA_PC_TWIST", "0")
+    m.precond_factor(Jd, 1.0, "theta_block")
+    x_one = m.precond_solve(b)
+    assert np.abs(x_tw - x_one).max() <= 1e-13 * np.abs(x_one).max()
+
+
 @pytest.mark.parametrize("dh", [2.1, 300.0])
 @pytest.mark.parametrize("Nz", [17, 32])
 def test_twisted_separator_inverse_on_stiff_stage_matrix(Nz, dh, monkeypatch):
