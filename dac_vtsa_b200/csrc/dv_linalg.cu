@@ -1168,8 +1168,9 @@ struct PcFrame {
 #define PA_DEPTH 2         // stages whose factors are in flight ahead of their use
 // Factors that do not stay in L2 (126 MB) from one sweep to the next are also prefetched into it, PA_AHEAD
 // stages ahead.  The line lies between 86 MB, where prefetching what is already there costs 4 % (12x12x48:
-// 27.4 -> 28.6 us), and 100 MB, where it gains 6 % (16x16x64 in FP32: 50.5 -> 47.4 us); at 117 MB 47.4 ->
-// 39.4 us, at 182 MB 57.8 -> 46.4 us (8 stages: 46.9, 16: 55.6).
+// 27.4 -> 28.6 us), and 94 MB, where it gains 23 % (4x64x48 in sectors: 33.4 -> 25.8 us; 16x16x64 in FP32, 100 MB:
+// 50.5 -> 47.4); at 162 MB 50.8 -> 36.8 us (5x64x64 in sectors), at 182 MB 57.6 -> 46.5 us (16x16x64; 8 stages
+// ahead: 46.9, 16: 55.6).
 #define PA_AHEAD 4
 #define PA_L2_BYTES (90ll << 20)
 #define PA_IO 4            // entries per thread whose loads the prologue / epilogue batch
@@ -1839,7 +1840,7 @@ static void launch_apply_tw(const PcGeom& g, dv_model* m, const TS* A, const dou
     const size_t table = sizeof(int4) * (size_t)(pa_stages(np, TW) + PA_DEPTH);
     size_t dyn = planes + table;
     auto kern = k_pc_apply<NJ, TS, TW, false>;
-    if constexpr (TW && NJ >= 3) {              // (smaller blocks add up to PA_L2_BYTES on no supported cross-section)
+    if constexpr (TW) {
         const int64_t bytes = (int64_t)sizeof(TS) * g.nparts * g.Nz * 5 * g.bs;
         if (m->tune.sweep_nbuf == 3 || (m->tune.sweep_nbuf != 2 && bytes > PA_L2_BYTES)) kern = k_pc_apply<NJ, TS, TW, true>;
     }

@@ -88,3 +88,34 @@ def test_gmres_graph_follows_the_sweep_prefetch():
     z3, with_prefetch = solve(3)
     assert torch.equal(z2, z3)
     assert not without & with_prefetch, (without, with_prefetch)
+
+
+@pytest.mark.parametrize("grid", [(1, 3, 9), (2, 3, 9), (7, 3, 9), (9, 3, 9)])
+def test_sweep_prefetch_is_honoured_at_every_block_size(grid):
+    """sweep_nbuf 2 and 3 select the sweep without and with the L2 prefetch for blocks of 7, 18, 37 and 49
+    unknowns (leading dimensions 16 to 64), with the same bits."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from dac_vtsa_b200 import autotune, host
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.jacobian import FDJacobian
+    from dac_vtsa_b200.model import TVSAModel
+    cfg = load_config(override_dict={"grid.Nr": grid[0], "grid.Ntheta": grid[1], "grid.Nz": grid[2]})
+    g = host.Grid.from_config(cfg)
+    st = host.seeded_state(cfg, g, host.get_backend(cfg), seed=2)
+    m = TVSAModel(cfg, g, host.get_backend(cfg), cfg.cycle[0], st)
+    y = torch.from_numpy(m.pack(st)).to(m.device)
+    m.precond_factor(FDJacobian(m).block(1.0, y), 0.05)
+    out = {}
+    for nbuf in (2, 3):
+        autotune.apply(m, {"sweep_nbuf": nbuf})
+        m.precond_solve(y)
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            out[nbuf] = m.precond_solve(y)
+            torch.cuda.synchronize()
+        names = {e.name.split("(dv::")[0] for e in p.events() if "k_pc_apply<" in e.name}
+        if not names:
+            pytest.skip("the profiler delivered no kernel names")
+        assert all(n.endswith("true, %s>" % ("true" if nbuf == 3 else "false")) for n in names), names
+    assert torch.equal(out[2], out[3])
