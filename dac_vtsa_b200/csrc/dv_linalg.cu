@@ -737,13 +737,16 @@ static __device__ __noinline__ int tm_inverse_blk(Team T, int nb, int ld, double
 }
 
 // Inverse of the block A into X, by a team of 4 warps (the pointers may have been exchanged in all
-// threads of the block: `odd`); blocked when X can hold two panels.
+// threads of the block: `odd`); blocked when X can hold two panels (24 nb doubles of nb ld) and the block is large
+// enough for panels to pay (nb >= 21 in its own ld; smaller ones where the partition's largest block sets ld).
 struct InvWork {
     double pv[8];
     int pi[8], perm[64], idx[64], pos[64], prow[16];
     unsigned pmask[4];
 };
-static __device__ __forceinline__ bool inv_blocked(int nb, int ld) { return 16 * nb + 8 * ld <= nb * ld; }
+static __device__ __forceinline__ bool inv_blocked(int nb, int ld) {
+    return 2 * PAN_LD <= ld && 16 * nb + 8 * ld <= nb * ld;
+}
 static __device__ __forceinline__ int tm_inverse(const Team& T, int nb, int ld, double* A, double* X, InvWork& W) {
     if (inv_blocked(nb, ld)) return tm_inverse_blk(T, nb, ld, A, X, W.pos, W.prow, W.pmask);
     return tm_inverse_unb(T, nb, ld, A, X, W.perm, W.idx, W.pv, W.pi);
