@@ -202,7 +202,7 @@ struct ChainP {
     bf16* Xbt;
     const bf16 *W1, *W2, *W3, *W4, *W4t, *W3t, *W2t;
     const float* P;       // parameters (biases)
-    int64_t rows_valid;   // rows at or beyond this are zero in every output and carry no loss
+    int64_t rows_valid;   // rows at or beyond this: no loss, zero activations and gradients; O is not written there
     float* out;           // O [rows][NOUT] (forward)
     const float* tgt;     // targets [rows][8]
     float dscale;         // dL/dO = dscale * (O - target)

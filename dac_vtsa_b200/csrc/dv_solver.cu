@@ -1349,7 +1349,9 @@ __device__ __forceinline__ double cg_sum(double (*ps)[GM_PS], int q) {
 
 // E: elements a thread has at most (0: any number, w then stays in memory between the passes).  E = 1: its
 // basis entries stay in registers over the passes; E > 1: they are fetched eight entries of every element at
-// a time (from L1 after the first pass).
+// a time (from L1 after the first pass).  Over solves of 30 steps, against E = 0: 8x8x32 (E = 1) 13.2 -> 9.7 us a
+// step, 12x12x48 (2) 23.6 -> 17.9, 16x16x64 (3) 42.9 -> 27.6.  Beds of more elements a thread (16x16x80: 4, 53 us
+// with E = 0) take E = 0: larger E were not built.
 template <int E>
 __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const double* __restrict__ V, int64_t ldv,
                                                     double* __restrict__ w, CgWord* xw, int kdim,
@@ -1678,8 +1680,8 @@ static int gmres_coop() {
     return v;
 }
 
-// The GMRES operator's launches inside the graph: the FP64 finite-difference matvec (three residual
-// kernels) or, with the mixed-precision operator, one FP32 assembled-Jacobian product.
+// The GMRES operator's launches inside the graph: the FP64 finite-difference matvec (one kernel of
+// tiles, or the three of the split residual) or, with the mixed-precision operator, one FP32 assembled-Jacobian product.
 static int op_capture(dv_model* m, Work& W, const double* dargs, double* out, cudaStream_t c) {
     if (m->op32) return launch_spmv32(m, W.u, W.s, 0.0, dargs, out, c, false);
     return matvec_capture(m, dargs, W.z, W.u, W.s, W.f, W.scal, out, c, W.tickets + 11);
@@ -2210,8 +2212,7 @@ static int newton_krylov(NewtonCtx& C, double t, const double* z0, const double*
         }
         // polish: further restart cycles until the polish tolerance (1e-3 of ||b||) or the cycle
         // limit.  Each cycle solves A P^-1 x_c = b0 - A P^-1 (x_1 + .. x_c-1), the linear residual
-        // of the summed solution recomputed from it (the speculation queued behind the first cycle
-        // reused the GMRES residual vector, and is void anyway); the Newton step is then formed
+        // of the summed solution recomputed from it; the Newton step is then formed
         // from x = sum x_c, as from a single cycle's solution.
         const int pcyc = std::min(std::max(C.o.polish_cycles, 1), 8);
         if (polish && info != 0 && pcyc > 1) {
