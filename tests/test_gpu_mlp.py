@@ -110,3 +110,66 @@ def test_product_kernel_over_ring_and_remainders(M, N, K):
     ref = A.astype(np.float64) @ B.astype(np.float64).T
     bound = K * 2.0 ** -24 * (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T)
     assert (np.abs(D - ref) <= bound + 2.0 ** -24 * np.abs(ref)).all()
+
+
+def _drawn(seed, step, count):
+    """Sample indices of a training batch: the library's hash of seed, step and row."""
+    with np.errstate(over="ignore"):
+        x = (np.uint64(seed) * np.uint64(0x9E3779B97F4A7C15) + np.uint64(step) * np.uint64(1000003)
+             + np.arange(4096, dtype=np.uint64))
+        x ^= x >> np.uint64(30)
+        x *= np.uint64(0xBF58476D1CE4E5B9)
+        x ^= x >> np.uint64(27)
+        x *= np.uint64(0x94D049BB133111EB)
+        x ^= x >> np.uint64(31)
+    return (x % np.uint64(count)).astype(np.int64)
+
+
+def test_training_step_on_a_drawn_batch_matches_oracle():
+    """The batch a training step draws (hash, scaled and clipped targets, its transposed copy) against the
+    oracle on the same rows: the loss of 70 steps at learning rate 0 (more than are read back together), and
+    every block of the gradient, recovered from Adam's first step p - lr g / (|g| + 1e-8).  Outputs and targets
+    of about 1e-5 keep |g| where that step is far from saturated: |g| from 1e-13 (a change of 1e-5, FP32
+    parameters resolve 1e-8 of it) to 1e-5 (1 - |step| = 1e-3, resolved to 1e-4).  Tolerances of the tests above."""
+    import json
+    from cases import build, golden
+    from dac_vtsa_b200.model import TVSAModel
+    from dac_vtsa_b200.predictor import NewtonPredictor
+    from dac_vtsa_b200.solver import TRBDF2
+    d = golden("trajectory_c0.npz")
+    meta = json.loads(str(d["s0_meta"]))
+    m, cfg = build(TVSAModel, json.loads(str(d["over"])), meta["step"], d["s0_P0"], meta["T_jacket_prev"],
+                   duration=meta["duration"])
+    net = NewtonPredictor(sample_capacity=1 << 14, seed=1)
+    integ = TRBDF2(m, cfg, h_max=cfg.solver.h_max_fraction * meta["duration"])
+    net.attach(integ, "adsorption", predict=False, record_stride=1)
+    integ.integrate(d["s0_y0"], meta["duration"], [meta["duration"]])
+    X, T = net.get_samples()
+    P = om.init_params(seed=9, scale_out=1e-5)
+    P[-om.NOUT:] *= 1e-4
+    nrm = net.params()[1]
+    nrm[13:19] = 1e5 * np.maximum(np.sqrt(np.mean(T[:, :6].astype(np.float64) ** 2, axis=0)), 1e-6)
+    nrm[19] = 2e-5
+    tgt = np.clip(T[:, :6].astype(np.float64) / nrm[13:19], -nrm[19], nrm[19]).astype(np.float32)
+    assert (np.abs(tgt) == np.float32(nrm[19])).any()
+    seed = 123456789
+    net.set_params(P, nrm)
+    hist = net.train(70, lr=0.0, seed=seed, keep_scales=True)
+    out, _ = om.forward(P, X)
+    err = ((out[:, :6] - tgt) ** 2).mean(axis=1)
+    ref = np.array([err[_drawn(seed, k, len(X))].mean() for k in range(70)])
+    assert np.ptp(ref) > 10 * 2e-3 * ref.mean()                  # the batches differ by more than the tolerance
+    assert np.abs(hist / ref - 1.0).max() < 2e-3
+    net.set_params(P, nrm)                                       # the optimiser starts again, with batch 0
+    net.train(1, lr=1.0, seed=seed, keep_scales=True)
+    step = P.astype(np.float64) - net.params()[0].astype(np.float64)
+    g = 1e-8 * step / (1.0 - np.abs(step))
+    rows = _drawn(seed, 0, len(X))
+    go, _ = om.gradient(P, X[rows], np.pad(tgt[rows], ((0, 0), (0, 2))))
+    o = 0
+    for name, shape in om.SIZES:
+        n = int(np.prod(shape))
+        a, b = g[o:o + n], go[o:o + n]
+        o += n
+        rel = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+        assert rel < 2e-2, (name, rel)
