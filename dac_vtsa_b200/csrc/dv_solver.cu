@@ -1304,10 +1304,10 @@ __device__ __forceinline__ void cg_publish(const double (&acc)[GM_KMAX + 1], int
     }
 }
 // every block's words of this epoch into ps: false, and bit 4 of *err, when a block's sums had not come within
-// `limit` polls of this thread (1 << 22: about three seconds)
+// `limit` polls of this thread (1 << 22: a few seconds)
 constexpr int CG_POLLS = 1 << 22;
 __device__ __forceinline__ bool cg_collect(const CgWord* x, int cnt, unsigned long long e, double (*ps)[GM_PS], int* err,
-                                           int limit = CG_POLLS) {
+                                           int limit) {
     const int items = (int)gridDim.x * cnt;
     int polls = 0;
     for (int i0 = threadIdx.x; i0 < items; i0 += 4 * VB) {
@@ -1355,7 +1355,7 @@ __device__ __forceinline__ double cg_sum(double (*ps)[GM_PS], int q) {
 template <int E>
 __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const double* __restrict__ V, int64_t ldv,
                                                     double* __restrict__ w, CgWord* xw, int kdim,
-                                                    cudaGraphConditionalHandle hnd, int* err) {
+                                                    cudaGraphConditionalHandle hnd, int* err, int polls) {
     if (st->done) return;                  // a step after the solve stopped (uniform over the grid)
     __shared__ double sm[VB / 32][GM_PS], h1[GM_PS], h2[GM_PS], rot[2][GM_PS];
     __shared__ double ps[CG_MAXB][GM_PS];
@@ -1450,7 +1450,7 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
         }
     }
     cg_publish(acc, m + 1, sm, x1, e);
-    bool ok = cg_collect(x1, m + 1, e, ps, err);
+    bool ok = cg_collect(x1, m + 1, e, ps, err, polls);
     cg_bar();
     if ((int)threadIdx.x <= m) h1[threadIdx.x] = cg_sum(ps, threadIdx.x);
     cg_bar();
@@ -1518,7 +1518,7 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
         }
     }
     cg_publish(acc, m, sm, x2, e);
-    ok = cg_collect(x2, m, e, ps, err) && ok;
+    ok = cg_collect(x2, m, e, ps, err, polls) && ok;
     cg_bar();
     if ((int)threadIdx.x < m) h2[threadIdx.x] = cg_sum(ps, threadIdx.x);
     __syncthreads();
@@ -1541,7 +1541,7 @@ __global__ void __launch_bounds__(CG_T) k_cgs_fused(int64_t n, GmDev* st, const 
     }
     cg_publish(acc, 1, sm, x3, e);
     if (blockIdx.x == 0) {                 // block-uniform
-        ok = cg_collect(x3, 1, e, ps, err) && ok;
+        ok = cg_collect(x3, 1, e, ps, err, polls) && ok;
         __syncthreads_or(ok ? 0 : 1);
     }
 }
@@ -1680,6 +1680,13 @@ static int gmres_coop() {
     return v;
 }
 
+// Poll limit of the Gram-Schmidt kernel's exchange: CG_POLLS, or DVTSA_CG_POLLS=<polls> from the environment at the
+// graph's capture (a test aid: a limit of a few polls makes a solve give up and report it)
+static int cg_polls() {
+    const char* e = getenv("DVTSA_CG_POLLS");
+    return e ? atoi(e) : CG_POLLS;
+}
+
 // The GMRES operator's launches inside the graph: the FP64 finite-difference matvec (one kernel of
 // tiles, or the three of the split residual) or, with the mixed-precision operator, one FP32 assembled-Jacobian product.
 static int op_capture(dv_model* m, Work& W, const double* dargs, double* out, cudaStream_t c) {
@@ -1762,7 +1769,7 @@ static int gm_build_once(dv_model* m, Work& W, int kdim) {
             auto kern = k_cgs_fused<0>;
             if (gmres_coop() == 1 && per <= 3) kern = per == 1 ? k_cgs_fused<1> : per == 2 ? k_cgs_fused<2> : k_cgs_fused<3>;
             if (cudaLaunchKernelEx(&cfg, kern, n, st, (const double*)W.V, ldv, W.wout, (CgWord*)W.cgx, kdim, hnd,
-                                   m->d_err) != cudaSuccess)
+                                   m->d_err, cg_polls()) != cudaSuccess)
                 coop_failed = true;
         } else {
             k_cgs_dots<<<g, VB, 0, c>>>(n, st, W.V, ldv, W.wout, W.part, W.tickets + 1, W.hbuf);

@@ -60,3 +60,37 @@ def test_gram_schmidt_exchange_gives_up_and_reports(polls):
     assert (bits.value, total.value) == (4, 0.0)
     assert lib.dv_selftest_exchange_timeout(1 << 22, 1, C.byref(total), C.byref(bits)) == 0, lib.dv_last_error()
     assert (bits.value, total.value) == (0, 768.0)
+
+
+@pytest.mark.parametrize("grid", [(8, 8, 12), (12, 12, 48)])
+def test_solve_whose_exchange_gave_up_reports_it_and_the_model_recovers(grid, monkeypatch):
+    """A GMRES graph captured with a limit of one poll: the exchange gives up inside a stage solve (other blocks'
+    sums take a trip through L2), the solve ends with the wait's error, and the same model, its graph captured
+    again with the usual limit, then gives the bits of a model that never failed."""
+    import torch
+    from dac_vtsa_b200 import autotune, host
+    from dac_vtsa_b200._lib import LibraryError
+    from dac_vtsa_b200.config import load_config
+    from dac_vtsa_b200.jacobian import FDJacobian
+    from dac_vtsa_b200.model import TVSAModel
+    cfg = load_config(override_dict={"grid.Nr": grid[0], "grid.Ntheta": grid[1], "grid.Nz": grid[2]})
+    g = host.Grid.from_config(cfg)
+    props = host.get_backend(cfg)
+    st = host.seeded_state(cfg, g, props, seed=2)
+
+    def model():
+        m = TVSAModel(cfg, g, props, cfg.cycle[0], st)
+        y = torch.from_numpy(m.pack(st)).to(m.device)
+        m.precond_factor(FDJacobian(m).block(1.0, y), 0.5)
+        return m, y
+
+    m, y = model()
+    ref = m.newton_stage(1.5, y, y, 0.5)
+    m, y = model()
+    monkeypatch.setenv("DVTSA_CG_POLLS", "-1")          # gives up after its first poll
+    with pytest.raises(LibraryError, match="exchange"):
+        m.newton_stage(1.5, y, y, 0.5)
+    monkeypatch.delenv("DVTSA_CG_POLLS")
+    autotune.apply(m, {"gmres_prefix": 2})              # (the graph is captured again)
+    z = m.newton_stage(1.5, y, y, 0.5)
+    assert torch.equal(z[0], ref[0]) and z[1] == ref[1] and z[2] == ref[2]
